@@ -224,6 +224,52 @@ def test_eaw_lattice_tiles_equal_direct_taps(core, size):
     assert np.array_equal(outs[0], outs[1])
 
 
+def eaw_stops(color, pos, nrm, iterations, phi, quirk=0):
+    """EAW with separate edge stops min(exp(-|d|^2 / phi), 1) in double precision (fmin: NaN distances stop
+    nothing)."""
+    h, w = color.shape[:2]
+    cur = color.astype(np.float64)
+    maps = [(m.astype(np.float64), f) for m, f in ((pos, phi[1]), (nrm, phi[2])) if m is not None]
+    with np.errstate(all="ignore"):
+        for i in range(iterations):
+            num, den = np.zeros_like(cur), np.zeros((h, w, 1))
+            for oy in range(-2, 3):
+                for ox in range(-2, 3):
+                    iy = np.clip(np.arange(h) + oy * 2 ** i, 0, h - 1)[:, None]
+                    ix = np.clip(np.arange(w) + ox * 2 ** i, 0, w - 1)[None, :]
+                    stop = lambda m, f: np.fmin(np.exp(-((m - m[iy, ix]) ** 2).sum(-1, keepdims=True) / np.float64(f)), 1.0)
+                    k = np.fmin(np.exp(-1.0 / np.float64(phi[0])), 1.0) if quirk else stop(cur, phi[0])
+                    for m, f in maps:
+                        k = k * stop(m, f)
+                    k = k * np.exp(-(ox * ox + oy * oy) / 2.0)
+                    num += k * cur[iy, ix]
+                    den += k
+            cur = num / den
+    return cur
+
+
+@pytest.mark.parametrize("w,h,iterations", [(1, 1, 3), (31, 17, 2), (33, 16, 4), (32, 15, 5), (64, 64, 3), (70, 130, 7)])
+@pytest.mark.parametrize("phi,quirk", [((5.0, 0.1, 0.1), 0), ((5.0, 0.1, 0.1), 1), ((0.0, 0.1, 0.1), 0),
+                                       ((5.0, -0.1, 0.1), 0)])
+def test_eaw_tiles_phi_and_non_finite_maps(core, w, h, iterations, phi, quirk):
+    """Sizes around the 32 x 16 lattice tiles, steps beyond the image, phi of zero and below (stops of one),
+    one or both maps, and infinities and NaN in the maps (a NaN distance stops nothing)."""
+    g = np.random.default_rng(5)
+    color = g.random((h, w, 4), np.float32)
+    pos, nrm = (g.random((h, w, 4), np.float32) * 0.5 for _ in range(2))
+    pos[h // 2, w // 2, 0] = np.inf
+    nrm[h // 3, w // 3, 1] = np.nan
+    for m in ((pos, nrm), (pos, None), (None, nrm), (None, None)):
+        d = [torch.from_numpy(a).cuda() if a is not None else None for a in (color, *m)]
+        out = torch.empty((h, w, 4), dtype=torch.float32, device="cuda")
+        assert core.lib.vpt_eaw_denoise_rgba(*(dptr(t) if t is not None else None for t in d), w, h, iterations, phi[0],
+                                             phi[1], phi[2], quirk, dptr(out), None) == 0
+        torch.cuda.synchronize()
+        # per pass 25 weights of a few ulp (2^x of arguments up to about 20: 2^-20) and sums of 25
+        assert np.allclose(out.cpu().numpy(), eaw_stops(color, m[0], m[1], iterations, phi, quirk), rtol=iterations * 4e-6,
+                           atol=1e-6)
+
+
 def test_eaw_rejects_an_output_that_overlaps_an_input(core):
     h, w = 16, 16
     imgs = [torch.rand((h, w, 4), device="cuda") for _ in range(3)]
