@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdint.h>
+#include <algorithm>
 #include <mutex>
 #include "vpt_denoise.h"
 #include "vpt_params.h"
@@ -62,14 +63,6 @@ void svgf_release(SvgfState& s) {
     s = SvgfState();
 }
 
-__device__ __forceinline__ float svgf_weight(float cd, float od, float phi_d, float3 cn, float3 on, float cc, float oc,
-                                             float phi_c) {
-    float wn = powf(fmaxf(0.0f, (cn.x * on.x + cn.y * on.y) + cn.z * on.z), 128.0f);
-    float wz = (phi_d == 0.0f) ? 0.0f : fabsf(cd - od) / phi_d;
-    float wc = fabsf(cc - oc) * 2.0f / phi_c;
-    return expf(0.0f - fmaxf(wc, 0.0f) - fmaxf(wz, 0.0f)) * wn;
-}
-
 struct SvgfCur {
     float4* noisy;     // rgba
     float2* motion;    // flow
@@ -80,7 +73,16 @@ struct SvgfCur {
     float4* temp;      // temp accum (rgb, variance)
     float4* ping;
     float4* pong;
+    float4* geo;       // normal.xyz, depth: one 16-byte read a tap
+    float *var0, *var1;  // variance (the w of the filtered image) as a plane of its own, ping / pong
 };
+
+constexpr int kSvgfPlaneFloats = 6;
+static void svgf_filter_planes(SvgfCur& c, float* base, int n) {
+    c.geo = reinterpret_cast<float4*>(base);
+    c.var0 = base + (size_t)n * 4;
+    c.var1 = base + (size_t)n * 5;
+}
 
 static SvgfCur svgf_cur(float* base, int n) {
     SvgfCur c;
@@ -93,9 +95,10 @@ static SvgfCur svgf_cur(float* base, int n) {
     c.motion = reinterpret_cast<float2*>(base + (size_t)n * 24);
     c.depth = base + (size_t)n * 26;
     c.fwidth = base + (size_t)n * 27;
+    svgf_filter_planes(c, base + (size_t)n * 28, n);
     return c;
 }
-constexpr int kSvgfCurFloats = 28;
+constexpr int kSvgfCurFloats = 28 + kSvgfPlaneFloats;
 
 struct Mat4 {
     float m[16];
@@ -239,97 +242,320 @@ __global__ void svgf_reproject_kernel(SvgfCur c, const float4* __restrict__ colo
     m1 = prev_m.x * (1.0f - a_m) + m1 * a_m;
     m2 = prev_m.y * (1.0f - a_m) + m2 * a_m;
     float var = fmaxf(0.0f, m2 - m1 * m1);
+    float4 geo = c.normal[i];
+    geo.w = c.depth[i];
+    c.geo[i] = geo;
     c.moments[i] = make_float4(m1, m2, hist_len, 0.0f);
     c.temp[i] = make_float4(last.x * (1.0f - a_c) + col.x * a_c, last.y * (1.0f - a_c) + col.y * a_c,
                             last.z * (1.0f - a_c) + col.z * a_c, var);
 }
 
-__global__ void svgf_filter_moments_kernel(SvgfCur c, float4* __restrict__ temp_out, int w, int h) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= w || y >= h) return;
-    int i = y * w + x;
-    float hl = c.moments[i].z;
-    float4 center = c.temp[i];
-    if (hl >= 4.0f) {
-        temp_out[i] = center;
-        return;
-    }
-    float cd = c.depth[i], cfw = c.fwidth[i];
-    float4 cn4 = c.normal[i];
-    float3 cn = make_float3(cn4.x, cn4.y, cn4.z);
-    float sw = 0.0f;
-    float3 sc = make_float3(0, 0, 0);
-    float2 sm = make_float2(0, 0);
-    for (int yy = -3; yy <= 3; yy++)
-        for (int xx = -3; xx <= 3; xx++) {
-            int qx = x + xx, qy = y + yy;
-            if (qx < 0 || qy < 0 || qx >= w || qy >= h) continue;
-            int q = qy * w + qx;
-            float4 oc = c.temp[q];
-            float4 om = c.moments[q];
-            float4 on = c.normal[q];
-            float wt = svgf_weight(cd, c.depth[q], fabsf(cfw) + 0.0001f, cn, make_float3(on.x, on.y, on.z), center.x,
-                                   oc.x, 10.0f);
-            sw += wt;
-            sc.x += wt * oc.x;
-            sc.y += wt * oc.y;
-            sc.z += wt * oc.z;
-            sm.x += wt * om.x;
-            sm.y += wt * om.y;
-        }
-    sw = fmaxf(sw, 1e-6f);
-    sc = make_float3(sc.x / sw, sc.y / sw, sc.z / sw);
-    sm = make_float2(sm.x / sw, sm.y / sw);
-    float var = sm.y - sm.x * sm.x;
-    var *= 4.0f / hl;
-    temp_out[i] = make_float4(sc.x, sc.y, sc.z, var);
+// The two edge-avoiding filters.  Both weigh a tap with
+//   max(0, n . n')^128 exp(-max(0, |z - z'| / phi_z) - max(0, |c - c'| * 2 / phi_c))
+// (compute_weight, svgf_common.glsl:29-41) and were bound by the instructions of powf, expf and two
+// divisions a tap, and by each tap's loads.  Here the power is seven squarings, the exponential the
+// special-function unit's 2^x of a sum scaled by log2(e), and the reciprocals of phi are formed once a
+// pixel.  A block stages its taps in shared memory, and a thread filters kSvgfRows vertically adjacent
+// pixels so that one read of a tap serves all of them.  Taps outside the image are staged with a zero
+// normal: their weight is 0, which is to skip them.  The max(0, .) also turn NaN distances into 0.
+// Measured, four frames of 1280 x 720 with five a-trous passes: 2785 us on the GPU (a pass 102, the moments filter
+// 134), 1413 so (50 and 56; each pass has 27 us of instructions).  Error against 64 bits over twelve sizes: image
+// 5.8e-7 (was 7.0e-7), colour history 1.5e-6 (1.9e-6).
+constexpr int kSvgfRows = 4;
+constexpr int kSvgfTileW = 32, kSvgfTileH = 16;
+constexpr int kSvgfThreads = kSvgfTileW * kSvgfTileH / kSvgfRows;
+constexpr float kLog2e = 1.4426950408889634f;
+
+// asynchronous copies into shared memory (all of a tile's are in flight before the wait); zeros when !valid
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src, bool valid) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;\n" ::"r"((uint32_t)__cvta_generic_to_shared(dst)),
+                 "l"(src), "n"(BYTES), "r"(valid ? BYTES : 0)
+                 : "memory");
 }
 
-__global__ void svgf_atrous_kernel(const float4* __restrict__ in, SvgfCur c, float4* __restrict__ out,
-                                   float4* __restrict__ color_hist, int w, int h, int iteration) {
-    int x = blockIdx.x * blockDim.x + threadIdx.x;
-    int y = blockIdx.y * blockDim.y + threadIdx.y;
-    if (x >= w || y >= h) return;
-    int i = y * w + x;
-    int step = 1 << iteration;
-    float4 cc = in[i];
-    const float kv2[2][2] = {{1.0f / 4.0f, 1.0f / 8.0f}, {1.0f / 8.0f, 1.0f / 16.0f}};
-    float fv = 0.0f;
-    for (int yy = -1; yy <= 1; yy++)
-        for (int xx = -1; xx <= 1; xx++) {
-            int qx = min(max(x + xx, 0), w - 1), qy = min(max(y + yy, 0), h - 1);
-            fv += in[qy * w + qx].w * kv2[abs(xx)][abs(yy)];
+__device__ __forceinline__ float exp2_sfu(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// x^128 for x >= 0.  A squaring doubles the relative error so far, so the first three carry their rounding
+// errors along (h + l = x^2k); the last four add about 3 ulp, as much as powf's own argument error.
+__device__ __forceinline__ float pow128(float x) {
+    float h = x * x, l = fmaf(x, x, -h);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+        const float h2 = h * h;
+        l = fmaf(h + h, l, fmaf(h, h, -h2));
+        h = h2;
+    }
+    h += l;
+    h *= h;
+    h *= h;
+    h *= h;
+    return h * h;
+}
+
+// normal and depth of a pixel in one float4; rc = 2 log2(e) / phi_c, rz = log2(e) / phi_z
+__device__ __forceinline__ float svgf_weight(float4 cg, float4 og, float rz, float cc, float oc, float rc) {
+    const float p = pow128(fmaxf(0.0f, fmaf(cg.z, og.z, fmaf(cg.y, og.y, cg.x * og.x))));
+    return exp2_sfu(0.0f - fmaxf(fabsf(cc - oc) * rc, 0.0f) - fmaxf(fabsf(cg.w - og.w) * rz, 0.0f)) * p;
+}
+
+// Spatial estimate of colour and variance for pixels with a history shorter than 4 frames (7 x 7 taps);
+// a block without such a pixel copies its colours.
+constexpr int kMomPatchW = kSvgfTileW + 6, kMomPatchH = kSvgfTileH + 6;
+
+__global__ void __launch_bounds__(kSvgfThreads) svgf_filter_moments_kernel(SvgfCur c, float4* __restrict__ temp_out,
+                                                                           int w, int h) {
+    __shared__ float4 sgeo[kMomPatchH][kMomPatchW];
+    __shared__ float4 scol[kMomPatchH][kMomPatchW];
+    __shared__ float2 smom[kMomPatchH][kMomPatchW];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int bx = blockIdx.x * kSvgfTileW, by = blockIdx.y * kSvgfTileH;
+    const int x = bx + lane, row0 = warp * kSvgfRows;
+    float hl[kSvgfRows];
+    bool young = false;
+#pragma unroll
+    for (int r = 0; r < kSvgfRows; r++) {
+        const int y = by + row0 + r;
+        hl[r] = x < w && y < h ? c.moments[y * w + x].z : 4.0f;
+        young = young || !(hl[r] >= 4.0f);
+    }
+    if (!__syncthreads_or(young)) {
+#pragma unroll
+        for (int r = 0; r < kSvgfRows; r++) {
+            const int y = by + row0 + r;
+            if (x < w && y < h) {
+                const float4 o = c.temp[y * w + x];
+                temp_out[y * w + x] = o;
+                c.var0[y * w + x] = o.w;
+            }
         }
-    float4 cn4 = c.normal[i];
-    float3 cn = make_float3(cn4.x, cn4.y, cn4.z);
-    float cz = c.depth[i], cfw = c.fwidth[i];
-    float phi_c = sqrtf(fmaxf(0.0f, 1e-10f + fv));
-    const float kvals[3] = {1.0f, 2.0f / 3.0f, 1.0f / 6.0f};
-    float accw = kvals[0] * kvals[0];
-    float4 sum = make_float4(cc.x * accw, cc.y * accw, cc.z * accw, cc.w * accw);
-    for (int yy = -2; yy <= 2; yy++)
-        for (int xx = -2; xx <= 2; xx++) {
-            int qx = x + xx * step, qy = y + yy * step;
-            bool inside = qx >= 0 && qy >= 0 && qx < w && qy < h;
-            if (!inside || (xx == 0 && yy == 0)) continue;
-            float kval = kvals[abs(xx)] * kvals[abs(yy)];
-            int q = qy * w + qx;
-            float4 oc = in[q];
-            float4 on = c.normal[q];
-            float len = sqrtf((float)(xx * xx + yy * yy));
-            float wt = svgf_weight(cz, c.depth[q], fabsf(cfw * len * (float)step) + 0.0001f, cn,
-                                   make_float3(on.x, on.y, on.z), cc.x, oc.x, phi_c) *
-                       kval;
-            sum.x += wt * oc.x;
-            sum.y += wt * oc.y;
-            sum.z += wt * oc.z;
-            sum.w += wt * wt * oc.w;
+        return;
+    }
+    for (int k = threadIdx.x; k < kMomPatchW * kMomPatchH; k += kSvgfThreads) {
+        const int j = k / kMomPatchW, i = k - j * kMomPatchW;
+        const int px = bx + i - 3, py = by + j - 3;
+        const bool v = px >= 0 && py >= 0 && px < w && py < h;
+        const int q = v ? py * w + px : 0;
+        copy_async<16>(&sgeo[j][i], &c.geo[q], v);
+        copy_async<16>(&scol[j][i], &c.temp[q], v);
+        copy_async<8>(&smom[j][i], &c.moments[q], v);
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    if (!__any_sync(0xffffffffu, young)) {
+#pragma unroll
+        for (int r = 0; r < kSvgfRows; r++) {
+            const int y = by + row0 + r;
+            if (x < w && y < h) {
+                const float4 o = c.temp[y * w + x];
+                temp_out[y * w + x] = o;
+                c.var0[y * w + x] = o.w;
+            }
+        }
+        return;
+    }
+    float4 cg[kSvgfRows];
+    float cl[kSvgfRows], rz[kSvgfRows], sw[kSvgfRows], s0[kSvgfRows], s1[kSvgfRows], s2[kSvgfRows], t1[kSvgfRows],
+        t2[kSvgfRows];
+#pragma unroll
+    for (int r = 0; r < kSvgfRows; r++) {
+        const int y = by + row0 + r;
+        cg[r] = sgeo[row0 + r + 3][lane + 3];
+        cl[r] = scol[row0 + r + 3][lane + 3].x;
+        rz[r] = kLog2e / ((x < w && y < h ? fabsf(c.fwidth[y * w + x]) : 0.0f) + 0.0001f);
+        sw[r] = s0[r] = s1[r] = s2[r] = t1[r] = t2[r] = 0.0f;
+    }
+    constexpr float rc = 2.0f * kLog2e / 10.0f;
+#pragma unroll 1
+    for (int ox = 0; ox < 7; ox++) {
+#pragma unroll
+        for (int j = 0; j < kSvgfRows + 6; j++) {
+            const float4 og = sgeo[row0 + j][lane + ox];
+            const float4 oc = scol[row0 + j][lane + ox];
+            const float2 m = smom[row0 + j][lane + ox];
+#pragma unroll
+            for (int r = 0; r < kSvgfRows; r++) {
+                if (j < r || j > r + 6) continue;
+                const float wt = svgf_weight(cg[r], og, rz[r], cl[r], oc.x, rc);
+                sw[r] += wt;
+                s0[r] = fmaf(wt, oc.x, s0[r]);
+                s1[r] = fmaf(wt, oc.y, s1[r]);
+                s2[r] = fmaf(wt, oc.z, s2[r]);
+                t1[r] = fmaf(wt, m.x, t1[r]);
+                t2[r] = fmaf(wt, m.y, t2[r]);
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kSvgfRows; r++) {
+        const int y = by + row0 + r;
+        if (x >= w || y >= h) continue;
+        const int i = y * w + x;
+        if (hl[r] >= 4.0f) {
+            const float4 o = c.temp[i];
+            temp_out[i] = o;
+            c.var0[i] = o.w;
+            continue;
+        }
+        const float s = fmaxf(sw[r], 1e-6f);
+        const float m1 = t1[r] / s, m2 = t2[r] / s;
+        float var = m2 - m1 * m1;
+        var *= 4.0f / hl[r];
+        temp_out[i] = make_float4(s0[r] / s, s1[r] / s, s2[r] / s, var);
+        c.var0[i] = var;
+    }
+}
+
+// One a-trous pass: 5 x 5 taps at step 2^iteration.  The taps of a pixel lie on the lattice of its residue
+// class modulo the step; a block takes 32 x 16 pixels of one class (at step >= 2 of two horizontally
+// adjacent ones, which share 32-byte sectors), as eaw_lattice_kernel does.
+constexpr int kAtrPatchH = kSvgfTileH + 4, kAtrPatchW = kSvgfTileW + 8;
+
+// variance over the 3 x 3 neighbourhood (clamped), weights 1/4, 1/8, 1/16, as 2 log2(e) / phi_c
+__device__ __forceinline__ float svgf_color_scale(const float* __restrict__ var, int x, int y, int w, int h) {
+    float fv = 0.0f;
+#pragma unroll
+    for (int yy = -1; yy <= 1; yy++)
+#pragma unroll
+        for (int xx = -1; xx <= 1; xx++) {
+            const int q = min(max(y + yy, 0), h - 1) * w + min(max(x + xx, 0), w - 1);
+            fv = fmaf(__ldg(var + q), 0.25f / (float)((1 + (xx != 0)) * (1 + (yy != 0))), fv);
+        }
+    return 2.0f * kLog2e / sqrtf(fmaxf(0.0f, 1e-10f + fv));
+}
+// log2(e) / phi_z of the taps at squared distance d2 = 1, 2, 4, 5, 8 (x the step): fw = |depth fwidth * step|
+__device__ __forceinline__ float svgf_depth_scale(float fw, int d2) {
+    return __fdividef(kLog2e, fw * sqrtf((float)d2) + 0.0001f);
+}
+// the a-trous kernel h(o), o = -2 .. 2
+__device__ constexpr float svgf_tap(int o) { return o == 0 ? 1.0f : (o * o == 1 ? 2.0f / 3.0f : 1.0f / 6.0f); }
+
+// The pass with every tap read from global memory: for steps so large that a class has few pixels (most of
+// a block's lattice tile would be empty).
+__global__ void svgf_atrous_direct_kernel(const float4* __restrict__ in, SvgfCur c, float4* __restrict__ out,
+                                          float4* __restrict__ color_hist, int w, int h, int iteration) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y * blockDim.y + threadIdx.y;
+    if (x >= w || y >= h) return;
+    const int i = y * w + x, step = 1 << iteration;
+    float4 sum = in[i];
+    const float4 cg = c.geo[i];
+    const float cl = sum.x, rc = svgf_color_scale(iteration & 1 ? c.var1 : c.var0, x, y, w, h), fw = fabsf(c.fwidth[i] * (float)step);
+    float accw = 1.0f;
+#pragma unroll
+    for (int oy = -2; oy <= 2; oy++)
+#pragma unroll
+        for (int ox = -2; ox <= 2; ox++) {
+            const int qx = x + ox * step, qy = y + oy * step;
+            if (qx < 0 || qy < 0 || qx >= w || qy >= h || (ox == 0 && oy == 0)) continue;
+            const int q = qy * w + qx;
+            const float4 og = c.geo[q], oc = in[q];
+            const float wt = svgf_weight(cg, og, svgf_depth_scale(fw, ox * ox + oy * oy), cl, oc.x, rc) *
+                             (svgf_tap(ox) * svgf_tap(oy));
+            sum.x = fmaf(wt, oc.x, sum.x);
+            sum.y = fmaf(wt, oc.y, sum.y);
+            sum.z = fmaf(wt, oc.z, sum.z);
+            sum.w = fmaf(wt * wt, oc.w, sum.w);
             accw += wt;
         }
-    float4 r = make_float4(sum.x / accw, sum.y / accw, sum.z / accw, sum.w / (accw * accw));
-    if (iteration == 0) color_hist[i] = r;
-    out[i] = r;
+    const float4 o = make_float4(sum.x / accw, sum.y / accw, sum.z / accw, sum.w / (accw * accw));
+    if (color_hist) color_hist[i] = o;
+    out[i] = o;
+    (iteration & 1 ? c.var0 : c.var1)[i] = o.w;
+}
+
+__global__ void __launch_bounds__(kSvgfThreads)
+    svgf_atrous_kernel(const float4* __restrict__ in, SvgfCur c, float4* __restrict__ out,
+                       float4* __restrict__ color_hist, int w, int h, int iteration, int tiles_x, int tiles_y) {
+    __shared__ float4 sgeo[kAtrPatchH][kAtrPatchW];
+    __shared__ float4 scol[kAtrPatchH][kAtrPatchW];
+    const int step = 1 << iteration;
+    const int classes = step > 1 ? 2 : 1, cols = kSvgfTileW / classes;
+    int b = blockIdx.x;
+    const int tx = b % tiles_x;
+    b /= tiles_x;
+    const int ty = b % tiles_y;
+    b /= tiles_y;
+    const int pairs = (min(step, w) + classes - 1) / classes;
+    const int rx = (b % pairs) * classes, ry = b / pairs;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int patch_w = (cols + 4) * classes;
+    for (int k = threadIdx.x; k < patch_w * kAtrPatchH; k += kSvgfThreads) {
+        const int j = k / patch_w, i = k - j * patch_w;
+        const int col = classes == 2 ? i >> 1 : i, cls = classes == 2 ? i & 1 : 0;
+        const int py = (ty * kSvgfTileH + j - 2) * step + ry, px = (tx * cols + col - 2) * step + rx + cls;
+        const bool v = px >= 0 && py >= 0 && px < w && py < h;
+        const int q = v ? py * w + px : 0;
+        copy_async<16>(&sgeo[j][i], &c.geo[q], v);
+        copy_async<16>(&scol[j][i], &in[q], v);
+    }
+    const int x = (tx * cols + lane / classes) * step + rx + lane % classes;
+    const int row0 = warp * kSvgfRows;
+    const int y0 = (ty * kSvgfTileH + row0) * step + ry;
+    const int cx = lane + 2 * classes;
+
+    // the pixels' own scales, while the copies are in flight (rows beyond the image take its last row, unused)
+    const float* var = iteration & 1 ? c.var1 : c.var0;
+    float rc[kSvgfRows], rz[kSvgfRows][5];
+#pragma unroll
+    for (int r = 0; r < kSvgfRows; r++) {
+        const int y = min(y0 + r * step, h - 1), xc = min(x, w - 1);
+        rc[r] = svgf_color_scale(var, xc, y, w, h);
+        const float fw = fabsf(c.fwidth[y * w + xc] * (float)step);
+        rz[r][0] = svgf_depth_scale(fw, 1);
+        rz[r][1] = svgf_depth_scale(fw, 2);
+        rz[r][2] = svgf_depth_scale(fw, 4);
+        rz[r][3] = svgf_depth_scale(fw, 5);
+        rz[r][4] = svgf_depth_scale(fw, 8);
+    }
+    asm volatile("cp.async.wait_all;\n" ::: "memory");
+    __syncthreads();
+    if (x >= w || y0 >= h) return;
+
+    float4 cg[kSvgfRows], sum[kSvgfRows];
+    float cl[kSvgfRows], accw[kSvgfRows];
+#pragma unroll
+    for (int r = 0; r < kSvgfRows; r++) {
+        cg[r] = sgeo[row0 + r + 2][cx];
+        sum[r] = scol[row0 + r + 2][cx];
+        cl[r] = sum[r].x;
+        accw[r] = 1.0f;
+    }
+#pragma unroll
+    for (int j = 0; j < kSvgfRows + 4; j++) {
+#pragma unroll
+        for (int ox = -2; ox <= 2; ox++) {
+            const float4 og = sgeo[row0 + j][cx + ox * classes];
+            const float4 oc = scol[row0 + j][cx + ox * classes];
+#pragma unroll
+            for (int r = 0; r < kSvgfRows; r++) {
+                const int oy = j - 2 - r;
+                if (oy < -2 || oy > 2 || (ox == 0 && oy == 0)) continue;
+                const int d2 = ox * ox + oy * oy;
+                const int cls = d2 == 1 ? 0 : d2 == 2 ? 1 : d2 == 4 ? 2 : d2 == 5 ? 3 : 4;
+                const float wt = svgf_weight(cg[r], og, rz[r][cls], cl[r], oc.x, rc[r]) *
+                                 (svgf_tap(ox) * svgf_tap(oy));
+                sum[r].x = fmaf(wt, oc.x, sum[r].x);
+                sum[r].y = fmaf(wt, oc.y, sum[r].y);
+                sum[r].z = fmaf(wt, oc.z, sum[r].z);
+                sum[r].w = fmaf(wt * wt, oc.w, sum[r].w);
+                accw[r] += wt;
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < kSvgfRows; r++) {
+        const int y = y0 + r * step;
+        if (y >= h) break;
+        const float4 o = make_float4(sum[r].x / accw[r], sum[r].y / accw[r], sum[r].z / accw[r],
+                                     sum[r].w / (accw[r] * accw[r]));
+        if (color_hist) color_hist[y * w + x] = o;
+        out[y * w + x] = o;
+        (iteration & 1 ? c.var0 : c.var1)[y * w + x] = o.w;
+    }
 }
 
 __global__ void svgf_update_history_kernel(SvgfCur c, float4* __restrict__ moments_hist,
@@ -343,7 +569,7 @@ __global__ void svgf_update_history_kernel(SvgfCur c, float4* __restrict__ momen
 
 cudaError_t svgf_filter_passes(SvgfCur c, float4* color_history, float4* moments_history, float4* normal_history,
                                float* depth_history, int w, int h, const SvgfSettings& s, cudaStream_t stream,
-                               const float4** result);
+                               float4* last, const float4** result);
 
 cudaError_t svgf_denoise_features(const float* color, const float* feat, uint32_t frames, int w, int h,
                                   const SvgfSettings& s, SvgfState& st, float* out_rgba, float** result,
@@ -381,35 +607,45 @@ cudaError_t svgf_denoise_features(const float* color, const float* feat, uint32_
     cudaError_t e = svgf_filter_passes(c, reinterpret_cast<float4*>(st.color_history),
                                        reinterpret_cast<float4*>(st.moments_history),
                                        reinterpret_cast<float4*>(st.normal_history), st.depth_history, w, h, s, stream,
-                                       &src);
+                                       nullptr, &src);
     *result = reinterpret_cast<float*>(const_cast<float4*>(src));
     return e;
 }
 
 // The filter passes of one SVGF frame on prepared maps (c.noisy / normal / depth / fwidth / motion)
-// and scratch (c.moments / temp / ping / pong); the result is c.temp, c.ping or c.pong.
+// and scratch (c.moments / temp / ping / pong); the result is c.temp, c.ping or c.pong, or `last` (may be
+// null; no input or history) when there is an a-trous pass to write it.
 cudaError_t svgf_filter_passes(SvgfCur c, float4* color_history, float4* moments_history, float4* normal_history,
                                float* depth_history, int w, int h, const SvgfSettings& s, cudaStream_t stream,
-                               const float4** result) {
+                               float4* last, const float4** result) {
     const int n = w * h;
     dim3 b(16, 16), g((w + 15) / 16, (h + 15) / 16);
     svgf_reproject_kernel<<<g, b, 0, stream>>>(c, color_history, moments_history, normal_history, depth_history, w, h,
                                                s.z_threshold, s.normal_threshold);
-    svgf_filter_moments_kernel<<<g, b, 0, stream>>>(c, c.ping, w, h);
-    cudaMemcpyAsync(c.temp, c.ping, (size_t)n * 16, cudaMemcpyDeviceToDevice, stream);
-    const float4* src = c.temp;
-    float4* bufs[2] = {c.ping, c.pong};
+    const dim3 tiles((w + kSvgfTileW - 1) / kSvgfTileW, (h + kSvgfTileH - 1) / kSvgfTileH);
+    svgf_filter_moments_kernel<<<tiles, kSvgfThreads, 0, stream>>>(c, c.ping, w, h);
+    const float4* src = c.ping;
+    float4* bufs[2] = {c.pong, c.temp};
     if (s.atrous_iterations < 1) {
-        cudaMemcpyAsync(color_history, c.temp, (size_t)n * 16, cudaMemcpyDeviceToDevice, stream);
+        cudaMemcpyAsync(color_history, c.ping, (size_t)n * 16, cudaMemcpyDeviceToDevice, stream);
     }
     for (int it = 0; it < s.atrous_iterations; it++) {
-        float4* dst = bufs[it & 1];
-        svgf_atrous_kernel<<<g, b, 0, stream>>>(src, c, dst, color_history, w, h, it);
+        float4* dst = last && it + 1 == s.atrous_iterations ? last : bufs[it & 1];
+        const int step = 1 << it, classes = step > 1 ? 2 : 1;
+        const int tiles_x = ((w + step - 1) / step + kSvgfTileW / classes - 1) / (kSvgfTileW / classes);
+        const int tiles_y = ((h + step - 1) / step + kSvgfTileH - 1) / kSvgfTileH;
+        const long long blocks = (long long)tiles_x * tiles_y * ((std::min(step, w) + classes - 1) / classes) * std::min(step, h);
+        float4* hist = it == 0 ? color_history : nullptr;
+        if (blocks * kSvgfTileW * kSvgfTileH <= 4LL * n)
+            svgf_atrous_kernel<<<(unsigned)blocks, kSvgfThreads, 0, stream>>>(src, c, dst, hist, w, h, it, tiles_x,
+                                                                              tiles_y);
+        else
+            svgf_atrous_direct_kernel<<<g, b, 0, stream>>>(src, c, dst, hist, w, h, it);
         src = dst;
     }
     svgf_update_history_kernel<<<(n + 255) / 256, 256, 0, stream>>>(c, moments_history, normal_history, depth_history,
                                                                      n);
-    count_launches(4 + (unsigned)s.atrous_iterations);
+    count_launches(3 + (unsigned)s.atrous_iterations);
     *result = src;
     return cudaGetLastError();
 }
@@ -751,7 +987,7 @@ extern "C" VptStatus vpt_svgf_filter(const float* noisy_rgba, const float* norma
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t n = (size_t)width * height;
     float* scratch = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&scratch), n * 16 * 4, s) != cudaSuccess) return VPT_ERR_OOM;
+    if (cudaMallocAsync(reinterpret_cast<void**>(&scratch), n * (16 + vpt::kSvgfPlaneFloats) * 4, s) != cudaSuccess) return VPT_ERR_OOM;
     vpt::SvgfCur c;
     c.noisy = reinterpret_cast<float4*>(const_cast<float*>(noisy_rgba));
     c.normal = reinterpret_cast<float4*>(const_cast<float*>(normal_rgba));
@@ -762,16 +998,31 @@ extern "C" VptStatus vpt_svgf_filter(const float* noisy_rgba, const float* norma
     c.temp = reinterpret_cast<float4*>(scratch + n * 4);
     c.ping = reinterpret_cast<float4*>(scratch + n * 8);
     c.pong = reinterpret_cast<float4*>(scratch + n * 12);
+    vpt::svgf_filter_planes(c, scratch + n * 16, (int)n);
     vpt::SvgfSettings st;
     st.z_threshold = z_threshold;
     st.normal_threshold = normal_threshold;
     st.atrous_iterations = iterations;
     const float4* res = nullptr;
+    // the last pass writes the output itself, unless the caller's output is one of the maps or histories
+    // that the passes still read
+    const struct {
+        const void* p;
+        size_t floats;
+    } held[] = {{noisy_rgba, 4}, {normal_rgba, 4}, {color_history, 4}, {moments_history, 4}, {normal_history, 4},
+                {depth, 1},      {depth_fwidth, 1}, {motion, 2},       {depth_history, 1}};
+    const uintptr_t o0 = reinterpret_cast<uintptr_t>(out_rgba);
+    bool direct = true;
+    for (const auto& b : held) {
+        const uintptr_t p0 = reinterpret_cast<uintptr_t>(b.p);
+        direct = direct && (o0 >= p0 + n * b.floats * 4 || p0 >= o0 + n * 16);
+    }
     cudaError_t e = vpt::svgf_filter_passes(c, reinterpret_cast<float4*>(color_history),
                                             reinterpret_cast<float4*>(moments_history),
                                             reinterpret_cast<float4*>(normal_history), depth_history, width, height, st,
-                                            s, &res);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(out_rgba, res, n * 16, cudaMemcpyDeviceToDevice, s);
+                                            s, direct ? reinterpret_cast<float4*>(out_rgba) : nullptr, &res);
+    if (e == cudaSuccess && reinterpret_cast<const float*>(res) != out_rgba)
+        e = cudaMemcpyAsync(out_rgba, res, n * 16, cudaMemcpyDeviceToDevice, s);
     cudaFreeAsync(scratch, s);
     return e == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
 }
