@@ -151,3 +151,30 @@ def test_three_scale_reconstruction_matches_reference_composition(ref_ops):
     got = kpn.inv_iter_denoise(x0, l0, l1, l2, lprev=lprev, prev=prev, reproj_uv=uv)
     assert got.shape == want.shape
     assert torch.allclose(got, want, rtol=1e-4, atol=1e-5)
+
+
+@pytest.mark.parametrize("k", [1, 3, 5, 7])
+@pytest.mark.parametrize("c,h,w", [(1, 8, 32), (2, 9, 33), (3, 7, 31), (4, 25, 97), (4, 1, 1)])
+def test_tiles_at_their_edges_match_oracle(k, c, h, w):
+    """The staged 32 x 8 tiles: a whole tile, one pixel more and less, several tiles, a single pixel; for odd
+    sizes the last row and column of the inv_iter base have no coarse pixel (base 0)."""
+    img, logits = rnd(2, c, h, w, seed=21), rnd(2, k * k, h, w, seed=22, scale=2.0)
+    for softmax in (True, False):
+        got = kpn.apply_kernels(cuda(img), cuda(logits), k, softmax).cpu().numpy()
+        # a sum of k * k products: k * k roundings of terms up to 2-norm |logits| |img|
+        assert np.allclose(got, bridge.kpn_apply(img, logits, k, softmax=softmax), rtol=RTOL, atol=k * k * ATOL)
+    lh, lw = max(1, h // 2), max(1, w // 2)
+    x_lo, pred = rnd(1, c, lh, lw, seed=23), rnd(1, c, lh, lw, seed=24)
+    fused = rnd(1, k * k + 3, h, w, seed=25, scale=2.0)
+    got = kpn.inv_iter(cuda(img[:1]), cuda(pred), cuda(x_lo), cuda(img[1:]), cuda(fused), k).cpu().numpy()
+    assert np.allclose(got, bridge.kpn_inv_iter(img[:1], pred, x_lo, img[1:], fused, k, True), rtol=RTOL, atol=ATOL)
+
+
+def test_apply_without_softmax_skips_taps_outside():
+    """An infinite weight on a tap outside the image is skipped, not multiplied by a staged zero."""
+    img = np.ones((1, 3, 12, 40), np.float32)
+    wts = np.full((1, 9, 12, 40), 1.0, np.float32)
+    wts[0, :3, 0, :] = np.inf   # the row above the first
+    wts[0, 2::3, :, -1] = np.inf  # the column right of the last
+    got = kpn.apply_kernels(cuda(img), cuda(wts), 3, softmax=False).cpu().numpy()
+    assert np.all(np.isfinite(got)) and got[0, 0, 5, 5] == 9.0 and got[0, 0, 0, 5] == 6.0 and got[0, 0, 0, 39] == 4.0
