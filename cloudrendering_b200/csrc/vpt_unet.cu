@@ -457,10 +457,10 @@ __global__ void __launch_bounds__(kThreads) conv_tile_kernel(const ConvArgs a) {
 __global__ void conv_finalize_kernel(const float* __restrict__ partial, int ksplit, long P, int cout,
                                      const float* __restrict__ bias, const bf16* __restrict__ mask, int relu,
                                      int out_f32, void* __restrict__ y) {
-    const long total = P * (cout / 4);
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const long p = i / (cout / 4);
-        const int c = (int)(i % (cout / 4)) * 4;
+    const uint32_t c4 = (uint32_t)cout / 4, total = (uint32_t)P * c4;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const size_t p = i / c4;
+        const int c = (int)(i - (uint32_t)p * c4) * 4;
         float4 acc = reinterpret_cast<const float4*>(partial + p * cout + c)[0];
         for (int k = 1; k < ksplit; ++k) {
             const float4 u = reinterpret_cast<const float4*>(partial + ((size_t)k * P + p) * cout + c)[0];
@@ -1237,13 +1237,15 @@ __global__ void rotate_weights_kernel(const bf16* __restrict__ w, bf16* __restri
 }
 
 // 2x2 average pooling, [n][h][w][c] -> [n][h/2][w/2][c]
+template <class I>
 __global__ void pool2_kernel(const bf16* __restrict__ in, bf16* __restrict__ out, int n, int h, int w, int c) {
     const int ho = h / 2, wo = w / 2, c8 = c / 8;
-    const long total = (long)n * ho * wo * c8;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int cc = (int)(i % c8) * 8;
-        const long pix = i / c8;
-        const int x = (int)(pix % wo), y = (int)((pix / wo) % ho), b = (int)(pix / ((long)wo * ho));
+    const I total = (I)n * ho * wo * c8;
+    for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const I pix = i / (I)c8;
+        const int cc = (int)(i - pix * c8) * 8;
+        const I row = pix / (I)wo, img = row / (I)ho;
+        const int x = (int)(pix - row * wo), y = (int)(row - img * ho), b = (int)img;
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (int dy = 0; dy < 2; ++dy)
             for (int dx = 0; dx < 2; ++dx) {
@@ -1254,20 +1256,22 @@ __global__ void pool2_kernel(const bf16* __restrict__ in, bf16* __restrict__ out
             }
 #pragma unroll
         for (int k = 0; k < 8; ++k) acc[k] *= 0.25f;
-        store8(out + pix * c + cc, acc);
+        store8(out + (size_t)pix * c + cc, acc);
     }
 }
 
 // out[n][y][x] = (lo[n][y/2][x/2] (ca channels), skip[n][y][x] (cs channels)): nearest upsampling
 // of the coarser level concatenated with the skip connection
+template <class I>
 __global__ void upcat_kernel(const bf16* __restrict__ lo, const bf16* __restrict__ skip, bf16* __restrict__ out,
                              int n, int h, int w, int ca, int cs) {
     const int c = ca + cs, c8 = c / 8;
-    const long total = (long)n * h * w * c8;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int cc = (int)(i % c8) * 8;
-        const long pix = i / c8;
-        const int x = (int)(pix % w), y = (int)((pix / w) % h), b = (int)(pix / ((long)w * h));
+    const I total = (I)n * h * w * c8;
+    for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const I pix = i / (I)c8;
+        const int cc = (int)(i - pix * c8) * 8;
+        const I row = pix / (I)w, img = row / (I)h;
+        const int x = (int)(pix - row * w), y = (int)(row - img * h), b = (int)img;
         const uint4* src;
         if (cc < ca)
             src = reinterpret_cast<const uint4*>(lo + (((size_t)b * (h / 2) + y / 2) * (w / 2) + x / 2) * ca + cc);
@@ -1279,14 +1283,16 @@ __global__ void upcat_kernel(const bf16* __restrict__ lo, const bf16* __restrict
 
 // backward of upcat for the coarse part: dlo[n][y][x][k] = (lo > 0) * sum of the 2x2 children's
 // gradient d[.][k] (k < ca); lo is the coarse level's ReLU output
+template <class I>
 __global__ void upcat_grad_lo_kernel(const bf16* __restrict__ d, const bf16* __restrict__ lo, bf16* __restrict__ dlo,
                                      int n, int h, int w, int ca, int cs) {
     const int ho = h / 2, wo = w / 2, c = ca + cs, c8 = ca / 8;
-    const long total = (long)n * ho * wo * c8;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int cc = (int)(i % c8) * 8;
-        const long pix = i / c8;
-        const int x = (int)(pix % wo), y = (int)((pix / wo) % ho), b = (int)(pix / ((long)wo * ho));
+    const I total = (I)n * ho * wo * c8;
+    for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const I pix = i / (I)c8;
+        const int cc = (int)(i - pix * c8) * 8;
+        const I row = pix / (I)wo, img = row / (I)ho;
+        const int x = (int)(pix - row * wo), y = (int)(row - img * ho), b = (int)img;
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
         for (int dy = 0; dy < 2; ++dy)
             for (int dx = 0; dx < 2; ++dx) {
@@ -1296,25 +1302,27 @@ __global__ void upcat_grad_lo_kernel(const bf16* __restrict__ d, const bf16* __r
                 for (int k = 0; k < 8; ++k) acc[k] += f[k];
             }
         float m[8];
-        load8(lo + pix * ca + cc, m);
+        load8(lo + (size_t)pix * ca + cc, m);
 #pragma unroll
         for (int k = 0; k < 8; ++k) acc[k] = m[k] > 0.0f ? acc[k] : 0.0f;
-        store8(dlo + pix * ca + cc, acc);
+        store8(dlo + (size_t)pix * ca + cc, acc);
     }
 }
 
 // gradient at an encoder level's ReLU output e (c channels): the skip part of the decoder's
 // concatenated gradient (d_cat[p][cat_off + k], row stride cat_c; may be null) plus the pooled
 // branch's gradient d_pool[n][y/2][x/2][k] / 4 (may be null), times (e > 0)
+template <class I>
 __global__ void encoder_grad_kernel(const bf16* __restrict__ d_cat, int cat_c, int cat_off,
                                     const bf16* __restrict__ d_pool, const bf16* __restrict__ e,
                                     bf16* __restrict__ out, int n, int h, int w, int c) {
     const int c8 = c / 8;
-    const long total = (long)n * h * w * c8;
-    for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
-        const int cc = (int)(i % c8) * 8;
-        const long pix = i / c8;
-        const int x = (int)(pix % w), y = (int)((pix / w) % h), b = (int)(pix / ((long)w * h));
+    const I total = (I)n * h * w * c8;
+    for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+        const I pix = i / (I)c8;
+        const int cc = (int)(i - pix * c8) * 8;
+        const I row = pix / (I)w, img = row / (I)h;
+        const int x = (int)(pix - row * w), y = (int)(row - img * h), b = (int)img;
         float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0}, f[8];
         if (d_cat) {
             load8(d_cat + (size_t)pix * cat_c + cat_off + cc, f);
@@ -1357,25 +1365,42 @@ __global__ void bias_grad_kernel(const bf16* __restrict__ dy, float* __restrict_
     }
 }
 
-// gradient of one layer into the flat fp32 gradient: g[co][t][ci] = sum_s wpart[s][t*cin+ci][co]
-// (fixed order over the splits) and gb[co] = sum_b bpart[b][co]
-__global__ void reduce_grads_kernel(const float* __restrict__ wpart, int splits, int m_pad, int cin, int cout,
-                                    const float* __restrict__ bpart, int bblocks, float* __restrict__ gw,
-                                    float* __restrict__ gb) {
-    const int nw = cout * 9 * cin;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nw + cout; i += gridDim.x * blockDim.x) {
-        float s = 0.0f;
-        if (i < nw) {
-            const int ci = i % cin, t = (i / cin) % 9, co = i / (9 * cin);
-            const size_t off = (size_t)(t * cin + ci) * cout + co;
-            for (int k = 0; k < splits; ++k) s += wpart[(size_t)k * m_pad * cout + off];
-            gw[i] = s;
-        } else {
-            const int co = i - nw;
-            if (bpart)
-                for (int k = 0; k < bblocks; ++k) s += bpart[(size_t)k * cout + co];
-            gb[co] = s;
-        }
+// gradient of one layer into the flat fp32 gradient: g[co][t][ci] = sum_s wpart[s][t*cin+ci][co] and
+// gb[co] = sum_b bpart[b][co], in a fixed order.  A warp sums 32 consecutive elements of the partials (its loads are
+// whole lines; reading by the gradient's own order, ci fastest, took a sector per lane): with 8 splits and more the
+// eight warps of a block take the splits s = warp, warp + 8, ... of the same elements and combine through shared
+// memory, with fewer each takes all splits of its own (64 pixels of 128 -> 128 channels, 1 split: eight warps on
+// the same elements made the layer's gradient 2.5 us slower).  Bound: the partials' bytes.  The 19 layers of a training
+// step of 8 images of 256 x 256: 437 us by the gradient's order, 160 us here.
+__global__ void __launch_bounds__(256) reduce_grads_kernel(const float* __restrict__ wpart, int splits, int m_pad,
+                                                           int cin, int cout, const float* __restrict__ bpart,
+                                                           int bblocks, float* __restrict__ gw,
+                                                           float* __restrict__ gb) {
+    __shared__ float part[8][32];
+    const int nw = cout * 9 * cin;  // a multiple of 256
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int wblocks = splits >= 8 ? nw / 32 : nw / 256;  // the blocks of the weights; then 32 biases a block
+    const bool weight = (int)blockIdx.x < wblocks;
+    const bool own = weight && splits < 8;  // a warp's elements are its own
+    const int j = own ? (int)blockIdx.x * 256 + (int)threadIdx.x : ((int)blockIdx.x - (weight ? 0 : wblocks)) * 32 + lane;
+    const float* src = weight ? wpart + j : bpart + j;
+    const size_t stride = weight ? (size_t)m_pad * cout : (size_t)cout;
+    const int count = weight ? splits : (bpart && j < cout ? bblocks : 0), step = own ? 1 : 8;
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = own ? 0 : warp; k < count; k += step) s += __ldg(src + (size_t)k * stride);
+    if (!own) {
+        part[warp][lane] = s;
+        __syncthreads();
+        if (warp > 0) return;
+#pragma unroll
+        for (int k = 1; k < 8; ++k) s += part[k][lane];
+    }
+    if (weight) {
+        const int m = j / cout, co = j - m * cout;  // m = t * cin + ci
+        gw[(size_t)co * 9 * cin + m] = s;
+    } else if (j < cout) {
+        gb[j] = s;
     }
 }
 
@@ -1768,6 +1793,15 @@ inline int grid_for(long work, int threads) {
     if (b < 1) b = 1;
     if (b > 148L * 16) b = 148L * 16;
     return (int)b;
+}
+
+// An elementwise kernel over `units` 16-byte units, with 32-bit indices where they suffice (a 64-bit division by a
+// runtime value is a long software routine, and these kernels divide several times per unit).
+template <class K32, class K64, class... A>
+void launch_units(long units, void* stream, K32 k32, K64 k64, A... args) {
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (units < (1L << 31)) k32<<<grid_for(units, 256), 256, 0, s>>>(args...);
+    else k64<<<grid_for(units, 256), 256, 0, s>>>(args...);
 }
 
 inline int pow2_cols(int n) {
@@ -2275,8 +2309,8 @@ VptStatus vpt_unet_rotate_weights(const void* w, void* wrot, int cin, int cout, 
 
 VptStatus vpt_unet_pool2(const void* in, void* out, int n, int h, int w, int c, void* stream) {
     if (!in || !out || n <= 0 || h <= 1 || w <= 1 || h % 2 || w % 2 || c <= 0 || c % 8) return VPT_ERR_ARG;
-    pool2_kernel<<<grid_for((long)n * (h / 2) * (w / 2) * (c / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const bf16*>(in), static_cast<bf16*>(out), n, h, w, c);
+    launch_units((long)n * (h / 2) * (w / 2) * (c / 8), stream, pool2_kernel<uint32_t>, pool2_kernel<unsigned long long>,
+                 static_cast<const bf16*>(in), static_cast<bf16*>(out), n, h, w, c);
     vpt::count_launches(1);
     return cudaGetLastError() == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
 }
@@ -2286,8 +2320,8 @@ VptStatus vpt_unet_upcat(const void* lo, const void* skip, void* out, int n, int
     if (!lo || !skip || !out || n <= 0 || h <= 1 || w <= 1 || h % 2 || w % 2 || ca <= 0 || ca % 8 || cs <= 0 ||
         cs % 8)
         return VPT_ERR_ARG;
-    upcat_kernel<<<grid_for((long)n * h * w * ((ca + cs) / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const bf16*>(lo), static_cast<const bf16*>(skip), static_cast<bf16*>(out), n, h, w, ca, cs);
+    launch_units((long)n * h * w * ((ca + cs) / 8), stream, upcat_kernel<uint32_t>, upcat_kernel<unsigned long long>,
+                 static_cast<const bf16*>(lo), static_cast<const bf16*>(skip), static_cast<bf16*>(out), n, h, w, ca, cs);
     vpt::count_launches(1);
     return cudaGetLastError() == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
 }
@@ -2297,10 +2331,8 @@ VptStatus vpt_unet_upcat_grad_lo(const void* d, const void* lo, void* dlo, int n
     if (!d || !lo || !dlo || n <= 0 || h <= 1 || w <= 1 || h % 2 || w % 2 || ca <= 0 || ca % 8 || cs <= 0 ||
         cs % 8)
         return VPT_ERR_ARG;
-    upcat_grad_lo_kernel<<<grid_for((long)n * (h / 2) * (w / 2) * (ca / 8), 256), 256, 0,
-                           static_cast<cudaStream_t>(stream)>>>(static_cast<const bf16*>(d),
-                                                                static_cast<const bf16*>(lo), static_cast<bf16*>(dlo),
-                                                                n, h, w, ca, cs);
+    launch_units((long)n * (h / 2) * (w / 2) * (ca / 8), stream, upcat_grad_lo_kernel<uint32_t>, upcat_grad_lo_kernel<unsigned long long>,
+                 static_cast<const bf16*>(d), static_cast<const bf16*>(lo), static_cast<bf16*>(dlo), n, h, w, ca, cs);
     vpt::count_launches(1);
     return cudaGetLastError() == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
 }
@@ -2310,9 +2342,8 @@ VptStatus vpt_unet_encoder_grad(const void* d_cat, int cat_c, int cat_off, const
     if (!e || !out || n <= 0 || h <= 0 || w <= 0 || c <= 0 || c % 8 || (d_cat && (cat_off % 8 || cat_c % 8)) ||
         (d_pool && (h % 2 || w % 2)))
         return VPT_ERR_ARG;
-    encoder_grad_kernel<<<grid_for((long)n * h * w * (c / 8), 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const bf16*>(d_cat), cat_c, cat_off, static_cast<const bf16*>(d_pool),
-        static_cast<const bf16*>(e), static_cast<bf16*>(out), n, h, w, c);
+    launch_units((long)n * h * w * (c / 8), stream, encoder_grad_kernel<uint32_t>, encoder_grad_kernel<unsigned long long>,
+                 static_cast<const bf16*>(d_cat), cat_c, cat_off, static_cast<const bf16*>(d_pool), static_cast<const bf16*>(e), static_cast<bf16*>(out), n, h, w, c);
     vpt::count_launches(1);
     return cudaGetLastError() == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
 }
@@ -2335,7 +2366,8 @@ VptStatus vpt_unet_reduce_grads(const float* wpartial, int splits, int cin, int 
         (bpartial && bblocks <= 0))
         return VPT_ERR_ARG;
     const int m_pad = (9 * cin + kBM - 1) / kBM * kBM;
-    reduce_grads_kernel<<<grid_for((long)cout * 9 * cin + cout, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
+    const int blocks = cout * 9 * cin / (splits >= 8 ? 32 : 256) + (cout + 31) / 32;
+    reduce_grads_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         wpartial, splits, m_pad, cin, cout, bpartial, bblocks, grad_w, grad_b);
     vpt::count_launches(1);
     return cudaGetLastError() == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;

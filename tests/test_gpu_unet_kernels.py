@@ -219,6 +219,57 @@ def test_conv_weight_grad(lib, case):
     close_f32(host(gb), uo.bias_grad(dy))
 
 
+EDGE_CASES = [
+    # n, h, w, cin, cout: rows of less than a K step, of whole steps and one pixel more, several columns; channel
+    # counts below, at and above the operand tiles (16 / 32 / 64 / 128), both operand roles, padded channel groups
+    (1, 1, 1, 16, 16),
+    (2, 3, 15, 16, 48),
+    (1, 5, 16, 48, 16),
+    (1, 7, 17, 32, 144),
+    (2, 4, 64, 80, 80),
+    (1, 3, 127, 144, 48),
+    (1, 2, 128, 16, 16),
+    (1, 9, 129, 48, 80),
+    (1, 3, 260, 80, 64),
+    (1, 30, 128, 176, 32),
+    (1, 3, 131, 112, 16),
+    (1, 5, 130, 32, 144),
+    (2, 5, 150, 96, 224),
+    (1, 128, 128, 96, 96),
+]
+
+
+@pytest.mark.parametrize("path", [0, 2])
+@pytest.mark.parametrize("case", EDGE_CASES)
+def test_conv_kernels_at_tile_edges(lib, request, case, path):
+    """Forward, input gradient and weight gradient through the kernels picked by shape and through the row
+    kernels wherever they apply (output channels in chunks, weight gradients of few pixels)."""
+    n, h, w, cin, cout = case
+    request.addfinalizer(lambda: lib.vpt_unet_set_conv_path(0))
+    assert lib.vpt_unet_set_conv_path(path) == 0
+    x, dy = uo.bf16(rng_data(31, n, h, w, cin)), uo.bf16(rng_data(32, n, h, w, cout))
+    wt = uo.bf16(rng_data(33, cout, 9, cin, scale=1.0 / np.sqrt(9 * cin)))
+    bias = rng_data(34, cout, scale=0.1)
+    d_x, d_dy, d_w, d_b = dev_bf16(x), dev_bf16(dy), dev_bf16(wt), dev_f32(bias)
+    y = torch.full((n, h, w, cout), float("nan"), dtype=torch.float32, device="cuda")
+    run(lib, "vpt_unet_conv3x3", ptr(d_x), ptr(d_w), ptr(d_b), None, ptr(y), n, h, w, cin, cout, 0, 1)
+    close_f32(host(y), uo.conv3x3(x, wt, bias=bias))
+    wrot = torch.empty((cin, 9, cout), dtype=torch.bfloat16, device="cuda")
+    assert lib.vpt_unet_rotate_weights(ptr(d_w), ptr(wrot), cin, cout, None) == 0
+    g = torch.full((n, h, w, cin), float("nan"), dtype=torch.float32, device="cuda")
+    run(lib, "vpt_unet_conv3x3", ptr(d_dy), ptr(wrot), None, ptr(d_x), ptr(g), n, h, w, cout, cin, 0, 1)
+    close_f32(host(g), uo.conv3x3_input_grad(dy, wt, mask=x))
+    splits, rows = lib.vpt_unet_wgrad_splits(n, h, w, cin, cout, 64), lib.vpt_unet_wgrad_rows(cin)
+    part = torch.full((splits, rows, cout), float("nan"), dtype=torch.float32, device="cuda")
+    run(lib, "vpt_unet_conv3x3_wgrad", ptr(d_x), ptr(d_dy), ptr(part), n, h, w, cin, cout, 64)
+    gw = torch.full((cout, 9, cin), float("nan"), dtype=torch.float32, device="cuda")
+    gb = torch.full((cout,), float("nan"), dtype=torch.float32, device="cuda")
+    assert lib.vpt_unet_reduce_grads(ptr(part), splits, cin, cout, None, 0, ptr(gw), ptr(gb), None) == 0
+    torch.cuda.synchronize()
+    close_f32(host(gw), uo.conv3x3_weight_grad(x, dy))
+    assert float(gb.abs().max()) == 0.0
+
+
 def test_pool_upcat_and_gradients(lib):
     n, h, w, ca, cs = 2, 10, 14, 32, 16
     e = uo.bf16(rng_data(10, n, h, w, cs))
