@@ -129,6 +129,26 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, uint64_t da, uint64_t 
         "l"(da), "l"(db), "r"(idesc), "r"(acc)
         : "memory");
 }
+// true in one lane of a converged warp.  The issuing warps run their loops with all lanes and enter the MMA
+// sequences through this: inside `if (lane == 0)` the compiler could not prove the operands warp-uniform and
+// moved every descriptor word to the uniform registers separately, about 250 cycles an MMA.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n.reg .pred P;\nelect.sync _|P, 0xffffffff;\nselp.u32 %0, 1, 0, P;\n}\n" : "=r"(p));
+    return p != 0;
+}
+
+// tcgen05.mma from descriptor halves.  No memory clobber: the MMA reads shared memory asynchronously
+// and is ordered by the mbarrier waits, tcgen05 fences and commits around it (which carry clobbers);
+// without one the issuing loop keeps its loop-invariant values in registers.
+__device__ __forceinline__ void mma_bf16_halves(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
+                                                uint32_t b_hi, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n.reg .pred p;\n.reg .b64 da, db;\nmov.b64 da, {%1, %2};\nmov.b64 db, {%3, %4};\n"
+        "setp.ne.b32 p, %6, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}\n" ::"r"(tmem_d),
+        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc));
+}
+
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n" ::"r"(bar)
                  : "memory");
@@ -182,7 +202,7 @@ __global__ void __launch_bounds__(kThreads) conv_tile_kernel(const ConvArgs a) {
     __shared__ uint64_t bars[kStages];
     __shared__ uint32_t tmem_slot;
 
-    const int tid = threadIdx.x;
+    const int tid = threadIdx.x, warp_u = __shfl_sync(0xffffffffu, tid >> 5, 0);
     const int P = a.n * a.h * a.w_;
     const int n_tile = a.n_tile;
     const uint32_t a_bytes = kBM * kBK * 2;
@@ -219,7 +239,7 @@ __global__ void __launch_bounds__(kThreads) conv_tile_kernel(const ConvArgs a) {
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
 
     // per-thread gather state
     int pn = 0, py = 0, px = 0;
@@ -347,17 +367,21 @@ __global__ void __launch_bounds__(kThreads) conv_tile_kernel(const ConvArgs a) {
         cp_async_wait<kStages - 2>();
         fence_proxy_async();
         if (__syncthreads_or(aborted)) break;
-        if (tid == 0) {
+        if (warp_u == 0) {
             tc_fence_after();
-            const uint32_t sA = sbase + slot * stage_bytes;
-            const uint32_t sB = sA + a_bytes;
-            const int steps = min(kBK / 16, (K - (s_first + s) * kBK + 15) / 16);
-            for (int j = 0; j < steps; ++j) {
-                const uint64_t da = smem_desc(sA + j * 2 * a_lbo, a_lbo, 128);
-                const uint64_t db = smem_desc(sB + j * 2 * b_lbo, b_lbo, 128);
-                mma_bf16(tmem, da, db, idesc, (s > 0 || j > 0) ? 1u : 0u);
+            if (elect_one()) {
+                const uint32_t sA = sbase + slot * stage_bytes;
+                const uint32_t sB = sA + a_bytes;
+                const int steps = min(kBK / 16, (K - (s_first + s) * kBK + 15) / 16);
+                const uint64_t da = smem_desc(sA, a_lbo, 128), db = smem_desc(sB, b_lbo, 128);
+                const uint32_t a_lo = (uint32_t)da, a_hi = (uint32_t)(da >> 32);
+                const uint32_t b_lo = (uint32_t)db, b_hi = (uint32_t)(db >> 32);
+                for (int j = 0; j < steps; ++j)  // 16 K: two 8-channel planes of each operand
+                    mma_bf16_halves(tmem, a_lo + (uint32_t)j * (a_lbo >> 3), a_hi, b_lo + (uint32_t)j * (b_lbo >> 3), b_hi,
+                                    idesc, (s > 0 || j > 0) ? 1u : 0u);
+                mma_commit(smem_u32(&bars[slot]));
             }
-            mma_commit(smem_u32(&bars[slot]));
+            __syncwarp();
         }
         issued = s;
         const int nxt = s + kStages - 1;
@@ -720,7 +744,7 @@ __global__ void __launch_bounds__(kThreads) conv_strip_kernel(const StripArgs a)
 //              swizzled K-major layout of that line width (pixel rows of 128 / 64 / 32 bytes), rows and
 //              pixels outside the image arriving as zeros; full[s] completes on the bytes, empty[s] is
 //              signalled by the tensor core once the last MMA reading the slot has completed;
-//   warps 1, 6 one lane each issues the 9 x cin/16 MMAs of every other output row (accumulator
+//   warps 1, 6 each issue the 9 x cin/16 MMAs of every other output row (accumulator
 //              index g: warp 1 the even, warp 6 the odd) into TMEM accumulator g % 2 (acc_full[b] on
 //              completion, after acc_empty[b]): one issuing thread is the bound for small N (about 93
 //              cycles per MMA against the tensor core's 48), two overlap their issue;
@@ -788,17 +812,6 @@ __device__ __forceinline__ uint64_t smem_desc_sw(uint32_t addr, uint32_t line) {
     return d;
 }
 
-// tcgen05.mma from descriptor halves.  No memory clobber: the MMA reads shared memory asynchronously
-// and is ordered by the mbarrier waits, tcgen05 fences and commits around it (which carry clobbers);
-// without one the issuing loop keeps its loop-invariant values in registers.
-__device__ __forceinline__ void mma_bf16_halves(uint32_t tmem_d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo,
-                                                uint32_t b_hi, uint32_t idesc, uint32_t acc) {
-    asm volatile(
-        "{\n.reg .pred p;\n.reg .b64 da, db;\nmov.b64 da, {%1, %2};\nmov.b64 db, {%3, %4};\n"
-        "setp.ne.b32 p, %6, 0;\ntcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %5, p;\n}\n" ::"r"(tmem_d),
-        "r"(a_lo), "r"(a_hi), "r"(b_lo), "r"(b_hi), "r"(idesc), "r"(acc));
-}
-
 // high word of smem_desc_sw: SBO = 8 lines, version, layout type of the line width (2 * channels)
 __device__ __forceinline__ uint32_t a_hi_of(int channels) {
     return (uint32_t)(smem_desc_sw(0, (uint32_t)channels * 2u) >> 32);
@@ -813,7 +826,7 @@ __global__ void __launch_bounds__(kWsThreads, 2) conv_ws_kernel(const __grid_con
     __shared__ uint32_t tmem_slot;
     __shared__ int fail_any;
     const StripArgs& a = wa.s;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int nkc = a.cin / 8;
     const uint32_t w_bytes = 9u * (uint32_t)a.cin * (uint32_t)a.cout * 2u;
     const uint32_t row_bytes = (uint32_t)wa.row_bytes;
@@ -846,7 +859,7 @@ __global__ void __launch_bounds__(kWsThreads, 2) conv_ws_kernel(const __grid_con
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
     const int total_segs = a.n * a.xtiles * a.segs_per_col;
     bool fail = false;
 
@@ -890,79 +903,69 @@ __global__ void __launch_bounds__(kWsThreads, 2) conv_ws_kernel(const __grid_con
             }
         }
     } else if (warp == 1 || warp == 6) {
-        if (lane == 0) {
-            const int mw = warp == 1 ? 0 : 1;  // this warp's accumulator parity
-            const uint32_t idesc = instr_desc(kBM, a.cout, 0, 0);
-            // descriptor words: A (swizzled, start field added per row / group / dx / step; LBO 1),
-            // B (no swizzle, LBO = one 8-channel plane of the weights, SBO 128)
-            const uint64_t bd0 = smem_desc(sw, (uint32_t)a.cout * 16u, 128);
-            const uint32_t b_hi = (uint32_t)(bd0 >> 32), b_lo0 = (uint32_t)bd0;
-            const uint32_t a_lo1 = 1u << 16;  // LBO field of the A descriptors
-            const uint32_t b_step = 2u * (uint32_t)a.cout, b_tap = (uint32_t)(nkc * a.cout), b_row = 3u * b_tap;
-            // per channel group (registers: every index below is a compile-time constant)
-            const int ngroups = wa.ngroups;
-            uint32_t g_ahi[kWsMaxGroups], g_aoff[kWsMaxGroups], g_line[kWsMaxGroups], g_boff[kWsMaxGroups];
-            int g_steps[kWsMaxGroups];
-#pragma unroll
-            for (int k = 0; k < kWsMaxGroups; ++k) {
-                const bool on = k < ngroups;
-                const int gw = on ? wa.gw[k] : 16;
-                g_ahi[k] = a_hi_of(gw);
-                g_aoff[k] = on ? (uint32_t)wa.goff[k] >> 4 : 0u;
-                g_line[k] = (uint32_t)gw >> 3;  // line bytes / 16
-                g_boff[k] = on ? (uint32_t)((wa.gc[k] >> 3) * a.cout) : 0u;
-                g_steps[k] = gw / 16;
-            }
-            int slot = 0;        // ring position of the segment's first row
-            uint32_t phase = 0;
-            long g = 0;          // accumulators used (both warps count every output row)
-            // Ring slots are released by both issuing warps (empty[] counts 2): after output row i
-            // its warp releases input rows i and i+1 (its last uses of them: it also computed row
-            // i-2, the other warp rows i-1 and i+1).  Rows without such a row get the arrival at the
-            // segment's start (input row 0 from the warp of row -1) or end (rows `rows`, `rows`+1).
-            auto own = [&](long gi) { return (int)(gi & 1) == mw; };
-            auto slot_of = [&](int r) { return (uint32_t)((slot + r) % ring); };
-            for (int seg = blockIdx.x; seg < total_segs && !fail; seg += gridDim.x) {
-                const WsSegment sgm = ws_segment(a, seg);
-                if (sgm.y0 >= sgm.y1) continue;
-                const int rows = sgm.y1 - sgm.y0;
-                const long g0 = g;
-                if (own(g0 - 1)) mbar_arrive(smem_u32(&empty[slot_of(0)]));
-                for (int i = 0; i < rows && !fail; ++i, ++g) {
-                    if (!own(g)) continue;
-                    // input rows i, i+1, i+2 of the segment (y-1, y, y+1)
-                    for (int k = 0; k <= 2; ++k) {
-                        const int pos = slot + i + k;
-                        const uint32_t ph = phase ^ (uint32_t)((pos / ring) & 1);
-                        if (!mbar_wait(smem_u32(&full[pos % ring]), ph)) fail = true;
-                    }
-                    const int b = (int)(g & 1);
-                    if (!fail && !mbar_wait(smem_u32(&acc_empty[b]), (uint32_t)(((g >> 1) & 1) ^ 1))) fail = true;
-                    if (fail) break;
-                    tc_fence_after();
+        const int mw = warp == 1 ? 0 : 1;  // this warp's accumulator parity
+        const uint32_t idesc = instr_desc(kBM, a.cout, 0, 0);
+        // descriptor words: A (swizzled, start field added per row / group / dx / step; LBO 1),
+        // B (no swizzle, LBO = one 8-channel plane of the weights, SBO 128)
+        const uint64_t bd0 = smem_desc(sw, (uint32_t)a.cout * 16u, 128);
+        const uint32_t b_hi = (uint32_t)(bd0 >> 32), b_lo0 = (uint32_t)bd0;
+        const uint32_t a_lo1 = 1u << 16;  // LBO field of the A descriptors
+        const uint32_t b_step = 2u * (uint32_t)a.cout, b_tap = (uint32_t)(nkc * a.cout), b_row = 3u * b_tap;
+        const int ngroups = wa.ngroups;
+        int slot = 0;        // ring position of the segment's first row
+        uint32_t phase = 0;
+        long g = 0;          // accumulators used (both warps count every output row)
+        // Ring slots are released by both issuing warps (empty[] counts 2): after output row i
+        // its warp releases input rows i and i+1 (its last uses of them: it also computed row
+        // i-2, the other warp rows i-1 and i+1).  Rows without such a row get the arrival at the
+        // segment's start (input row 0 from the warp of row -1) or end (rows `rows`, `rows`+1).
+        auto own = [&](long gi) { return (int)(gi & 1) == mw; };
+        auto slot_of = [&](int r) { return (uint32_t)((slot + r) % ring); };
+        for (int seg = blockIdx.x; seg < total_segs && !fail; seg += gridDim.x) {
+            const WsSegment sgm = ws_segment(a, seg);
+            if (sgm.y0 >= sgm.y1) continue;
+            const int rows = sgm.y1 - sgm.y0;
+            const long g0 = g;
+            if (own(g0 - 1) && elect_one()) mbar_arrive(smem_u32(&empty[slot_of(0)]));
+            __syncwarp();
+            for (int i = 0; i < rows && !fail; ++i, ++g) {
+                if (!own(g)) continue;
+                // input rows i, i+1, i+2 of the segment (y-1, y, y+1)
+                bool ok = true;
+                for (int k = 0; k <= 2; ++k) {
+                    const int pos = slot + i + k;
+                    const uint32_t ph = phase ^ (uint32_t)((pos / ring) & 1);
+                    ok = ok && mbar_wait(smem_u32(&full[pos % ring]), ph);
+                }
+                const int b = (int)(g & 1);
+                ok = ok && mbar_wait(smem_u32(&acc_empty[b]), (uint32_t)(((g >> 1) & 1) ^ 1));
+                if (!__all_sync(0xffffffffu, ok)) {
+                    fail = true;
+                    break;
+                }
+                tc_fence_after();
+                if (elect_one()) {
                     const uint32_t dacc = tmem + (uint32_t)b * acc_cols;
                     // descriptors walk affinely: per channel group, A's start advances by one pixel
                     // row per dx and 32 bytes per 16-channel step, B's by a tap (nkc * cout * 16
                     // bytes) per dx and two 8-channel planes per step
                     uint32_t acc = 0;
-#pragma unroll 1
                     for (int dy = 0; dy < 3; ++dy) {
                         const uint32_t row16 = (sring + slot_of(i + dy) * row_bytes) >> 4;
-#pragma unroll
-                        for (int k = 0; k < kWsMaxGroups; ++k) {
-                            if (k >= ngroups) break;
-                            const uint32_t al0 = a_lo1 + row16 + g_aoff[k];
-                            const uint32_t bl0 = b_lo0 + (uint32_t)dy * b_row + g_boff[k];
+                        for (int k = 0; k < ngroups; ++k) {
+                            const int gw = wa.gw[k];
+                            const uint32_t ahi = a_hi_of(gw);
+                            uint32_t al = a_lo1 + row16 + ((uint32_t)wa.goff[k] >> 4);
+                            uint32_t bl = b_lo0 + (uint32_t)dy * b_row + (uint32_t)((wa.gc[k] >> 3) * a.cout);
 #pragma unroll
                             for (int dx = 0; dx < 3; ++dx) {
-                                const uint32_t al = al0 + (uint32_t)dx * g_line[k], bl = bl0 + (uint32_t)dx * b_tap;
-#pragma unroll
-                                for (int j = 0; j < 4; ++j) {
-                                    if (j >= g_steps[k]) break;
-                                    mma_bf16_halves(dacc, al + 2u * (uint32_t)j, g_ahi[k], bl + (uint32_t)j * b_step,
-                                                    b_hi, idesc, acc);
+                                for (int jj = 0; jj < gw / 16; ++jj) {
+                                    mma_bf16_halves(dacc, al + 2u * (uint32_t)jj, ahi, bl + (uint32_t)jj * b_step, b_hi,
+                                                    idesc, acc);
                                     acc = 1;
                                 }
+                                al += (uint32_t)gw >> 3;
+                                bl += b_tap;
                             }
                         }
                     }
@@ -970,20 +973,25 @@ __global__ void __launch_bounds__(kWsThreads, 2) conv_ws_kernel(const __grid_con
                     mma_commit(smem_u32(&empty[slot_of(i)]));
                     mma_commit(smem_u32(&empty[slot_of(i + 1)]));
                 }
-                if (fail) break;
+                __syncwarp();
+            }
+            if (fail) break;
+            if (elect_one()) {
                 if (own(g0 + rows - 1)) mma_commit(smem_u32(&empty[slot_of(rows + 1)]));
                 if (own(g0 + rows)) {
                     mma_commit(smem_u32(&empty[slot_of(rows)]));
                     mma_commit(smem_u32(&empty[slot_of(rows + 1)]));
                 }
-                const int adv = slot + rows + 2;
-                slot = adv % ring;
-                phase ^= (uint32_t)((adv / ring) & 1);
             }
-            // every MMA this warp issued has completed before TMEM is released
-            mma_commit(smem_u32(&done_bar[mw]));
-            if (!mbar_wait(smem_u32(&done_bar[mw]), 0)) fail = true;
+            __syncwarp();
+            const int adv = slot + rows + 2;
+            slot = adv % ring;
+            phase ^= (uint32_t)((adv / ring) & 1);
         }
+        // every MMA this warp issued has completed before TMEM is released
+        if (elect_one()) mma_commit(smem_u32(&done_bar[mw]));
+        __syncwarp();
+        if (!mbar_wait(smem_u32(&done_bar[mw]), 0)) fail = true;
     } else if (warp >= 2 && warp <= 5) {
         const int quarter = warp & 3;
         long g = 0;
@@ -1001,6 +1009,368 @@ __global__ void __launch_bounds__(kWsThreads, 2) conv_ws_kernel(const __grid_con
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
+            }
+        }
+    }
+    if (fail) atomicOr(&fail_any, 1);
+    tc_fence_before();
+    __syncthreads();
+    if (fail_any && tid == 0 && a.err) atomicExch(a.err, (int)VPT_ERR_ITER_LIMIT);
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, (uint32_t)a.tmem_cols);
+    }
+}
+
+
+// ---------------------------------------------------------------------------------------------
+// the warp-specialised row-strip convolution with stacked rows
+// ---------------------------------------------------------------------------------------------
+// conv_ws_kernel issues 9 x cin/16 MMAs of N = cout columns a row, and an MMA takes the same time for every N up to
+// 96 (its issue, about 93 cycles; the tensor core's own minimum is 48).  This kernel turns the sum over dy around:
+// the three output rows y-1, y, y+1 that read input row y have adjacent accumulators, and one MMA of N = 3 cout
+// columns adds input row y's contribution to all of them, its B operand being the taps dy = +1, 0, -1 stacked:
+// 3 x cin/16 (+ 1) MMAs a row.  A launch computes `cout` <= 80 of the layer's output channels.
+//   Layer, us, 8 images of 256 x 256 (conv_ws_kernel / here): 96 -> 32 93.0 / 56.0, 32 -> 32 29.0 / 23.3, 16 -> 32
+// 24.2 / 18.6; one image of 256 x 256, 32 -> 32 10.0 / 10.2, 48 -> 48 at half that size 17.2 / 13.2.  Bound: 8 us
+// to start, load the weights and drain, then the bytes (32 -> 32 67 MB, 10 us at 6.65 TB/s; 96 -> 32 134 MB, 20 us)
+// and the MMAs' issue (96 -> 32: 19 of about 90 cycles a row and 28 rows an SM, 25 us), which overlap in part.
+//   ring      input rows as in conv_ws_kernel, but a slot is free again after its own row's MMAs: two slots do.
+//   TMEM      a ring of `blocks` accumulators of cout columns, output row g of the CTA in block g % blocks;
+//             three adjacent rows are contiguous columns except around the ring's end (then two MMAs).
+//   first use an output row's first MMA (its dy = -1 taps, dx = -1, first 16 channels) overwrites its block,
+//             so that step is split into N = cout (overwrite) and the older rows (accumulate).
+//   sets      with many input channels (longer sums in the accumulator's fp32) the channel groups alternate
+//             between two such rings, which the epilogue adds.
+//   order     one thread issues every MMA, so an accumulator's updates and the commits behind them are in
+//             order: after input row q's MMAs one commit frees its ring slot, one hands row q-2 (counted
+//             from the segment's start) to the epilogue.
+// Warps: 0 loads input rows, 1 issues, 2-9 run the epilogue (two teams of four take the rows alternately: one
+// team, 2700 cycles a row of 32 channels, was the kernel's bound).  The weights are copied by warps 1-9 while
+// the first rows arrive.  Every wait is bounded, as in conv_ws_kernel.
+constexpr int kStackThreads = 320;  // producer, issuer, 8 epilogue warps
+constexpr int kStackMaxBlocks = 8;
+constexpr int kStackMaxCout = 80;  // 3 cout <= 256 columns
+
+struct StackArgs {
+    WsArgs ws;
+    int ring, blocks;
+    int sets;  // 2: the channel groups alternate between two accumulator rings, added in the epilogue
+    int co0, cout_total;  // first output channel of this launch, channels per pixel of y
+};
+
+// The image columns (at most 128 pixels wide) of a batch, their rows taken as one sequence that the CTAs split
+// evenly: CTA i owns rows [i R / G, (i + 1) R / G), in segments of one column each.
+struct RowRange {
+    int row, end, h, xtiles;
+    __device__ __forceinline__ RowRange(int n, int h_, int xtiles_) : h(h_), xtiles(xtiles_) {
+        const long rows = (long)n * xtiles_ * h_;
+        row = (int)(rows * blockIdx.x / gridDim.x);
+        end = (int)(rows * (blockIdx.x + 1) / gridDim.x);
+    }
+    __device__ __forceinline__ bool next(WsSegment& g) {
+        if (row >= end) return false;
+        const int col = row / h;
+        g.n_img = col / xtiles;
+        g.x0 = (col % xtiles) * kBM;
+        g.y0 = row - col * h;
+        g.y1 = min(h, g.y0 + (end - row));
+        row += g.y1 - g.y0;
+        return true;
+    }
+};
+
+// Epilogue of one accumulator row for this warp's 32 pixels (at: offset of the lane's pixel and this
+// launch's first channel): partial sums
+// of earlier passes, bias, ReLU, mask, store.  set2: column offset of a second accumulator that is added (0 = none).
+__device__ __forceinline__ void stack_epilogue(const StripArgs& a, const float* bias, uint32_t tacc, uint32_t set2,
+                                               size_t at, bool ok, const uint4 (&mask)[kStackMaxCout / 8]) {
+#pragma unroll
+    for (int k = 0; k < kStackMaxCout / 16; ++k) {
+        const int c0 = 16 * k;
+        if (c0 >= a.cout) break;
+        float v[16];
+        tmem_ld16(tacc + (uint32_t)c0, v);
+        if (set2) {
+            float v2[16];
+            tmem_ld16(tacc + set2 + (uint32_t)c0, v2);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += v2[i];
+        }
+        if (!ok) continue;
+        if (a.part_in) {
+            const float4* src = reinterpret_cast<const float4*>(a.part_in + at + c0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const float4 t = src[i];
+                v[4 * i] += t.x;
+                v[4 * i + 1] += t.y;
+                v[4 * i + 2] += t.z;
+                v[4 * i + 3] += t.w;
+            }
+        }
+        if (a.part_out) {
+            float4* dst = reinterpret_cast<float4*>(a.part_out + at + c0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+            continue;
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] += bias[c0 + i];
+        if (a.relu) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
+        }
+        if (a.mask) {
+            const uint4 m4[2] = {mask[2 * k], mask[2 * k + 1]};
+            const bf16* mb = reinterpret_cast<const bf16*>(m4);
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] = __bfloat162float(mb[i]) > 0.0f ? v[i] : 0.0f;
+        }
+        if (a.out_f32) {
+            float4* dst = reinterpret_cast<float4*>(static_cast<float*>(a.y) + at + c0);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        } else {
+            uint4 o[2];
+            __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(o);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) ob[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+            uint4* dst = reinterpret_cast<uint4*>(static_cast<bf16*>(a.y) + at + c0);
+            dst[0] = o[0];
+            dst[1] = o[1];
+        }
+    }
+}
+
+__global__ void __launch_bounds__(kStackThreads, 2)
+    conv_stack_kernel(const __grid_constant__ CUtensorMap map64, const __grid_constant__ CUtensorMap map32,
+                      const __grid_constant__ CUtensorMap map16, const __grid_constant__ StackArgs st) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ uint64_t full[kWsMaxRing], empty[kWsMaxRing], acc_full[kStackMaxBlocks], acc_empty[kStackMaxBlocks],
+        done_bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int fail_any;
+    __shared__ __align__(16) float s_bias[kStackMaxCout];
+    const WsArgs& wa = st.ws;
+    const StripArgs& a = wa.s;
+    const int ring = st.ring, blocks = st.blocks;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int nkc = a.cin / 8, cout = a.cout;
+    const uint32_t w_bytes = 9u * (uint32_t)a.cin * (uint32_t)cout * 2u;
+    const uint32_t row_bytes = (uint32_t)wa.row_bytes;
+    const uint32_t sw = smem_u32(smem);
+    const uint32_t sring = sw + ((w_bytes + 1023u) & ~1023u);
+    if (tid == 0) {
+        for (int k = 0; k < ring; ++k) {
+            mbar_init(smem_u32(&full[k]), 1);
+            mbar_init(smem_u32(&empty[k]), 1);
+        }
+        for (int k = 0; k < blocks; ++k) {
+            mbar_init(smem_u32(&acc_full[k]), 1);
+            mbar_init(smem_u32(&acc_empty[k]), 4);  // one arrival per epilogue warp
+        }
+        mbar_init(smem_u32(&done_bar), 1);
+        fail_any = 0;
+        fence_mbar_init();
+    }
+    if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), (uint32_t)a.tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    bool fail = false;
+
+    if (warp > 0) {
+        // weights: unit (dx, kc, p, co), p = 2 - dy, at (((dx * nkc + kc) * 3 + p) * cout + co) * 16
+        for (int q = tid - 32; q < 9 * nkc * cout; q += kStackThreads - 32) {
+            const int co = q % cout;
+            int rest = q / cout;
+            const int p = rest % 3;
+            rest /= 3;
+            const int kc = rest % nkc, dx = rest / nkc;
+            const int t = (2 - p) * 3 + dx;
+            cp_async16(sw + (uint32_t)q * 16u, a.w + ((size_t)(st.co0 + co) * 9 + t) * a.cin_total + a.c0 + kc * 8,
+                       true);
+        }
+        for (int c = tid - 32; c < cout; c += kStackThreads - 32) s_bias[c] = a.bias ? a.bias[st.co0 + c] : 0.0f;
+        cp_async_commit();
+        cp_async_wait<0>();
+        fence_proxy_async();
+        asm volatile("bar.sync 1, %0;\n" ::"n"(kStackThreads - 32) : "memory");
+    }
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int slot = 0;
+            uint32_t phase = 0;
+            long issued = 0;
+            RowRange range(a.n, a.h, a.xtiles);
+            WsSegment g;
+            while (!fail && range.next(g)) {
+                for (int yy = g.y0 - 1; yy <= g.y1; ++yy) {
+                    if (!mbar_wait(smem_u32(&empty[slot]), phase ^ 1u)) {
+                        fail = true;
+                        break;
+                    }
+                    const uint32_t dst = sring + (uint32_t)slot * row_bytes;
+                    const uint32_t fb = smem_u32(&full[slot]);
+                    mbar_arrive_expect_tx(fb, (uint32_t)wa.tx_bytes);
+                    for (int k = 0; k < wa.ngroups; ++k) {
+                        const CUtensorMap* m = wa.gw[k] == 64 ? &map64 : (wa.gw[k] == 32 ? &map32 : &map16);
+                        tma_load_4d(dst + (uint32_t)wa.goff[k], m, a.c0 + wa.gc[k], g.x0 - 1, yy, g.n_img, fb);
+                    }
+                    ++issued;
+                    if (++slot == ring) {
+                        slot = 0;
+                        phase ^= 1u;
+                    }
+                }
+            }
+            // the last loads (one per slot at most) have landed before the CTA can exit
+            const long tail = issued < ring ? issued : ring;
+            for (long k = 1; k <= tail; ++k) {
+                int sl = slot - (int)k;
+                uint32_t ph = phase;
+                if (sl < 0) {
+                    sl += ring;
+                    ph ^= 1u;
+                }
+                if (!mbar_wait(smem_u32(&full[sl]), ph)) fail = true;
+            }
+        }
+    } else if (warp == 1) {
+        // descriptor words: A (swizzled, start field added per row / group / dx / step; LBO 1), B (no
+        // swizzle, LBO = one 8-channel plane of 3 cout rows, SBO 128)
+        const uint32_t n3 = 3u * (uint32_t)cout;
+        const uint64_t bd0 = smem_desc(sw, n3 * 16u, 128);
+        const uint32_t b_hi = (uint32_t)(bd0 >> 32), b_lo0 = (uint32_t)bd0;
+        const uint32_t a_lo1 = 1u << 16;
+        const uint32_t b_step = 2u * n3, b_dx = (uint32_t)nkc * n3;
+        const uint32_t id1 = instr_desc(kBM, cout, 0, 0);
+        const uint32_t id_n = (uint32_t)(cout >> 3) << 17;  // one more block of columns
+        const int ngroups = wa.ngroups;
+        const uint32_t set_cols = (uint32_t)(blocks * cout);
+        int slot = 0;
+        uint32_t phase = 0;
+        int blk0 = 0;        // block of the segment's first output row
+        uint32_t use0 = 0;   // parity of that block's use count
+        RowRange range(a.n, a.h, a.xtiles);
+        WsSegment sgm;
+        while (!fail && range.next(sgm)) {
+            const int rows = sgm.y1 - sgm.y0;
+            // block of output rows q - 2 and q, and the use parity of the latter's
+            int b2 = blk0, b0 = blk0;
+            uint32_t u0 = use0;
+            for (int q = 0; q < rows + 2; ++q) {
+                const int lo = q < 2 ? 0 : q - 2, hi = min(q, rows - 1);  // output rows that read input row q
+                const int blo = q < 2 ? blk0 : b2;                        // block of row lo
+                const bool fresh = q < rows;                              // row q starts here
+                bool ok = mbar_wait(smem_u32(&full[slot]), phase);
+                if (fresh) ok = ok && mbar_wait(smem_u32(&acc_empty[b0]), u0 ^ 1u);
+                if (!__all_sync(0xffffffffu, ok)) {
+                    fail = true;
+                    break;
+                }
+                tc_fence_after();
+                if (elect_one()) {
+                    const uint32_t row16 = (sring + (uint32_t)slot * row_bytes) >> 4;
+                    const int cnt = hi - lo + 1;
+                    const int n_first = min(cnt, blocks - blo);  // columns up to the ring's end, then the rest
+                    const int n_rest = cnt - n_first;
+                    const uint32_t p0 = (uint32_t)((2 - q + lo) * cout), p_rest = p0 + (uint32_t)(n_first * cout);
+                    const uint32_t id_first = id1 + (uint32_t)(n_first - 1) * id_n;
+                    const uint32_t id_rest = id1 + (uint32_t)(n_rest - 1) * id_n;
+                    for (int k = 0; k < ngroups; ++k) {
+                        const int gw = wa.gw[k];
+                        const uint32_t ahi = a_hi_of(gw);
+                        const uint32_t line16 = (uint32_t)gw >> 3;
+                        // the channel groups alternate between the sets; a set's first step overwrites
+                        const uint32_t acc0 = tmem + (st.sets == 2 ? (uint32_t)(k & 1) * set_cols : 0u);
+                        bool first = fresh && k < st.sets;
+                        uint32_t al = a_lo1 + row16 + ((uint32_t)wa.goff[k] >> 4);
+                        uint32_t bl = b_lo0 + (uint32_t)(wa.gc[k] >> 3) * n3;
+#pragma unroll
+                        for (int dx = 0; dx < 3; ++dx) {
+                            uint32_t aj = al, bj = bl;
+                            for (int j = 0; j < gw / 16; ++j) {
+                                if (first) {  // the new row overwrites its block, the older ones accumulate
+                                    first = false;
+                                    for (int i = lo; i <= hi; ++i) {
+                                        const int bi = blo + (i - lo) < blocks ? blo + (i - lo) : blo + (i - lo) - blocks;
+                                        mma_bf16_halves(acc0 + (uint32_t)(bi * cout), aj, ahi,
+                                                        bj + (uint32_t)((2 - q + i) * cout), b_hi, id1, i < q ? 1u : 0u);
+                                    }
+                                } else {
+                                    mma_bf16_halves(acc0 + (uint32_t)(blo * cout), aj, ahi, bj + p0, b_hi, id_first, 1u);
+                                    if (n_rest > 0) mma_bf16_halves(acc0, aj, ahi, bj + p_rest, b_hi, id_rest, 1u);
+                                }
+                                aj += 2u;
+                                bj += b_step;
+                            }
+                            al += line16;
+                            bl += b_dx;
+                        }
+                    }
+                    mma_commit(smem_u32(&empty[slot]));
+                    if (q >= 2) mma_commit(smem_u32(&acc_full[b2]));
+                }
+                __syncwarp();
+                if (++slot == ring) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+                if (q >= 2 && ++b2 == blocks) b2 = 0;
+                if (fresh && ++b0 == blocks) {
+                    b0 = 0;
+                    u0 ^= 1u;
+                }
+            }
+            blk0 = b0;
+            use0 = u0;
+        }
+        // every MMA this warp issued has completed before TMEM is released
+        if (elect_one()) mma_commit(smem_u32(&done_bar));
+        __syncwarp();
+        if (!mbar_wait(smem_u32(&done_bar), 0)) fail = true;
+    } else {
+        // two teams of four warps take the rows alternately; before it waits for its row a warp has the row's
+        // ReLU mask on the way
+        const int quarter = warp & 3, team = (warp - 2) >> 2;
+        const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+        int b = 0, turn = 0;
+        uint32_t u = 0;
+        RowRange range(a.n, a.h, a.xtiles);
+        WsSegment sgm;
+        while (!fail && range.next(sgm)) {
+            const int x = sgm.x0 + quarter * 32 + lane;
+            const bool ok = x < a.w_;
+            for (int y = sgm.y0; y < sgm.y1; ++y) {
+                if (turn == team) {
+                    const size_t at = (((size_t)sgm.n_img * a.h + y) * a.w_ + (ok ? x : 0)) * st.cout_total + st.co0;
+                    uint4 mask[kStackMaxCout / 8];
+                    if (a.mask) {
+#pragma unroll
+                        for (int k = 0; k < kStackMaxCout / 8; ++k)
+                            if (k * 8 < cout) mask[k] = __ldg(reinterpret_cast<const uint4*>(a.mask + at) + k);
+                    }
+                    const bool full_ok = mbar_wait(smem_u32(&acc_full[b]), u);
+                    if (!__all_sync(0xffffffffu, full_ok)) {
+                        fail = true;
+                        break;
+                    }
+                    tc_fence_after();
+                    stack_epilogue(a, s_bias, tmem + lanes + (uint32_t)(b * cout),
+                                   st.sets == 2 ? (uint32_t)(blocks * cout) : 0u, at, ok, mask);
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
+                }
+                turn ^= 1;
+                if (++b == blocks) {
+                    b = 0;
+                    u ^= 1u;
+                }
             }
         }
     }
@@ -2040,6 +2410,29 @@ inline WsGroups ws_groups_of(int cin) {
 inline size_t ws_weight_bytes(int cin, int cout) { return (9ul * cin * cout * 2 + 1023) & ~(size_t)1023; }
 inline size_t ws_row_bytes(int cin) { return (size_t)ws_groups_of(cin).row_bytes; }
 
+// accumulator sets of the stacked kernel: 99 or more accumulations in one would round more than the two
+// passes over channel groups that such layers took
+inline int stack_sets(int cin) { return cin > 96 ? 2 : 1; }
+
+// The stacked kernel (cout <= kStackMaxCout a launch): a ring slot is free again after its own row's MMAs, so two slots
+// do; two CTAs per SM when each gets three (their issuing threads overlap) and at least four accumulators.
+bool stack_config(int cin, int cout, int& per_sm, int& ring) {
+    const size_t rb = ws_row_bytes(cin), wb = ws_weight_bytes(cin, cout);
+    per_sm = 0;
+    ring = 0;
+    if (rb == 0) return false;
+    for (int occ = 2; occ >= 1; --occ) {
+        const size_t budget = std::min(kSmPerSm / occ - kWsStatic, kSmPerCta);
+        if (wb >= budget || 512 / occ / (cout * stack_sets(cin)) < 4) continue;
+        const int r = (int)std::min<size_t>(kWsMaxRing, (budget - wb) / rb);
+        if (r < (occ == 2 ? 3 : 2)) continue;
+        per_sm = occ;
+        ring = r;
+        return true;
+    }
+    return false;
+}
+
 // CTAs per SM and ring depth: the most rows in flight per SM (CTAs x (ring - 3)), then more CTAs;
 // TMEM holds two accumulators per CTA.  false when not even one CTA with a 4-slot ring fits.
 bool ws_config(int cin, int cout, int& per_sm, int& ring) {
@@ -2065,31 +2458,58 @@ bool ws_config(int cin, int cout, int& per_sm, int& ring) {
     return per_sm > 0;
 }
 
-// input-channel passes for the warp-specialised kernel (0 = not eligible).  Several passes re-stream
-// an fp32 partial: measured faster than the gather kernel for up to 64 output channels (176 -> 32,
-// 160 -> 64), slower for 96 -> 96 and 224 -> 96.
-inline int ws_groups(int width, int cin, int cout, bool any = false) {
-    if (width < kBM || cout > 256) return 0;
+
+// How the warp-specialised kernels take a layer.  Input channels: one pass where the weights and the rings fit,
+// else up to 4 passes through an fp32 partial, which beat the gather kernel for up to 64 output channels only
+// (measured).  Output channels: conv_stack_kernel for up to 80 of them, in chunks of at most 80 (each launch reads
+// the input again) or all of them in conv_ws_kernel (chunk = 0) beyond.  us, gather or conv_ws / chunks, at 128 pixels
+// a row:
+//   conv_ws does not fit (gather, whose CTAs hold all outputs of 128 pixels)   chunks from 64 rows a chunk
+//     96 -> 96    64 rows 24.2 / 25.4   128 rows 29.4 / 25.7   512 rows 64.7 / 36.1   4,096 rows 458 / 117
+//     96 -> 224  128 rows 40.4 / 53.1   256 rows 78.7 / 57.7   512 rows 155 / 73.7    4,096 rows 1097 / 211
+//   conv_ws fits                                                 chunks for N > 96 (its MMAs get longer), 16 rows an SM
+//     48 -> 144  512 rows 29.6 / 31.9   1,024 rows 46.5 / 39.8   4,096 rows 189 / 100
+//     32 -> 176  512 rows 26.8 / 38.9   2,048 rows 68.0 / 67.8   4,096 rows 166 / 130, its fp32 outputs 173 / 128
+//     32 -> 96   512 rows 19.2 / 22.6   2,048 rows 42.8 / 38.5   4,096 rows 68.0 / 63.4, with the ReLU mask 94 / 107
+struct StackPlan {
+    int groups = 0, chunk = 0;  // groups = 0: not eligible
+};
+inline StackPlan stack_plan(int n_img, int h, int width, int cin, int cout, bool any = false) {
+    StackPlan p;
+    if (width < kBM || cout > 256) return p;
+    const long rows = (long)n_img * ((width + kBM - 1) / kBM) * h;
     for (int g = 1; g <= 4; ++g) {
+        if (g > 1 && cout > 64 && !any) return p;
         const int cg = (cin / 16 + g - 1) / g * 16;
-        int occ, ring;
-        if (ws_config(cg, cout, occ, ring)) return (g == 1 || cout <= 64 || any) ? g : 0;
+        int occ, ring, chunk = 0, chunks = 0;
+        for (int n = (cout + kStackMaxCout - 1) / kStackMaxCout; n <= 4 && !chunk; ++n) {
+            const int c = (cout / 16 + n - 1) / n * 16;
+            if (!stack_config(cg, c, occ, ring)) continue;
+            chunk = c;
+            chunks = n;
+        }
+        const bool ws = cout > kStackMaxCout && ws_config(cg, cout, occ, ring);
+        if (ws && !(chunk && cout > 96 && rows >= 16L * sm_count())) {
+            p.groups = g;
+            return p;
+        }
+        if (!chunk) continue;
+        if (chunks > 1 && rows < 64L * chunks && !any) return p;
+        p.groups = g;
+        p.chunk = chunk;
+        return p;
     }
-    return 0;
+    return p;
 }
 
-cudaError_t launch_ws_pass(StripArgs a, cudaStream_t s) {
-    int per_sm = 0, ring = 0;
-    if (!ws_config(a.cin, a.cout, per_sm, ring)) return cudaErrorInvalidValue;
-    WsArgs wa{};
+// the tensor maps (widths 64, 32, 16) and the channel groups of a pass
+bool encode_groups(const StripArgs& a, WsArgs& wa, CUtensorMap (&maps)[3]) {
     const WsGroups gr = ws_groups_of(a.cin);
-    CUtensorMap maps[3];  // widths 64, 32, 16
     memset(maps, 0, sizeof(maps));
     bool have[3] = {false, false, false};
     for (int k = 0; k < gr.n; ++k) {
         const int mi = gr.w[k] == 64 ? 0 : (gr.w[k] == 32 ? 1 : 2);
-        if (!have[mi] && !encode_rows(&maps[mi], a.x, a.n, a.h, a.w_, a.cin_total, gr.w[k]))
-            return cudaErrorInvalidValue;
+        if (!have[mi] && !encode_rows(&maps[mi], a.x, a.n, a.h, a.w_, a.cin_total, gr.w[k])) return false;
         have[mi] = true;
         wa.gc[k] = gr.c[k];
         wa.gw[k] = gr.w[k];
@@ -2098,25 +2518,60 @@ cudaError_t launch_ws_pass(StripArgs a, cudaStream_t s) {
     wa.ngroups = gr.n;
     wa.row_bytes = gr.row_bytes;
     wa.tx_bytes = gr.tx;
+    return true;
+}
+
+// the shared memory of a launch: at least what holds the CTAs per SM to per_sm (TMEM is sized for that many)
+inline size_t ws_smem(int cin, int cout, int per_sm, int ring) {
+    const size_t need = ws_weight_bytes(cin, cout) + (size_t)ring * ws_row_bytes(cin);
+    return std::max(need, std::min(kSmPerCta, kSmPerSm / (per_sm + 1) - kWsStatic + 1024));
+}
+
+cudaError_t launch_ws(StripArgs a, cudaStream_t s) {
+    int per_sm = 0, ring = 0;
+    WsArgs wa{};
+    CUtensorMap maps[3];
+    if (!ws_config(a.cin, a.cout, per_sm, ring) || !encode_groups(a, wa, maps)) return cudaErrorInvalidValue;
     a.tmem_cols = 2 * pow2_cols(a.cout);
     const int slots = sm_count() * per_sm;
     int total = 0;
     strip_segments(a.n, a.h, a.w_, slots, a.xtiles, a.seg_rows, a.segs_per_col, total);
-    const int grid = min(total, slots);
     wa.s = a;
-    // at least the shared memory that holds the CTAs per SM to per_sm (TMEM is sized for that many)
-    const size_t need = ws_weight_bytes(a.cin, a.cout) + (size_t)ring * ws_row_bytes(a.cin);
-    const size_t smem = std::max(need, std::min(kSmPerCta, kSmPerSm / (per_sm + 1) - kWsStatic + 1024));
-    cudaError_t e = cudaFuncSetAttribute(conv_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const size_t smem = ws_smem(a.cin, a.cout, per_sm, ring);
+    const cudaError_t e = cudaFuncSetAttribute(conv_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
-    conv_ws_kernel<<<grid, kWsThreads, smem, s>>>(maps[0], maps[1], maps[2], wa, ring);
+    conv_ws_kernel<<<min(total, slots), kWsThreads, smem, s>>>(maps[0], maps[1], maps[2], wa, ring);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
+// output channels [co0, co0 + cout) of the cout_total of a layer (a.cout is set here)
+cudaError_t launch_stack(StripArgs a, int co0, int cout, int cout_total, cudaStream_t s) {
+    a.cout = cout;
+    StackArgs sa{};
+    int per_sm = 0;
+    CUtensorMap maps[3];
+    if (!stack_config(a.cin, cout, per_sm, sa.ring) || !encode_groups(a, sa.ws, maps)) return cudaErrorInvalidValue;
+    a.tmem_cols = 512 / per_sm;  // the CTAs of an SM share its 512 columns
+    a.xtiles = (a.w_ + kBM - 1) / kBM;
+    sa.sets = stack_sets(a.cin);
+    sa.blocks = std::min(kStackMaxBlocks, a.tmem_cols / (cout * sa.sets));
+    sa.co0 = co0;
+    sa.cout_total = cout_total;
+    sa.ws.s = a;
+    const long rows = (long)a.n * a.xtiles * a.h;
+    const int grid = (int)std::min<long>(std::max<long>(1, rows / 2), sm_count() * per_sm);  // at least two rows each
+    const size_t smem = ws_smem(a.cin, cout, per_sm, sa.ring);
+    const cudaError_t e = cudaFuncSetAttribute(conv_stack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    conv_stack_kernel<<<grid, kStackThreads, smem, s>>>(maps[0], maps[1], maps[2], sa);
     count_launches(1);
     return cudaGetLastError();
 }
 
 static int g_strip_kernel = 0;  // 0: warp-specialised (TMA) strips, 1: the cp.async strip kernel
 
-cudaError_t launch_strip(const ConvArgs& c, int groups, cudaStream_t s) {
+cudaError_t launch_strip(const ConvArgs& c, int groups, int chunk, cudaStream_t s) {
     StripArgs a{};
     a.x = c.x;
     a.w = c.w;
@@ -2126,6 +2581,14 @@ cudaError_t launch_strip(const ConvArgs& c, int groups, cudaStream_t s) {
     a.w_ = c.w_;
     a.cout = c.cout;
     a.cin_total = c.cin;
+    auto pass = [&](const StripArgs& p) {
+        if (g_strip_kernel != 0) return launch_strip_pass(p, s);
+        if (chunk == 0) return launch_ws(p, s);
+        cudaError_t e = cudaSuccess;
+        for (int co = 0; co < c.cout && e == cudaSuccess; co += chunk)
+            e = launch_stack(p, co, min(chunk, c.cout - co), c.cout, s);
+        return e;
+    };
     if (groups <= 1) {
         a.cin = c.cin;
         a.bias = c.bias;
@@ -2133,7 +2596,7 @@ cudaError_t launch_strip(const ConvArgs& c, int groups, cudaStream_t s) {
         a.y = c.y;
         a.relu = c.relu;
         a.out_f32 = c.out_f32;
-        return g_strip_kernel == 0 ? launch_ws_pass(a, s) : launch_strip_pass(a, s);
+        return pass(a);
     }
     // fp32 partial sum of the earlier groups (stream-ordered scratch)
     float* part = nullptr;
@@ -2155,7 +2618,7 @@ cudaError_t launch_strip(const ConvArgs& c, int groups, cudaStream_t s) {
             p.relu = c.relu;
             p.out_f32 = c.out_f32;
         }
-        e = g_strip_kernel == 0 ? launch_ws_pass(p, s) : launch_strip_pass(p, s);
+        e = pass(p);
     }
     const cudaError_t f = cudaFreeAsync(part, s);
     return e != cudaSuccess ? e : f;
@@ -2196,10 +2659,12 @@ VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, cons
     a.out_f32 = out_f32;
     // row strips: the warp-specialised kernel's tensor map wants a 16-byte aligned base
     const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0;
-    const int groups = g_strip_kernel == 0 ? (aligned ? ws_groups(width, cin, cout, g_force_strip) : 0)
-                                           : strip_groups(width, cin, cout, g_force_strip);
-    if (groups > 0 && !g_force_gather)
-        return launch_strip(a, groups, static_cast<cudaStream_t>(stream)) == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
+    StackPlan plan;
+    if (g_strip_kernel != 0) plan.groups = strip_groups(width, cin, cout, g_force_strip);
+    else if (aligned) plan = stack_plan(n, h, width, cin, cout, g_force_strip);
+    if (plan.groups > 0 && !g_force_gather)
+        return launch_strip(a, plan.groups, plan.chunk, static_cast<cudaStream_t>(stream)) == cudaSuccess ? VPT_OK
+                                                                                                       : VPT_ERR_CUDA;
     const long P = (long)n * h * width;
     const unsigned gx = (unsigned)((P + kBM - 1) / kBM), gy = (unsigned)((cout + a.n_tile - 1) / a.n_tile);
     // small grids (the deep levels): split the K stages over more CTAs, raw fp32 sums finished by
