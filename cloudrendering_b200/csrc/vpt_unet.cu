@@ -166,6 +166,14 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
 }
 
+// 32 lanes x 16 columns of zeros (the caller waits with tcgen05.wait::st)
+__device__ __forceinline__ void tmem_zero16(uint32_t taddr) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};\n" ::"r"(taddr),
+        "r"(0)
+        : "memory");
+}
+
 // ---------------------------------------------------------------------------------------------
 // the implicit-GEMM convolution tile
 // ---------------------------------------------------------------------------------------------
@@ -1385,192 +1393,273 @@ __global__ void __launch_bounds__(kStackThreads, 2)
 }
 
 // ---------------------------------------------------------------------------------------------
-// the row-strip weight gradient (images at least 128 pixels wide)
+// the weight gradient on image rows
 // ---------------------------------------------------------------------------------------------
-// dw[co][t][ci] = sum over pixels p of dy[p][co] * x[p + off(t)][ci].  Per output row y of a 128-pixel
-// column: the 128 pixels are the K dimension; for tap (dy, dx) the x operand is the row strip of
-// input row y+dy-1 shifted by dx pixels (descriptor start + dx * 16 bytes, as in the forward strip
-// kernel), the dy operand is output-gradient row y.  Both operands are MN-major (8-channel planes of
-// 16-byte pixel rows: LBO = 128 between 8-pixel groups, SBO = plane stride between channel groups).
-// ROLE 0: A = x (M = input channels m0 .. m0+ma, zero planes beyond), B = dy (N = output channels);
-// ROLE 1: A = dy (M = output channels m0 .. m0+ma), B = x (N = input channels).  Each tap t of
-// [t0, t1) accumulates in its own TMEM block (columns (t - t0) * N) over every row the CTA owns; the
-// CTA writes its sums to partial[blockIdx.x][t * cin + ci][co] at the end (reduced in fixed order by
-// reduce_grads_kernel).  M = 64 accumulators occupy lanes 0-15 of each 32-lane quarter of TMEM.
-constexpr int kDyRing = 3;
-constexpr int kDyPlane = kBM * 16;  // 2048 bytes: 128 pixels x 16 bytes
+// dw[co][t][ci] = sum over pixels p of dy[p][co] * x[p + off(t)][ci].  Pixels are K: a CTA walks the rows of
+// an image column at most 128 pixels wide, every row a contraction over its pixels in steps of 16, and sums
+// all its rows in TMEM.  Both operands are rows as they lie in memory, [pixel][channels], read by the TMA
+// into the MN-major swizzled layout (channels contiguous: MN; pixels: K), lines of 32 or 16 channels.  A tap's
+// horizontal shift dx is a start moved by dx pixel lines, as in conv_stack_kernel; pixels and channels outside
+// arrive as zeros.
+//   One tensor (U) is the A operand, M = 64 or 128 of its channels; of the other (S) a chunk of at most 32
+// channels is B, of the three rows that meet U's row in the three vertical taps at once: the rows lie in
+// consecutive ring slots, so B's channel groups are the slots and one MMA of N = 3 x 32 columns serves
+// three taps (two MMAs where the ring wraps).  Accumulators: one block of 3 x 32 columns per dx.
+//   role 0: U = x, S = dy (row r of x meets rows r-1, r, r+1 of dy);
+//   role 1: U = dy, S = x (row y of dy meets rows y-1, y, y+1 of x).
+// The role with fewer passes (U chunks x S chunks, blockIdx.y) is taken.
+// Warps: 0 loads (TMA), 1-3 issue the MMAs of dx = 0, 1, 2 (one thread's issue, about 93 cycles an MMA, is the
+// bound of N <= 96), 4-7 zero the accumulators at the start and write the CTA's sums to
+// partial[blockIdx.x][t * cin + ci][co] at the end (reduced in fixed order by reduce_grads_kernel).  M = 64
+// accumulators occupy lanes 0-15 of each 32-lane quarter of TMEM.
+//   Kernel and reduction, us, 8 images of 256 x 256 (the strip kernel that copied both rows into 8-channel planes
+// and issued one MMA a tap and 16 pixels, or the gather kernel below 64 channels / here): 96 -> 32 179 / 65,
+// 32 -> 32 176 / 50, 16 -> 32 134 / 49, 32 -> 176 380 / 153; 144 -> 48 at half that size 200 / 94.  Bound: the rows'
+// bytes (96 -> 32: 134 MB, 20 us) and the MMAs (24 a row and 28 rows an SM), which overlap, then writing the
+// accumulators.
+constexpr int kWgThreads = 256;
+constexpr int kWgMaxRing = 8;
+constexpr int kWgURing = 3;
 
-struct WgradStripArgs {
-    const bf16* x;      // [n][h][w][cin]
-    const bf16* dy;     // [n][h][w][cout]
-    float* partial;     // [splits][m_pad][cout]
+struct WgradArgs {
+    float* partial;  // [gridDim.x][m_pad][cout]
     int* err;
-    int n, h, w_, cin, cout;
-    int m0, ma;         // A channel range (input channels for role 0, output channels for role 1), ma 64 / 128
-    int t0, t1;         // taps of this pass
-    int xplanes, dyplanes;  // 8-channel planes per x strip / dy row in shared memory
-    int m_pad;
-    int xtiles, seg_rows, segs_per_col, tmem_cols;
+    int n, h, w_, cin, cout, m_pad;
+    int role;
+    int s_group;               // channels of an S chunk: 32, or 16 when S has 16
+    int u_chunks, s_chunks;    // blockIdx.y = u_chunk * s_chunks + s_chunk
+    int ksteps;                // 16-pixel steps of a row
+    int xtiles;
+    int u_slot, u_group_bytes, s_slot, s_ring;  // shared-memory strides; ring depth of S
+    int u_lines, s_lines;      // pixel lines of a row (the x tensor's rows carry a halo of one)
+    int tmem_cols;
 };
 
-template <int ROLE>
-__global__ void __launch_bounds__(kThreads) wgrad_strip_kernel(const WgradStripArgs a) {
-    extern __shared__ __align__(1024) uint8_t smem[];
-    __shared__ uint64_t bars[2];
-    __shared__ uint32_t tmem_slot;
-    const int tid = threadIdx.x;
-    const int N = ROLE == 0 ? a.cout : a.cin;
-    const uint32_t xrow = (uint32_t)a.xplanes * kPlane, dyrow = (uint32_t)a.dyplanes * kDyPlane;
-    const uint32_t sx = smem_u32(smem);
-    const uint32_t sdy = sx + kRing * xrow;
-    // channels gathered into the strips: x planes [x_c0, x_c0 + 8 * x_real), dy planes likewise
-    const int x_c0 = ROLE == 0 ? a.m0 : 0;
-    const int x_real = ROLE == 0 ? min(a.ma, a.cin - a.m0) / 8 : a.cin / 8;
-    const int dy_c0 = ROLE == 0 ? 0 : a.m0;
-    const int dy_real = ROLE == 0 ? a.cout / 8 : min(a.ma, a.cout - a.m0) / 8;
+// MN-major swizzled descriptor: lines of `line` bytes (128 / 64 / 32: 64 / 32 / 16 channels), 8-pixel groups
+// 8 lines apart (SBO), channel groups `lbo` bytes apart
+__device__ __forceinline__ uint64_t smem_desc_mn(uint32_t line, uint32_t lbo) {
+    uint64_t d = (uint64_t)((lbo >> 4) & 0x3FFFu) << 16;
+    d |= (uint64_t)(((8u * line) >> 4) & 0x3FFFu) << 32;
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)(line == 128 ? 2 : (line == 64 ? 4 : 6)) << 61;
+    return d;
+}
 
+__global__ void __launch_bounds__(kWgThreads, 1)
+    wgrad_rows_kernel(const __grid_constant__ CUtensorMap umap, const __grid_constant__ CUtensorMap smap,
+                      const __grid_constant__ WgradArgs a) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ uint64_t u_full[kWgURing], u_empty[kWgURing], s_full[kWgMaxRing], s_empty[kWgMaxRing], done_bar[3];
+    __shared__ uint32_t tmem_slot;
+    __shared__ int fail_any;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int u_total = a.role == 0 ? a.cin : a.cout;
+    const int u0 = ((int)blockIdx.y / a.s_chunks) * 128, s0 = ((int)blockIdx.y % a.s_chunks) * a.s_group;
+    const int ma = u_total - u0 > 64 ? 128 : 64;
+    const int n3 = 3 * a.s_group;
+    const uint32_t su = smem_u32(smem), ss = su + (uint32_t)(kWgURing * a.u_slot);
     if (tid == 0) {
-        mbar_init(smem_u32(&bars[0]), 1);
-        mbar_init(smem_u32(&bars[1]), 1);
+        for (int k = 0; k < kWgURing; ++k) {
+            mbar_init(smem_u32(&u_full[k]), 1);
+            mbar_init(smem_u32(&u_empty[k]), 3);  // one release per issuing warp
+        }
+        for (int k = 0; k < a.s_ring; ++k) {
+            mbar_init(smem_u32(&s_full[k]), 1);
+            mbar_init(smem_u32(&s_empty[k]), 3);
+        }
+        for (int k = 0; k < 3; ++k) mbar_init(smem_u32(&done_bar[k]), 1);
+        fail_any = 0;
         fence_mbar_init();
     }
-    if (tid < 32) tmem_alloc(smem_u32(&tmem_slot), (uint32_t)a.tmem_cols);
-    // zero the padding planes of every ring slot once (the gathers never write them)
-    {
-        uint4* base = reinterpret_cast<uint4*>(smem);
-        const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-        for (int slot = 0; slot < kRing; ++slot)
-            for (int q = tid; q < (a.xplanes - x_real) * kStripPix; q += kThreads)
-                base[(slot * xrow + (uint32_t)(x_real + q / kStripPix) * kPlane) / 16 + q % kStripPix] = z;
-        for (int slot = 0; slot < kDyRing; ++slot)
-            for (int q = tid; q < (a.dyplanes - dy_real) * kBM; q += kThreads)
-                base[(kRing * xrow + slot * dyrow + (uint32_t)(dy_real + q / kBM) * kDyPlane) / 16 + q % kBM] = z;
-    }
-    fence_proxy_async();
+    if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), (uint32_t)a.tmem_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
-    const uint32_t tmem = tmem_slot;
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    bool fail = false;
+    if (warp >= 4) {
+        const uint32_t trow = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        for (int c = 0; c < 3 * n3; c += 16) tmem_zero16(trow + (uint32_t)c);
+        asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory");
+        tc_fence_before();
+    }
+    if (warp != 0) asm volatile("bar.sync 1, %0;\n" ::"n"(kWgThreads - 32) : "memory");
 
-    auto load_x = [&](int n_img, int yy, int x0) {
-        const uint32_t base = sx + (uint32_t)(((yy + 1) % kRing + kRing) % kRing) * xrow;
-        const bool row_ok = yy >= 0 && yy < a.h;
-        for (int q = tid; q < kStripPix * x_real; q += kThreads) {
-            const int r = q % kStripPix, kc = q / kStripPix;
-            const int xx = x0 - 1 + r;
-            const bool v = row_ok && xx >= 0 && xx < a.w_;
-            const bf16* src = v ? a.x + (((size_t)n_img * a.h + yy) * a.w_ + xx) * a.cin + x_c0 + kc * 8 : a.x;
-            cp_async16(base + (uint32_t)kc * kPlane + (uint32_t)r * 16u, src, v);
-        }
-    };
-    auto load_dy = [&](int n_img, int yy, int x0) {
-        const uint32_t base = sdy + (uint32_t)(yy % kDyRing) * dyrow;
-        for (int q = tid; q < kBM * dy_real; q += kThreads) {
-            const int r = q % kBM, kc = q / kBM;
-            const int xx = x0 + r;
-            const bool v = yy < a.h && xx < a.w_;
-            const bf16* src = v ? a.dy + (((size_t)n_img * a.h + yy) * a.w_ + xx) * a.cout + dy_c0 + kc * 8 : a.dy;
-            cp_async16(base + (uint32_t)kc * kDyPlane + (uint32_t)r * 16u, src, v);
-        }
-    };
-
-    const uint32_t idesc = instr_desc(a.ma, N, 1, 1);
-    // MN-major descriptor words (LBO = 128 between 8-pixel groups, SBO = plane stride); start fields 0
-    const uint64_t xd0 = smem_desc(0, 128, kPlane), dd0 = smem_desc(0, 128, kDyPlane);
-    const uint32_t x_lo = (uint32_t)xd0, x_hi = (uint32_t)(xd0 >> 32);
-    const uint32_t d_lo = (uint32_t)dd0, d_hi = (uint32_t)(dd0 >> 32);
-    const int total_segs = a.n * a.xtiles * a.segs_per_col;
-    long g = 0;
-    int fail = 0;
-    for (int seg = blockIdx.x; seg < total_segs && !fail; seg += gridDim.x) {
-        const int col = seg / a.segs_per_col, part = seg % a.segs_per_col;
-        const int n_img = col / a.xtiles, x0 = (col % a.xtiles) * kBM;
-        const int y0 = part * a.seg_rows, y1 = min(a.h, y0 + a.seg_rows);
-        if (y0 >= y1) continue;
-        if (g > 0) {  // the previous segment's MMAs have read their rows
-            if (!mbar_wait(smem_u32(&bars[(g - 1) & 1]), (uint32_t)(((g - 1) >> 1) & 1))) fail = 1;
-            if (__syncthreads_or(fail)) break;
-        }
-        load_x(n_img, y0 - 1, x0);
-        load_x(n_img, y0, x0);
-        load_x(n_img, y0 + 1, x0);
-        load_dy(n_img, y0, x0);
-        cp_async_commit();
-        if (y0 + 2 <= y1) load_x(n_img, y0 + 2, x0);
-        if (y0 + 1 < y1) load_dy(n_img, y0 + 1, x0);
-        cp_async_commit();
-        for (int yrow = y0; yrow < y1; ++yrow, ++g) {
-            cp_async_wait<1>();
-            fence_proxy_async();
-            tc_fence_before();
-            if (__syncthreads_or(fail)) break;
-            if (tid == 0) {
-                tc_fence_after();
-                // descriptor halves: the start fields walk 256 bytes (16 pixels) per K step; the x
-                // strip of tap (dyy, dxx) starts dxx pixels (16 bytes) into the slot of row yrow+dyy
-                const uint32_t d16 = (sdy + (uint32_t)(yrow % kDyRing) * dyrow) >> 4;
-                for (int t = a.t0; t < a.t1; ++t) {
-                    const int dyy = t / 3, dxx = t - 3 * dyy;
-                    const uint32_t x16 = ((sx + (uint32_t)((yrow + dyy) % kRing) * xrow) >> 4) + (uint32_t)dxx;
-                    const uint32_t dacc = tmem + (uint32_t)((t - a.t0) * N);
-#pragma unroll
-                    for (int j = 0; j < kBM / 16; ++j) {
-                        const uint32_t xl = x_lo + x16 + 16u * (uint32_t)j, dl = d_lo + d16 + 16u * (uint32_t)j;
-                        const uint32_t acc = (g == 0 && j == 0) ? 0u : 1u;
-                        if (ROLE == 0) mma_bf16_halves(dacc, xl, x_hi, dl, d_hi, idesc, acc);
-                        else mma_bf16_halves(dacc, dl, d_hi, xl, x_hi, idesc, acc);
+    // Row order of a segment [y0, y1) (both roles): steps r = first .. last of U's rows; before step r the S
+    // rows up to r + 1 are there.  Role 0: r = y0 - 1 .. y1, S rows y0 .. y1 - 1; role 1: r = y0 .. y1 - 1, S
+    // rows y0 - 1 .. y1.  An S row is released after the step that follows it.
+    if (warp == 0) {
+        if (lane == 0) {
+            const int ugroups = ma / 32;
+            const uint32_t u_tx = (uint32_t)(ugroups * a.u_lines * 64), s_tx = (uint32_t)(a.s_lines * a.s_group * 2);
+            int us = 0, sl = 0;
+            uint32_t uph = 0, sph = 0;
+            long ui = 0, si = 0;
+            auto load_s = [&](const WsSegment& g, int row) {
+                if (!mbar_wait(smem_u32(&s_empty[sl]), sph ^ 1u)) {
+                    fail = true;
+                    return;
+                }
+                const uint32_t fb = smem_u32(&s_full[sl]);
+                mbar_arrive_expect_tx(fb, s_tx);
+                tma_load_4d(ss + (uint32_t)(sl * a.s_slot), &smap, s0, g.x0 - (a.role == 1 ? 1 : 0), row, g.n_img, fb);
+                ++si;
+                if (++sl == a.s_ring) {
+                    sl = 0;
+                    sph ^= 1u;
+                }
+            };
+            RowRange range(a.n, a.h, a.xtiles);
+            WsSegment g;
+            while (!fail && range.next(g)) {
+                const int r0 = a.role == 0 ? g.y0 - 1 : g.y0, r1 = a.role == 0 ? g.y1 : g.y1 - 1;
+                const int slo = a.role == 0 ? g.y0 : g.y0 - 1, shi = a.role == 0 ? g.y1 - 1 : g.y1;
+                int next = slo;
+                for (int r = r0; r <= r1 && !fail; ++r) {
+                    while (next <= min(r + 1, shi) && !fail) load_s(g, next++);
+                    if (fail || !mbar_wait(smem_u32(&u_empty[us]), uph ^ 1u)) {
+                        fail = true;
+                        break;
+                    }
+                    const uint32_t fb = smem_u32(&u_full[us]);
+                    mbar_arrive_expect_tx(fb, u_tx);
+                    for (int k = 0; k < ugroups; ++k)
+                        tma_load_4d(su + (uint32_t)(us * a.u_slot + k * a.u_group_bytes), &umap, u0 + 32 * k,
+                                    g.x0 - (a.role == 0 ? 1 : 0), r, g.n_img, fb);
+                    ++ui;
+                    if (++us == kWgURing) {
+                        us = 0;
+                        uph ^= 1u;
                     }
                 }
-                mma_commit(smem_u32(&bars[g & 1]));
             }
-            if (yrow > y0) {  // the previous row's MMAs are done: its x and dy slots are free
-                if (!mbar_wait(smem_u32(&bars[(g - 1) & 1]), (uint32_t)(((g - 1) >> 1) & 1))) fail = 1;
-                if (__syncthreads_or(fail)) break;
+            // the last loads (one per slot at most) have landed before the CTA can exit
+            for (long k = 1; k <= min(ui, (long)kWgURing); ++k) {
+                int q = us - (int)k;
+                uint32_t ph = uph;
+                if (q < 0) {
+                    q += kWgURing;
+                    ph ^= 1u;
+                }
+                if (!mbar_wait(smem_u32(&u_full[q]), ph)) fail = true;
             }
-            if (yrow + 3 <= y1) load_x(n_img, yrow + 3, x0);
-            if (yrow + 2 < y1) load_dy(n_img, yrow + 2, x0);
-            cp_async_commit();
-        }
-    }
-    cp_async_wait<0>();
-    bool done = true;
-    if (g > 0) done = mbar_wait(smem_u32(&bars[(g - 1) & 1]), (uint32_t)(((g - 1) >> 1) & 1));
-    fail = __syncthreads_or(fail || !done);
-    tc_fence_after();
-    if (!fail) {
-        // accumulator rows: M = 128 -> lane = row; M = 64 -> lanes 0-15 of each warp quarter
-        const int warp = tid >> 5, lane = tid & 31;
-        const int row = a.ma == 128 ? warp * 32 + lane : (lane < 16 ? warp * 16 + lane : -1);
-        const uint32_t trow = tmem + ((uint32_t)(warp * 32) << 16);
-        float* part = a.partial + (size_t)blockIdx.x * a.m_pad * a.cout;
-        for (int t = a.t0; t < a.t1; ++t) {
-            for (int c0 = 0; c0 < N; c0 += 16) {
-                float v[16];
-                tmem_ld16(trow + (uint32_t)((t - a.t0) * N + c0), v);
-                if (row < 0) continue;
-                if (g == 0) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = 0.0f;
+            for (long k = 1; k <= min(si, (long)a.s_ring); ++k) {
+                int q = sl - (int)k;
+                uint32_t ph = sph;
+                if (q < 0) {
+                    q += a.s_ring;
+                    ph ^= 1u;
                 }
-                if (ROLE == 0) {
-                    const int ci = a.m0 + row;
-                    if (ci >= a.cin) continue;
-                    float4* dst = reinterpret_cast<float4*>(part + (size_t)(t * a.cin + ci) * a.cout + c0);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                } else {
-                    const int co = a.m0 + row;
-                    if (co >= a.cout) continue;
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) part[(size_t)(t * a.cin + c0 + i) * a.cout + co] = v[i];
-                }
+                if (!mbar_wait(smem_u32(&s_full[q]), ph)) fail = true;
             }
         }
+    } else if (warp <= 3) {
+        tc_fence_after();
+        const int dx = warp - 1;
+        const uint32_t s_line = (uint32_t)a.s_group * 2u;
+        const uint64_t ud = smem_desc_mn(64, (uint32_t)a.u_group_bytes), sd = smem_desc_mn(s_line, (uint32_t)a.s_slot);
+        const uint32_t u_hi = (uint32_t)(ud >> 32), s_hi = (uint32_t)(sd >> 32);
+        // the x tensor's rows start at x0 - 1: its start moves by dx lines
+        const uint32_t u_lo = (uint32_t)ud + ((su + (a.role == 0 ? (uint32_t)dx * 64u : 0u)) >> 4);
+        const uint32_t s_lo = (uint32_t)sd + ((ss + (a.role == 1 ? (uint32_t)dx * s_line : 0u)) >> 4);
+        const uint32_t u_step = 64, s_step = s_line;  // 16 lines, in 16-byte units
+        const uint32_t id1 = instr_desc(ma, a.s_group, 1, 1), id_n = (uint32_t)(a.s_group >> 3) << 17;
+        const uint32_t dacc = tmem + (uint32_t)(dx * n3);
+        int us = 0;
+        uint32_t uph = 0;
+        int ws = 0;         // ring slot of the oldest S row in use
+        uint32_t wph = 0;   // its phase
+        RowRange range(a.n, a.h, a.xtiles);
+        WsSegment g;
+        while (!fail && range.next(g)) {
+            const int r0 = a.role == 0 ? g.y0 - 1 : g.y0, r1 = a.role == 0 ? g.y1 : g.y1 - 1;
+            const int slo = a.role == 0 ? g.y0 : g.y0 - 1, shi = a.role == 0 ? g.y1 - 1 : g.y1;
+            int oldest = slo;  // S row in slot ws
+            for (int r = r0; r <= r1; ++r) {
+                const int lo = max(r - 1, slo), hi = min(r + 1, shi);  // S rows of this step (lo == oldest)
+                bool ok = mbar_wait(smem_u32(&u_full[us]), uph);
+                for (int k = 0; k <= hi - oldest; ++k) {
+                    const int q = ws + k < a.s_ring ? ws + k : ws + k - a.s_ring;
+                    ok = ok && mbar_wait(smem_u32(&s_full[q]), ws + k < a.s_ring ? wph : wph ^ 1u);
+                }
+                if (!__all_sync(0xffffffffu, ok)) {
+                    fail = true;
+                    break;
+                }
+                tc_fence_after();
+                // S row r - 1 is last used here; the segment's last step releases the rest
+                const int keep = r == r1 ? shi + 1 : max(r, slo);
+                if (elect_one()) {
+                    const int cnt = hi - lo + 1, n_first = min(cnt, a.s_ring - ws), n_rest = cnt - n_first;
+                    const uint32_t d0 = dacc + (uint32_t)((lo - (r - 1)) * a.s_group);
+                    const uint32_t d1 = d0 + (uint32_t)(n_first * a.s_group);
+                    const uint32_t id_first = id1 + (uint32_t)(n_first - 1) * id_n;
+                    const uint32_t id_rest = id1 + (uint32_t)(n_rest - 1) * id_n;
+                    uint32_t ul = u_lo + ((uint32_t)(us * a.u_slot) >> 4);
+                    uint32_t sl = s_lo + ((uint32_t)(ws * a.s_slot) >> 4), sw = s_lo;
+                    for (int j = 0; j < a.ksteps; ++j) {
+                        mma_bf16_halves(d0, ul, u_hi, sl, s_hi, id_first, 1u);
+                        if (n_rest > 0) mma_bf16_halves(d1, ul, u_hi, sw, s_hi, id_rest, 1u);
+                        ul += u_step;
+                        sl += s_step;
+                        sw += s_step;
+                    }
+                    mma_commit(smem_u32(&u_empty[us]));
+                    for (int k = 0; k < keep - oldest; ++k)
+                        mma_commit(smem_u32(&s_empty[ws + k < a.s_ring ? ws + k : ws + k - a.s_ring]));
+                }
+                __syncwarp();
+                if (++us == kWgURing) {
+                    us = 0;
+                    uph ^= 1u;
+                }
+                for (; oldest < keep; ++oldest)
+                    if (++ws == a.s_ring) {
+                        ws = 0;
+                        wph ^= 1u;
+                    }
+            }
+        }
+        // every MMA this warp issued has completed before TMEM is read or released
+        if (elect_one()) mma_commit(smem_u32(&done_bar[dx]));
+        __syncwarp();
+        if (!mbar_wait(smem_u32(&done_bar[dx]), 0)) fail = true;
     }
-    if (fail && tid == 0 && a.err) atomicExch(a.err, (int)VPT_ERR_ITER_LIMIT);
+    if (fail) atomicOr(&fail_any, 1);
     tc_fence_before();
     __syncthreads();
-    if (tid < 32) {
+    tc_fence_after();
+    if (warp >= 4 && !fail_any) {
+        const int q = warp & 3;
+        const int row = ma == 128 ? q * 32 + lane : (lane < 16 ? q * 16 + lane : -1);
+        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+        const int s_total = a.role == 0 ? a.cout : a.cin;
+        const bool ok = row >= 0 && u0 + row < u_total;
+        float* part = a.partial + (size_t)blockIdx.x * a.m_pad * a.cout;
+        for (int dx = 0; dx < 3; ++dx)
+            for (int p = 0; p < 3; ++p) {
+                const int t = (a.role == 0 ? 2 - p : p) * 3 + dx;
+                for (int c = 0; c < a.s_group; c += 16) {
+                    float v[16];
+                    tmem_ld16(trow + (uint32_t)(dx * n3 + p * a.s_group + c), v);  // whole warp, uniform
+                    if (!ok || s0 + c >= s_total) continue;  // (channel counts are multiples of 16)
+                    if (a.role == 0) {
+                        float4* dst = reinterpret_cast<float4*>(part + (size_t)(t * a.cin + u0 + row) * a.cout + s0 + c);
+#pragma unroll
+                        for (int i = 0; i < 4; ++i)
+                            dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+                    } else {
+#pragma unroll
+                        for (int i = 0; i < 16; ++i)
+                            part[(size_t)(t * a.cin + s0 + c + i) * a.cout + u0 + row] = v[i];
+                    }
+                }
+            }
+    }
+    if (fail_any && tid == 0 && a.err) atomicExch(a.err, (int)VPT_ERR_ITER_LIMIT);
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, (uint32_t)a.tmem_cols);
     }
@@ -2228,38 +2317,42 @@ inline int strip_groups(int width, int cin, int cout, bool any = false) {
     return 0;
 }
 
-// Weight-gradient plan on row strips: the role (which tensor is A), the A channel chunks of at most
-// 128 (M = 64 or 128), tap groups so that taps x N <= 512 TMEM columns, and the shared memory of the
-// largest pass; 0 passes = not eligible (the gather kernel serves it).
+// Weight gradients of fewer pixels than this take the gather kernel, whose launch has work for every SM there:
+// a CTA of the row kernel sets up nine accumulators and writes them all, however few rows it gets.  Kernel and
+// reduction, us, gather / rows: 64 pixels of 128 -> 128 channels 12.4 / 19.2, 1,024 pixels of 96 -> 96 18.8 / 21.7,
+// 3,200 pixels of 96 -> 96 27.9 / 25.2, 4,096 pixels of 48 -> 48 18.9 / 15.3.
+constexpr long kWgradRowsMinPixels = 2048;
+
+// Weight-gradient plan on image rows: the role with fewer passes and the CTAs of a pass.
 struct WgradPlan {
-    int role = 0, chunks = 0, taps_per = 9, groups = 1, passes = 0;
-    size_t smem = 0;
+    int role = 0, s_group = 32, u_chunks = 1, s_chunks = 1, passes = 1;
+    int kpix = kBM, xtiles = 1, grid = 1;
 };
 
-constexpr size_t kWgradSmemLimit = 220 * 1024;
-
-inline WgradPlan wgrad_plan(int width, int cin, int cout, bool any_width = false) {
-    WgradPlan best;
-    if (width < kBM) return best;
-    // with fewer than 64 channels on both sides the per-row MMAs are too small (M = 64, N = 32) to
-    // beat the gather kernel (measured); any_width lifts the rule
-    if (!any_width && cin < 64 && cout < 64) return best;
+inline WgradPlan wgrad_plan(int n, int h, int w, int cin, int cout, int sms) {
+    WgradPlan p;
+    int best = 0;
     for (int role = 0; role < 2; ++role) {
-        const int mtot = role == 0 ? cin : cout, N = role == 0 ? cout : cin;
-        if (N > 256) continue;
-        WgradPlan p;
-        p.role = role;
-        p.chunks = (mtot + 127) / 128;
-        const int ma = mtot > 64 ? 128 : 64;  // largest chunk
-        p.taps_per = min(9, 512 / N);
-        p.groups = (9 + p.taps_per - 1) / p.taps_per;
-        p.passes = p.chunks * p.groups;
-        const int xplanes = role == 0 ? ma / 8 : cin / 8, dyplanes = role == 0 ? cout / 8 : ma / 8;
-        p.smem = (size_t)kRing * xplanes * kPlane + (size_t)kDyRing * dyplanes * kDyPlane;
-        if (p.smem > kWgradSmemLimit) continue;
-        if (best.passes == 0 || p.passes < best.passes) best = p;
+        const int u = role == 0 ? cin : cout, sc = role == 0 ? cout : cin;
+        const int uc = (u + 127) / 128, sn = (sc + 31) / 32;
+        if (best == 0 || uc * sn < best) {
+            best = uc * sn;
+            p.role = role;
+            p.s_group = sc == 16 ? 16 : 32;
+            p.u_chunks = uc;
+            p.s_chunks = sn;
+        }
     }
-    return best;
+    p.passes = best;
+    p.kpix = std::min(kBM, (w + 15) / 16 * 16);
+    p.xtiles = (w + kBM - 1) / kBM;
+    // CTAs per pass: enough to fill the SMs with all passes, and so many (up to one per SM) that a CTA's
+    // accumulators take about 64 additions each: longer fp32 sums in TMEM round more than the partials' sum
+    const int cols = n * p.xtiles;
+    const long steps = (long)cols * h * (p.kpix / 16);
+    const int ctas = (int)std::max<long>(std::max(1, sms / best), std::min<long>(sms, (steps + 63) / 64));
+    p.grid = (int)std::min<long>((long)cols * h, ctas);
+    return p;
 }
 
 inline void strip_segments(int n, int h, int w, int slots, int& xtiles, int& seg_rows, int& segs_per_col,
@@ -2272,55 +2365,6 @@ inline void strip_segments(int n, int h, int w, int slots, int& xtiles, int& seg
     seg_rows = (h + spc - 1) / spc;
     segs_per_col = (h + seg_rows - 1) / seg_rows;
     total = cols * segs_per_col;
-}
-
-inline int wgrad_strip_grid(int n, int h, int w) {
-    int xt, sr, spc, total;
-    strip_segments(n, h, w, sm_count(), xt, sr, spc, total);
-    return min(total, sm_count());
-}
-
-cudaError_t launch_wgrad_strip(const bf16* x, const bf16* dy, float* partial, int* err, int n, int h, int w, int cin,
-                               int cout, const WgradPlan& plan, cudaStream_t s) {
-    WgradStripArgs a{};
-    a.x = x;
-    a.dy = dy;
-    a.partial = partial;
-    a.err = err;
-    a.n = n;
-    a.h = h;
-    a.w_ = w;
-    a.cin = cin;
-    a.cout = cout;
-    a.m_pad = (9 * cin + kBM - 1) / kBM * kBM;
-    const int slots = sm_count();
-    int total = 0;
-    strip_segments(n, h, w, slots, a.xtiles, a.seg_rows, a.segs_per_col, total);
-    const int grid = min(total, slots);
-    const int mtot = plan.role == 0 ? cin : cout, N = plan.role == 0 ? cout : cin;
-    cudaError_t e = cudaSuccess;
-    for (int c = 0; c < plan.chunks && e == cudaSuccess; ++c) {
-        a.m0 = c * 128;
-        a.ma = (mtot - a.m0) > 64 ? 128 : 64;
-        a.xplanes = plan.role == 0 ? a.ma / 8 : cin / 8;
-        a.dyplanes = plan.role == 0 ? cout / 8 : a.ma / 8;
-        const size_t smem = (size_t)kRing * a.xplanes * kPlane + (size_t)kDyRing * a.dyplanes * kDyPlane;
-        for (int gidx = 0; gidx < plan.groups && e == cudaSuccess; ++gidx) {
-            a.t0 = gidx * plan.taps_per;
-            a.t1 = min(9, a.t0 + plan.taps_per);
-            a.tmem_cols = pow2_cols((a.t1 - a.t0) * N);
-            if (plan.role == 0) {
-                e = cudaFuncSetAttribute(wgrad_strip_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (e == cudaSuccess) wgrad_strip_kernel<0><<<grid, kThreads, smem, s>>>(a);
-            } else {
-                e = cudaFuncSetAttribute(wgrad_strip_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-                if (e == cudaSuccess) wgrad_strip_kernel<1><<<grid, kThreads, smem, s>>>(a);
-            }
-            count_launches(1);
-            if (e == cudaSuccess) e = cudaGetLastError();
-        }
-    }
-    return e;
 }
 
 cudaError_t launch_strip_pass(StripArgs a, cudaStream_t s) {
@@ -2380,6 +2424,63 @@ bool encode_rows(CUtensorMap* map, const bf16* x, int n, int h, int w, int c, in
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(x), dims, strides, box, estr,
               CU_TENSOR_MAP_INTERLEAVE_NONE, sz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+// One tensor of a weight gradient, [n][h][w][c] bf16, as rows of `lines` pixels x `group` channels (64, 32 or
+// 16: 128, 64 or 32-byte swizzled lines)
+bool encode_wgrad(CUtensorMap* map, const bf16* x, int n, int h, int w, int c, int group, int lines) {
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return false;
+    const cuuint64_t dims[4] = {(cuuint64_t)c, (cuuint64_t)w, (cuuint64_t)h, (cuuint64_t)n};
+    const cuuint64_t strides[3] = {(cuuint64_t)c * 2, (cuuint64_t)w * c * 2, (cuuint64_t)h * w * c * 2};
+    const cuuint32_t box[4] = {(cuuint32_t)group, (cuuint32_t)lines, 1, 1};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<bf16*>(x), dims, strides, box, estr,
+              CU_TENSOR_MAP_INTERLEAVE_NONE,
+              group == 64 ? CU_TENSOR_MAP_SWIZZLE_128B
+                          : (group == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B),
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* partial, int* err, int n, int h, int w, int cin,
+                              int cout, const WgradPlan& p, cudaStream_t s) {
+    WgradArgs a{};
+    a.partial = partial;
+    a.err = err;
+    a.n = n;
+    a.h = h;
+    a.w_ = w;
+    a.cin = cin;
+    a.cout = cout;
+    a.m_pad = (9 * cin + kBM - 1) / kBM * kBM;
+    a.role = p.role;
+    a.s_group = p.s_group;
+    a.u_chunks = p.u_chunks;
+    a.s_chunks = p.s_chunks;
+    a.ksteps = p.kpix / 16;
+    a.xtiles = p.xtiles;
+    a.u_lines = p.kpix + (p.role == 0 ? 2 : 0);
+    a.s_lines = p.kpix + (p.role == 1 ? 2 : 0);
+    // group and slot strides: whole 1024-byte blocks (the swizzle acts on absolute addresses)
+    auto up = [](int b) { return (b + 1023) / 1024 * 1024; };
+    a.u_group_bytes = up(a.u_lines * 64);
+    const int u_total = p.role == 0 ? cin : cout;
+    a.u_slot = a.u_group_bytes * (u_total > 64 ? 4 : 2);
+    a.s_slot = up(a.s_lines * p.s_group * 2);
+    a.s_ring = kWgMaxRing;
+    const size_t smem = (size_t)kWgURing * a.u_slot + (size_t)a.s_ring * a.s_slot;
+    a.tmem_cols = pow2_cols(9 * p.s_group);
+    CUtensorMap umap, smap;
+    const bf16* ut = p.role == 0 ? x : dy;
+    const bf16* st = p.role == 0 ? dy : x;
+    if (!encode_wgrad(&umap, ut, n, h, w, u_total, 32, a.u_lines) ||
+        !encode_wgrad(&smap, st, n, h, w, p.role == 0 ? cout : cin, p.s_group, a.s_lines))
+        return cudaErrorInvalidValue;
+    cudaError_t e = cudaFuncSetAttribute(wgrad_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    wgrad_rows_kernel<<<dim3((unsigned)p.grid, (unsigned)p.passes), kWgThreads, smem, s>>>(umap, smap, a);
+    count_launches(1);
+    return cudaGetLastError();
 }
 
 constexpr size_t kSmPerSm = 233472;   // shared memory of one SM (bytes)
@@ -2633,6 +2734,10 @@ static bool g_force_gather = false;  // conv path 1: the gather kernels everywhe
 static bool g_force_strip = false;   // conv path 2: the strip kernels wherever they apply
 static int g_conv_ksplit = 0;        // gather convolution K splits: 0 automatic, 1 none, k > 1 forced
 
+static bool wgrad_on_rows(int n, int h, int w) {
+    return !g_force_gather && (g_force_strip || (long)n * h * w >= kWgradRowsMinPixels);
+}
+
 extern "C" {
 
 VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, const void* mask, void* y, int n, int h,
@@ -2745,10 +2850,12 @@ VptStatus vpt_unet_conv3x3_wgrad(const void* x, const void* dy, float* partial, 
     a.pix_per_split = pixels_per_split;
     const int mtiles = (9 * cin + kBM - 1) / kBM;
     a.m_pad = mtiles * kBM;
-    const WgradPlan plan = wgrad_plan(width, cin, cout, g_force_strip);
-    if (plan.passes > 0 && !g_force_gather)
-        return launch_wgrad_strip(a.x, a.w, partial, err, n, h, width, cin, cout, plan,
-                                  static_cast<cudaStream_t>(stream)) == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
+    if (wgrad_on_rows(n, h, width)) {  // (its tensor maps want aligned tensors)
+        if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(dy) % 16) return VPT_ERR_ARG;
+        const WgradPlan plan = wgrad_plan(n, h, width, cin, cout, sm_count());
+        return launch_wgrad_rows(a.x, a.w, partial, err, n, h, width, cin, cout, plan,
+                                 static_cast<cudaStream_t>(stream)) == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
+    }
     const long P = (long)n * h * width;
     const dim3 grid((unsigned)mtiles, (unsigned)((cout + a.n_tile - 1) / a.n_tile),
                     (unsigned)((P + pixels_per_split - 1) / pixels_per_split));
@@ -2759,7 +2866,7 @@ int vpt_unet_wgrad_rows(int cin) { return (9 * cin + kBM - 1) / kBM * kBM; }
 
 int vpt_unet_wgrad_splits(int n, int h, int width, int cin, int cout, int pixels_per_split) {
     if (n <= 0 || h <= 0 || width <= 0 || pixels_per_split <= 0) return 0;
-    if (!g_force_gather && wgrad_plan(width, cin, cout, g_force_strip).passes > 0) return wgrad_strip_grid(n, h, width);
+    if (wgrad_on_rows(n, h, width)) return wgrad_plan(n, h, width, cin, cout, sm_count()).grid;
     const long P = (long)n * h * width;
     return (int)((P + pixels_per_split - 1) / pixels_per_split);
 }
