@@ -327,15 +327,11 @@ __global__ void __launch_bounds__(kTraceBlock) trace_persistent_kernel(const __g
 
 
 // ---------------------------------------------------------------------------------------------
-// Per-lane path refill schedule (delta, ratio and NEE trackers).
-//
-// Each loop iteration advances every live lane by ONE tentative collision.  A lane whose path ends
-// (escape, absorption, bounce cap) writes the film and takes the next path id at the top of the
-// next iteration, so the 32 lanes of a warp keep executing the same step code instead of waiting
-// for the warp's longest path.  NEE shadow rays are a second mode of the same step: the free-path
-// sample and the density lookup are shared code for primary and shadow lanes.  Random numbers are
-// drawn in exactly the order of the recursive trackers (vpt_trackers.cuh), so every path is the same
-// path.  Path ids come from a global counter in warp batches of 64 (one atomic per 64 paths).
+// Per-lane path refill schedules: a persistent warp whose lanes take a new path id each when their path has
+// ended (escape, absorption, bounce cap), so that the 32 lanes keep executing the same step code instead of
+// waiting for the warp's longest path.  Shadow rays are a second mode of the same step: the free-path sample
+// and the density lookup are shared code for primary and shadow lanes.  Random numbers are drawn in exactly
+// the order of the recursive trackers (vpt_trackers.cuh), so every path is the same path.
 enum : int { kModePrimary = 0, kModeShadow = 1, kModeShadowEss = 2 };
 
 // Block walk of shadow_transmittance_ess (NeeTransmittance.glsl:173-228): the block of the entry
@@ -376,25 +372,6 @@ VPT_DEV void refill_finish(const TraceParams& P, size_t pix, F3 L, bool& has) {
         atomicAdd(P.film_sq + pix * 3 + 2, (double)L.z * (double)L.z);
     }
     has = false;
-}
-
-// Shadow ray done: add the light sample (f = weight * T with weight = pdf_phase / pdf_light for the
-// sky, or the light probability factor times pdf_phase for a light; NextEventTracking.glsl:348-369)
-// and resume the primary path at the scatter point with the sampled direction.
-VPT_DEV void end_shadow(const TraceParams& P, F3& color, F3& x, F3& w, float& d, F3 xp, F3 nw, float dp,
-                        float weight, float ts, int light, int& mode) {
-    const float f = weight * ts;
-    const F3 l = light >= 0 ? light_radiance(P, xp, light) : sky_and_sun(P, w);
-    color = color + f3(f * l.x, f * l.y, f * l.z);
-    x = xp;
-    w = nw;
-    d = dp;
-    mode = kModePrimary;
-    float tmin, tmax;
-    if (ray_box_p(P, x, w, tmin, tmax)) {
-        x = x + w * tmin;
-        d = tmax - tmin;
-    }
 }
 
 // Where the parameters of a path come from: one scene (the kernel's constant parameter block) or a
@@ -438,12 +415,436 @@ VPT_DEV void flush_counters_to(unsigned long long* counters, int* error_flags, u
     if (guard_hit) atomicOr(error_flags, kErrIterLimit);
 }
 
+// ---------------------------------------------------------------------------------------------
+// The event loop (delta, ratio, decomposition and next event tracking).
+//
+// A path is long runs of tentative collisions (free path, lookup, accept or not) between rare, long
+// events: a scatter (phase function, new ray interval, for next event tracking a light sample), the end
+// of a shadow ray, the end of the path.  Run as they occur, an event's 100 to 300 instructions hold up the
+// whole warp for the one or two lanes that have it in an iteration.  So a lane with an event waits: the
+// others go on colliding until kEventShare eighths of the warp's live lanes wait, and then the events run
+// together.  (The paths' own order of operations and random numbers is that of the recursive trackers in
+// vpt_trackers.cuh: a lane that waits draws nothing.)  Path ids come from a global counter in batches of
+// `batch`; lanes beyond `lanes` stay empty, so that a launch with fewer paths than resident lanes spreads
+// over all warps.
+enum : int {
+    kPendNone = 0,
+    kPendScatter,  // a real collision that scatters, at x
+    kPendAbsorb,   // one that absorbs, at x
+    kPendEscape,   // the path left the volume along w
+    kPendShadow,   // the shadow ray along w is done
+    kPendEnd       // the path ends with `color` (step guard)
+};
+
 template <int TRACKER, int INTERP, int GRID, bool TF, class SRC>
-VPT_DEV void refill_loop(const SRC& src, uint64_t total, unsigned long long* work_counter,
-                         unsigned long long* counters, int* error_flags, int refill_min) {
+VPT_DEV void event_loop(const SRC& src, uint64_t total, unsigned long long* work_counter,
+                        unsigned long long* counters, int* error_flags, int refill_min, int batch, int lanes) {
     // next event tracking; kNextEvent + 100: its sky shadow rays skip the occupancy grid's empty blocks
     constexpr bool kNee = TRACKER == kNextEvent || TRACKER == kNextEvent + 100;
     constexpr bool kEss = TRACKER == kNextEvent + 100;
+    constexpr bool kDec = TRACKER == kDecomposition;
+    // events run once kEventShare eighths of the warp's live lanes wait (measured, 1 .. 5 eighths: delta tracking of
+    // a 512^3 grid 57.6 ms at 2, 56.5 at 3, 59.6 at 4; of a sparse grid 14.6 at 2, 15.5 at 3, 17.2 at 4; next event
+    // tracking 23.1 at 1, 22.6 at 2, 25.4 at 3)
+    constexpr int kEventShare = kNee ? 2 : (!kDec && GRID == kNanoVdb ? 2 : 3);
+    static_assert(kEventShare >= 1 && kEventShare <= 8, "0 would never let a lane collide");
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    const F3 zero = f3(0.0f, 0.0f, 0.0f);
+
+    // warp-uniform local batch of path ids
+    unsigned long long q_base = 0;
+    int q_left = 0;
+
+    bool has = false, exhausted = lane >= lanes;
+    int pend = kPendNone;
+    Rng rng;
+    F3 x = zero, w = zero, color = zero, xp = zero, nw = zero;
+    float d = 0.0f, dp = 0.0f, trans = 1.0f, weight = 0.0f;
+    float ts = 1.0f;  // shadow ray: transmittance so far; at a waiting collision: its density
+    float shadow_dist = 0.0f, shadow_max = 0.0f;  // distance walked / light distance (light shadow rays)
+    int mode = kModePrimary, bounces = 0, light = -1;
+    bool ev = false;
+    // block walk of decomposition tracking and of empty-space-skipping shadow rays, one boundary or one
+    // tentative collision per step: current block, the block whose data is held, inside a block or at a
+    // boundary, its length, distance sampled so far (decomposition: the residual clock) from entry bx0
+    int bx = 0, by = 0, bz = 0, ox = 0, oy = 0, oz = 0;
+    bool empty = false, in_block = false;
+    float bt = 0.0f, bd = 0.0f;
+    F3 bx0 = zero;
+    // decomposition tracking: the block's normalised min / max density, its control and residual
+    // extinctions and the control clock
+    float dc_min = 0.0f, dc_max = 0.0f, mu_c = 1.0f, mu_r = 1.0f, t_c = 0.0f;
+    int scene = 0;
+    uint32_t steps = 0;
+    size_t pix = 0;
+    uint32_t lookups = 0, paths = 0;
+    bool guard_hit = false;
+
+    while (true) {
+        // ---- refill lanes without a path ----
+        const bool need = !has && !exhausted;
+        const unsigned m = __ballot_sync(FULL, need);
+        unsigned live = __ballot_sync(FULL, has);
+        // refill once `refill_min` lanes wait (the refill step is long and divergent), or when no lane of the
+        // warp holds a path
+        if (m && (__popc(m) >= refill_min || !live)) {
+            const int n = __popc(m);
+            const int r = __popc(m & lt_mask);
+            unsigned long long fresh = 0;
+            if (n > q_left) {
+                unsigned long long b = 0;
+                if (lane == 0) b = atomicAdd(work_counter, (unsigned long long)batch);
+                fresh = __shfl_sync(FULL, b, 0);
+            }
+            if (need) {
+                unsigned long long p = r < q_left ? q_base + (unsigned long long)r
+                                                  : fresh + (unsigned long long)(r - q_left);
+                uint32_t frame;
+                int px, py;
+                const bool done = p >= total;
+                int s = 0;
+                if (!done) s = src.locate(p);
+                const TraceParams& P = src.scene(s);
+                if (done) {
+                    exhausted = true;
+                } else if (decode_path(P, p, frame, px, py)) {
+                    scene = s;
+                    const uint32_t w_u = (uint32_t)P.width, h_u = (uint32_t)P.height;
+                    uint32_t seed = (P.global_frame + frame) * w_u * h_u + (uint32_t)px + (uint32_t)py * w_u;
+                    seed += P.seed_offset;
+                    rng = rng_init(seed);
+                    float rx = rng_next(rng);
+                    float ry = rng_next(rng);
+                    float sx = (2.0f * ((float)px + rx)) / (float)P.width - 1.0f;
+                    float sy = (2.0f * ((float)py + ry)) / (float)P.height - 1.0f;
+                    camera_ray(P, sx, sy, x, w);
+                    pix = (size_t)py * P.width + px;
+                    paths++;
+                    steps = 0;
+                    bounces = 0;
+                    trans = 1.0f;
+                    color = zero;
+                    ev = false;
+                    mode = kModePrimary;
+                    in_block = false;
+                    has = true;
+                    pend = kPendNone;
+                    float tmin, tmax;
+                    if constexpr (kDec) {
+                        // analogDecompositionTracking: entry through the box shrunk by 1e-6, then the
+                        // supervoxel walk (its first block's bounds are read)
+                        const F3 eps = f3(1e-6f, 1e-6f, 1e-6f);
+                        if (ray_box(P.box_min + eps, P.box_max - eps, x, w, tmin, tmax)) {
+                            x = x + w * tmin;
+                            ess_first_block(P, x, bx, by, bz);
+                            ox = oy = oz = -1;
+                        } else {
+                            pend = kPendEscape;
+                        }
+                    } else if (ray_box_p(P, x, w, tmin, tmax)) {
+                        x = x + w * tmin;
+                        d = tmax - tmin;
+                    } else {
+                        pend = kPendEscape;
+                    }
+                }
+            }
+            if (n > q_left) {
+                q_base = fresh + (unsigned long long)(n - q_left);
+                q_left = batch - (n - q_left);
+            } else {
+                q_base += (unsigned long long)n;
+                q_left -= n;
+            }
+            live = __ballot_sync(FULL, has);
+        }
+        if (!live) {
+            if (__all_sync(FULL, exhausted)) break;
+            continue;
+        }
+
+        // ---- collisions, until enough lanes wait with an event ----
+        const int live_n = __popc(live);
+        while (__popc(__ballot_sync(FULL, pend != kPendNone)) * 8 < live_n * kEventShare) {
+            if (!has || pend != kPendNone) continue;
+            const TraceParams& P = src.scene(scene);
+            Sampler<INTERP, GRID, TF> sample{P};
+            if (++steps > P.max_steps) {
+                guard_hit = true;
+                pend = kPendEnd;
+                continue;
+            }
+            if constexpr (kEss) {
+                if (mode == kModeShadowEss) {
+                    if (!in_block) {  // at a block boundary (or the entry point)
+                        if (bx < 0 || by < 0 || bz < 0 || bx >= P.svx || by >= P.svy || bz >= P.svz) {
+                            pend = kPendShadow;
+                            continue;
+                        }
+                        const F3 smin = P.box_min + f3((float)bx, (float)by, (float)bz) * P.sv_world;
+                        const F3 smax = smin + P.sv_world;
+                        float tmin_sv = 0.0f, tmax_sv = 0.0f;
+                        ray_box(smin, smax, x, w, tmin_sv, tmax_sv);
+                        bd = tmax_sv - tmin_sv;
+                        x = x + w * tmin_sv;
+                        if (ox != bx || oy != by || oz != bz) {
+                            empty = __ldg(P.occupancy + ((size_t)bz * P.svy + by) * P.svx + bx) == 0;
+                            ox = bx;
+                            oy = by;
+                            oz = bz;
+                        }
+                        if (empty) {
+                            x = x + w * bd;
+                            ess_next_block(P, x, w, bx, by, bz);
+                        } else {
+                            bx0 = x;
+                            bt = 0.0f;
+                            in_block = true;
+                        }
+                        continue;
+                    }
+                    bt -= m_log(fmaxf(0.0000000001f, 1.0f - rng_next(rng))) * P.inv_extinction;
+                    if (bt >= bd) {
+                        x = (P.ess_ref_compat ? x : bx0) + w * bd;
+                        in_block = false;
+                        ess_next_block(P, x, w, bx, by, bz);
+                        continue;
+                    }
+                    const F3 xn = (P.ess_ref_compat ? x : bx0) + w * bt;
+                    const float dens = sample(xn, rng);
+                    lookups++;
+                    x = xn;
+                    ts *= 1.0f - dens;
+                    continue;
+                }
+            }
+            if constexpr (kDec) {
+                // the supervoxel walk of track_decomposition, one block boundary or one step of the two
+                // competing exponential clocks (control t_c, residual t_r) per step
+                if (!in_block) {
+                    if (bx < 0 || by < 0 || bz < 0 || bx >= P.svx || by >= P.svy || bz >= P.svz) {
+                        pend = kPendEscape;
+                        continue;
+                    }
+                    const F3 smin = P.box_min + f3((float)bx, (float)by, (float)bz) * P.sv_world;
+                    const F3 smax = smin + P.sv_world;
+                    float tmin_sv = 0.0f, tmax_sv = 0.0f;
+                    ray_box(smin, smax, x, w, tmin_sv, tmax_sv);
+                    bd = tmax_sv - tmin_sv;
+                    x = x + w * tmin_sv;
+                    if (ox != bx || oy != by || oz != bz) {
+                        const float2 mm = __ldg(reinterpret_cast<const float2*>(P.sv_data) +
+                                                ((size_t)bz * P.svy + by) * P.svx + bx);
+                        dc_min = mm.x;
+                        dc_max = mm.y;
+                        ox = bx;
+                        oy = by;
+                        oz = bz;
+                    }
+                    if (dc_max < 1e-5f) {
+                        x = x + w * bd;
+                        sv_step(smin, smax, x, w, bx, by, bz);
+                    } else {
+                        mu_c = fmaxf(0.0000000001f, P.extinction * dc_min);
+                        mu_r = fmaxf(0.0000000001f, P.extinction * dc_max - mu_c);
+                        t_c = -m_log(fmaxf(0.0000000001f, 1.0f - rng_next(rng))) / mu_c;
+                        bt = 0.0f;  // t_r
+                        in_block = true;
+                    }
+                    continue;
+                }
+                bt -= m_log(fmaxf(0.0000000001f, 1.0f - rng_next(rng))) / mu_r;
+                if (t_c >= bd && bt >= bd) {
+                    x = x + w * bd;
+                    in_block = false;
+                    const F3 smin = P.box_min + f3((float)bx, (float)by, (float)bz) * P.sv_world;
+                    sv_step(smin, smin + P.sv_world, x, w, bx, by, bz);
+                    continue;
+                }
+                const F3 xs = x + w * fminf(t_c, bt);
+                bool collision = true;
+                if (!(t_c <= bt)) {
+                    const float dens = sample(xs, rng);
+                    lookups++;
+                    collision = rng_next(rng) * mu_r < P.extinction * dens - mu_c;
+                }
+                if (collision) {
+                    x = xs;
+                    pend = kPendScatter;
+                }
+                continue;
+            }
+            const float t = free_path(rng, P.inv_extinction);
+            bool escape = t > d;
+            if (kNee && mode == kModeShadow && light >= 0) {
+                shadow_dist += t;
+                escape = escape || shadow_dist > shadow_max;
+            }
+            if (escape) {
+                pend = kNee && mode == kModeShadow ? kPendShadow : kPendEscape;
+                continue;
+            }
+            x = x + w * t;
+            const float density = sample(x, rng);
+            lookups++;
+            if (kNee && mode == kModeShadow) {
+                ts *= 1.0f - density;
+                d -= t;
+                continue;
+            }
+            const float xi = rng_next(rng);
+            if (TRACKER != kRatio && xi < P.absorb_albedo * density) {
+                // transfer function: the absorbed path ends with its emission (DeltaTracking.glsl:293-301)
+                if (TF && !(kNee && P.emission)) color = color + sample.tf_emission();
+                pend = kPendAbsorb;
+            } else if (xi < density) {
+                ts = density;
+                pend = kPendScatter;
+            } else {
+                d -= t;
+            }
+        }
+
+        // ---- the events of the waiting lanes ----
+        if (pend == kPendNone) continue;
+        const TraceParams& P = src.scene(scene);
+        F3 L = zero;
+        bool end = false;
+        if (pend == kPendEscape || (kNee && pend == kPendShadow)) {
+            const bool shadow = kNee && pend == kPendShadow;
+            if (shadow && light >= 0) L = light_radiance(P, xp, light);
+            else L = sky_and_sun(P, w);
+            if (shadow) {
+                // the light sample (f = weight * T with weight = pdf_phase / pdf_light for the sky, or the
+                // light probability factor times pdf_phase for a light; NextEventTracking.glsl:348-369);
+                // the path goes on at the scatter point with the sampled direction
+                const float f = weight * ts;
+                color = color + f3(f * L.x, f * L.y, f * L.z);
+                x = xp;
+                w = nw;
+                d = dp;
+                mode = kModePrimary;
+                float tmin, tmax;
+                if (ray_box_p(P, x, w, tmin, tmax)) {
+                    x = x + w * tmin;
+                    d = tmax - tmin;
+                }
+            } else {
+                if (kNee) L = ev ? color : color + L;
+                else if (TRACKER == kRatio) L = L * trans;
+                end = true;
+            }
+        } else if (pend == kPendScatter) {
+            if constexpr (kDec) {
+                end = rng_next(rng) < P.absorb_albedo || (P.max_bounces > 0 && ++bounces > P.max_bounces);
+                if (!end) {
+                    w = sample_phase(rng, P.g, w);
+                    bt = 0.0f;
+                    t_c = -m_log(fmaxf(0.0000000001f, 1.0f - rng_next(rng))) / mu_c;
+                    const F3 smin = P.box_min + f3((float)bx, (float)by, (float)bz) * P.sv_world;
+                    float tmin_sv = 0.0f, tmax_sv = 0.0f;
+                    ray_box(smin, smin + P.sv_world, x, w, tmin_sv, tmax_sv);
+                    bd = tmax_sv - tmin_sv;
+                }
+            } else if (P.max_bounces > 0 && ++bounces > P.max_bounces) {
+                L = kNee ? color : zero;
+                end = true;
+            } else {
+                if (TRACKER == kRatio) {
+                    const float pa = P.absorb_albedo * ts;
+                    const float ps = P.albedo * ts;
+                    trans *= 1.0f - pa / (pa + ps);
+                }
+                const F3 out = sample_phase(rng, P.g, w);
+                ev = true;
+                bool cast = true;  // the shadow ray needs a walk
+                if (kNee) {
+                    nw = out;
+                    bool to_light = false;
+                    float prob_factor = 1.0f, pdf_light = 0.0f, light_dist = 0.0f;
+                    int light_idx = 0;
+                    if (P.num_lights > 0) {
+                        to_light = P.env_is_black ? true : (rng_next(rng) > 0.5f);
+                        prob_factor = P.env_is_black ? 1.0f : 2.0f;
+                    }
+                    F3 dir;
+                    if (to_light) dir = light_direction(P, x, rng, light_idx, prob_factor, light_dist);
+                    else dir = importance_sample_sky(P, rng, pdf_light);
+                    const float pdf_phase = evaluate_phase(P.g, w, dir);
+                    if (P.num_lights > 0)
+                        weight = to_light ? prob_factor * pdf_phase : (prob_factor * pdf_phase) / pdf_light;
+                    else weight = pdf_phase / pdf_light;
+                    light = to_light ? light_idx : -1;
+                    shadow_max = light_dist;
+                    xp = x;
+                    dp = d;
+                    w = dir;
+                    ts = 1.0f;
+                    mode = kModeShadow;
+                    if (kEss && !to_light) {
+                        // shadow_transmittance_ess: entry through the box shrunk by 1e-6, the entry block is
+                        // walked as occupied
+                        const F3 eps = f3(1e-6f, 1e-6f, 1e-6f);
+                        float tmin, tmax;
+                        if (ray_box(P.box_min + eps, P.box_max - eps, x, w, tmin, tmax)) {
+                            x = x + w * tmin;
+                            ess_first_block(P, x, bx, by, bz);
+                            ox = bx;
+                            oy = by;
+                            oz = bz;
+                            empty = false;
+                            in_block = false;
+                            mode = kModeShadowEss;
+                        } else {
+                            pend = kPendShadow;  // no shadow steps: transmittance 1
+                        }
+                        cast = false;
+                    }
+                } else {
+                    w = out;
+                }
+                if (cast) {
+                    float tmin, tmax;
+                    if (ray_box_p(P, x, w, tmin, tmax)) {
+                        x = x + w * tmin;
+                        d = tmax - tmin;
+                        if (kNee) shadow_dist = tmin;
+                    } else if (kNee) {
+                        // no shadow steps (and no random numbers), like calculateTransmittance
+                        pend = kPendShadow;
+                    }
+                }
+            }
+            if (kNee && pend == kPendShadow) continue;
+        } else if (pend == kPendAbsorb) {
+            // USE_EMISSION (NextEventTracking.glsl:296-301): the absorbed path ends with the emission
+            L = color;
+            if (kNee && P.emission) {
+                Sampler<INTERP, GRID, TF> sample{P};
+                L = color + sample.emission(x, rng);
+            }
+            end = true;
+        } else {
+            L = color;
+            end = true;
+        }
+        pend = kPendNone;
+        if (end) {
+            refill_finish<TRACKER>(P, pix, L, has);
+        }
+    }
+    flush_counters_to(counters, error_flags, paths, lookups, guard_hit);
+}
+
+// ---------------------------------------------------------------------------------------------
+// The refill loop of the other per-lane schedules: delta tracking with isosurfaces (kDeltaIso) and the
+// unbiased residual ratio tracker (kResidualRatioNee).  Each loop iteration advances every live lane by one
+// tentative collision or cell boundary, events included.
+template <int TRACKER, int INTERP, int GRID, bool TF, class SRC>
+VPT_DEV void refill_loop(const SRC& src, uint64_t total, unsigned long long* work_counter,
+                         unsigned long long* counters, int* error_flags, int refill_min) {
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -456,8 +857,8 @@ VPT_DEV void refill_loop(const SRC& src, uint64_t total, unsigned long long* wor
     bool has = false, exhausted = false;
     Rng rng;
     F3 x = zero, w = zero, color = zero, xp = zero, nw = zero;
-    float d = 0.0f, dp = 0.0f, trans = 1.0f, ts = 1.0f, weight = 0.0f;
-    float shadow_dist = 0.0f, shadow_max = 0.0f;  // distance walked / light distance (light shadow rays)
+    float d = 0.0f, ts = 1.0f, weight = 0.0f;
+    float shadow_max = 0.0f;  // light distance (shadow rays)
     int mode = kModePrimary, bounces = 0, light = -1;
     bool ev = false;
     // isosurface state (kDeltaIso): surface throughput, sign at the first point after the last event,
@@ -466,16 +867,9 @@ VPT_DEV void refill_loop(const SRC& src, uint64_t total, unsigned long long* wor
     float iso_last = 0.0f;
     bool iso_first = true;
     int iso_it = 0;
-    // empty-space-skipping shadow ray (kEss), the walk of shadow_transmittance_ess one step per
-    // iteration: current block, the block whose occupancy `empty` holds, inside an occupied block or
-    // at a block boundary, distance sampled so far from the block entry x0, the block's length
-    int bx = 0, by = 0, bz = 0, ox = 0, oy = 0, oz = 0;
-    bool empty = false, in_block = false;
-    float bt = 0.0f, bd = 0.0f;
-    F3 bx0 = zero;
-    // decomposition tracking (the same block walk): the block's normalised min / max density, its
-    // control and residual extinctions and the control clock (bt is the residual clock)
-    float dc_min = 0.0f, dc_max = 0.0f, mu_c = 1.0f, mu_r = 1.0f, t_c = 0.0f;
+    // unbiased residual ratio tracking: inside a cell, the distance sampled so far
+    bool in_block = false;
+    float bt = 0.0f;
     // unbiased residual ratio tracking: the Amanatides-Woo supervoxel walk of the current free flight
     // or shadow ray (started lazily), its axis and cell, the distance reached, the walk's length
     SvWalk sw;
@@ -530,7 +924,6 @@ VPT_DEV void refill_loop(const SRC& src, uint64_t total, unsigned long long* wor
                     paths++;
                     steps = 0;
                     bounces = 0;
-                    trans = 1.0f;
                     color = zero;
                     ev = false;
                     mode = kModePrimary;
@@ -541,20 +934,7 @@ VPT_DEV void refill_loop(const SRC& src, uint64_t total, unsigned long long* wor
                     iso_it = 0;
                     float tmin, tmax;
                     has = true;
-                    if constexpr (TRACKER == kDecomposition) {
-                        // analogDecompositionTracking: entry through the box shrunk by 1e-6, then the
-                        // supervoxel walk (its first block's bounds are read)
-                        const F3 eps = f3(1e-6f, 1e-6f, 1e-6f);
-                        if (ray_box(P.box_min + eps, P.box_max - eps, x, w, tmin, tmax)) {
-                            x = x + w * tmin;
-                            ess_first_block(P, x, bx, by, bz);
-                            ox = oy = oz = -1;
-                            in_block = false;
-                        } else {
-                            F3 L = sky_and_sun(P, w);
-                            refill_finish<TRACKER>(P, pix, L, has);
-                        }
-                    } else if (ray_box_p(P, x, w, tmin, tmax)) {
+                    if (ray_box_p(P, x, w, tmin, tmax)) {
                         x = x + w * tmin;
                         d = tmax - tmin;
                     } else {
@@ -586,52 +966,8 @@ VPT_DEV void refill_loop(const SRC& src, uint64_t total, unsigned long long* wor
         }
         if (++steps > P.max_steps) {
             guard_hit = true;
-            refill_finish<TRACKER>(P, pix, (kNee || TRACKER == kResidualRatioNee) ? color : zero, has);
+            refill_finish<TRACKER>(P, pix, TRACKER == kResidualRatioNee ? color : zero, has);
             continue;
-        }
-        if constexpr (kEss) {
-            if (mode == kModeShadowEss) {
-                if (!in_block) {  // at a block boundary (or the entry point)
-                    if (bx < 0 || by < 0 || bz < 0 || bx >= P.svx || by >= P.svy || bz >= P.svz) {
-                        end_shadow(P, color, x, w, d, xp, nw, dp, weight, ts, light, mode);
-                        continue;
-                    }
-                    const F3 smin = P.box_min + f3((float)bx, (float)by, (float)bz) * P.sv_world;
-                    const F3 smax = smin + P.sv_world;
-                    float tmin_sv = 0.0f, tmax_sv = 0.0f;
-                    ray_box(smin, smax, x, w, tmin_sv, tmax_sv);
-                    bd = tmax_sv - tmin_sv;
-                    x = x + w * tmin_sv;
-                    if (ox != bx || oy != by || oz != bz) {
-                        empty = __ldg(P.occupancy + ((size_t)bz * P.svy + by) * P.svx + bx) == 0;
-                        ox = bx;
-                        oy = by;
-                        oz = bz;
-                    }
-                    if (empty) {
-                        x = x + w * bd;
-                        ess_next_block(P, x, w, bx, by, bz);
-                    } else {
-                        bx0 = x;
-                        bt = 0.0f;
-                        in_block = true;
-                    }
-                    continue;
-                }
-                bt -= m_log(fmaxf(0.0000000001f, 1.0f - rng_next(rng))) * P.inv_extinction;
-                if (bt >= bd) {
-                    x = (P.ess_ref_compat ? x : bx0) + w * bd;
-                    in_block = false;
-                    ess_next_block(P, x, w, bx, by, bz);
-                    continue;
-                }
-                const F3 xn = (P.ess_ref_compat ? x : bx0) + w * bt;
-                const float dens = sample(xn, rng);
-                lookups++;
-                x = xn;
-                ts *= 1.0f - dens;
-                continue;
-            }
         }
         if constexpr (TRACKER == kResidualRatioNee) {
             // track_residual_ratio_nee one step per iteration: a free flight by delta tracking with each
@@ -751,198 +1087,39 @@ VPT_DEV void refill_loop(const SRC& src, uint64_t total, unsigned long long* wor
             }
             continue;
         }
-        if constexpr (TRACKER == kDecomposition) {
-            // the supervoxel walk of track_decomposition, one block boundary or one step of the two
-            // competing exponential clocks (control t_c, residual t_r) per iteration
-            if (!in_block) {
-                if (bx < 0 || by < 0 || bz < 0 || bx >= P.svx || by >= P.svy || bz >= P.svz) {
-                    refill_finish<TRACKER>(P, pix, sky_and_sun(P, w), has);
-                    continue;
-                }
-                const F3 smin = P.box_min + f3((float)bx, (float)by, (float)bz) * P.sv_world;
-                const F3 smax = smin + P.sv_world;
-                float tmin_sv = 0.0f, tmax_sv = 0.0f;
-                ray_box(smin, smax, x, w, tmin_sv, tmax_sv);
-                bd = tmax_sv - tmin_sv;
-                x = x + w * tmin_sv;
-                if (ox != bx || oy != by || oz != bz) {
-                    const float2 mm = __ldg(reinterpret_cast<const float2*>(P.sv_data) +
-                                            ((size_t)bz * P.svy + by) * P.svx + bx);
-                    dc_min = mm.x;
-                    dc_max = mm.y;
-                    ox = bx;
-                    oy = by;
-                    oz = bz;
-                }
-                if (dc_max < 1e-5f) {
-                    x = x + w * bd;
-                    sv_step(smin, smax, x, w, bx, by, bz);
-                } else {
-                    mu_c = fmaxf(0.0000000001f, P.extinction * dc_min);
-                    mu_r = fmaxf(0.0000000001f, P.extinction * dc_max - mu_c);
-                    t_c = -m_log(fmaxf(0.0000000001f, 1.0f - rng_next(rng))) / mu_c;
-                    bt = 0.0f;  // t_r
-                    in_block = true;
-                }
+        if constexpr (TRACKER == kDeltaIso) {
+            const float t = free_path(rng, P.inv_extinction);
+            if (t > d) {
+                refill_finish<TRACKER>(P, pix, iw * sky_and_sun(P, w), has);
                 continue;
             }
-            bt -= m_log(fmaxf(0.0000000001f, 1.0f - rng_next(rng))) / mu_r;
-            if (t_c >= bd && bt >= bd) {
-                x = x + w * bd;
-                in_block = false;
-                const F3 smin = P.box_min + f3((float)bx, (float)by, (float)bz) * P.sv_world;
-                sv_step(smin, smin + P.sv_world, x, w, bx, by, bz);
+            const F3 xn = x + w * t;
+            const float density = sample(xn, rng);
+            lookups++;
+            float tmax_unused = 0.0f;
+            if (iso_segment(P, sample, rng, x, xn, density, w, d, tmax_unused, iw, iso_last, iso_first, lookups,
+                            nullptr)) {
+                if (iw.x < 1e-3f && iw.y < 1e-3f && iw.z < 1e-3f) refill_finish<TRACKER>(P, pix, zero, has);
                 continue;
             }
-            const F3 xs = x + w * fminf(t_c, bt);
-            bool collision;
-            if (t_c <= bt) {
-                collision = true;
-            } else {
-                const float dens = sample(xs, rng);
-                lookups++;
-                collision = rng_next(rng) * mu_r < P.extinction * dens - mu_c;
-            }
-            if (collision) {
-                x = xs;
-                if (rng_next(rng) < P.absorb_albedo) {
-                    refill_finish<TRACKER>(P, pix, zero, has);
-                    continue;
-                }
+            x = xn;
+            const float xi = rng_next(rng);
+            if (xi < P.absorb_albedo * density) {
+                refill_finish<TRACKER>(P, pix, zero, has);
+            } else if (xi < density) {
                 if (P.max_bounces > 0 && ++bounces > P.max_bounces) {
                     refill_finish<TRACKER>(P, pix, zero, has);
                     continue;
                 }
                 w = sample_phase(rng, P.g, w);
-                bt = 0.0f;
-                t_c = -m_log(fmaxf(0.0000000001f, 1.0f - rng_next(rng))) / mu_c;
-                const F3 smin = P.box_min + f3((float)bx, (float)by, (float)bz) * P.sv_world;
-                float tmin_sv = 0.0f, tmax_sv = 0.0f;
-                ray_box(smin, smin + P.sv_world, x, w, tmin_sv, tmax_sv);
-                bd = tmax_sv - tmin_sv;
-            }
-            continue;
-        }
-        const float t = free_path(rng, P.inv_extinction);
-        bool escape = t > d;
-        if (kNee && mode == kModeShadow && light >= 0) {
-            shadow_dist += t;
-            escape = escape || shadow_dist > shadow_max;
-        }
-        float density = 0.0f;
-        if (!escape) {
-            F3 xn = x + w * t;
-            density = sample(xn, rng);
-            lookups++;
-            if constexpr (TRACKER == kDeltaIso) {
-                float tmax_unused = 0.0f;
-                if (iso_segment(P, sample, rng, x, xn, density, w, d, tmax_unused, iw, iso_last, iso_first, lookups,
-                                nullptr)) {
-                    if (iw.x < 1e-3f && iw.y < 1e-3f && iw.z < 1e-3f) refill_finish<TRACKER>(P, pix, zero, has);
-                    continue;
-                }
-            }
-            x = xn;
-        }
-        if (kNee && mode == kModeShadow) {
-            if (!escape) {
-                ts *= 1.0f - density;
-                d -= t;
-                continue;
-            }
-            end_shadow(P, color, x, w, d, xp, nw, dp, weight, ts, light, mode);
-            continue;
-        }
-        if (escape) {
-            F3 L;
-            if (kNee) L = ev ? color : color + sky_and_sun(P, w);
-            else if (TRACKER == kRatio) L = sky_and_sun(P, w) * trans;
-            else if (TRACKER == kDeltaIso) L = iw * sky_and_sun(P, w);
-            else L = sky_and_sun(P, w);
-            refill_finish<TRACKER>(P, pix, L, has);
-            continue;
-        }
-        const float xi = rng_next(rng);
-        if (TRACKER != kRatio && xi < P.absorb_albedo * density) {
-            // USE_EMISSION (NextEventTracking.glsl:296-301): the absorbed NEE path ends with the emission
-            F3 L = zero;
-            if (kNee) {
-                L = P.emission ? color + sample.emission(x, rng) : (P.tf ? color + sample.tf_emission() : color);
-            } else if (P.tf) {  // delta tracking (DeltaTracking.glsl:293-301)
-                L = sample.tf_emission();
-            }
-            refill_finish<TRACKER>(P, pix, L, has);
-            continue;
-        }
-        if (xi < density) {
-            if (P.max_bounces > 0 && ++bounces > P.max_bounces) {
-                refill_finish<TRACKER>(P, pix, kNee ? color : zero, has);
-                continue;
-            }
-            float tmin, tmax;
-            if (kNee) {
-                nw = sample_phase(rng, P.g, w);
-                ev = true;
-                bool to_light = false;
-                float prob_factor = 1.0f, pdf_light = 0.0f, light_dist = 0.0f;
-                int light_idx = 0;
-                if (P.num_lights > 0) {
-                    to_light = P.env_is_black ? true : (rng_next(rng) > 0.5f);
-                    prob_factor = P.env_is_black ? 1.0f : 2.0f;
-                }
-                F3 dir;
-                if (to_light) dir = light_direction(P, x, rng, light_idx, prob_factor, light_dist);
-                else dir = importance_sample_sky(P, rng, pdf_light);
-                const float pdf_phase = evaluate_phase(P.g, w, dir);
-                if (P.num_lights > 0) weight = to_light ? prob_factor * pdf_phase : (prob_factor * pdf_phase) / pdf_light;
-                else weight = pdf_phase / pdf_light;
-                light = to_light ? light_idx : -1;
-                shadow_max = light_dist;
-                xp = x;
-                dp = d;
-                w = dir;
-                ts = 1.0f;
-                mode = kModeShadow;
-                if (kEss && !to_light) {
-                    // shadow_transmittance_ess: entry through the box shrunk by 1e-6, the entry block is
-                    // walked as occupied
-                    const F3 eps = f3(1e-6f, 1e-6f, 1e-6f);
-                    if (ray_box(P.box_min + eps, P.box_max - eps, x, w, tmin, tmax)) {
-                        x = x + w * tmin;
-                        ess_first_block(P, x, bx, by, bz);
-                        ox = bx;
-                        oy = by;
-                        oz = bz;
-                        empty = false;
-                        in_block = false;
-                        mode = kModeShadowEss;
-                    } else {
-                        end_shadow(P, color, x, w, d, xp, nw, dp, weight, ts, light, mode);
-                    }
-                    continue;
-                }
+                float tmin, tmax;
                 if (ray_box_p(P, x, w, tmin, tmax)) {
                     x = x + w * tmin;
                     d = tmax - tmin;
-                    shadow_dist = tmin;
-                } else {
-                    // no shadow steps (and no random numbers), like calculateTransmittance
-                    end_shadow(P, color, x, w, d, xp, nw, dp, weight, ts, light, mode);
                 }
-                continue;
+            } else {
+                d -= t;
             }
-            if (TRACKER == kRatio) {
-                float pa = P.absorb_albedo * density;
-                float ps = P.albedo * density;
-                trans *= 1.0f - pa / (pa + ps);
-            }
-            w = sample_phase(rng, P.g, w);
-            if (ray_box_p(P, x, w, tmin, tmax)) {
-                x = x + w * tmin;
-                d = tmax - tmin;
-            }
-        } else {
-            d -= t;
         }
     }
     flush_counters_to(counters, error_flags, paths, lookups, guard_hit);
@@ -954,6 +1131,14 @@ __global__ void __launch_bounds__(kTraceBlock) trace_refill_kernel(const __grid_
                                        P.counters, P.error_flags, P.refill_min);
 }
 
+template <int TRACKER, int INTERP, int GRID, bool TF>
+__global__ void __launch_bounds__(kTraceBlock) trace_event_kernel(const __grid_constant__ TraceParams P, uint64_t total,
+                                                                  int batch, int lanes) {
+    event_loop<TRACKER, INTERP, GRID, TF>(OneScene{P}, total,
+                                                reinterpret_cast<unsigned long long*>(P.work_counter), P.counters,
+                                                P.error_flags, P.refill_min, batch, lanes);
+}
+
 // Many independent scenes (own grid, camera, image size, spp, medium) traced by one persistent
 // launch: lanes refill from one id space that concatenates the scenes' paths.  The total path count
 // is read from offsets[num], so a captured launch serves any frame counts.
@@ -962,8 +1147,8 @@ __global__ void __launch_bounds__(kTraceBlock) trace_batch_kernel(const TracePar
                                                                   const unsigned long long* __restrict__ offsets,
                                                                   int num, unsigned long long* work_counter,
                                                                   unsigned long long* counters, int* error_flags) {
-    refill_loop<TRACKER, INTERP, GRID, false>(SceneBatch{scenes, offsets, num}, __ldg(offsets + num), work_counter, counters,
-                                       error_flags, scenes[0].refill_min);
+    event_loop<TRACKER, INTERP, GRID, false>(SceneBatch{scenes, offsets, num}, __ldg(offsets + num), work_counter,
+                                                    counters, error_flags, scenes[0].refill_min, kRefillBatch, 32);
 }
 
 
@@ -1001,14 +1186,15 @@ static cudaError_t batch_tracker(const BatchLaunch& b, cudaStream_t s) {
         default: return cudaErrorNotSupported;
     }
 }
-template <int TRACKER, int INTERP, int GRID, bool TF>
-static int refill_blocks(int requested) {
+// One wave of resident blocks of `kernel` (SMs x blocks per SM from the occupancy calculator, kept in
+// `per_sm`), or the requested number.
+template <class K>
+static int resident_blocks(K* kernel, int& per_sm, int requested) {
     if (requested > 0) return requested;
-    static int per_sm = 0;
     if (per_sm == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_refill_kernel<TRACKER, INTERP, GRID, TF>, kTraceBlock,
-                                                      0);
-        if (per_sm <= 0) per_sm = 1;
+        int n = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, kernel, kTraceBlock, 0);
+        per_sm = n > 0 ? n : 1;
     }
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
@@ -1016,17 +1202,48 @@ static int refill_blocks(int requested) {
     return per_sm * sms;
 }
 
+// share: paths per resident warp
+template <int TRACKER, int INTERP, int GRID, bool TF>
+static cudaError_t launch_events(const TraceParams& P, uint64_t total, int blocks, uint64_t share, cudaStream_t stream) {
+    // Ids per warp: batches of 64 when every warp gets several, of 32 when it gets few (a finer balance at the
+    // end).  Decomposition tracking with fewer paths than resident lanes spreads them over all warps, since a
+    // warp's time is that of its longest path and of the code its lanes do not share: 64^2 paths 455 -> 360 us,
+    // 128^2 498 -> 395, 256^2 620 -> 600 on the 256^3 cloud.  Next event tracking does not gain from it.
+    constexpr bool kSpread = TRACKER == kDecomposition;
+    const int lanes = share >= 32 || !kSpread ? 32 : (share < 4 ? 4 : (int)share + 1);
+    const int batch = share >= 256 ? kRefillBatch : lanes;
+    cudaMemsetAsync(P.work_counter, 0, sizeof(unsigned long long), stream);
+    trace_event_kernel<TRACKER, INTERP, GRID, TF><<<blocks, kTraceBlock, 0, stream>>>(P, total, batch, lanes);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
 template <int TRACKER, int INTERP, int GRID, bool TF>
 static cudaError_t launch_trace_t(const TraceParams& P, int schedule, int features, int persistent_blocks,
                                   cudaStream_t stream) {
     uint64_t total = padded_paths(P.width, P.height, P.num_frames);
-    constexpr bool kRefillable = TRACKER == kDelta || TRACKER == kRatio || TRACKER == kNextEvent ||
-                                 TRACKER == kNextEvent + 100 || TRACKER == kDeltaIso ||
-                                 ((TRACKER == kDecomposition || TRACKER == kResidualRatioNee) && GRID != kNanoVdb);
+    constexpr bool kEvents = TRACKER == kDelta || TRACKER == kRatio || TRACKER == kNextEvent ||
+                             TRACKER == kNextEvent + 100 || (TRACKER == kDecomposition && GRID != kNanoVdb);
+    constexpr bool kRefillable = TRACKER == kDeltaIso || (TRACKER == kResidualRatioNee && GRID != kNanoVdb);
+    if constexpr (kEvents) {
+        if (schedule == kScheduleRefill && !features) {
+            static int per_sm = 0;
+            const int blocks = resident_blocks(trace_event_kernel<TRACKER, INTERP, GRID, TF>, per_sm, persistent_blocks);
+            const uint64_t share = total / ((uint64_t)blocks * (kTraceBlock / 32));
+            // Delta and ratio tracking with fewer than five paths per resident lane: the launch lasts as long as
+            // its longest path, whose steps are shortest on persistent batches (nothing to wait for): 256^2 paths of
+            // the 128^3 cloud 580 against 655 us, 512^2 690 / 810, 2 x 512^2 930 / 1040, 4 x 512^2 1370 / 1360,
+            // 8 x 512^2 2290 / 2200.  The other trackers' events make batches two to three times slower at any size.
+            constexpr bool kShortEvents = TRACKER == kDelta || TRACKER == kRatio;
+            if (!kShortEvents || share >= 160 || persistent_blocks > 0)
+                return launch_events<TRACKER, INTERP, GRID, TF>(P, total, blocks, share, stream);
+        }
+    }
     // the refill loop's surface check has no closing surfaces (CLOSE_ISOSURFACES): persistent batches then
     if (schedule == kScheduleRefill && kRefillable && !features && !P.iso_close) {
         if constexpr (kRefillable) {
-            int blocks = refill_blocks<TRACKER, INTERP, GRID, TF>(persistent_blocks);
+            static int per_sm = 0;
+            const int blocks = resident_blocks(trace_refill_kernel<TRACKER, INTERP, GRID, TF>, per_sm, persistent_blocks);
             cudaMemsetAsync(P.work_counter, 0, sizeof(unsigned long long), stream);
             trace_refill_kernel<TRACKER, INTERP, GRID, TF><<<blocks, kTraceBlock, 0, stream>>>(P, total);
             count_launches(1);
@@ -1039,19 +1256,8 @@ static cudaError_t launch_trace_t(const TraceParams& P, int schedule, int featur
         trace_tiles_kernel<TRACKER, INTERP, GRID, TF><<<(unsigned)blocks, kTraceBlock, 0, stream>>>(P, features);
         count_launches(1);
     } else {
-        if (persistent_blocks <= 0) {
-            // one wave of resident blocks: SMs x blocks per SM from the occupancy calculator
-            static int per_sm = 0;
-            if (per_sm == 0) {
-                cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, trace_persistent_kernel<TRACKER, INTERP, GRID, TF>,
-                                                              kTraceBlock, 0);
-                if (per_sm <= 0) per_sm = 1;
-            }
-            int dev = 0, sms = 148;
-            cudaGetDevice(&dev);
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-            persistent_blocks = per_sm * sms;
-        }
+        static int per_sm = 0;
+        persistent_blocks = resident_blocks(trace_persistent_kernel<TRACKER, INTERP, GRID, TF>, per_sm, persistent_blocks);
         cudaMemsetAsync(P.work_counter, 0, sizeof(unsigned long long), stream);
         trace_persistent_kernel<TRACKER, INTERP, GRID, TF><<<persistent_blocks, kTraceBlock, 0, stream>>>(P, features,
                                                                                                            total);

@@ -473,6 +473,31 @@ def test_schedules_trace_identical_paths(core_dr, mode):
         assert np.allclose(films[0], f, rtol=1e-12, atol=1e-12)
 
 
+@pytest.mark.parametrize("size", [(1, 1), (5, 3), (33, 7), (64, 48)])
+@pytest.mark.parametrize("interp", ["nearest", "stochastic", "trilinear"])
+@pytest.mark.parametrize("mode", ["delta", "ratio", "nee", "nee_lights", "nee_ess", "decomposition"])
+def test_deferred_events_trace_identical_paths(core_dr, mode, interp, size):
+    """The refill schedule's loop that defers path events traces the paths of the tile schedule: launches of less
+    than a path per lane (the decomposition tracker spreads those over the warps), of part of a warp and of
+    several waves, and one block per SM (which also takes the
+    small delta and ratio launches to this loop).  Same film up to the order of the FP64 additions."""
+    core = core_dr
+    kw = dict(PATH_CASES["nee_lights"]) if mode == "nee_lights" else dict(mode=mode)
+    if mode == "nee_ess":
+        kw = dict(mode="nee", use_ess=True)
+    sp = fbm_scene(width=size[0], height=size[1], **dict(kw, interp=interp))
+    setup_core(core, sp)
+    films = []
+    for sched, blocks in ((0.0, 0.0), (2.0, 0.0), (2.0, 1.0)):
+        core("vpt_set_option", b"schedule", sched)
+        core("vpt_set_option", b"persistent_blocks_per_sm", blocks)
+        films.append(gpu_render(core, sp, 3, stats=False)[0])
+    core("vpt_set_option", b"persistent_blocks_per_sm", 0.0)
+    core("vpt_set_option", b"schedule", 2.0)
+    for f in films[1:]:
+        assert np.allclose(films[0], f, rtol=1e-12, atol=1e-12)
+
+
 @pytest.mark.parametrize("interp", ["nearest", "stochastic", "trilinear"])
 @pytest.mark.parametrize("sched", [1, 2])
 @pytest.mark.parametrize("mode", ["delta", "ratio", "nee", "nee_ess", "decomposition", "rrt_unbiased"])
