@@ -447,6 +447,8 @@ VPT_DEV void event_loop(const SRC& src, uint64_t total, unsigned long long* work
     // a 512^3 grid 57.6 ms at 2, 56.5 at 3, 59.6 at 4; of a sparse grid 14.6 at 2, 15.5 at 3, 17.2 at 4; next event
     // tracking 23.1 at 1, 22.6 at 2, 25.4 at 3)
     constexpr int kEventShare = kNee ? 2 : (!kDec && GRID == kNanoVdb ? 2 : 3);
+    // collisions a shadow ray goes ahead of its lookups (a trilinear lookup is eight fetches)
+    constexpr int kAhead = kNee ? (INTERP == kTrilinear ? 2 : 4) : 1;
     static_assert(kEventShare >= 1 && kEventShare <= 8, "0 would never let a lane collide");
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -676,24 +678,42 @@ VPT_DEV void event_loop(const SRC& src, uint64_t total, unsigned long long* work
                 }
                 continue;
             }
-            const float t = free_path(rng, P.inv_extinction);
-            bool escape = t > d;
-            if (kNee && mode == kModeShadow && light >= 0) {
-                shadow_dist += t;
-                escape = escape || shadow_dist > shadow_max;
+            // A shadow ray's collisions do not depend on the densities met on the way, only its transmittance
+            // does: its lanes go up to kAhead collisions on with the lookups in flight, and take the densities
+            // into the transmittance afterwards, in order.
+            const bool shadow = kNee && mode == kModeShadow;
+            float dens[kAhead], t = 0.0f;
+#pragma unroll
+            for (int u = 0; u < kAhead; u++) {
+                dens[u] = 0.0f;
+                if (u > 0 && (!shadow || pend != kPendNone)) continue;
+                if (u > 0 && ++steps > P.max_steps) {
+                    guard_hit = true;
+                    pend = kPendEnd;
+                    continue;
+                }
+                t = free_path(rng, P.inv_extinction);
+                bool escape = t > d;
+                if (kNee && shadow && light >= 0) {
+                    shadow_dist += t;
+                    escape = escape || shadow_dist > shadow_max;
+                }
+                if (escape) {
+                    pend = shadow ? kPendShadow : kPendEscape;
+                    continue;
+                }
+                x = x + w * t;
+                dens[u] = sample(x, rng);
+                lookups++;
+                if (shadow) d -= t;
             }
-            if (escape) {
-                pend = kNee && mode == kModeShadow ? kPendShadow : kPendEscape;
+            if (shadow) {
+#pragma unroll
+                for (int u = 0; u < kAhead; u++) ts *= 1.0f - dens[u];
                 continue;
             }
-            x = x + w * t;
-            const float density = sample(x, rng);
-            lookups++;
-            if (kNee && mode == kModeShadow) {
-                ts *= 1.0f - density;
-                d -= t;
-                continue;
-            }
+            if (pend != kPendNone) continue;
+            const float density = dens[0];
             const float xi = rng_next(rng);
             if (TRACKER != kRatio && xi < P.absorb_albedo * density) {
                 // transfer function: the absorbed path ends with its emission (DeltaTracking.glsl:293-301)

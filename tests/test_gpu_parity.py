@@ -479,7 +479,7 @@ def test_schedules_trace_identical_paths(core_dr, mode):
 def test_deferred_events_trace_identical_paths(core_dr, mode, interp, size):
     """The refill schedule's loop that defers path events traces the paths of the tile schedule: launches of less
     than a path per lane (the decomposition tracker spreads those over the warps), of part of a warp and of
-    several waves, and one block per SM (which also takes the
+    several waves, shadow rays that walk ahead of their lookups, and one block per SM (which also takes the
     small delta and ratio launches to this loop).  Same film up to the order of the FP64 additions."""
     core = core_dr
     kw = dict(PATH_CASES["nee_lights"]) if mode == "nee_lights" else dict(mode=mode)
