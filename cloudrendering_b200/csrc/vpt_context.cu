@@ -17,6 +17,7 @@
 #include "vpt_kernels.h"
 #include "vpt_params.h"
 #include "vpt_denoise.h"
+#include "vpt_scratch.h"
 #include "vpt_sparse.h"
 
 using vpt::F3;
@@ -40,6 +41,11 @@ struct DevBuf {
         release();
         if (n == 0) return cudaSuccess;
         cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T));
+        if (e == cudaErrorMemoryAllocation) {  // once more without the scratch that is kept between calls
+            cudaGetLastError();
+            vpt::scratch_trim();
+            e = cudaMalloc(reinterpret_cast<void**>(&ptr), n * sizeof(T));
+        }
         if (e != cudaSuccess) {
             ptr = nullptr;
             return e;
@@ -1046,6 +1052,7 @@ void vpt_destroy(VptContext* ctx) {
     ctx->error_flags.release();
     ctx->work_counter.release();
     vpt::svgf_release(ctx->svgf_state);
+    vpt::scratch_trim();
     delete ctx;
 }
 
@@ -2392,7 +2399,7 @@ VptStatus vpt_eaw_denoise_rgba(const float* color, const float* position, const 
         return cudaMemcpyAsync(out, color, bytes, cudaMemcpyDeviceToDevice, s) == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
     }
     float* scratch = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&scratch), bytes, s) != cudaSuccess) return VPT_ERR_OOM;
+    if (vpt::scratch_alloc(reinterpret_cast<void**>(&scratch), bytes, s) != cudaSuccess) return VPT_ERR_OOM;
     vpt::EawSettings st;
     st.iterations = iterations;
     st.phi_color = phi_color;

@@ -15,6 +15,7 @@
 #include "vpt_denoise.h"
 #include "vpt_params.h"
 #include "vpt_kernels.h"
+#include "vpt_scratch.h"
 #include "../../include/vpt_b200.h"
 
 namespace vpt {
@@ -987,7 +988,8 @@ extern "C" VptStatus vpt_svgf_filter(const float* noisy_rgba, const float* norma
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const size_t n = (size_t)width * height;
     float* scratch = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&scratch), n * (16 + vpt::kSvgfPlaneFloats) * 4, s) != cudaSuccess) return VPT_ERR_OOM;
+    if (vpt::scratch_alloc(reinterpret_cast<void**>(&scratch), n * (16 + vpt::kSvgfPlaneFloats) * 4, s) != cudaSuccess)
+        return VPT_ERR_OOM;
     vpt::SvgfCur c;
     c.noisy = reinterpret_cast<float4*>(const_cast<float*>(noisy_rgba));
     c.normal = reinterpret_cast<float4*>(const_cast<float*>(normal_rgba));

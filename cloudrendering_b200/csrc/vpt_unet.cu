@@ -36,6 +36,7 @@
 #include <string.h>
 #include "../../include/vpt_b200.h"
 #include "vpt_kernels.h"
+#include "vpt_scratch.h"
 
 namespace vpt {
 namespace unet {
@@ -2702,7 +2703,7 @@ cudaError_t launch_strip(const ConvArgs& c, int groups, int chunk, cudaStream_t 
     // fp32 partial sum of the earlier groups (stream-ordered scratch)
     float* part = nullptr;
     const size_t bytes = (size_t)c.n * c.h * c.w_ * c.cout * sizeof(float);
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&part), bytes, s);
+    cudaError_t e = vpt::scratch_alloc(reinterpret_cast<void**>(&part), bytes, s);
     if (e != cudaSuccess) return e;
     const int cg = (c.cin / 16 + groups - 1) / groups * 16;
     for (int g = 0, c0 = 0; c0 < c.cin && e == cudaSuccess; ++g, c0 += cg) {
@@ -2785,7 +2786,7 @@ VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, cons
     if (ksplit == 1)
         return launch_tile<kConv>(a, dim3(gx, gy, 1), s) == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
     float* part = nullptr;
-    if (cudaMallocAsync(reinterpret_cast<void**>(&part), (size_t)ksplit * P * cout * sizeof(float), s) != cudaSuccess)
+    if (vpt::scratch_alloc(reinterpret_cast<void**>(&part), (size_t)ksplit * P * cout * sizeof(float), s) != cudaSuccess)
         return VPT_ERR_OOM;
     a.ksplit = ksplit;
     a.partial = part;
