@@ -310,6 +310,78 @@ __global__ void supervoxel_stats_kernel(const float* __restrict__ dens, int nx, 
     if (out_occ) out_occ[idx] = hi < 1e-5f ? 0 : 1;
 }
 
+// The same numbers for supervoxels of 8 (the default), a warp for 32 of them along x.  A thread's loads above are 8
+// voxels apart, one sector each, and one after the other: 91 us for 256 x 256 x 200 voxels.  Here a lane reads its
+// rows as two 16-byte words, all rows of a z plane at once, and its neighbours' voxels of the halo come by shuffles
+// (the warp's two ends load theirs); every lane still adds its own voxels in z-y-x order.  14 us for those voxels (52 MB, 8 us); copying the
+// planes through shared memory word by word took 89.
+template <int HALO>
+__global__ void __launch_bounds__(128) supervoxel8_kernel(const float* __restrict__ dens, int nx, int ny, int nz,
+                                                          int svx, int svy, int svz, float* __restrict__ out_min,
+                                                          float* __restrict__ out_max, float* __restrict__ out_avg,
+                                                          uint8_t* __restrict__ out_occ) {
+    constexpr int SIDE = 8 + 2 * HALO;
+    const int lane = threadIdx.x & 31;
+    const int runs = (svx + 31) / 32;
+    const long run = (long)blockIdx.x * 4 + (threadIdx.x >> 5);  // x run fastest, then y, then z
+    if (run >= (long)runs * svy * svz) return;
+    const int bx = (int)(run % runs) * 32 + lane, by = (int)(run / runs % svy), bz = (int)(run / runs / svy);
+    const int x0 = bx * 8;
+    const bool a_ok = x0 < nx, b_ok = x0 + 4 < nx;  // nx is a multiple of 4
+    const int xe = lane == 0 ? x0 - 1 : x0 + 8;     // the halo voxel an end lane loads itself
+    const bool e_ok = HALO && (lane == 0 || lane == 31) && xe >= 0 && xe < nx;
+    float lo = 3.402823466e+38f, hi = -3.402823466e+38f, sum = 0.0f;
+    for (int p = 0; p < SIDE; ++p) {
+        const int z = bz * 8 - HALO + p;
+        float4 a[SIDE], b[SIDE];
+        float e[SIDE];
+#pragma unroll
+        for (int r = 0; r < SIDE; ++r) {
+            const int y = by * 8 - HALO + r;
+            const bool ok = z >= 0 && z < nz && y >= 0 && y < ny;
+            const float* row = dens + ((size_t)(ok ? z : 0) * ny + (ok ? y : 0)) * nx;
+            a[r] = ok && a_ok ? __ldg(reinterpret_cast<const float4*>(row + x0)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            b[r] = ok && b_ok ? __ldg(reinterpret_cast<const float4*>(row + x0 + 4)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (HALO) e[r] = ok && e_ok ? __ldg(row + xe) : 0.0f;
+        }
+#pragma unroll
+        for (int r = 0; r < SIDE; ++r) {
+            auto add = [&](float v) {
+                lo = fminf(lo, v);
+                hi = fmaxf(hi, v);
+                sum += v;
+            };
+            float left = 0.0f, right = 0.0f;
+            if (HALO) {
+                left = __shfl_up_sync(0xffffffffu, b[r].w, 1);
+                right = __shfl_down_sync(0xffffffffu, a[r].x, 1);
+                if (lane == 0) left = e[r];
+                if (lane == 31) right = e[r];
+                add(left);
+            }
+            add(a[r].x);
+            add(a[r].y);
+            add(a[r].z);
+            add(a[r].w);
+            add(b[r].x);
+            add(b[r].y);
+            add(b[r].z);
+            add(b[r].w);
+            if (HALO) add(right);
+        }
+    }
+    if (bx >= svx) return;
+    const int idx = (bz * svy + by) * svx + bx;
+    const float avg = sum / (float)(SIDE * SIDE * SIDE);
+    if ((nx % 8 != 0 && bx == svx - 1) || (ny % 8 != 0 && by == svy - 1) || (nz % 8 != 0 && bz == svz - 1)) {
+        lo = 0.0f;
+    }
+    out_min[idx] = lo;
+    out_max[idx] = hi;
+    if (out_avg) out_avg[idx] = avg;
+    if (out_occ) out_occ[idx] = hi < 1e-5f ? 0 : 1;
+}
+
 // Residual-ratio-tracking control and residual extinctions (SuperVoxelGrid.cpp:218-256):
 // mu_r_bar = max(mu_max - mu_min, 0.1), mu_c = clamp(mu_min + mu_r_bar * gamma^(1/(D mu_r_bar) - 1),
 // mu_min, mu_avg) with gamma = 2, D = sqrt(3) * sv.
@@ -525,6 +597,13 @@ cudaError_t launch_fbm(float* out, int nx, int ny, int nz, const int* perm512, c
 
 cudaError_t launch_supervoxel_stats(const float* dens, int nx, int ny, int nz, int sv, int svx, int svy, int svz,
                                     int halo, float* mn, float* mx, float* avg, uint8_t* occ, cudaStream_t s) {
+    if (sv == 8 && nx % 4 == 0 && reinterpret_cast<uintptr_t>(dens) % 16 == 0) {  // whole 16-byte words
+        const long runs = (long)((svx + 31) / 32) * svy * svz;
+        auto kernel = halo ? supervoxel8_kernel<1> : supervoxel8_kernel<0>;
+        kernel<<<(unsigned)((runs + 3) / 4), 128, 0, s>>>(dens, nx, ny, nz, svx, svy, svz, mn, mx, avg, occ);
+        count_launches(1);
+        return cudaGetLastError();
+    }
     int total = svx * svy * svz;
     supervoxel_stats_kernel<<<(total + 127) / 128, 128, 0, s>>>(dens, nx, ny, nz, sv, svx, svy, svz, halo, mn, mx,
                                                                 avg, occ);

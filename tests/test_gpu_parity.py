@@ -71,6 +71,15 @@ def test_supervoxel_grid_bit_exact(core, shape, sv, halo):
     assert np.allclose(got[0::2], ref[0::2], rtol=2e-7, atol=0)
 
 
+@pytest.mark.parametrize("halo", [0, 1])
+@pytest.mark.parametrize("shape,sv", [((17, 10, 264), 8), ((8, 7, 4), 8), ((9, 8, 256), 8), ((9, 8, 260), 8),
+                                      ((24, 31, 516), 8), ((9, 8, 257), 8), ((8, 8, 8), 7)])
+def test_supervoxel_runs_bit_exact(core, shape, sv, halo):
+    """Runs of 32 supervoxels of 8 voxels: ragged ends, less than a supervoxel, whole and barely begun runs; rows
+    that are not whole 16-byte words and other sizes, which one thread a supervoxel sums."""
+    test_supervoxel_grid_bit_exact(core, shape, sv, halo)
+
+
 @pytest.mark.parametrize("key", sorted(__import__("tests.harness", fromlist=["_"]).supervoxel_golden()))
 def test_supervoxel_grid_matches_reference_builder(core, key):
     """The core's supervoxel builders against SuperVoxelGrid.cpp compiled unmodified (fixture
