@@ -205,6 +205,44 @@ __device__ __forceinline__ void pixel_coords(int p, int h, int w, int& n, int& y
     n = t / h;
 }
 
+// 16 output channels from co of pixel p: the split's raw sums, or bias, ReLU, mask and store
+__device__ __forceinline__ void conv_store(const ConvArgs& a, int P, int p, int co, float (&v)[16]) {
+    if (a.partial) {  // split-K: raw sums, finished by conv_finalize_kernel
+        float4* dst = reinterpret_cast<float4*>(a.partial + ((size_t)blockIdx.z * P + p) * a.cout + co);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+        return;
+    }
+    if (a.bias) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] += a.bias[co + i];
+    }
+    if (a.relu) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
+    }
+    if (a.mask) {
+        const uint4* mp = reinterpret_cast<const uint4*>(a.mask + (size_t)p * a.cout + co);
+        const uint4 m4[2] = {mp[0], mp[1]};
+        const bf16* mb = reinterpret_cast<const bf16*>(m4);
+#pragma unroll
+        for (int i = 0; i < 16; ++i) v[i] = __bfloat162float(mb[i]) > 0.0f ? v[i] : 0.0f;
+    }
+    if (a.out_f32) {
+        float4* dst = reinterpret_cast<float4*>(static_cast<float*>(a.y) + (size_t)p * a.cout + co);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
+    } else {
+        uint4 o[2];
+        __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(o);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) ob[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<bf16*>(a.y) + (size_t)p * a.cout + co);
+        dst[0] = o[0];
+        dst[1] = o[1];
+    }
+}
+
 template <int MODE, int kStages>
 __global__ void __launch_bounds__(kThreads) conv_tile_kernel(const ConvArgs a) {
     extern __shared__ __align__(1024) uint8_t smem[];
@@ -431,41 +469,7 @@ __global__ void __launch_bounds__(kThreads) conv_tile_kernel(const ConvArgs a) {
             if (MODE == kConv) {
                 const int p = m0 + r;
                 if (p >= P) continue;
-                if (a.partial) {  // split-K: raw sums, finished by conv_finalize_kernel
-                    float4* dst = reinterpret_cast<float4*>(a.partial + ((size_t)blockIdx.z * P + p) * a.cout + co);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i)
-                        dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                    continue;
-                }
-                if (a.bias) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] += a.bias[co + i];
-                }
-                if (a.relu) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = fmaxf(v[i], 0.0f);
-                }
-                if (a.mask) {
-                    const uint4* mp = reinterpret_cast<const uint4*>(a.mask + (size_t)p * a.cout + co);
-                    const uint4 m4[2] = {mp[0], mp[1]};
-                    const bf16* mb = reinterpret_cast<const bf16*>(m4);
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) v[i] = __bfloat162float(mb[i]) > 0.0f ? v[i] : 0.0f;
-                }
-                if (a.out_f32) {
-                    float4* dst = reinterpret_cast<float4*>(static_cast<float*>(a.y) + (size_t)p * a.cout + co);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) dst[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                } else {
-                    uint4 o[2];
-                    __nv_bfloat162* ob = reinterpret_cast<__nv_bfloat162*>(o);
-#pragma unroll
-                    for (int i = 0; i < 8; ++i) ob[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
-                    uint4* dst = reinterpret_cast<uint4*>(static_cast<bf16*>(a.y) + (size_t)p * a.cout + co);
-                    dst[0] = o[0];
-                    dst[1] = o[1];
-                }
+                conv_store(a, P, p, co, v);
             } else {
                 const int m = m0 + r;
                 if (m >= M) continue;
@@ -1387,6 +1391,164 @@ __global__ void __launch_bounds__(kStackThreads, 2)
     tc_fence_before();
     __syncthreads();
     if (fail_any && tid == 0 && a.err) atomicExch(a.err, (int)VPT_ERR_ITER_LIMIT);
+    if (warp == 1) {
+        tc_fence_after();
+        tmem_dealloc(tmem, (uint32_t)a.tmem_cols);
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// the convolution on boxes of 128 pixels (TMA-fed tiles)
+// ---------------------------------------------------------------------------------------------
+// conv_tile_kernel's tiles (128 pixels x up to 256 output channels a CTA, K split over blockIdx.z for small grids) for
+// images whose 128 consecutive pixels are a box: widths that divide 128 (whole rows, whole images where they are
+// smaller) and multiples of 128.  A stage is one tap and up to 64 input channels: the box moved by (dx, dy), whose
+// pixels outside the image arrive as zeros, and the tap's weights, both loaded by the tensor-memory-access unit
+// into K-major swizzled lines of `cw` channels, four stages ahead; the gather kernel's threads compute 64 addresses
+// and copies each a stage and meet at a barrier for it.
+// Warps: 0 loads, 1 issues, 2-5 the epilogue.  Every wait is bounded, as in conv_ws_kernel.
+//   us, gather kernel / here: 96 -> 96 8 images of 64 x 64 33.5 / 15.6, 224 -> 96 71 / 23, 96 -> 224 80 / 31; 128 -> 128
+// 8 images of 16 x 16 17.3 / 13.1, one of 4 x 4 12.7 / 8.2; 224 -> 96 one image of 128 x 128 61 / 15.  Bound: the stages' bytes
+// from L2 (28 KB for 96 channels) for large grids, the latency of a tile's serial stages for small ones.
+constexpr int kBoxThreads = 192;
+constexpr int kBoxStages = 4;
+
+struct BoxArgs {
+    ConvArgs c;
+    int cw;              // channels of a stage: 64, 32 or 16 (the last stage of a tap may hold fewer)
+    int bh, bn;          // rows and images of a box
+};
+
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], "
+        "[%5];\n" ::"r"(dst),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(bar)
+        : "memory");
+}
+
+__global__ void __launch_bounds__(kBoxThreads)
+    conv_box_kernel(const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap wmap,
+                    const __grid_constant__ BoxArgs b) {
+    extern __shared__ __align__(1024) uint8_t smem[];
+    __shared__ uint64_t full[kBoxStages], empty[kBoxStages], done_bar;
+    __shared__ uint32_t tmem_slot;
+    __shared__ int fail_any;
+    const ConvArgs& a = b.c;
+    const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
+    const int P = a.n * a.h * a.w_, n0 = blockIdx.y * a.n_tile;
+    const int chunks = (a.cin + b.cw - 1) / b.cw;
+    int first = 0, nk = 9 * chunks;
+    if (a.ksplit > 1) {
+        const int per = (nk + a.ksplit - 1) / a.ksplit;
+        first = blockIdx.z * per;
+        nk = max(0, min(nk, first + per) - first);
+    }
+    const uint32_t a_bytes = (uint32_t)(kBM * b.cw * 2), b_bytes = (uint32_t)(a.n_tile * b.cw * 2);
+    const uint32_t stage_bytes = a_bytes + ((b_bytes + 1023u) & ~1023u);
+    const uint32_t sbase = smem_u32(smem);
+    if (tid == 0) {
+        for (int k = 0; k < kBoxStages; ++k) {
+            mbar_init(smem_u32(&full[k]), 1);
+            mbar_init(smem_u32(&empty[k]), 1);
+        }
+        mbar_init(smem_u32(&done_bar), 1);
+        fail_any = 0;
+        fence_mbar_init();
+    }
+    if (warp == 1) tmem_alloc(smem_u32(&tmem_slot), (uint32_t)a.tmem_cols);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const uint32_t tmem = __shfl_sync(0xffffffffu, tmem_slot, 0);
+    bool fail = false;
+
+    if (warp == 0) {
+        if (lane == 0) {
+            int img, y0, x0;
+            pixel_coords((int)blockIdx.x * kBM, a.h, a.w_, img, y0, x0);
+            int slot = 0, issued = 0;
+            uint32_t phase = 0;
+            int tap = first / chunks, chunk = first - tap * chunks;
+            for (int k = 0; k < nk; ++k) {
+                if (!mbar_wait(smem_u32(&empty[slot]), phase ^ 1u)) {
+                    fail = true;
+                    break;
+                }
+                const uint32_t dst = sbase + (uint32_t)slot * stage_bytes, fb = smem_u32(&full[slot]);
+                mbar_arrive_expect_tx(fb, a_bytes + b_bytes);
+                const int dy = tap / 3;
+                tma_load_4d(dst, &xmap, chunk * b.cw, x0 + tap - 3 * dy - 1, y0 + dy - 1, img, fb);
+                tma_load_3d(dst + a_bytes, &wmap, chunk * b.cw, tap, n0, fb);
+                ++issued;
+                if (++chunk == chunks) {
+                    chunk = 0;
+                    ++tap;
+                }
+                if (++slot == kBoxStages) {
+                    slot = 0;
+                    phase ^= 1u;
+                }
+            }
+            // the last loads (one per slot at most) have landed before the CTA can exit
+            for (int k = 1; k <= min(issued, kBoxStages); ++k) {
+                int q = slot - k;
+                uint32_t ph = phase;
+                if (q < 0) {
+                    q += kBoxStages;
+                    ph ^= 1u;
+                }
+                if (!mbar_wait(smem_u32(&full[q]), ph)) fail = true;
+            }
+        }
+    } else if (warp == 1) {
+        const uint32_t idesc = instr_desc(kBM, a.n_tile, 0, 0), hi = a_hi_of(b.cw), lbo = 1u << 16;
+        int slot = 0, chunk = first % chunks;
+        uint32_t phase = 0;
+        for (int k = 0; k < nk; ++k) {
+            const bool ok = mbar_wait(smem_u32(&full[slot]), phase);
+            if (!__all_sync(0xffffffffu, ok)) {
+                fail = true;
+                break;
+            }
+            tc_fence_after();
+            if (elect_one()) {
+                const uint32_t sA = (sbase + (uint32_t)slot * stage_bytes) >> 4;
+                const uint32_t al = lbo + sA, bl = lbo + sA + (a_bytes >> 4);
+                const int steps = min(b.cw, a.cin - chunk * b.cw) / 16;
+                for (int j = 0; j < steps; ++j)
+                    mma_bf16_halves(tmem, al + 2u * (uint32_t)j, hi, bl + 2u * (uint32_t)j, hi, idesc,
+                                    (k > 0 || j > 0) ? 1u : 0u);
+                mma_commit(smem_u32(&empty[slot]));
+            }
+            __syncwarp();
+            if (++chunk == chunks) chunk = 0;
+            if (++slot == kBoxStages) {
+                slot = 0;
+                phase ^= 1u;
+            }
+        }
+        // every MMA issued has completed before TMEM is read or released
+        if (elect_one()) mma_commit(smem_u32(&done_bar));
+        __syncwarp();
+        if (!mbar_wait(smem_u32(&done_bar), 0)) fail = true;
+    }
+    if (fail) atomicOr(&fail_any, 1);
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp >= 2 && !fail_any) {
+        const int q = warp & 3, p = (int)blockIdx.x * kBM + q * 32 + lane;
+        const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+        for (int c0 = 0; c0 < a.n_tile; c0 += 16) {
+            float v[16] = {};  // an empty K range contributes zeros
+            if (nk > 0) tmem_ld16(trow + (uint32_t)c0, v);  // whole warp, uniform
+            if (p < P && n0 + c0 < a.cout) conv_store(a, P, p, n0 + c0, v);
+        }
+    }
+    if (fail_any && tid == 0 && a.err) atomicExch(a.err, (int)VPT_ERR_ITER_LIMIT);
+    tc_fence_before();
+    __syncthreads();
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem, (uint32_t)a.tmem_cols);
@@ -2781,6 +2943,50 @@ cudaError_t launch_stack(StripArgs a, int co0, int cout, int cout_total, cudaStr
     return cudaGetLastError();
 }
 
+// the box of 128 consecutive pixels of an image batch: rows and images, or false where they are not one
+inline bool conv_box(int n, int h, int w, int& bh, int& bn) {
+    bh = bn = 1;
+    if (w % kBM == 0) return true;
+    if (kBM % w) return false;
+    const int rows = kBM / w;
+    bh = std::min(rows, h);
+    bn = rows / bh;
+    return h % bh == 0 && rows % bh == 0;
+}
+
+cudaError_t launch_box(const ConvArgs& a, int bh, int bn, dim3 grid, cudaStream_t s) {
+    EncodeTiledFn fn = encode_tiled();
+    if (!fn) return cudaErrorInvalidValue;
+    BoxArgs b{};
+    b.c = a;
+    b.bh = bh;
+    b.bn = bn;
+    b.cw = a.cin <= 16 ? 16 : (a.cin <= 32 ? 32 : 64);
+    const CUtensorMapSwizzle sz = b.cw == 64 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                             : (b.cw == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
+    const cuuint64_t c = (cuuint64_t)a.cin, w = (cuuint64_t)a.w_, h = (cuuint64_t)a.h;
+    const cuuint64_t xdims[4] = {c, w, h, (cuuint64_t)a.n}, xstr[3] = {c * 2, w * c * 2, h * w * c * 2};
+    const cuuint32_t xbox[4] = {(cuuint32_t)b.cw, (cuuint32_t)std::min(a.w_, kBM), (cuuint32_t)bh, (cuuint32_t)bn};
+    const cuuint64_t wdims[3] = {c, 9, (cuuint64_t)a.cout}, wstr[2] = {c * 2, 9 * c * 2};
+    const cuuint32_t wbox[3] = {(cuuint32_t)b.cw, 1, (cuuint32_t)a.n_tile};
+    const cuuint32_t one[4] = {1, 1, 1, 1};
+    CUtensorMap xmap, wmap;
+    auto encode = [&](CUtensorMap* m, int rank, const bf16* p, const cuuint64_t* dims, const cuuint64_t* str,
+                      const cuuint32_t* box) {
+        return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, rank, const_cast<bf16*>(p), dims, str, box, one,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, sz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!encode(&xmap, 4, a.x, xdims, xstr, xbox) || !encode(&wmap, 3, a.w, wdims, wstr, wbox))
+        return cudaErrorInvalidValue;
+    const size_t smem = (size_t)kBoxStages * ((size_t)kBM * b.cw * 2 + ((size_t)a.n_tile * b.cw * 2 + 1023) / 1024 * 1024);
+    const cudaError_t e = cudaFuncSetAttribute(conv_box_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    conv_box_kernel<<<grid, kBoxThreads, smem, s>>>(xmap, wmap, b);
+    count_launches(1);
+    return cudaGetLastError();
+}
+
 static int g_strip_kernel = 0;  // 0: warp-specialised (TMA) strips, 1: the cp.async strip kernel
 
 cudaError_t launch_strip(const ConvArgs& c, int groups, int chunk, cudaStream_t s) {
@@ -2885,7 +3091,9 @@ VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, cons
     const unsigned gx = (unsigned)((P + kBM - 1) / kBM), gy = (unsigned)((cout + a.n_tile - 1) / a.n_tile);
     // small grids (the deep levels): split the K stages over more CTAs, raw fp32 sums finished by
     // conv_finalize_kernel in a fixed order
-    const int nk = (9 * cin + kBK - 1) / kBK;
+    int bh = 1, bn = 1;
+    const bool box = !g_force_gather && aligned && reinterpret_cast<uintptr_t>(w) % 16 == 0 && conv_box(n, h, width, bh, bn);
+    const int nk = box ? 9 * ((cin + kBK - 1) / kBK) : (9 * cin + kBK - 1) / kBK;
     const int sms = sm_count();
     const long tiles = (long)gx * gy;
     int ksplit = 1;
@@ -2894,13 +3102,16 @@ VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, cons
         ksplit = (int)std::max<long>(1, std::min<long>(std::min<long>(8, (2L * sms + tiles - 1) / tiles), nk / 2));
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     if (ksplit == 1)
-        return launch_tile<kConv>(a, dim3(gx, gy, 1), s) == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
+        return (box ? launch_box(a, bh, bn, dim3(gx, gy, 1), s) : launch_tile<kConv>(a, dim3(gx, gy, 1), s)) == cudaSuccess
+                   ? VPT_OK
+                   : VPT_ERR_CUDA;
     float* part = nullptr;
     if (vpt::scratch_alloc(reinterpret_cast<void**>(&part), (size_t)ksplit * P * cout * sizeof(float), s) != cudaSuccess)
         return VPT_ERR_OOM;
     a.ksplit = ksplit;
     a.partial = part;
-    cudaError_t e = launch_tile<kConv>(a, dim3(gx, gy, (unsigned)ksplit), s);
+    const dim3 grid(gx, gy, (unsigned)ksplit);
+    cudaError_t e = box ? launch_box(a, bh, bn, grid, s) : launch_tile<kConv>(a, grid, s);
     if (e == cudaSuccess) {
         conv_finalize_kernel<<<grid_for(P * (cout / 4), 256), 256, 0, s>>>(part, ksplit, P, cout, bias,
                                                                           static_cast<const bf16*>(mask), relu,

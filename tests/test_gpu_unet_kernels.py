@@ -236,6 +236,14 @@ EDGE_CASES = [
     (1, 5, 130, 32, 144),
     (2, 5, 150, 96, 224),
     (1, 128, 128, 96, 96),
+    # boxes of 128 pixels: part of the last box's images, a box a row / rows of one image, split K, two column tiles,
+    # stages of 16, 32 and 64 channels and of less
+    (3, 4, 8, 48, 32),
+    (1, 6, 64, 224, 96),
+    (2, 16, 16, 128, 128),
+    (5, 1, 2, 32, 16),
+    (1, 4, 32, 16, 272),
+    (1, 3, 128, 160, 96),
 ]
 
 
