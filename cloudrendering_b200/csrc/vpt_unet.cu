@@ -24,7 +24,9 @@
 // pass and the bf16 / fp32 store.  Forward and input-gradient tiles have K-major operands (k
 // contiguous: channels of one pixel); the weight-gradient tile has MN-major operands (channels
 // contiguous, pixels along K) and writes per-split fp32 partial sums that the optimiser reduces in a
-// fixed order (deterministic).
+// fixed order (deterministic).  That is conv_tile_kernel, which takes any shape; most layers go through the kernels
+// further down whose operands the tensor-memory-access unit loads: boxes of 128 pixels (conv_box_kernel), row
+// strips (conv_stack_kernel, conv_ws_kernel) and the weight gradient on image rows (wgrad_rows_kernel).
 //
 // Every mbarrier wait is bounded: on expiry the kernel records VPT_ERR_ITER_LIMIT in *err, waits
 // (bounded) for the MMAs it issued, frees its TMEM and returns.
@@ -2836,8 +2838,15 @@ bool ws_config(int cin, int cout, int& per_sm, int& ring) {
 // How the warp-specialised kernels take a layer.  Input channels: one pass where the weights and the rings fit,
 // else up to 4 passes through an fp32 partial, which beat the gather kernel for up to 64 output channels only
 // (measured).  Output channels: conv_stack_kernel for up to 80 of them, in chunks of at most 80 (each launch reads
-// the input again) or all of them in conv_ws_kernel (chunk = 0) beyond.  us, gather or conv_ws / chunks, at 128 pixels
-// a row:
+// the input again) or all of them in conv_ws_kernel (chunk = 0) beyond.
+// Up to two rows of 128 pixels an SM conv_box_kernel takes the layer (groups = 0) where the width is a multiple of 128: every
+// tile has a CTA of its own, while these kernels read three rows for one and start with all nine taps' weights;
+// up to four rows an SM with more than 80 output channels and no half-empty stages.  us, these kernels / boxes:
+//     96 -> 32  128 rows 12.0 / 8.3   256 rows 13.2 / 10.4  512 rows 17.8 / 18.3  1,024 rows 24.1 / 35.1
+//     48 -> 48  128 rows 9.7 / 7.2    256 rows 10.1 / 9.6   512 rows 14.8 / 17.5  1,024 rows 16.9 / 31.7
+//     96 -> 96  128 rows 25.8 / 10.3  256 rows 28.7 / 15.6  512 rows 36.7 / 28.4  1,024 rows 50.1 / 53.6
+//     48 -> 96  256 rows 17.7 / 14.6  512 rows 18.5 / 23.1;  16 -> 32  256 rows 6.8 / 7.0  512 rows 7.8 / 9.8
+// us, gather or conv_ws / chunks, at 128 pixels a row:
 //   conv_ws does not fit (gather, whose CTAs hold all outputs of 128 pixels)   chunks from 64 rows a chunk
 //     96 -> 96    64 rows 24.2 / 25.4   128 rows 29.4 / 25.7   512 rows 64.7 / 36.1   4,096 rows 458 / 117
 //     96 -> 224  128 rows 40.4 / 53.1   256 rows 78.7 / 57.7   512 rows 155 / 73.7    4,096 rows 1097 / 211
@@ -2852,6 +2861,11 @@ inline StackPlan stack_plan(int n_img, int h, int width, int cin, int cout, bool
     StackPlan p;
     if (width < kBM || cout > 256) return p;
     const long rows = (long)n_img * ((width + kBM - 1) / kBM) * h;
+    if (!any && width % kBM == 0) {
+        const long sms = sm_count();
+        if (rows <= 2 * sms && cin > 16) return p;
+        if (rows <= 4 * sms && cout > kStackMaxCout && cin % 32 == 0) return p;
+    }
     for (int g = 1; g <= 4; ++g) {
         if (g > 1 && cout > 64 && !any) return p;
         const int cg = (cin / 16 + g - 1) / g * 16;

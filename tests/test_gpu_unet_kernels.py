@@ -244,6 +244,7 @@ EDGE_CASES = [
     (5, 1, 2, 32, 16),
     (1, 4, 32, 16, 272),
     (1, 3, 128, 160, 96),
+    (2, 5, 256, 64, 48),
 ]
 
 
