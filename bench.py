@@ -1114,7 +1114,7 @@ def run_reference(args):
 
 def profile_trace(spp):
     """Two launches of the delta tracker on the bench scene (1 frame, then `spp` frames) for ncu:
-    `ncu -k regex:trace_refill -s 1 -c 1 ... python bench.py --profile-trace SPP` captures the second."""
+    `ncu -k regex:trace_event -s 1 -c 1 ... python bench.py --profile-trace SPP` captures the second."""
     import torch
     from cloudrendering_b200 import vpt, _lib
     torch.cuda.set_device(0)

@@ -1410,8 +1410,8 @@ __global__ void __launch_bounds__(kStackThreads, 2)
 // and copies each a stage and meet at a barrier for it.
 // Warps: 0 loads, 1 issues, 2-5 the epilogue.  Every wait is bounded, as in conv_ws_kernel.
 //   us, gather kernel / here: 96 -> 96 8 images of 64 x 64 33.5 / 15.6, 224 -> 96 71 / 23, 96 -> 224 80 / 31; 128 -> 128
-// 8 images of 16 x 16 17.3 / 13.1, one of 4 x 4 12.7 / 8.2; 224 -> 96 one image of 128 x 128 61 / 15.  Bound: the stages' bytes
-// from L2 (28 KB for 96 channels) for large grids, the latency of a tile's serial stages for small ones.
+// 8 images of 16 x 16 17.3 / 13.1, one of 4 x 4 12.7 / 8.2; 224 -> 96 one image of 128 x 128 61 / 15.  Bound: the
+// stages' bytes from L2 (28 KB for 96 channels) for large grids, the latency of a tile's serial stages for small ones.
 constexpr int kBoxThreads = 192;
 constexpr int kBoxStages = 4;
 
@@ -1972,9 +1972,23 @@ __global__ void bias_grad_kernel(const bf16* __restrict__ dy, float* __restrict_
     const int lane_c = threadIdx.x % c8, group = threadIdx.x / c8, groups = blockDim.x / c8;
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
     if (group < groups) {
-        for (long p = (long)blockIdx.x * groups + group; p < P; p += (long)gridDim.x * groups) {
+        // eight loads at a time (with one, two blocks an SM keep 8 KB in flight; the sums' order does not change): the
+        // 19 layers of a training step of 8 images of 256 x 256 144 -> 128 us
+        const long step = (long)gridDim.x * groups;
+        const bf16* src = dy + lane_c * 8;
+        long p = (long)blockIdx.x * groups + group;
+        for (; p + 7 * step < P; p += 8 * step) {
+            float f[8][8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) load8(src + (p + u * step) * c, f[u]);
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+                for (int k = 0; k < 8; ++k) acc[k] += f[u][k];
+        }
+        for (; p < P; p += step) {
             float f[8];
-            load8(dy + p * c + lane_c * 8, f);
+            load8(src + p * c, f);
 #pragma unroll
             for (int k = 0; k < 8; ++k) acc[k] += f[k];
         }
@@ -2839,9 +2853,9 @@ bool ws_config(int cin, int cout, int& per_sm, int& ring) {
 // else up to 4 passes through an fp32 partial, which beat the gather kernel for up to 64 output channels only
 // (measured).  Output channels: conv_stack_kernel for up to 80 of them, in chunks of at most 80 (each launch reads
 // the input again) or all of them in conv_ws_kernel (chunk = 0) beyond.
-// Up to two rows of 128 pixels an SM conv_box_kernel takes the layer (groups = 0) where the width is a multiple of 128: every
-// tile has a CTA of its own, while these kernels read three rows for one and start with all nine taps' weights;
-// up to four rows an SM with more than 80 output channels and no half-empty stages.  us, these kernels / boxes:
+// Up to two rows of 128 pixels an SM conv_box_kernel takes the layer (groups = 0) where the width is a multiple of
+// 128: every tile has a CTA of its own, while these kernels read three rows for one and start with all nine taps'
+// weights; up to four rows an SM with more than 80 output channels and no half-empty stages.  us, these / boxes:
 //     96 -> 32  128 rows 12.0 / 8.3   256 rows 13.2 / 10.4  512 rows 17.8 / 18.3  1,024 rows 24.1 / 35.1
 //     48 -> 48  128 rows 9.7 / 7.2    256 rows 10.1 / 9.6   512 rows 14.8 / 17.5  1,024 rows 16.9 / 31.7
 //     96 -> 96  128 rows 25.8 / 10.3  256 rows 28.7 / 15.6  512 rows 36.7 / 28.4  1,024 rows 50.1 / 53.6
@@ -3106,7 +3120,8 @@ VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, cons
     // small grids (the deep levels): split the K stages over more CTAs, raw fp32 sums finished by
     // conv_finalize_kernel in a fixed order
     int bh = 1, bn = 1;
-    const bool box = !g_force_gather && aligned && reinterpret_cast<uintptr_t>(w) % 16 == 0 && conv_box(n, h, width, bh, bn);
+    const bool box = !g_force_gather && aligned && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
+                     conv_box(n, h, width, bh, bn);
     const int nk = box ? 9 * ((cin + kBK - 1) / kBK) : (9 * cin + kBK - 1) / kBK;
     const int sms = sm_count();
     const long tiles = (long)gx * gy;
@@ -3239,7 +3254,8 @@ VptStatus vpt_unet_upcat_grad_lo(const void* d, const void* lo, void* dlo, int n
     if (!d || !lo || !dlo || n <= 0 || h <= 1 || w <= 1 || h % 2 || w % 2 || ca <= 0 || ca % 8 || cs <= 0 ||
         cs % 8)
         return VPT_ERR_ARG;
-    launch_units((long)n * (h / 2) * (w / 2) * (ca / 8), stream, upcat_grad_lo_kernel<uint32_t>, upcat_grad_lo_kernel<unsigned long long>,
+    launch_units((long)n * (h / 2) * (w / 2) * (ca / 8), stream, upcat_grad_lo_kernel<uint32_t>,
+                 upcat_grad_lo_kernel<unsigned long long>,
                  static_cast<const bf16*>(d), static_cast<const bf16*>(lo), static_cast<bf16*>(dlo), n, h, w, ca, cs);
     vpt::count_launches(1);
     return cudaGetLastError() == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
@@ -3251,7 +3267,8 @@ VptStatus vpt_unet_encoder_grad(const void* d_cat, int cat_c, int cat_off, const
         (d_pool && (h % 2 || w % 2)))
         return VPT_ERR_ARG;
     launch_units((long)n * h * w * (c / 8), stream, encoder_grad_kernel<uint32_t>, encoder_grad_kernel<unsigned long long>,
-                 static_cast<const bf16*>(d_cat), cat_c, cat_off, static_cast<const bf16*>(d_pool), static_cast<const bf16*>(e), static_cast<bf16*>(out), n, h, w, c);
+                 static_cast<const bf16*>(d_cat), cat_c, cat_off, static_cast<const bf16*>(d_pool),
+                 static_cast<const bf16*>(e), static_cast<bf16*>(out), n, h, w, c);
     vpt::count_launches(1);
     return cudaGetLastError() == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
 }

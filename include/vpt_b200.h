@@ -503,14 +503,15 @@ VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, cons
 /* Selects the convolution kernels: 0 (default) = by shape (the persistent row-strip kernels for images
  * at least 128 pixels wide where they are measured faster; input channels in up to 4 groups through an
  * fp32 partial allocated on the stream; the weight gradient on image rows for 2,048 pixels and more),
- * 1 = the per-tile gather kernels everywhere, 2 = the row kernels wherever they apply. */
+ * 1 = the per-tile gather kernels everywhere, 2 = the row kernels wherever they apply.  (By default tiles
+ * whose 128 pixels are a box of rows or images are loaded by the tensor-memory-access unit.) */
 VptStatus vpt_unet_set_conv_path(int path);
 /* Row-strip convolution kernel: 0 (default) = warp-specialised (input rows loaded by the tensor-memory-
  * access unit into a ring; up to 80 output channels a launch with the three output rows that read an input
  * row in one MMA, or all of them one row at a time; input channel groups when the weights and the ring do
  * not fit), 1 = the cp.async row-strip kernel. */
 VptStatus vpt_unet_set_strip_kernel(int kind);
-/* K splits of the per-tile gather convolution: 0 (default) = by grid size (grids of at most half an SM wave
+/* K splits of the per-tile convolutions: 0 (default) = by grid size (grids of at most half an SM wave
  * split their K stages over up to 8 CTAs, whose fp32 sums, allocated on the stream, are added in split
  * order before the bias / ReLU / mask epilogue), 1 = never, k > 1 = always k (at most the K stages). */
 VptStatus vpt_unet_set_conv_ksplit(int ksplit);
