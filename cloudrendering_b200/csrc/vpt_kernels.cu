@@ -313,8 +313,8 @@ __global__ void supervoxel_stats_kernel(const float* __restrict__ dens, int nx, 
 // The same numbers for supervoxels of 8 (the default), a warp for 32 of them along x.  A thread's loads above are 8
 // voxels apart, one sector each, and one after the other: 91 us for 256 x 256 x 200 voxels.  Here a lane reads its
 // rows as two 16-byte words, all rows of a z plane at once, and its neighbours' voxels of the halo come by shuffles
-// (the warp's two ends load theirs); every lane still adds its own voxels in z-y-x order.  14 us for those voxels (52 MB, 8 us); copying the
-// planes through shared memory word by word took 89.
+// (the warp's two ends load theirs); every lane still adds its own voxels in z-y-x order.  14 us for those voxels
+// (52 MB, 8 us); copying the planes through shared memory word by word took 89.
 template <int HALO>
 __global__ void __launch_bounds__(128) supervoxel8_kernel(const float* __restrict__ dens, int nx, int ny, int nz,
                                                           int svx, int svy, int svz, float* __restrict__ out_min,

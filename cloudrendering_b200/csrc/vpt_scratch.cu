@@ -3,9 +3,9 @@
 //
 // The device's default pool returns its memory at every synchronisation (release threshold 0), so that the next
 // call maps it again: 0.5 ms of a 1920 x 1080 EAW call that starts on an idle device (0.94 ms; 0.46 ms when calls
-// follow one another, and here either way).  These calls allocate from a pool of their own, one per device, which keeps up to
-// kScratchKeep bytes across synchronisations.  The pool orders reuse between streams and threads by itself; a
-// destroyed context and an allocation that fails for want of memory give it back (scratch_trim).
+// follow one another, and here either way).  These calls allocate from a pool of their own, one per device, which
+// keeps up to kScratchKeep bytes across synchronisations.  The pool orders reuse between streams and threads by
+// itself; a destroyed context and an allocation that fails for want of memory give it back (scratch_trim).
 #include "vpt_scratch.h"
 
 #include <mutex>

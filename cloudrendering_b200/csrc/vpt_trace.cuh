@@ -447,7 +447,9 @@ VPT_DEV void event_loop(const SRC& src, uint64_t total, unsigned long long* work
     // a 512^3 grid 57.6 ms at 2, 56.5 at 3, 59.6 at 4; of a sparse grid 14.6 at 2, 15.5 at 3, 17.2 at 4; next event
     // tracking 23.1 at 1, 22.6 at 2, 25.4 at 3)
     constexpr int kEventShare = kNee ? 2 : (!kDec && GRID == kNanoVdb ? 2 : 3);
-    // collisions a shadow ray goes ahead of its lookups (a trilinear lookup is eight fetches)
+    // collisions a shadow ray goes ahead of its lookups (a trilinear lookup is eight fetches); measured, stochastic
+    // lookups of a 512^3 grid: 23.6 ms at 1, 22.5 at 2, 19.1 at 4, 19.4 at 6 (events one by one 26.4); 256^2 paths of a
+    // 128^3 grid 12.7 / 10.0 / 9.0 / 9.2 ms
     constexpr int kAhead = kNee ? (INTERP == kTrilinear ? 2 : 4) : 1;
     static_assert(kEventShare >= 1 && kEventShare <= 8, "0 would never let a lane collide");
     const unsigned FULL = 0xffffffffu;
