@@ -2120,249 +2120,139 @@ __global__ void pack_input_kernel(const float* __restrict__ radiance, const floa
 //   dL/dlogit_j = s_j (g . x_j - g . d),  g_c = 2 (d_c - t_c) / (t_c^2 + eps) * inv_count
 // logits: [P][hc] fp32 (NHWC, hc >= k*k a multiple of 8, channels k*k.. unused, their gradient 0);
 // x, t, out: [n][3][h][w] fp32.  The softmax is recomputed per pass (no per-tap arrays in registers).
-// One block per 64-pixel row segment at a time (grid-stride).  The segment's logits (contiguous in NHWC) are staged in
-// shared memory by asynchronous copies, a warp per pixel row, at a row stride of hc + 4 floats; the KS x (64 + KS - 1)
-// radiance window likewise, with zeros outside the image (an out-of-image tap adds to the normalisation only).
-// Eight lanes take two neighbouring pixels, each lane the kernel rows rl and rl + 8 of both, and combine by
-// shuffles: the logits go to registers once, and a window row of KS + 1 floats, read 8 bytes at a time, serves both
-// pixels (2.6 shared-memory wavefronts a tap; a lane per pixel and row that read the logits for the maximum and again
-// for the exponential took 5).  With the logits in registers their buffer takes the next segment while this one is
-// computed; the window has two buffers, the logit gradients their own, and leave as coalesced bf16 rows.
-// Bank spread: the logit stride is 4 (mod 8) with an odd quotient, so four pairs start 8 banks apart and the eight
-// rows (KS odd) fall on the 8 banks between; the window row length is 8 (mod 16), so the four rows of a half warp
-// start 8 banks apart and its four pairs take 2 banks each.
-// Asynchronous copies by fixed units and columns a thread: by warp rows, with 64-bit divisions a segment, the copies
-// took half of the instructions.  us, a lane per pixel and row / here: 512 x 512 with 13 x 13 taps 82 / 70, 8 images of
-// 256 x 256 with their gradients 303 / 242; 5 x 5 taps 37 / 31.  Bound: instruction issue (nine a tap; 188 MB of
-// logits and radiance would be 28 us).
+// One block per 64-pixel row segment at a time (grid-stride): the segment's logits (contiguous in
+// NHWC) are staged in shared memory by asynchronous copies, a warp per pixel row, at a row stride of
+// hc + 4 floats; the KS x (64 + KS - 1) radiance window likewise, with zeros outside the image (an
+// out-of-image tap adds to the normalisation only).  Four lanes per pixel take the kernel rows
+// sub, sub + 4, ... (columns unrolled: window offsets are immediates) and combine by shuffles.  Bank
+// spread: the logit stride is 4 (mod 8) with an odd quotient, so the warp's 8 pixels start on banks
+// 0, 4, .., 28 and the lanes' rows (KS odd) add 0..3; the window row length is 8 (mod 16), so the
+// lanes' window rows start 8 banks apart.  The logit gradients overwrite the staged logits and leave
+// as coalesced bf16 rows.
 constexpr int kHeadSeg = 64;
 
 __host__ __device__ constexpr int head_window_row(int ks) {  // >= kHeadSeg + ks - 1, = 8 (mod 16)
     return (kHeadSeg + ks - 1 + 7) / 16 * 16 + 8;
 }
 
-// over the lanes of a pixel pair (the eight kernel rows: lane bits 2 .. 4)
-__device__ __forceinline__ float row_sum(float v) {
-    v += __shfl_xor_sync(0xffffffffu, v, 4);
-    v += __shfl_xor_sync(0xffffffffu, v, 8);
-    return v + __shfl_xor_sync(0xffffffffu, v, 16);
-}
-__device__ __forceinline__ float row_max(float v) {
-    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 4));
-    v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 8));
-    return fmaxf(v, __shfl_xor_sync(0xffffffffu, v, 16));
-}
-
-// shared memory of kpn_head_kernel: logits, two radiance windows, the bf16 logit gradients (training only)
-__host__ __device__ constexpr size_t head_smem(int ks, int hc, bool train) {
-    return ((size_t)kHeadSeg * (hc + 4) + 2 * 3 * ks * head_window_row(ks)) * sizeof(float) +
-           (train ? (size_t)kHeadSeg * (hc + 8) * sizeof(bf16) : 0);
+__device__ __forceinline__ float quad_sum(float v) {
+    v += __shfl_xor_sync(0xffffffffu, v, 1);
+    return v + __shfl_xor_sync(0xffffffffu, v, 2);
 }
 
 template <int KS>
-__global__ void __launch_bounds__(256, 2) kpn_head_kernel(const float* __restrict__ logits, int hc,
-                                                          const float* __restrict__ x,
-                                                          const float* __restrict__ target, float* __restrict__ out,
-                                                          bf16* __restrict__ dlogits, float* __restrict__ loss_partial,
-                                                          int n, int h, int w, float eps, float inv_count) {
+__global__ void __launch_bounds__(256) kpn_head_kernel(const float* __restrict__ logits, int hc,
+                                                       const float* __restrict__ x, const float* __restrict__ target,
+                                                       float* __restrict__ out, bf16* __restrict__ dlogits,
+                                                       float* __restrict__ loss_partial, int n, int h, int w,
+                                                       float eps, float inv_count) {
     constexpr int RW = head_window_row(KS), WIN = KS * RW, TAPS = KS * KS, RAD = KS / 2;
-    constexpr int ROWS = (KS + 7) / 8;  // kernel rows of a lane
-    extern __shared__ __align__(16) float hsm[];
-    const int stride = hc + 4, dstride = hc + 8;
+    extern __shared__ float hsm[];
+    const int stride = hc + 4;
     float* lsm = hsm;                       // [kHeadSeg][stride]
-    float* rsm = hsm + kHeadSeg * stride;   // [2][3][KS][RW]
-    bf16* dsm = reinterpret_cast<bf16*>(rsm + 2 * 3 * WIN);  // [kHeadSeg][dstride] (training)
+    float* rsm = hsm + kHeadSeg * stride;   // [3][KS][RW]
     const long plane = (long)h * w;
     const int segs_w = (w + kHeadSeg - 1) / kHeadSeg;
     const long nseg = (long)n * h * segs_w;
-    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-    const int rl = lane >> 2, pl = warp * 8 + (lane & 3) * 2;  // first kernel row, first pixel of the pair
+    const int t = threadIdx.x, pl = t >> 2, sub = t & 3, warp = t >> 5, lane = t & 31;
     const int q4 = hc / 4;
     float local = 0.0f;
-    // the segment's place, moved on by gridDim.x without further divisions
-    struct Place {
-        long b;
-        int y, sx;
-    };
-    auto place = [&](long sg) {
+    for (long sg = blockIdx.x; sg < nseg; sg += gridDim.x) {
+        const int sx = (int)(sg % segs_w);
         const long row = sg / segs_w;
-        return Place{row / h, (int)(row % h), (int)(sg - row * segs_w)};
-    };
-    const Place step = place(gridDim.x);
-    auto advance = [&](Place p) {
-        p.sx += step.sx;
-        p.y += step.y;
-        p.b += step.b;
-        if (p.sx >= segs_w) {
-            p.sx -= segs_w;
-            ++p.y;
-        }
-        if (p.y >= h) {
-            p.y -= h;
-            ++p.b;
-        }
-        return p;
-    };
-    // asynchronous copies of a segment: 16-byte units t, t + 256, ... of its logits, and of the window a column of
-    // one channel a thread
-    const int unit_p = t / q4, unit_c = t - unit_p * q4, unit_dp = 256 / q4, unit_dc = 256 - unit_dp * q4;
-    constexpr int COLS = kHeadSeg + KS - 1;
-    const int wch = t / COLS, wcol = t - wch * COLS;
-    auto stage = [&](const Place& pc, float* win) {
-        const int x0 = pc.sx * kHeadSeg, np = min(kHeadSeg, w - x0);
-        const float4* lg4 = reinterpret_cast<const float4*>(logits + ((pc.b * h + pc.y) * w + x0) * hc) + t;
-        for (int p = unit_p, c = unit_c; p < np; lg4 += 256) {
-            cp_async16_stream(smem_u32(lsm + p * stride + 4 * c), lg4);
-            p += unit_dp;
-            c += unit_dc;
-            if (c >= q4) {
-                c -= q4;
-                ++p;
-            }
-        }
-        if (wch < 3) {
-            const float* xb = x + pc.b * 3 * plane;
-            const int xq = x0 + wcol - RAD;
-            const bool col_ok = xq >= 0 && xq < w;
-            const float* src = xb + wch * plane + (long)(pc.y - RAD) * w + xq;
-            uint32_t dst = smem_u32(win + wch * WIN + wcol);
-#pragma unroll
-            for (int r = 0; r < KS; ++r, src += w, dst += 4 * RW) {
-                const bool v = col_ok && pc.y + r >= RAD && pc.y + r < h + RAD;
-                cp_async4(dst, v ? src : xb, v);
-            }
-        }
-    };
-    if (target)  // the channels past the taps have no gradient
-        for (int k = t; k < kHeadSeg * (hc - TAPS); k += 256)
-            dsm[k / (hc - TAPS) * dstride + TAPS + k % (hc - TAPS)] = __float2bfloat16_rn(0.0f);
-    Place at = place(blockIdx.x);
-    if (blockIdx.x < nseg) stage(at, rsm);
-    cp_async_commit();
-    int buf = 0;
-    for (long sg = blockIdx.x; sg < nseg; sg += gridDim.x, buf ^= 1) {
-        const int y = at.y, x0 = at.sx * kHeadSeg, np = min(kHeadSeg, w - x0);
-        const long b = at.b;
+        const int y = (int)(row % h);
+        const long b = row / h;
+        const int x0 = sx * kHeadSeg, np = min(kHeadSeg, w - x0);
         const long p0 = (b * h + y) * w + x0;
+        __syncthreads();  // the previous segment is done with shared memory
+        // asynchronous copies: every copy of the block is in flight before the first wait
+        const float4* lg4 = reinterpret_cast<const float4*>(logits + p0 * hc);
+        for (int p = warp; p < np; p += 8) {
+            const float4* src = lg4 + (long)p * q4;
+            const uint32_t dst = smem_u32(lsm + p * stride);
+            for (int c = lane; c < q4; c += 32) cp_async16_stream(dst + 16 * c, src + c);
+        }
+        const float* xb = x + b * 3 * plane;
+        for (int rr = warp; rr < 3 * KS; rr += 8) {  // window row rr = c * KS + r
+            const int c = rr / KS, r = rr - c * KS;
+            const int yy = y + r - RAD;
+            const bool row_ok = yy >= 0 && yy < h;
+            const float* src = xb + c * plane + (long)(row_ok ? yy : 0) * w;
+            const uint32_t dst = smem_u32(rsm + rr * RW);
+            for (int xx = lane; xx < kHeadSeg + KS - 1; xx += 32) {
+                const int xq = x0 + xx - RAD;
+                const bool v = row_ok && xq >= 0 && xq < w;
+                cp_async4(dst + 4 * xx, v ? src + xq : xb, v);
+            }
+        }
+        cp_async_commit();
         cp_async_wait<0>();
         __syncthreads();
-        float e[2][ROWS][KS];  // the lane's logits, then their exponentials
-        float mx[2] = {-INFINITY, -INFINITY};
+        const bool pv = pl < np;
+        const float* lp = lsm + pl * stride;
+        const float* rp = rsm + pl;
+        float mx = -INFINITY;
+        if (pv)
+            for (int r = sub; r < KS; r += 4) {
 #pragma unroll
-        for (int i = 0; i < 2; ++i)
-#pragma unroll
-            for (int q = 0; q < ROWS; ++q) {
-                const int r = rl + 8 * q;
-                if (r >= KS) continue;
-                const float* lp = lsm + (pl + i) * stride + r * KS;
+                for (int c = 0; c < KS; ++c) mx = fmaxf(mx, lp[r * KS + c]);
+            }
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+        mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+        float sum = 0.0f, d0 = 0.0f, d1 = 0.0f, d2 = 0.0f;
+        if (pv)
+            for (int r = sub; r < KS; r += 4) {
+                const float* lr = lp + r * KS;
+                const float* xr = rp + r * RW;
 #pragma unroll
                 for (int c = 0; c < KS; ++c) {
-                    e[i][q][c] = lp[c];
-                    mx[i] = fmaxf(mx[i], e[i][q][c]);
+                    const float e = __expf(lr[c] - mx);
+                    sum += e;
+                    d0 += e * xr[c];
+                    d1 += e * xr[WIN + c];
+                    d2 += e * xr[2 * WIN + c];
                 }
             }
-        __syncthreads();  // the logits are in registers, and the other window is done with
-        at = advance(at);
-        if (sg + gridDim.x < nseg) stage(at, rsm + (buf ^ 1) * 3 * WIN);
-        cp_async_commit();
-        const float* rp = rsm + buf * 3 * WIN + pl;
-        float sum[2] = {0.0f, 0.0f}, d[2][3] = {};
-        mx[0] = row_max(mx[0]);
-        mx[1] = row_max(mx[1]);
-#pragma unroll
-        for (int q = 0; q < ROWS; ++q) {
-            const int r = rl + 8 * q;
-            if (r >= KS) continue;
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-                for (int c = 0; c < KS; ++c) {
-                    e[i][q][c] = __expf(e[i][q][c] - mx[i]);
-                    sum[i] += e[i][q][c];
-                }
-#pragma unroll
-            for (int ch = 0; ch < 3; ++ch) {
-                float v[KS + 1];
-                const float2* src = reinterpret_cast<const float2*>(rp + ch * WIN + r * RW);
-#pragma unroll
-                for (int c = 0; c < (KS + 1) / 2; ++c) {
-                    const float2 u = src[c];
-                    v[2 * c] = u.x;
-                    v[2 * c + 1] = u.y;
-                }
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-#pragma unroll
-                    for (int c = 0; c < KS; ++c) d[i][ch] += e[i][q][c] * v[c + i];
-            }
-        }
-        float inv[2];
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-            inv[i] = 1.0f / row_sum(sum[i]);
-#pragma unroll
-            for (int ch = 0; ch < 3; ++ch) d[i][ch] = row_sum(d[i][ch]) * inv[i];
-        }
-        const long q0 = (long)y * w + x0 + pl;
-        if (out) {  // lane rows 0 .. 5: channel rl / 2 of pixel rl % 2
-            const int ch = rl >> 1, i = rl & 1;
-            const float v0 = ch == 0 ? d[0][0] : (ch == 1 ? d[0][1] : d[0][2]);
-            const float v1 = ch == 0 ? d[1][0] : (ch == 1 ? d[1][1] : d[1][2]);
-            if (ch < 3 && pl + i < np) out[(b * 3 + ch) * plane + q0 + i] = i ? v1 : v0;
-        }
+        sum = quad_sum(sum);
+        d0 = quad_sum(d0);
+        d1 = quad_sum(d1);
+        d2 = quad_sum(d2);
+        const float inv = 1.0f / sum;
+        const float d[3] = {d0 * inv, d1 * inv, d2 * inv};
+        const long q = (long)y * w + x0 + pl;
+        if (pv && out && sub < 3) out[(b * 3 + sub) * plane + q] = sub == 0 ? d[0] : (sub == 1 ? d[1] : d[2]);
         if (target) {
-            float g[2][3], gd[2];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const bool pv = pl + i < np;
-#pragma unroll
+            float g[3] = {0.0f, 0.0f, 0.0f};
+            if (pv) {
                 for (int c = 0; c < 3; ++c) {
-                    const float tg = pv ? target[(b * 3 + c) * plane + q0 + i] : 0.0f;
+                    const float tg = target[(b * 3 + c) * plane + q];
                     const float den = tg * tg + eps;
-                    const float err = d[i][c] - tg;
-                    if (pv && rl == 0) local += err * err / den * inv_count;
-                    g[i][c] = 2.0f * err / den * inv_count;
+                    const float e = d[c] - tg;
+                    if (sub == 0) local += e * e / den * inv_count;
+                    g[c] = 2.0f * e / den * inv_count;
                 }
-                // summed like gx below: the two cancel exactly where one tap has all the weight
-                gd[i] = fmaf(g[i][2], d[i][2], fmaf(g[i][1], d[i][1], g[i][0] * d[i][0]));
             }
+            const float gd = g[0] * d[0] + g[1] * d[1] + g[2] * d[2];
+            float* lw = lsm + pl * stride;
+            for (int r = sub; r < KS; r += 4) {
+                float* lr = lw + r * KS;
+                const float* xr = rp + r * RW;
 #pragma unroll
-            for (int q = 0; q < ROWS; ++q) {
-                const int r = rl + 8 * q;
-                if (r >= KS) continue;
-                float gx[2][KS] = {};
-#pragma unroll
-                for (int ch = 0; ch < 3; ++ch) {
-                    float v[KS + 1];
-                    const float2* src = reinterpret_cast<const float2*>(rp + ch * WIN + r * RW);
-#pragma unroll
-                    for (int c = 0; c < (KS + 1) / 2; ++c) {
-                        const float2 u = src[c];
-                        v[2 * c] = u.x;
-                        v[2 * c + 1] = u.y;
-                    }
-#pragma unroll
-                    for (int i = 0; i < 2; ++i)
-#pragma unroll
-                        for (int c = 0; c < KS; ++c) gx[i][c] = fmaf(g[i][ch], v[c + i], gx[i][c]);
+                for (int c = 0; c < KS; ++c) {
+                    const float gx = g[0] * xr[c] + g[1] * xr[WIN + c] + g[2] * xr[2 * WIN + c];
+                    lr[c] = pv ? __expf(lr[c] - mx) * inv * (gx - gd) : 0.0f;
                 }
-#pragma unroll
-                for (int i = 0; i < 2; ++i)
-#pragma unroll
-                    for (int c = 0; c < KS; ++c)
-                        dsm[(pl + i) * dstride + r * KS + c] =
-                            __float2bfloat16_rn(e[i][q][c] * inv[i] * (gx[i][c] - gd[i]));
             }
+            for (int j = TAPS + sub; j < hc; j += 4) lw[j] = 0.0f;
             __syncthreads();
-            const int d8 = hc / 8, dp = 256 / d8, dc = 256 - dp * d8;
-            uint4* drow = reinterpret_cast<uint4*>(dlogits + p0 * hc) + t;
-            for (int p = t / d8, c = t - p * d8; p < np; drow += 256) {
-                *drow = *reinterpret_cast<const uint4*>(dsm + p * dstride + 8 * c);
-                p += dp;
-                c += dc;
-                if (c >= d8) {
-                    c -= d8;
-                    ++p;
+            for (int p = warp; p < np; p += 8) {
+                const float* srow = lsm + p * stride;
+                bf16* drow = dlogits + (p0 + p) * hc;
+                for (int c = lane * 8; c < hc; c += 256) {
+                    const float4 u = *reinterpret_cast<const float4*>(srow + c);
+                    const float4 v = *reinterpret_cast<const float4*>(srow + c + 4);
+                    const float f[8] = {u.x, u.y, u.z, u.w, v.x, v.y, v.z, v.w};
+                    store8(drow + c, f);
                 }
             }
         }
@@ -3339,7 +3229,8 @@ VptStatus vpt_unet_kpn_head(const float* logits, int head_channels, int kernel_s
     // row segments, which the blocks stride over)
     const int blocks = grid_for((long)n * h * w, 256);
     const float inv_count = 1.0f / (3.0f * (float)n * (float)h * (float)w);
-    const size_t smem = head_smem(kernel_size, head_channels, target != nullptr);
+    const size_t smem =
+        ((size_t)kHeadSeg * (head_channels + 4) + 3 * kernel_size * head_window_row(kernel_size)) * sizeof(float);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     bf16* dl = static_cast<bf16*>(dlogits);
     cudaError_t e = cudaErrorInvalidValue;

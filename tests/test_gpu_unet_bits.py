@@ -1,0 +1,77 @@
+"""The learned denoiser's sums in their recorded order, bit for bit.
+
+A convolution's fp32 sum depends on its order in the last place, and a network amplifies that: one flipped bf16
+rounding or ReLU mask in an early layer moves a training step's gradient by several per cent, which is as far as it is
+from its 64-bit value.  So the order is part of the results: whichever kernel takes a shape adds the same products in
+the same order.  The digests below are of results recorded on a B200 (148 SMs, which fixes the number of
+partial sums) with the kernels that defined the order."""
+import ctypes
+import hashlib
+
+import numpy as np
+import pytest
+import torch
+
+from cloudrendering_b200 import _lib
+from oracle import unet_oracle as uo
+
+pytestmark = pytest.mark.gpu
+
+
+def ptr(t):
+    return ctypes.c_void_p(t.data_ptr()) if t is not None else None
+
+
+def normal(seed, *shape, scale=1.0):
+    return (np.random.default_rng(seed).standard_normal(shape) * scale).astype(np.float32)
+
+
+def f32(a):
+    return torch.from_numpy(np.ascontiguousarray(a, np.float32)).cuda()
+
+
+def bf16(a):
+    return torch.from_numpy(uo.bf16(np.asarray(a, np.float32))).to(torch.bfloat16).cuda().contiguous()
+
+
+def digest(*tensors):
+    h = hashlib.sha256()
+    for t in tensors:
+        h.update((t.float() + 0.0).contiguous().cpu().numpy().tobytes())  # (+ 0: -0 and 0 are one value)
+    return h.hexdigest()[:16]
+
+
+# ---- the kernel head ----
+def head_digest(lib, n, h, w, ks):
+    hc = (ks * ks + 7) // 8 * 8
+    g = np.random.default_rng(40)
+    rad = f32(g.exponential(1.0, (n, 3, h, w)) * (g.random((n, 3, h, w)) < 0.7))
+    target = f32(g.exponential(1.0, (n, 3, h, w)))
+    logits = f32(normal(41, n, h, w, hc, scale=2.0))
+    out = torch.empty((n, 3, h, w), device="cuda")
+    dl = torch.empty((n, h, w, hc), dtype=torch.bfloat16, device="cuda")
+    lp = torch.empty(lib.vpt_unet_head_blocks(n, h, w), device="cuda")
+    assert lib.vpt_unet_kpn_head(ptr(logits), hc, ks, ptr(rad), ptr(target), ptr(out), ptr(dl), ptr(lp), n, h, w,
+                                 ctypes.c_float(1e-2), None) == 0
+    torch.cuda.synchronize()
+    return digest(out, dl)
+
+
+COMPUTE = {"head": head_digest}
+# (what, sizes): the digest
+RECORDED = {
+    ("head", 2, 9, 130, 13): "43e0284da028c99d",
+    ("head", 1, 33, 70, 5): "96607ab2ed513255",
+    ("head", 1, 6, 64, 15): "0a8f679207c8b013",
+}
+
+
+@pytest.fixture(scope="module")
+def lib():
+    torch.cuda.init()
+    return _lib.load()
+
+
+@pytest.mark.parametrize("key", RECORDED, ids=lambda k: "-".join(map(str, k)))
+def test_results_as_recorded(lib, key):
+    assert COMPUTE[key[0]](lib, *key[1:]) == RECORDED[key]
