@@ -2004,35 +2004,61 @@ __global__ void bias_grad_kernel(const bf16* __restrict__ dy, float* __restrict_
 }
 
 // gradient of one layer into the flat fp32 gradient: g[co][t][ci] = sum_s wpart[s][t*cin+ci][co] and
-// gb[co] = sum_b bpart[b][co], in a fixed order.  A warp sums 32 consecutive elements of the partials (its loads are
-// whole lines; reading by the gradient's own order, ci fastest, took a sector per lane): with 8 splits and more the
-// eight warps of a block take the splits s = warp, warp + 8, ... of the same elements and combine through shared
-// memory, with fewer each takes all splits of its own (64 pixels of 128 -> 128 channels, 1 split: eight warps on
-// the same elements made the layer's gradient 2.5 us slower).  Bound: the partials' bytes.  The 19 layers of a training
-// step of 8 images of 256 x 256: 437 us by the gradient's order, 160 us here.
+// gb[co] = sum_b bpart[b][co], every sum one after the other from the first partial to the last.  The loads are whole
+// lines, by the partials' own order (by the gradient's, ci fastest, they took a sector per lane).  A thread adds its own
+// element's partials, 16 loads in flight, where the layer has an element for every lane of 128 blocks; below that, and
+// for the biases, the eight warps of a block have 16 partials each of the same 32 elements on the way and put them into
+// shared memory, where the first warp adds them while the next ones arrive.  Bound: the partials' bytes.  The
+// 19 layers of a training step of 8 images of 256 x 256: 457 us by the gradient's order, 160 here (most of it
+// the launches' 8 us each); all layers through shared memory 216.
+constexpr int kReduceChunk = 128;  // partials in shared memory
+
+__host__ __device__ constexpr bool reduce_shared(int splits, int nw) { return splits >= 8 && nw < 32768; }
+
 __global__ void __launch_bounds__(256) reduce_grads_kernel(const float* __restrict__ wpart, int splits, int m_pad,
                                                            int cin, int cout, const float* __restrict__ bpart,
                                                            int bblocks, float* __restrict__ gw,
                                                            float* __restrict__ gb) {
-    __shared__ float part[8][32];
+    __shared__ float part[kReduceChunk][32];
     const int nw = cout * 9 * cin;  // a multiple of 256
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int wblocks = splits >= 8 ? nw / 32 : nw / 256;  // the blocks of the weights; then 32 biases a block
+    // the blocks of the weights; then 32 biases a block
+    const int wblocks = reduce_shared(splits, nw) ? nw / 32 : nw / 256;
     const bool weight = (int)blockIdx.x < wblocks;
-    const bool own = weight && splits < 8;  // a warp's elements are its own
+    const bool own = weight && !reduce_shared(splits, nw);  // a thread's element is its own
     const int j = own ? (int)blockIdx.x * 256 + (int)threadIdx.x : ((int)blockIdx.x - (weight ? 0 : wblocks)) * 32 + lane;
     const float* src = weight ? wpart + j : bpart + j;
     const size_t stride = weight ? (size_t)m_pad * cout : (size_t)cout;
-    const int count = weight ? splits : (bpart && j < cout ? bblocks : 0), step = own ? 1 : 8;
+    const bool in = weight || j < cout;
+    const int count = weight ? splits : (bpart ? bblocks : 0);
     float s = 0.0f;
-#pragma unroll 8
-    for (int k = own ? 0 : warp; k < count; k += step) s += __ldg(src + (size_t)k * stride);
-    if (!own) {
-        part[warp][lane] = s;
-        __syncthreads();
-        if (warp > 0) return;
+    if (own) {
+#pragma unroll 16
+        for (int k = 0; k < count; ++k) s += __ldg(src + (size_t)k * stride);
+    } else {
+        constexpr int kMine = kReduceChunk / 8;
+        float v[kMine];
+        auto load = [&](int k0) {
 #pragma unroll
-        for (int k = 1; k < 8; ++k) s += part[k][lane];
+            for (int i = 0; i < kMine; ++i) {
+                const int k = k0 + 8 * i + warp;
+                v[i] = in && k < count ? __ldg(src + (size_t)k * stride) : 0.0f;
+            }
+        };
+        load(0);
+        for (int k0 = 0; k0 < count; k0 += kReduceChunk) {
+#pragma unroll
+            for (int i = 0; i < kMine; ++i) part[8 * i + warp][lane] = v[i];
+            __syncthreads();
+            if (k0 + kReduceChunk < count) load(k0 + kReduceChunk);
+            if (warp == 0) {
+                const int n = min(kReduceChunk, count - k0);
+#pragma unroll 8
+                for (int k = 0; k < n; ++k) s += part[k][lane];
+            }
+            __syncthreads();
+        }
+        if (warp > 0) return;
     }
     if (weight) {
         const int m = j / cout, co = j - m * cout;  // m = t * cin + ci
@@ -3181,7 +3207,7 @@ VptStatus vpt_unet_reduce_grads(const float* wpartial, int splits, int cin, int 
         (bpartial && bblocks <= 0))
         return VPT_ERR_ARG;
     const int m_pad = (9 * cin + kBM - 1) / kBM * kBM;
-    const int blocks = cout * 9 * cin / (splits >= 8 ? 32 : 256) + (cout + 31) / 32;
+    const int blocks = cout * 9 * cin / (reduce_shared(splits, cout * 9 * cin) ? 32 : 256) + (cout + 31) / 32;
     reduce_grads_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         wpartial, splits, m_pad, cin, cout, bpartial, bblocks, grad_w, grad_b);
     vpt::count_launches(1);

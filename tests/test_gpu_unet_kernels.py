@@ -373,3 +373,26 @@ def test_adam(lib):
     for got, ref in ((host(tp), rp), (host(tm1), rm1), (host(tm2), rm2)):
         assert np.all(np.abs(got - ref) <= 1e-6 * np.abs(ref) + 4 * 2.0 ** -23 * np.abs(ref).max())
     assert np.array_equal(host(pb), uo.bf16(host(tp).astype(np.float32)))
+
+
+@pytest.mark.parametrize("splits,cin,cout,bblocks", [(1, 16, 16, 1), (7, 32, 48, 9), (8, 16, 32, 8), (9, 48, 16, 127),
+                                                     (128, 16, 32, 128), (129, 32, 16, 129), (300, 16, 80, 257),
+                                                     (148, 32, 32, 0), (21, 64, 64, 3)])
+def test_partial_sums_are_added_in_order(lib, splits, cin, cout, bblocks):
+    """Every gradient is its partials' fp32 sum from the first to the last, bit for bit."""
+    rows = lib.vpt_unet_wgrad_rows(cin)
+    part, bpart = rng_data(81, splits, rows, cout), rng_data(82, max(1, bblocks), cout)
+    d_part, d_b = dev_f32(part), dev_f32(bpart)
+    gw = torch.full((cout, 9, cin), float("nan"), device="cuda")
+    gb = torch.full((cout,), float("nan"), device="cuda")
+    assert lib.vpt_unet_reduce_grads(ptr(d_part), splits, cin, cout, ptr(d_b) if bblocks else None, bblocks, ptr(gw),
+                                     ptr(gb), None) == 0
+    torch.cuda.synchronize()
+    want = np.zeros((rows, cout), np.float32)
+    for p in part:
+        want = want + p
+    bias = np.zeros(cout, np.float32)
+    for p in bpart[:bblocks]:
+        bias = bias + p
+    assert np.array_equal(gw.cpu().numpy(), want[:9 * cin].reshape(9, cin, cout).transpose(2, 0, 1))
+    assert np.array_equal(gb.cpu().numpy(), bias)
