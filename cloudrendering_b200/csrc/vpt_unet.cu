@@ -1560,9 +1560,9 @@ __global__ void __launch_bounds__(kBoxThreads)
 // ---------------------------------------------------------------------------------------------
 // the weight gradient on image rows
 // ---------------------------------------------------------------------------------------------
-// dw[co][t][ci] = sum over pixels p of dy[p][co] * x[p + off(t)][ci].  Pixels are K: a CTA walks the rows of
-// an image column at most 128 pixels wide, every row a contraction over its pixels in steps of 16, and sums
-// all its rows in TMEM.  Both operands are rows as they lie in memory, [pixel][channels], read by the TMA
+// dw[co][t][ci] = sum over pixels p of dy[p][co] * x[p + off(t)][ci].  Pixels are K: a CTA walks segments of rows of
+// an image column 128 pixels wide, every row a contraction over its pixels in steps of 16, and sums
+// all its rows in TMEM, one after the other.  Both operands are rows as they lie in memory, [pixel][channels], read by the TMA
 // into the MN-major swizzled layout (channels contiguous: MN; pixels: K), lines of 32 or 16 channels.  A tap's
 // horizontal shift dx is a start moved by dx pixel lines, as in conv_stack_kernel; pixels and channels outside
 // arrive as zeros.
@@ -1593,11 +1593,26 @@ struct WgradArgs {
     int role;
     int s_group;               // channels of an S chunk: 32, or 16 when S has 16
     int u_chunks, s_chunks;    // blockIdx.y = u_chunk * s_chunks + s_chunk
-    int ksteps;                // 16-pixel steps of a row
-    int xtiles;
+    int xtiles, seg_rows, segs_per_col;  // segments of seg_rows rows of a column; CTA i takes i, i + gridDim.x, ...
     int u_slot, u_group_bytes, s_slot, s_ring;  // shared-memory strides; ring depth of S
     int u_lines, s_lines;      // pixel lines of a row (the x tensor's rows carry a halo of one)
     int tmem_cols;
+};
+
+// the segments of a CTA in order
+struct SegWalk {
+    const WgradArgs& a;
+    int seg = (int)blockIdx.x;
+    __device__ __forceinline__ bool next(WsSegment& g) {
+        if (seg >= a.n * a.xtiles * a.segs_per_col) return false;
+        const int col = seg / a.segs_per_col, part = seg - col * a.segs_per_col;
+        g.n_img = col / a.xtiles;
+        g.x0 = (col % a.xtiles) * kBM;
+        g.y0 = part * a.seg_rows;
+        g.y1 = min(a.h, g.y0 + a.seg_rows);
+        seg += (int)gridDim.x;
+        return true;
+    }
 };
 
 // MN-major swizzled descriptor: lines of `line` bytes (128 / 64 / 32: 64 / 32 / 16 channels), 8-pixel groups
@@ -1674,7 +1689,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
                     sph ^= 1u;
                 }
             };
-            RowRange range(a.n, a.h, a.xtiles);
+            SegWalk range{a};
             WsSegment g;
             while (!fail && range.next(g)) {
                 const int r0 = a.role == 0 ? g.y0 - 1 : g.y0, r1 = a.role == 0 ? g.y1 : g.y1 - 1;
@@ -1734,7 +1749,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
         uint32_t uph = 0;
         int ws = 0;         // ring slot of the oldest S row in use
         uint32_t wph = 0;   // its phase
-        RowRange range(a.n, a.h, a.xtiles);
+        SegWalk range{a};
         WsSegment g;
         while (!fail && range.next(g)) {
             const int r0 = a.role == 0 ? g.y0 - 1 : g.y0, r1 = a.role == 0 ? g.y1 : g.y1 - 1;
@@ -1762,7 +1777,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
                     const uint32_t id_rest = id1 + (uint32_t)(n_rest - 1) * id_n;
                     uint32_t ul = u_lo + ((uint32_t)(us * a.u_slot) >> 4);
                     uint32_t sl = s_lo + ((uint32_t)(ws * a.s_slot) >> 4), sw = s_lo;
-                    for (int j = 0; j < a.ksteps; ++j) {
+                    for (int j = 0; j < kBM / 16; ++j) {
                         mma_bf16_halves(d0, ul, u_hi, sl, s_hi, id_first, 1u);
                         if (n_rest > 0) mma_bf16_halves(d1, ul, u_hi, sw, s_hi, id_rest, 1u);
                         ul += u_step;
@@ -2522,22 +2537,43 @@ inline int strip_groups(int width, int cin, int cout, bool any = false) {
     return 0;
 }
 
-// Weight gradients of fewer pixels than this take the gather kernel, whose launch has work for every SM there:
-// a CTA of the row kernel sets up nine accumulators and writes them all, however few rows it gets.  Kernel and
-// reduction, us, gather / rows: 64 pixels of 128 -> 128 channels 12.4 / 19.2, 1,024 pixels of 96 -> 96 18.8 / 21.7,
-// 3,200 pixels of 96 -> 96 27.9 / 25.2, 4,096 pixels of 48 -> 48 18.9 / 15.3.
-constexpr long kWgradRowsMinPixels = 2048;
+inline void strip_segments(int n, int h, int w, int slots, int& xtiles, int& seg_rows, int& segs_per_col,
+                           int& total) {
+    xtiles = (w + kBM - 1) / kBM;
+    const int cols = n * xtiles;
+    const int want = max(cols, 2 * slots);
+    int spc = (want + cols - 1) / cols;
+    spc = min(spc, max(1, h / 4));
+    seg_rows = (h + spc - 1) / spc;
+    segs_per_col = (h + seg_rows - 1) / seg_rows;
+    total = cols * segs_per_col;
+}
 
-// Weight-gradient plan on image rows: the role with fewer passes and the CTAs of a pass.
+// The rule and the split of the weight gradient on image rows.  Which pixels a partial holds, and their order, are part
+// of the result: one flipped rounding in the sum of a layer is as large as the error of a training step.  So
+// images at least 128 pixels wide with 64 channels on a side are split by segments of rows, one partial for each CTA of
+// a pass, where five 130-pixel rows of x and three 128-pixel rows of dy with their channels (one of the two in
+// chunks of 64 or 128) take at most 220 KB; everything else in runs of pixels_per_split (conv_tile_kernel).
+// `any`: also with fewer channels.
+inline bool wgrad_by_rows(int width, int cin, int cout, bool any) {
+    if (width < kBM || (!any && cin < 64 && cout < 64)) return false;
+    for (int role = 0; role < 2; ++role) {
+        const int u = role == 0 ? cin : cout, sc = role == 0 ? cout : cin;
+        const int chunk = u > 64 ? 128 : 64, xc = role == 0 ? chunk : cin, dyc = role == 0 ? cout : chunk;
+        if (sc <= 256 && 5 * kStripPix * 2 * xc + 3 * kBM * 2 * dyc <= 220 * 1024) return true;
+    }
+    return false;
+}
+
 struct WgradPlan {
     int role = 0, s_group = 32, u_chunks = 1, s_chunks = 1, passes = 1;
-    int kpix = kBM, xtiles = 1, grid = 1;
+    int xtiles = 1, seg_rows = 1, segs_per_col = 1, grid = 1;
 };
 
 inline WgradPlan wgrad_plan(int n, int h, int w, int cin, int cout, int sms) {
     WgradPlan p;
     int best = 0;
-    for (int role = 0; role < 2; ++role) {
+    for (int role = 0; role < 2; ++role) {  // the role with fewer passes
         const int u = role == 0 ? cin : cout, sc = role == 0 ? cout : cin;
         const int uc = (u + 127) / 128, sn = (sc + 31) / 32;
         if (best == 0 || uc * sn < best) {
@@ -2549,27 +2585,10 @@ inline WgradPlan wgrad_plan(int n, int h, int w, int cin, int cout, int sms) {
         }
     }
     p.passes = best;
-    p.kpix = std::min(kBM, (w + 15) / 16 * 16);
-    p.xtiles = (w + kBM - 1) / kBM;
-    // CTAs per pass: enough to fill the SMs with all passes, and so many (up to one per SM) that a CTA's
-    // accumulators take about 64 additions each: longer fp32 sums in TMEM round more than the partials' sum
-    const int cols = n * p.xtiles;
-    const long steps = (long)cols * h * (p.kpix / 16);
-    const int ctas = (int)std::max<long>(std::max(1, sms / best), std::min<long>(sms, (steps + 63) / 64));
-    p.grid = (int)std::min<long>((long)cols * h, ctas);
+    int total = 0;
+    strip_segments(n, h, w, sms, p.xtiles, p.seg_rows, p.segs_per_col, total);
+    p.grid = std::min(total, sms);
     return p;
-}
-
-inline void strip_segments(int n, int h, int w, int slots, int& xtiles, int& seg_rows, int& segs_per_col,
-                           int& total) {
-    xtiles = (w + kBM - 1) / kBM;
-    const int cols = n * xtiles;
-    const int want = max(cols, 2 * slots);
-    int spc = (want + cols - 1) / cols;
-    spc = min(spc, max(1, h / 4));
-    seg_rows = (h + spc - 1) / spc;
-    segs_per_col = (h + seg_rows - 1) / seg_rows;
-    total = cols * segs_per_col;
 }
 
 cudaError_t launch_strip_pass(StripArgs a, cudaStream_t s) {
@@ -2662,10 +2681,11 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* partial, int
     a.s_group = p.s_group;
     a.u_chunks = p.u_chunks;
     a.s_chunks = p.s_chunks;
-    a.ksteps = p.kpix / 16;
     a.xtiles = p.xtiles;
-    a.u_lines = p.kpix + (p.role == 0 ? 2 : 0);
-    a.s_lines = p.kpix + (p.role == 1 ? 2 : 0);
+    a.seg_rows = p.seg_rows;
+    a.segs_per_col = p.segs_per_col;
+    a.u_lines = kBM + (p.role == 0 ? 2 : 0);
+    a.s_lines = kBM + (p.role == 1 ? 2 : 0);
     // group and slot strides: whole 1024-byte blocks (the swizzle acts on absolute addresses)
     auto up = [](int b) { return (b + 1023) / 1024 * 1024; };
     a.u_group_bytes = up(a.u_lines * 64);
@@ -2995,8 +3015,8 @@ static bool g_force_gather = false;  // conv path 1: the gather kernels everywhe
 static bool g_force_strip = false;   // conv path 2: the strip kernels wherever they apply
 static int g_conv_ksplit = 0;        // gather convolution K splits: 0 automatic, 1 none, k > 1 forced
 
-static bool wgrad_on_rows(int n, int h, int w) {
-    return !g_force_gather && (g_force_strip || (long)n * h * w >= kWgradRowsMinPixels);
+static bool wgrad_on_rows(int w, int cin, int cout) {
+    return !g_force_gather && wgrad_by_rows(w, cin, cout, g_force_strip);
 }
 
 extern "C" {
@@ -3117,7 +3137,7 @@ VptStatus vpt_unet_conv3x3_wgrad(const void* x, const void* dy, float* partial, 
     a.pix_per_split = pixels_per_split;
     const int mtiles = (9 * cin + kBM - 1) / kBM;
     a.m_pad = mtiles * kBM;
-    if (wgrad_on_rows(n, h, width)) {  // (its tensor maps want aligned tensors)
+    if (wgrad_on_rows(width, cin, cout)) {  // (its tensor maps want aligned tensors)
         if (reinterpret_cast<uintptr_t>(x) % 16 || reinterpret_cast<uintptr_t>(dy) % 16) return VPT_ERR_ARG;
         const WgradPlan plan = wgrad_plan(n, h, width, cin, cout, sm_count());
         return launch_wgrad_rows(a.x, a.w, partial, err, n, h, width, cin, cout, plan,
@@ -3133,7 +3153,7 @@ int vpt_unet_wgrad_rows(int cin) { return (9 * cin + kBM - 1) / kBM * kBM; }
 
 int vpt_unet_wgrad_splits(int n, int h, int width, int cin, int cout, int pixels_per_split) {
     if (n <= 0 || h <= 0 || width <= 0 || pixels_per_split <= 0) return 0;
-    if (wgrad_on_rows(n, h, width)) return wgrad_plan(n, h, width, cin, cout, sm_count()).grid;
+    if (wgrad_on_rows(width, cin, cout)) return wgrad_plan(n, h, width, cin, cout, sm_count()).grid;
     const long P = (long)n * h * width;
     return (int)((P + pixels_per_split - 1) / pixels_per_split);
 }

@@ -41,6 +41,13 @@ def digest(*tensors):
     return h.hexdigest()[:16]
 
 
+def call(lib, name, *args):
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert getattr(lib, name)(*args, ptr(err), None) == 0, name
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0, name
+
+
 # ---- the kernel head ----
 def head_digest(lib, n, h, w, ks):
     hc = (ks * ks + 7) // 8 * 8
@@ -57,12 +64,38 @@ def head_digest(lib, n, h, w, ks):
     return digest(out, dl)
 
 
-COMPUTE = {"head": head_digest}
+# ---- weight gradients ----
+def split_pixels(lib, pixels, cin):
+    """The training loop's pixels per split."""
+    tiles = lib.vpt_unet_wgrad_rows(cin) // 128
+    splits = max(1, min((pixels + 63) // 64, (2 * 148 + tiles - 1) // tiles))
+    return ((pixels + splits - 1) // splits + 63) // 64 * 64
+
+
+def wgrad_digest(lib, n, h, w, cin, cout):
+    x, dy = bf16(normal(61, n, h, w, cin)), bf16(normal(62, n, h, w, cout))
+    pps = split_pixels(lib, n * h * w, cin)
+    splits, rows = lib.vpt_unet_wgrad_splits(n, h, w, cin, cout, pps), lib.vpt_unet_wgrad_rows(cin)
+    part = torch.zeros((splits, rows, cout), device="cuda")
+    call(lib, "vpt_unet_conv3x3_wgrad", ptr(x), ptr(dy), ptr(part), n, h, w, cin, cout, pps)
+    return digest(part[:, :9 * cin])
+
+
+COMPUTE = {"head": head_digest, "wgrad": wgrad_digest}
 # (what, sizes): the digest
 RECORDED = {
     ("head", 2, 9, 130, 13): "43e0284da028c99d",
     ("head", 1, 33, 70, 5): "96607ab2ed513255",
     ("head", 1, 6, 64, 15): "0a8f679207c8b013",
+    ("wgrad", 8, 96, 256, 96, 32): "a0dcfe46e0ade327",
+    ("wgrad", 2, 80, 224, 96, 32): "68d25f01401e2d07",
+    ("wgrad", 1, 37, 130, 64, 64): "1b001b1a681183d3",
+    ("wgrad", 1, 64, 128, 160, 64): "d4636b2e89e0de43",
+    ("wgrad", 2, 50, 200, 32, 176): "3f2207bf578b20f5",
+    ("wgrad", 2, 64, 256, 32, 32): "ff406f1095b659ae",
+    ("wgrad", 1, 96, 150, 16, 32): "297b0026b330b4d6",
+    ("wgrad", 4, 40, 112, 64, 64): "5af21771fd023618",
+    ("wgrad", 8, 32, 32, 128, 128): "1a14c8b49fae70ea",
 }
 
 

@@ -396,3 +396,24 @@ def test_partial_sums_are_added_in_order(lib, splits, cin, cout, bblocks):
         bias = bias + p
     assert np.array_equal(gw.cpu().numpy(), want[:9 * cin].reshape(9, cin, cout).transpose(2, 0, 1))
     assert np.array_equal(gb.cpu().numpy(), bias)
+
+
+@pytest.mark.parametrize("case", [(2, 40, 64, 32, 48, 1024), (1, 50, 100, 96, 64, 448), (1, 30, 130, 32, 32, 640),
+                                  (1, 9, 256, 16, 48, 128), (4, 32, 32, 144, 272, 64)])
+def test_weight_gradient_of_runs_of_pixels(lib, case):
+    """Images narrower than 128 pixels, and layers of few channels, have a partial for each pixels_per_split pixels: that
+    many, and each the weight gradient of its own pixels."""
+    n, h, w, cin, cout, pps = case
+    P = n * h * w
+    splits, rows = -(-P // pps), lib.vpt_unet_wgrad_rows(cin)
+    assert lib.vpt_unet_wgrad_splits(n, h, w, cin, cout, pps) == splits
+    x, dy = uo.bf16(rng_data(83, n, h, w, cin)), uo.bf16(rng_data(84, n, h, w, cout))
+    d_x, d_dy = dev_bf16(x), dev_bf16(dy)
+    part = torch.full((splits + 1, rows, cout), -7.0, device="cuda")
+    run(lib, "vpt_unet_conv3x3_wgrad", ptr(d_x), ptr(d_dy), ptr(part), n, h, w, cin, cout, pps)
+    assert bool((part[splits] == -7.0).all())  # nothing beyond
+    for k in sorted({0, splits // 2, splits - 1}):
+        own = np.zeros((P, cout))
+        own[k * pps:(k + 1) * pps] = dy.reshape(P, cout)[k * pps:(k + 1) * pps]
+        ref = uo.conv3x3_weight_grad(x, own.reshape(n, h, w, cout))
+        close_f32(host(part[k, :9 * cin]), ref.transpose(1, 2, 0).reshape(9 * cin, cout))
