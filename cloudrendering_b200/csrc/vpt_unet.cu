@@ -493,13 +493,14 @@ __global__ void __launch_bounds__(kThreads) conv_tile_kernel(const ConvArgs a) {
 
 // Split-K convolution: y = act(bias + sum over the splits of partial[s]) (fixed order), times the
 // ReLU-derivative mask, stored bf16 or fp32; 4 channels per thread.
+template <class I>
 __global__ void conv_finalize_kernel(const float* __restrict__ partial, int ksplit, long P, int cout,
                                      const float* __restrict__ bias, const bf16* __restrict__ mask, int relu,
                                      int out_f32, void* __restrict__ y) {
-    const uint32_t c4 = (uint32_t)cout / 4, total = (uint32_t)P * c4;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
+    const I c4 = (I)(cout / 4), total = (I)P * c4;
+    for (I i = (I)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
         const size_t p = i / c4;
-        const int c = (int)(i - (uint32_t)p * c4) * 4;
+        const int c = (int)(i - (I)p * c4) * 4;
         float4 acc = reinterpret_cast<const float4*>(partial + p * cout + c)[0];
         for (int k = 1; k < ksplit; ++k) {
             const float4 u = reinterpret_cast<const float4*>(partial + ((size_t)k * P + p) * cout + c)[0];
@@ -1055,8 +1056,10 @@ __global__ void __launch_bounds__(kWsThreads, 2) conv_ws_kernel(const __grid_con
 //             three adjacent rows are contiguous columns except around the ring's end (then two MMAs).
 //   first use an output row's first MMA (its dy = -1 taps, dx = -1, first 16 channels) overwrites its block,
 //             so that step is split into N = cout (overwrite) and the older rows (accumulate).
-//   sets      with many input channels (longer sums in the accumulator's fp32) the channel groups alternate
-//             between two such rings, which the epilogue adds.
+//   sums      an output's products are added row by row, in a row by channel group and in a group by tap, as
+//             conv_ws_kernel adds them; or (by_tap) by tap and in a tap by channel, as conv_tile_kernel does.  A layer
+//             of two passes over its input channels (ConvOrder) has a ring of accumulators for each, which the
+//             epilogue adds.
 //   order     one thread issues every MMA, so an accumulator's updates and the commits behind them are in
 //             order: after input row q's MMAs one commit frees its ring slot, one hands row q-2 (counted
 //             from the segment's start) to the epilogue.
@@ -1070,7 +1073,8 @@ constexpr int kStackMaxCout = 80;  // 3 cout <= 256 columns
 struct StackArgs {
     WsArgs ws;
     int ring, blocks;
-    int sets;  // 2: the channel groups alternate between two accumulator rings, added in the epilogue
+    int groups0;  // channel groups of the first pass (all of them: one ring of accumulators)
+    int by_tap;   // order of an input row's products
     int co0, cout_total;  // first output channel of this launch, channels per pixel of y
 };
 
@@ -1266,6 +1270,8 @@ __global__ void __launch_bounds__(kStackThreads, 2)
         const uint32_t id_n = (uint32_t)(cout >> 3) << 17;  // one more block of columns
         const int ngroups = wa.ngroups;
         const uint32_t set_cols = (uint32_t)(blocks * cout);
+        // the (group, dx) pairs of a row: dx inner, or the group inner
+        const int by_tap = st.by_tap;
         int slot = 0;
         uint32_t phase = 0;
         int blk0 = 0;        // block of the segment's first output row
@@ -1296,35 +1302,38 @@ __global__ void __launch_bounds__(kStackThreads, 2)
                     const uint32_t p0 = (uint32_t)((2 - q + lo) * cout), p_rest = p0 + (uint32_t)(n_first * cout);
                     const uint32_t id_first = id1 + (uint32_t)(n_first - 1) * id_n;
                     const uint32_t id_rest = id1 + (uint32_t)(n_rest - 1) * id_n;
-                    for (int k = 0; k < ngroups; ++k) {
+                    int k = 0, dx = 0;
+                    for (int u = 0; u < 3 * ngroups; ++u) {
                         const int gw = wa.gw[k];
                         const uint32_t ahi = a_hi_of(gw);
-                        const uint32_t line16 = (uint32_t)gw >> 3;
-                        // the channel groups alternate between the sets; a set's first step overwrites
-                        const uint32_t acc0 = tmem + (st.sets == 2 ? (uint32_t)(k & 1) * set_cols : 0u);
-                        bool first = fresh && k < st.sets;
-                        uint32_t al = a_lo1 + row16 + ((uint32_t)wa.goff[k] >> 4);
-                        uint32_t bl = b_lo0 + (uint32_t)(wa.gc[k] >> 3) * n3;
-#pragma unroll
-                        for (int dx = 0; dx < 3; ++dx) {
-                            uint32_t aj = al, bj = bl;
-                            for (int j = 0; j < gw / 16; ++j) {
-                                if (first) {  // the new row overwrites its block, the older ones accumulate
-                                    first = false;
-                                    for (int i = lo; i <= hi; ++i) {
-                                        const int bi = blo + (i - lo) < blocks ? blo + (i - lo) : blo + (i - lo) - blocks;
-                                        mma_bf16_halves(acc0 + (uint32_t)(bi * cout), aj, ahi,
-                                                        bj + (uint32_t)((2 - q + i) * cout), b_hi, id1, i < q ? 1u : 0u);
-                                    }
-                                } else {
-                                    mma_bf16_halves(acc0 + (uint32_t)(blo * cout), aj, ahi, bj + p0, b_hi, id_first, 1u);
-                                    if (n_rest > 0) mma_bf16_halves(acc0, aj, ahi, bj + p_rest, b_hi, id_rest, 1u);
+                        // a ring of accumulators for each pass; its first step overwrites the new row's
+                        const uint32_t acc0 = tmem + (k >= st.groups0 ? set_cols : 0u);
+                        bool first = fresh && dx == 0 && (k == 0 || k == st.groups0);
+                        uint32_t aj = a_lo1 + row16 + ((uint32_t)wa.goff[k] >> 4) + (uint32_t)dx * ((uint32_t)gw >> 3);
+                        uint32_t bj = b_lo0 + (uint32_t)(wa.gc[k] >> 3) * n3 + (uint32_t)dx * b_dx;
+                        for (int j = 0; j < gw / 16; ++j) {
+                            if (first) {  // the new row overwrites its block, the older ones accumulate
+                                first = false;
+                                for (int i = lo; i <= hi; ++i) {
+                                    const int bi = blo + (i - lo) < blocks ? blo + (i - lo) : blo + (i - lo) - blocks;
+                                    mma_bf16_halves(acc0 + (uint32_t)(bi * cout), aj, ahi,
+                                                    bj + (uint32_t)((2 - q + i) * cout), b_hi, id1, i < q ? 1u : 0u);
                                 }
-                                aj += 2u;
-                                bj += b_step;
+                            } else {
+                                mma_bf16_halves(acc0 + (uint32_t)(blo * cout), aj, ahi, bj + p0, b_hi, id_first, 1u);
+                                if (n_rest > 0) mma_bf16_halves(acc0, aj, ahi, bj + p_rest, b_hi, id_rest, 1u);
                             }
-                            al += line16;
-                            bl += b_dx;
+                            aj += 2u;
+                            bj += b_step;
+                        }
+                        if (by_tap) {
+                            if (++k == ngroups) {
+                                k = 0;
+                                ++dx;
+                            }
+                        } else if (++dx == 3) {
+                            dx = 0;
+                            ++k;
                         }
                     }
                     mma_commit(smem_u32(&empty[slot]));
@@ -1376,7 +1385,7 @@ __global__ void __launch_bounds__(kStackThreads, 2)
                     }
                     tc_fence_after();
                     stack_epilogue(a, s_bias, tmem + lanes + (uint32_t)(b * cout),
-                                   st.sets == 2 ? (uint32_t)(blocks * cout) : 0u, at, ok, mask);
+                                   st.groups0 < wa.ngroups ? (uint32_t)(blocks * cout) : 0u, at, ok, mask);
                     tc_fence_before();
                     __syncwarp();
                     if (lane == 0) mbar_arrive(smem_u32(&acc_empty[b]));
@@ -1407,7 +1416,8 @@ __global__ void __launch_bounds__(kStackThreads, 2)
 // smaller) and multiples of 128.  A stage is one tap and up to 64 input channels: the box moved by (dx, dy), whose
 // pixels outside the image arrive as zeros, and the tap's weights, both loaded by the tensor-memory-access unit
 // into K-major swizzled lines of `cw` channels, four stages ahead; the gather kernel's threads compute 64 addresses
-// and copies each a stage and meet at a barrier for it.
+// and copies each a stage and meet at a barrier for it.  The stages follow the layer's order of products (ConvOrder):
+// by tap and channel, or as the row-strip kernels add them, with an accumulator for each pass over the channels.
 // Warps: 0 loads, 1 issues, 2-5 the epilogue.  Every wait is bounded, as in conv_ws_kernel.
 //   us, gather kernel / here: 96 -> 96 8 images of 64 x 64 33.5 / 15.6, 224 -> 96 71 / 23, 96 -> 224 80 / 31; 128 -> 128
 // 8 images of 16 x 16 17.3 / 13.1, one of 4 x 4 12.7 / 8.2; 224 -> 96 one image of 128 x 128 61 / 15.  Bound: the
@@ -1417,8 +1427,66 @@ constexpr int kBoxStages = 4;
 
 struct BoxArgs {
     ConvArgs c;
-    int cw;              // channels of a stage: 64, 32 or 16 (the last stage of a tap may hold fewer)
+    int cw;              // channels of a stage: 64, 32 or 16 (a stage may use fewer)
     int bh, bn;          // rows and images of a box
+    int passes, pass_ch; // order of the row-strip kernels: passes over pass_ch input channels each (0: by tap and channel)
+    int kper;            // by tap: K (= tap * cin + channel) of a split
+};
+
+// The stages of a CTA in the layer's order of products.
+struct BoxWalk {
+    const BoxArgs& b;
+    int tap = 0, ci = 0, len = 0;  // the stage: tap, first channel, channels
+    int pass = -1;                 // its pass (by tap: 0)
+    bool first = false;            // the first of its pass
+    int k = 0, kend = 0;           // by tap: K so far, end of the split
+    int c = 0, d = 0;              // by pass: channel within the pass, 3 dy + dx
+
+    __device__ __forceinline__ explicit BoxWalk(const BoxArgs& b_) : b(b_) {
+        if (b.passes) return;
+        k = min((int)blockIdx.z * b.kper, 9 * b.c.cin);
+        kend = min(k + b.kper, 9 * b.c.cin);
+        tap = k / b.c.cin;
+        ci = k - tap * b.c.cin;
+    }
+    __device__ __forceinline__ bool next() {
+        if (!b.passes) {
+            ci += len;
+            if (ci == b.c.cin) {
+                ci = 0;
+                ++tap;
+            }
+            if (k >= kend) return false;
+            len = min(min(b.cw, b.c.cin - ci), kend - k);
+            k += len;
+            first = pass < 0;
+            pass = 0;
+            return true;
+        }
+        // dy, channel group (64, then 32, then 16), dx
+        int width = min(b.pass_ch, b.c.cin - max(pass, 0) * b.pass_ch);
+        first = pass < 0;
+        if (first) {
+            pass = 0;
+        } else if (++d % 3 == 0) {
+            c += len;
+            if (c < width) {
+                d -= 3;
+            } else {
+                c = 0;
+                if (d == 9) {
+                    d = 0;
+                    if (++pass == b.passes) return false;
+                    first = true;
+                    width = min(b.pass_ch, b.c.cin - pass * b.pass_ch);
+                }
+            }
+        }
+        tap = d;
+        ci = pass * b.pass_ch + c;
+        len = width - c >= 64 ? 64 : (width - c >= 32 ? 32 : 16);
+        return true;
+    }
 };
 
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int c0, int c1, int c2, uint32_t bar) {
@@ -1439,13 +1507,6 @@ __global__ void __launch_bounds__(kBoxThreads)
     const ConvArgs& a = b.c;
     const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
     const int P = a.n * a.h * a.w_, n0 = blockIdx.y * a.n_tile;
-    const int chunks = (a.cin + b.cw - 1) / b.cw;
-    int first = 0, nk = 9 * chunks;
-    if (a.ksplit > 1) {
-        const int per = (nk + a.ksplit - 1) / a.ksplit;
-        first = blockIdx.z * per;
-        nk = max(0, min(nk, first + per) - first);
-    }
     const uint32_t a_bytes = (uint32_t)(kBM * b.cw * 2), b_bytes = (uint32_t)(a.n_tile * b.cw * 2);
     const uint32_t stage_bytes = a_bytes + ((b_bytes + 1023u) & ~1023u);
     const uint32_t sbase = smem_u32(smem);
@@ -1471,22 +1532,18 @@ __global__ void __launch_bounds__(kBoxThreads)
             pixel_coords((int)blockIdx.x * kBM, a.h, a.w_, img, y0, x0);
             int slot = 0, issued = 0;
             uint32_t phase = 0;
-            int tap = first / chunks, chunk = first - tap * chunks;
-            for (int k = 0; k < nk; ++k) {
+            BoxWalk g(b);
+            while (g.next()) {
                 if (!mbar_wait(smem_u32(&empty[slot]), phase ^ 1u)) {
                     fail = true;
                     break;
                 }
                 const uint32_t dst = sbase + (uint32_t)slot * stage_bytes, fb = smem_u32(&full[slot]);
                 mbar_arrive_expect_tx(fb, a_bytes + b_bytes);
-                const int dy = tap / 3;
-                tma_load_4d(dst, &xmap, chunk * b.cw, x0 + tap - 3 * dy - 1, y0 + dy - 1, img, fb);
-                tma_load_3d(dst + a_bytes, &wmap, chunk * b.cw, tap, n0, fb);
+                const int dy = g.tap / 3;
+                tma_load_4d(dst, &xmap, g.ci, x0 + g.tap - 3 * dy - 1, y0 + dy - 1, img, fb);
+                tma_load_3d(dst + a_bytes, &wmap, g.ci, g.tap, n0, fb);
                 ++issued;
-                if (++chunk == chunks) {
-                    chunk = 0;
-                    ++tap;
-                }
                 if (++slot == kBoxStages) {
                     slot = 0;
                     phase ^= 1u;
@@ -1505,9 +1562,10 @@ __global__ void __launch_bounds__(kBoxThreads)
         }
     } else if (warp == 1) {
         const uint32_t idesc = instr_desc(kBM, a.n_tile, 0, 0), hi = a_hi_of(b.cw), lbo = 1u << 16;
-        int slot = 0, chunk = first % chunks;
+        int slot = 0;
         uint32_t phase = 0;
-        for (int k = 0; k < nk; ++k) {
+        BoxWalk g(b);
+        while (g.next()) {
             const bool ok = mbar_wait(smem_u32(&full[slot]), phase);
             if (!__all_sync(0xffffffffu, ok)) {
                 fail = true;
@@ -1517,14 +1575,13 @@ __global__ void __launch_bounds__(kBoxThreads)
             if (elect_one()) {
                 const uint32_t sA = (sbase + (uint32_t)slot * stage_bytes) >> 4;
                 const uint32_t al = lbo + sA, bl = lbo + sA + (a_bytes >> 4);
-                const int steps = min(b.cw, a.cin - chunk * b.cw) / 16;
-                for (int j = 0; j < steps; ++j)
-                    mma_bf16_halves(tmem, al + 2u * (uint32_t)j, hi, bl + 2u * (uint32_t)j, hi, idesc,
-                                    (k > 0 || j > 0) ? 1u : 0u);
+                const uint32_t dacc = tmem + (uint32_t)(g.pass * a.n_tile);
+                for (int j = 0; j < g.len / 16; ++j)
+                    mma_bf16_halves(dacc, al + 2u * (uint32_t)j, hi, bl + 2u * (uint32_t)j, hi, idesc,
+                                    (!g.first || j > 0) ? 1u : 0u);
                 mma_commit(smem_u32(&empty[slot]));
             }
             __syncwarp();
-            if (++chunk == chunks) chunk = 0;
             if (++slot == kBoxStages) {
                 slot = 0;
                 phase ^= 1u;
@@ -1542,9 +1599,16 @@ __global__ void __launch_bounds__(kBoxThreads)
     if (warp >= 2 && !fail_any) {
         const int q = warp & 3, p = (int)blockIdx.x * kBM + q * 32 + lane;
         const uint32_t trow = tmem + ((uint32_t)(q * 32) << 16);
+        const bool any = b.passes || (int)blockIdx.z * b.kper < 9 * a.cin;
         for (int c0 = 0; c0 < a.n_tile; c0 += 16) {
             float v[16] = {};  // an empty K range contributes zeros
-            if (nk > 0) tmem_ld16(trow + (uint32_t)c0, v);  // whole warp, uniform
+            if (any) tmem_ld16(trow + (uint32_t)c0, v);  // whole warp, uniform
+            if (b.passes == 2) {
+                float v2[16];
+                tmem_ld16(trow + (uint32_t)(a.n_tile + c0), v2);
+#pragma unroll
+                for (int i = 0; i < 16; ++i) v[i] += v2[i];
+            }
             if (p < P && n0 + c0 < a.cout) conv_store(a, P, p, n0 + c0, v);
         }
     }
@@ -2736,20 +2800,35 @@ inline WsGroups ws_groups_of(int cin) {
 inline size_t ws_weight_bytes(int cin, int cout) { return (9ul * cin * cout * 2 + 1023) & ~(size_t)1023; }
 inline size_t ws_row_bytes(int cin) { return (size_t)ws_groups_of(cin).row_bytes; }
 
-// accumulator sets of the stacked kernel: 99 or more accumulations in one would round more than the two
-// passes over channel groups that such layers took
-inline int stack_sets(int cin) { return cin > 96 ? 2 : 1; }
+// the groups of `passes` (1 or 2) passes over the channels in one launch, pass by pass
+inline int pass_channels(int cin, int passes) { return (cin / 16 + passes - 1) / passes * 16; }
+inline WsGroups ws_groups_of(int cin, int passes) {
+    if (passes == 1) return ws_groups_of(cin);
+    const int cg = pass_channels(cin, 2);
+    WsGroups g = ws_groups_of(cg);
+    const WsGroups g1 = ws_groups_of(cin - cg);
+    if (!g.row_bytes || !g1.row_bytes || g.n + g1.n > kWsMaxGroups) return WsGroups();
+    for (int k = 0; k < g1.n; ++k) {
+        g.c[g.n + k] = cg + g1.c[k];
+        g.w[g.n + k] = g1.w[k];
+        g.off[g.n + k] = g.row_bytes + g1.off[k];
+    }
+    g.n += g1.n;
+    g.row_bytes += g1.row_bytes;
+    g.tx += g1.tx;
+    return g;
+}
 
 // The stacked kernel (cout <= kStackMaxCout a launch): a ring slot is free again after its own row's MMAs, so two slots
 // do; two CTAs per SM when each gets three (their issuing threads overlap) and at least four accumulators.
-bool stack_config(int cin, int cout, int& per_sm, int& ring) {
-    const size_t rb = ws_row_bytes(cin), wb = ws_weight_bytes(cin, cout);
+bool stack_config(int cin, int cout, int passes, int& per_sm, int& ring) {
+    const size_t rb = (size_t)ws_groups_of(cin, passes).row_bytes, wb = ws_weight_bytes(cin, cout);
     per_sm = 0;
     ring = 0;
     if (rb == 0) return false;
     for (int occ = 2; occ >= 1; --occ) {
         const size_t budget = std::min(kSmPerSm / occ - kWsStatic, kSmPerCta);
-        if (wb >= budget || 512 / occ / (cout * stack_sets(cin)) < 4) continue;
+        if (wb >= budget || 512 / occ / (cout * passes) < 4) continue;
         const int r = (int)std::min<size_t>(kWsMaxRing, (budget - wb) / rb);
         if (r < (occ == 2 ? 3 : 2)) continue;
         per_sm = occ;
@@ -2785,64 +2864,95 @@ bool ws_config(int cin, int cout, int& per_sm, int& ring) {
 }
 
 
-// How the warp-specialised kernels take a layer.  Input channels: one pass where the weights and the rings fit,
-// else up to 4 passes through an fp32 partial, which beat the gather kernel for up to 64 output channels only
-// (measured).  Output channels: conv_stack_kernel for up to 80 of them, in chunks of at most 80 (each launch reads
-// the input again) or all of them in conv_ws_kernel (chunk = 0) beyond.
-// Up to two rows of 128 pixels an SM conv_box_kernel takes the layer (groups = 0) where the width is a multiple of
-// 128: every tile has a CTA of its own, while these kernels read three rows for one and start with all nine taps'
-// weights; up to four rows an SM with more than 80 output channels and no half-empty stages.  us, these / boxes:
-//     96 -> 32  128 rows 12.0 / 8.3   256 rows 13.2 / 10.4  512 rows 17.8 / 18.3  1,024 rows 24.1 / 35.1
-//     48 -> 48  128 rows 9.7 / 7.2    256 rows 10.1 / 9.6   512 rows 14.8 / 17.5  1,024 rows 16.9 / 31.7
-//     96 -> 96  128 rows 25.8 / 10.3  256 rows 28.7 / 15.6  512 rows 36.7 / 28.4  1,024 rows 50.1 / 53.6
-//     48 -> 96  256 rows 17.7 / 14.6  512 rows 18.5 / 23.1;  16 -> 32  256 rows 6.8 / 7.0  512 rows 7.8 / 9.8
-// us, gather or conv_ws / chunks, at 128 pixels a row:
-//   conv_ws does not fit (gather, whose CTAs hold all outputs of 128 pixels)   chunks from 64 rows a chunk
-//     96 -> 96    64 rows 24.2 / 25.4   128 rows 29.4 / 25.7   512 rows 64.7 / 36.1   4,096 rows 458 / 117
-//     96 -> 224  128 rows 40.4 / 53.1   256 rows 78.7 / 57.7   512 rows 155 / 73.7    4,096 rows 1097 / 211
-//   conv_ws fits                                                 chunks for N > 96 (its MMAs get longer), 16 rows an SM
-//     48 -> 144  512 rows 29.6 / 31.9   1,024 rows 46.5 / 39.8   4,096 rows 189 / 100
-//     32 -> 176  512 rows 26.8 / 38.9   2,048 rows 68.0 / 67.8   4,096 rows 166 / 130, its fp32 outputs 173 / 128
-//     32 -> 96   512 rows 19.2 / 22.6   2,048 rows 42.8 / 38.5   4,096 rows 68.0 / 63.4, with the ReLU mask 94 / 107
-struct StackPlan {
-    int groups = 0, chunk = 0;  // groups = 0: not eligible
-};
-inline StackPlan stack_plan(int n_img, int h, int width, int cin, int cout, bool any = false) {
-    StackPlan p;
-    if (width < kBM || cout > 256) return p;
-    const long rows = (long)n_img * ((width + kBM - 1) / kBM) * h;
-    if (!any && width % kBM == 0) {
-        const long sms = sm_count();
-        if (rows <= 2 * sms && cin > 16) return p;
-        if (rows <= 4 * sms && cout > kStackMaxCout && cin % 32 == 0) return p;
-    }
+// input-channel passes of the row-strip kernels (0: the layer is not theirs).  Several passes, summed through an fp32
+// partial: measured faster than the gather kernel for up to 64 output channels (176 -> 32, 160 -> 64), slower
+// for 96 -> 96 and 224 -> 96.
+inline int ws_passes(int width, int cin, int cout, bool any) {
+    if (width < kBM || cout > 256) return 0;
     for (int g = 1; g <= 4; ++g) {
-        if (g > 1 && cout > 64 && !any) return p;
-        const int cg = (cin / 16 + g - 1) / g * 16;
-        int occ, ring, chunk = 0, chunks = 0;
-        for (int n = (cout + kStackMaxCout - 1) / kStackMaxCout; n <= 4 && !chunk; ++n) {
-            const int c = (cout / 16 + n - 1) / n * 16;
-            if (!stack_config(cg, c, occ, ring)) continue;
-            chunk = c;
-            chunks = n;
+        int occ, ring;
+        if (ws_config(pass_channels(cin, g), cout, occ, ring)) return (g == 1 || cout <= 64 || any) ? g : 0;
+    }
+    return 0;
+}
+
+// The order of a layer's sums.  It is part of the result and a function of the layer and the image alone, whichever
+// kernel adds: fp32 sums in another order differ by 2e-7, which flips a few bf16 roundings and ReLU masks a layer, and
+// twenty layers make that 2 to 4 % of a training step's gradient - as far as it is from its 64-bit value.
+//   passes > 0: input channels in this many equal passes (the last may be smaller), whose sums are added in order; in
+//   a pass by image row (dy), channel group (64, then 32, then 16 channels), dx, channel.
+//   passes = 0: by K = tap * cin + channel, in ksplit runs of whole 64s, whose sums are added in order.
+struct ConvOrder {
+    int passes = 0, ksplit = 1;
+};
+
+// How the row-strip kernels take a layer.  Output channels: conv_stack_kernel for up to 80 of them, in chunks of at most
+// 80 (each launch reads the input again) or all of them in conv_ws_kernel (chunk = 0) beyond.  One or two passes over the
+// input channels in one launch where the weights and the rings fit, else a launch each through an fp32 partial.
+// us on one image up to 256 rows of 128 pixels, images of 256 rows beyond (boxes in the layer's order; "before": conv_ws
+// or, where it does not fit, the gather kernel, both without the kernels below):
+//                 rows  128: stack, box, before   256              512              1,024            4,096
+//     32 -> 32           8.3   6.4   9.6    8.9   7.0   9.6  10.2   8.9  10.2  12.3  14.3  11.9   24   41   29
+//     48 -> 48          11.0   9.5  12.2   11.7  17.7  12.3  14.8  30.2  12.7  18.7  57.0  19.7   37  249   72
+//     96 -> 32          13.3   9.0  14.4   14.9  10.2  14.6  18.5  18.8  14.8  24.8  35.2  24.1   67  122   94
+//    160 -> 64          39.1  15.3  44.9   41.3  19.3  46.0  55.4  36.8  46.9  73.9  70.2  75.0  209  261  307
+//    176 -> 32          20.4  14.1  30.9   21.3  16.0  31.4  29.0  30.2  32.1  37.8  57.7  49.6  109  214  211
+//     96 -> 96          25.8  11.4  29.3   28.7  15.3  33.1  36.7  28.3  64.6  52.0  54.1   128  142  194  459
+//     96 -> 224         53.1  16.6  40.3   57.7  30.5  79.2  73.7  57.6   156  96.1   102   275  235  385 1095
+//     32 -> 176         25.4  10.4  25.6   25.7  12.1  25.9  26.7  22.5  27.1  42.0  44.9  42.3  129  150  163
+// conv_box_kernel (on = false), whose tiles have a CTA each while these kernels read three rows for one and start with
+// all nine taps' weights, where the width is a multiple of 128: up to two rows an SM, beyond one unless its stages would
+// be more than half empty (48 channels in groups of 32 and 16); up to four with more than 80 output channels; up to
+// eight with two passes and more than 48.  conv_ws_kernel: between two and four rows an SM (eight from 96 input channels
+// on) for one pass of 48 input channels and more into at most 48; for 81 to 96 output channels; and for more of
+// fewer than 16 rows an SM.  Output chunks from 64 rows a chunk.
+struct StackPlan {
+    bool on = false;
+    int launches = 1;  // passes over the input channels with a launch each
+    int chunk = 0;
+};
+inline StackPlan stack_plan(int n_img, int h, int width, int cin, int cout, const ConvOrder& order, bool any) {
+    StackPlan p;
+    if (width < kBM || cout > 256 || order.ksplit > 1) return p;
+    const long rows = (long)n_img * ((width + kBM - 1) / kBM) * h;
+    const long sms = sm_count();
+    if (!any && width % kBM == 0 && order.passes <= 2) {
+        const bool filled = order.passes == 0 || 2 * cin >= 64 * ws_groups_of(cin, order.passes).n;
+        if (rows <= 2 * sms && cin > 16 && (filled || rows <= sms)) return p;
+        if (rows <= 4 * sms && cout > kStackMaxCout && cin % 32 == 0) return p;
+        if (rows <= 8 * sms && order.passes == 2 && cout > 48) return p;
+    }
+    // fewest output chunks of conv_stack_kernel with `passes` passes over c input channels
+    int chunks = 0;
+    auto fit = [&](int c, int passes) {
+        int occ, ring;
+        for (chunks = (cout + kStackMaxCout - 1) / kStackMaxCout; chunks <= 4; ++chunks) {
+            const int n = (cout / 16 + chunks - 1) / chunks * 16;
+            if (stack_config(c, n, passes, occ, ring)) return n;
         }
-        const bool ws = cout > kStackMaxCout && ws_config(cg, cout, occ, ring);
-        if (ws && !(chunk && cout > 96 && rows >= 16L * sm_count())) {
-            p.groups = g;
-            return p;
-        }
-        if (!chunk) continue;
-        if (chunks > 1 && rows < 64L * chunks && !any) return p;
-        p.groups = g;
-        p.chunk = chunk;
+        return 0;
+    };
+    if (order.passes <= 2) p.chunk = fit(cin, std::max(1, order.passes));
+    if (order.passes == 0) {
+        p.on = p.chunk > 0 && (chunks == 1 || rows >= 64L * chunks || any);
         return p;
     }
+    if (!p.chunk && order.passes > 1) {
+        p.launches = order.passes;
+        p.chunk = fit(pass_channels(cin, order.passes), 1);
+    }
+    // conv_ws_kernel fits (ws_passes)
+    const bool narrow = order.passes == 1 && cin >= 48 && cout <= 48 && rows > 2 * sms && rows <= (cin >= 96 ? 8 : 4) * sms;
+    const bool chunked = cout <= kStackMaxCout ? any || !narrow : cout > 96 && rows >= 16 * sms;
+    if (!chunked || (chunks > 1 && rows < 64L * chunks && !any)) p.chunk = 0;
+    if (!p.chunk) p.launches = order.passes;
+    p.on = true;
     return p;
 }
 
-// the tensor maps (widths 64, 32, 16) and the channel groups of a pass
-bool encode_groups(const StripArgs& a, WsArgs& wa, CUtensorMap (&maps)[3]) {
-    const WsGroups gr = ws_groups_of(a.cin);
+// the tensor maps (widths 64, 32, 16) and the channel groups of a launch
+bool encode_groups(const StripArgs& a, int passes, WsArgs& wa, CUtensorMap (&maps)[3]) {
+    const WsGroups gr = ws_groups_of(a.cin, passes);
     memset(maps, 0, sizeof(maps));
     bool have[3] = {false, false, false};
     for (int k = 0; k < gr.n; ++k) {
@@ -2860,8 +2970,8 @@ bool encode_groups(const StripArgs& a, WsArgs& wa, CUtensorMap (&maps)[3]) {
 }
 
 // the shared memory of a launch: at least what holds the CTAs per SM to per_sm (TMEM is sized for that many)
-inline size_t ws_smem(int cin, int cout, int per_sm, int ring) {
-    const size_t need = ws_weight_bytes(cin, cout) + (size_t)ring * ws_row_bytes(cin);
+inline size_t ws_smem(int cin, int cout, int passes, int per_sm, int ring) {
+    const size_t need = ws_weight_bytes(cin, cout) + (size_t)ring * ws_groups_of(cin, passes).row_bytes;
     return std::max(need, std::min(kSmPerCta, kSmPerSm / (per_sm + 1) - kWsStatic + 1024));
 }
 
@@ -2869,13 +2979,13 @@ cudaError_t launch_ws(StripArgs a, cudaStream_t s) {
     int per_sm = 0, ring = 0;
     WsArgs wa{};
     CUtensorMap maps[3];
-    if (!ws_config(a.cin, a.cout, per_sm, ring) || !encode_groups(a, wa, maps)) return cudaErrorInvalidValue;
+    if (!ws_config(a.cin, a.cout, per_sm, ring) || !encode_groups(a, 1, wa, maps)) return cudaErrorInvalidValue;
     a.tmem_cols = 2 * pow2_cols(a.cout);
     const int slots = sm_count() * per_sm;
     int total = 0;
     strip_segments(a.n, a.h, a.w_, slots, a.xtiles, a.seg_rows, a.segs_per_col, total);
     wa.s = a;
-    const size_t smem = ws_smem(a.cin, a.cout, per_sm, ring);
+    const size_t smem = ws_smem(a.cin, a.cout, 1, per_sm, ring);
     const cudaError_t e = cudaFuncSetAttribute(conv_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     conv_ws_kernel<<<min(total, slots), kWsThreads, smem, s>>>(maps[0], maps[1], maps[2], wa, ring);
@@ -2883,23 +2993,27 @@ cudaError_t launch_ws(StripArgs a, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-// output channels [co0, co0 + cout) of the cout_total of a layer (a.cout is set here)
-cudaError_t launch_stack(StripArgs a, int co0, int cout, int cout_total, cudaStream_t s) {
+// output channels [co0, co0 + cout) of the cout_total of a layer (a.cout is set here); passes: of this launch, 0 = the
+// products by tap
+cudaError_t launch_stack(StripArgs a, int co0, int cout, int cout_total, int passes, cudaStream_t s) {
+    const int sets = std::max(1, passes);
     a.cout = cout;
     StackArgs sa{};
     int per_sm = 0;
     CUtensorMap maps[3];
-    if (!stack_config(a.cin, cout, per_sm, sa.ring) || !encode_groups(a, sa.ws, maps)) return cudaErrorInvalidValue;
+    if (!stack_config(a.cin, cout, sets, per_sm, sa.ring) || !encode_groups(a, sets, sa.ws, maps))
+        return cudaErrorInvalidValue;
     a.tmem_cols = 512 / per_sm;  // the CTAs of an SM share its 512 columns
     a.xtiles = (a.w_ + kBM - 1) / kBM;
-    sa.sets = stack_sets(a.cin);
-    sa.blocks = std::min(kStackMaxBlocks, a.tmem_cols / (cout * sa.sets));
+    sa.groups0 = sets == 2 ? ws_groups_of(pass_channels(a.cin, 2)).n : sa.ws.ngroups;
+    sa.by_tap = passes == 0;
+    sa.blocks = std::min(kStackMaxBlocks, a.tmem_cols / (cout * sets));
     sa.co0 = co0;
     sa.cout_total = cout_total;
     sa.ws.s = a;
     const long rows = (long)a.n * a.xtiles * a.h;
     const int grid = (int)std::min<long>(std::max<long>(1, rows / 2), sm_count() * per_sm);  // at least two rows each
-    const size_t smem = ws_smem(a.cin, cout, per_sm, sa.ring);
+    const size_t smem = ws_smem(a.cin, cout, sets, per_sm, sa.ring);
     const cudaError_t e = cudaFuncSetAttribute(conv_stack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     conv_stack_kernel<<<grid, kStackThreads, smem, s>>>(maps[0], maps[1], maps[2], sa);
@@ -2918,13 +3032,18 @@ inline bool conv_box(int n, int h, int w, int& bh, int& bn) {
     return h % bh == 0 && rows % bh == 0;
 }
 
-cudaError_t launch_box(const ConvArgs& a, int bh, int bn, dim3 grid, cudaStream_t s) {
+cudaError_t launch_box(const ConvArgs& a, const ConvOrder& order, int bh, int bn, dim3 grid, cudaStream_t s) {
     EncodeTiledFn fn = encode_tiled();
     if (!fn) return cudaErrorInvalidValue;
     BoxArgs b{};
     b.c = a;
     b.bh = bh;
     b.bn = bn;
+    b.passes = order.passes;
+    b.pass_ch = order.passes ? pass_channels(a.cin, order.passes) : 0;
+    const int k64 = (9 * a.cin + 63) / 64;
+    b.kper = (k64 + order.ksplit - 1) / order.ksplit * 64;
+    if (order.passes == 2) b.c.tmem_cols = pow2_cols(2 * a.n_tile);
     b.cw = a.cin <= 16 ? 16 : (a.cin <= 32 ? 32 : 64);
     const CUtensorMapSwizzle sz = b.cw == 64 ? CU_TENSOR_MAP_SWIZZLE_128B
                                              : (b.cw == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B);
@@ -2953,7 +3072,8 @@ cudaError_t launch_box(const ConvArgs& a, int bh, int bn, dim3 grid, cudaStream_
 
 static int g_strip_kernel = 0;  // 0: warp-specialised (TMA) strips, 1: the cp.async strip kernel
 
-cudaError_t launch_strip(const ConvArgs& c, int groups, int chunk, cudaStream_t s) {
+// groups: passes over the input channels with a launch each; passes, chunk: of a launch (launch_stack)
+cudaError_t launch_strip(const ConvArgs& c, int groups, int chunk, int passes, cudaStream_t s) {
     StripArgs a{};
     a.x = c.x;
     a.w = c.w;
@@ -2968,7 +3088,7 @@ cudaError_t launch_strip(const ConvArgs& c, int groups, int chunk, cudaStream_t 
         if (chunk == 0) return launch_ws(p, s);
         cudaError_t e = cudaSuccess;
         for (int co = 0; co < c.cout && e == cudaSuccess; co += chunk)
-            e = launch_stack(p, co, min(chunk, c.cout - co), c.cout, s);
+            e = launch_stack(p, co, min(chunk, c.cout - co), c.cout, passes, s);
         return e;
     };
     if (groups <= 1) {
@@ -2985,7 +3105,7 @@ cudaError_t launch_strip(const ConvArgs& c, int groups, int chunk, cudaStream_t 
     const size_t bytes = (size_t)c.n * c.h * c.w_ * c.cout * sizeof(float);
     cudaError_t e = vpt::scratch_alloc(reinterpret_cast<void**>(&part), bytes, s);
     if (e != cudaSuccess) return e;
-    const int cg = (c.cin / 16 + groups - 1) / groups * 16;
+    const int cg = pass_channels(c.cin, groups);
     for (int g = 0, c0 = 0; c0 < c.cin && e == cudaSuccess; ++g, c0 += cg) {
         const bool last = c0 + cg >= c.cin;
         StripArgs p = a;
@@ -3045,42 +3165,46 @@ VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, cons
     a.out_f32 = out_f32;
     // row strips: the warp-specialised kernel's tensor map wants a 16-byte aligned base
     const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0;
-    StackPlan plan;
-    if (g_strip_kernel != 0) plan.groups = strip_groups(width, cin, cout, g_force_strip);
-    else if (aligned) plan = stack_plan(n, h, width, cin, cout, g_force_strip);
-    if (plan.groups > 0 && !g_force_gather)
-        return launch_strip(a, plan.groups, plan.chunk, static_cast<cudaStream_t>(stream)) == cudaSuccess ? VPT_OK
-                                                                                                       : VPT_ERR_CUDA;
+    const cudaStream_t s = static_cast<cudaStream_t>(stream);
+    auto status = [](cudaError_t e) { return e == cudaSuccess ? VPT_OK : VPT_ERR_CUDA; };
+    if (g_strip_kernel != 0 && !g_force_gather) {
+        const int groups = strip_groups(width, cin, cout, g_force_strip);
+        if (groups > 0) return status(launch_strip(a, groups, 0, 0, s));
+    }
     const long P = (long)n * h * width;
     const unsigned gx = (unsigned)((P + kBM - 1) / kBM), gy = (unsigned)((cout + a.n_tile - 1) / a.n_tile);
-    // small grids (the deep levels): split the K stages over more CTAs, raw fp32 sums finished by
-    // conv_finalize_kernel in a fixed order
+    const int sms = sm_count();
+    const long tiles = (long)gx * gy;
+    ConvOrder order;
+    if (g_strip_kernel == 0 && !g_force_gather && aligned) order.passes = ws_passes(width, cin, cout, g_force_strip);
+    if (order.passes == 0) {
+        // small grids (the deep levels): K split over more CTAs, raw fp32 sums finished by conv_finalize_kernel
+        const int nk = (9 * cin + kBK - 1) / kBK;
+        if (g_conv_ksplit > 1) order.ksplit = std::min(g_conv_ksplit, nk);
+        else if (g_conv_ksplit == 0 && 2 * tiles <= sms)  // under half a wave: about two CTAs per SM (measured)
+            order.ksplit = (int)std::max<long>(1, std::min<long>(std::min<long>(8, (2L * sms + tiles - 1) / tiles), nk / 2));
+    }
+    if (g_strip_kernel == 0 && !g_force_gather && aligned) {
+        const StackPlan plan = stack_plan(n, h, width, cin, cout, order, g_force_strip);
+        if (plan.on)
+            return status(launch_strip(a, plan.launches, plan.chunk, plan.launches > 1 ? 1 : order.passes, s));
+    }
     int bh = 1, bn = 1;
     const bool box = !g_force_gather && aligned && reinterpret_cast<uintptr_t>(w) % 16 == 0 &&
                      conv_box(n, h, width, bh, bn);
-    const int nk = box ? 9 * ((cin + kBK - 1) / kBK) : (9 * cin + kBK - 1) / kBK;
-    const int sms = sm_count();
-    const long tiles = (long)gx * gy;
-    int ksplit = 1;
-    if (g_conv_ksplit > 1) ksplit = std::min(g_conv_ksplit, nk);
-    else if (g_conv_ksplit == 0 && 2 * tiles <= sms)  // under half a wave: about two CTAs per SM (measured)
-        ksplit = (int)std::max<long>(1, std::min<long>(std::min<long>(8, (2L * sms + tiles - 1) / tiles), nk / 2));
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int ksplit = order.ksplit;
     if (ksplit == 1)
-        return (box ? launch_box(a, bh, bn, dim3(gx, gy, 1), s) : launch_tile<kConv>(a, dim3(gx, gy, 1), s)) == cudaSuccess
-                   ? VPT_OK
-                   : VPT_ERR_CUDA;
+        return status(box ? launch_box(a, order, bh, bn, dim3(gx, gy, 1), s) : launch_tile<kConv>(a, dim3(gx, gy, 1), s));
     float* part = nullptr;
     if (vpt::scratch_alloc(reinterpret_cast<void**>(&part), (size_t)ksplit * P * cout * sizeof(float), s) != cudaSuccess)
         return VPT_ERR_OOM;
     a.ksplit = ksplit;
     a.partial = part;
     const dim3 grid(gx, gy, (unsigned)ksplit);
-    cudaError_t e = box ? launch_box(a, bh, bn, grid, s) : launch_tile<kConv>(a, grid, s);
+    cudaError_t e = box ? launch_box(a, order, bh, bn, grid, s) : launch_tile<kConv>(a, grid, s);
     if (e == cudaSuccess) {
-        conv_finalize_kernel<<<grid_for(P * (cout / 4), 256), 256, 0, s>>>(part, ksplit, P, cout, bias,
-                                                                          static_cast<const bf16*>(mask), relu,
-                                                                          out_f32, y);
+        launch_units(P * (cout / 4), stream, conv_finalize_kernel<uint32_t>, conv_finalize_kernel<unsigned long long>,
+                     (const float*)part, ksplit, P, cout, bias, static_cast<const bf16*>(mask), relu, out_f32, y);
         e = cudaGetLastError();
     }
     const cudaError_t f = cudaFreeAsync(part, s);
