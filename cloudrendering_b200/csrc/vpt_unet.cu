@@ -36,6 +36,8 @@
 #include <math.h>
 #include <stdint.h>
 #include <string.h>
+#include <atomic>
+#include <type_traits>
 #include "../../include/vpt_b200.h"
 #include "vpt_kernels.h"
 #include "vpt_scratch.h"
@@ -2553,11 +2555,31 @@ inline int pow2_cols(int n) {
     return c;
 }
 
+constexpr size_t kSmPerSm = 233472;   // shared memory of one SM (bytes)
+constexpr size_t kSmPerCta = 232448;  // largest shared memory of one CTA
+
+// Raises a kernel's limit of dynamic shared memory to all that a CTA can have, once on every device.  The limit is state
+// of the process that every launch is checked against: set to the size of each launch, one thread could lower it
+// between another's setting and its launch.  It is a limit only, and does not change what a launch occupies.
+template <auto Kernel>
+cudaError_t allow_smem() {
+    static std::atomic<unsigned long long> done{0};  // a bit a device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+    if (done.load(std::memory_order_acquire) & bit) return cudaSuccess;
+    cudaFuncAttributes attr;
+    if ((e = cudaFuncGetAttributes(&attr, Kernel)) != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kSmPerCta - attr.sharedSizeBytes));
+    if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_release);
+    return e;
+}
+
 template <int MODE, int STAGES>
 cudaError_t launch_tile_n(const ConvArgs& a, dim3 grid, cudaStream_t s) {
     const size_t smem = (size_t)STAGES * (kBM * kBK * 2 + (size_t)a.n_tile * kBK * 2);
-    cudaError_t e = cudaFuncSetAttribute(conv_tile_kernel<MODE, STAGES>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem<conv_tile_kernel<MODE, STAGES>>();
     if (e != cudaSuccess) return e;
     conv_tile_kernel<MODE, STAGES><<<grid, kThreads, smem, s>>>(a);
     count_launches(1);
@@ -2671,7 +2693,7 @@ cudaError_t launch_strip_pass(StripArgs a, cudaStream_t s) {
     a.segs_per_col = (a.h + a.seg_rows - 1) / a.seg_rows;
     const int total = cols * a.segs_per_col;
     const int grid = min(total, slots);
-    cudaError_t e = cudaFuncSetAttribute(conv_strip_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem<conv_strip_kernel>();
     if (e != cudaSuccess) return e;
     conv_strip_kernel<<<grid, kThreads, smem, s>>>(a);
     count_launches(1);
@@ -2684,16 +2706,14 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 
 EncodeTiledFn encode_tiled() {
-    static EncodeTiledFn fn = nullptr;
-    static bool tried = false;
-    if (!tried) {
-        tried = true;
+    static const EncodeTiledFn fn = []() -> EncodeTiledFn {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-            q == cudaDriverEntryPointSuccess)
-            fn = reinterpret_cast<EncodeTiledFn>(p);
-    }
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            return nullptr;
+        return reinterpret_cast<EncodeTiledFn>(p);
+    }();
     return fn;
 }
 
@@ -2765,15 +2785,13 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* partial, int
     if (!encode_wgrad(&umap, ut, n, h, w, u_total, 32, a.u_lines) ||
         !encode_wgrad(&smap, st, n, h, w, p.role == 0 ? cout : cin, p.s_group, a.s_lines))
         return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(wgrad_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem<wgrad_rows_kernel>();
     if (e != cudaSuccess) return e;
     wgrad_rows_kernel<<<dim3((unsigned)p.grid, (unsigned)p.passes), kWgThreads, smem, s>>>(umap, smap, a);
     count_launches(1);
     return cudaGetLastError();
 }
 
-constexpr size_t kSmPerSm = 233472;   // shared memory of one SM (bytes)
-constexpr size_t kSmPerCta = 232448;  // largest dynamic shared memory of one CTA
 constexpr size_t kWsStatic = 2048;    // static shared memory + the per-CTA reservation, rounded up
 
 // a pass's channels as groups of 64, then 32, then 16 (each a 1024-byte aligned buffer of 130 lines)
@@ -2986,7 +3004,7 @@ cudaError_t launch_ws(StripArgs a, cudaStream_t s) {
     strip_segments(a.n, a.h, a.w_, slots, a.xtiles, a.seg_rows, a.segs_per_col, total);
     wa.s = a;
     const size_t smem = ws_smem(a.cin, a.cout, 1, per_sm, ring);
-    const cudaError_t e = cudaFuncSetAttribute(conv_ws_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem<conv_ws_kernel>();
     if (e != cudaSuccess) return e;
     conv_ws_kernel<<<min(total, slots), kWsThreads, smem, s>>>(maps[0], maps[1], maps[2], wa, ring);
     count_launches(1);
@@ -3014,7 +3032,7 @@ cudaError_t launch_stack(StripArgs a, int co0, int cout, int cout_total, int pas
     const long rows = (long)a.n * a.xtiles * a.h;
     const int grid = (int)std::min<long>(std::max<long>(1, rows / 2), sm_count() * per_sm);  // at least two rows each
     const size_t smem = ws_smem(a.cin, cout, sets, per_sm, sa.ring);
-    const cudaError_t e = cudaFuncSetAttribute(conv_stack_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem<conv_stack_kernel>();
     if (e != cudaSuccess) return e;
     conv_stack_kernel<<<grid, kStackThreads, smem, s>>>(maps[0], maps[1], maps[2], sa);
     count_launches(1);
@@ -3063,7 +3081,7 @@ cudaError_t launch_box(const ConvArgs& a, const ConvOrder& order, int bh, int bn
     if (!encode(&xmap, 4, a.x, xdims, xstr, xbox) || !encode(&wmap, 3, a.w, wdims, wstr, wbox))
         return cudaErrorInvalidValue;
     const size_t smem = (size_t)kBoxStages * ((size_t)kBM * b.cw * 2 + ((size_t)a.n_tile * b.cw * 2 + 1023) / 1024 * 1024);
-    const cudaError_t e = cudaFuncSetAttribute(conv_box_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    const cudaError_t e = allow_smem<conv_box_kernel>();
     if (e != cudaSuccess) return e;
     conv_box_kernel<<<grid, kBoxThreads, smem, s>>>(xmap, wmap, b);
     count_launches(1);
@@ -3136,7 +3154,7 @@ static bool g_force_strip = false;   // conv path 2: the strip kernels wherever 
 static int g_conv_ksplit = 0;        // gather convolution K splits: 0 automatic, 1 none, k > 1 forced
 
 static bool wgrad_on_rows(int w, int cin, int cout) {
-    return !g_force_gather && wgrad_by_rows(w, cin, cout, g_force_strip);
+    return !g_force_gather && wgrad_by_rows(w, cin, cout, g_force_strip) && encode_tiled();
 }
 
 extern "C" {
@@ -3163,8 +3181,8 @@ VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, cons
     a.tmem_cols = pow2_cols(a.n_tile);
     a.relu = relu;
     a.out_f32 = out_f32;
-    // row strips: the warp-specialised kernel's tensor map wants a 16-byte aligned base
-    const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0;
+    // tensor maps want a 16-byte aligned base (and the driver's encoder)
+    const bool aligned = reinterpret_cast<uintptr_t>(x) % 16 == 0 && encode_tiled();
     const cudaStream_t s = static_cast<cudaStream_t>(stream);
     auto status = [](cudaError_t e) { return e == cudaSuccess ? VPT_OK : VPT_ERR_CUDA; };
     if (g_strip_kernel != 0 && !g_force_gather) {
@@ -3404,23 +3422,22 @@ VptStatus vpt_unet_kpn_head(const float* logits, int head_channels, int kernel_s
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     bf16* dl = static_cast<bf16*>(dlogits);
     cudaError_t e = cudaErrorInvalidValue;
-    auto go = [&](auto kernel) {
-        if (smem > 48 * 1024 &&
-            cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
-            return cudaErrorInvalidValue;
-        kernel<<<blocks, 256, smem, s>>>(logits, head_channels, radiance, target, out, dl, loss_partial, n, h, w,
+    auto go = [&](auto size) {
+        constexpr int kSize = decltype(size)::value;
+        if (allow_smem<kpn_head_kernel<kSize>>() != cudaSuccess) return cudaErrorInvalidValue;
+        kpn_head_kernel<kSize><<<blocks, 256, smem, s>>>(logits, head_channels, radiance, target, out, dl, loss_partial, n, h, w,
                                          eps, inv_count);
         return cudaGetLastError();
     };
     switch (kernel_size) {
-        case 1: e = go(kpn_head_kernel<1>); break;
-        case 3: e = go(kpn_head_kernel<3>); break;
-        case 5: e = go(kpn_head_kernel<5>); break;
-        case 7: e = go(kpn_head_kernel<7>); break;
-        case 9: e = go(kpn_head_kernel<9>); break;
-        case 11: e = go(kpn_head_kernel<11>); break;
-        case 13: e = go(kpn_head_kernel<13>); break;
-        case 15: e = go(kpn_head_kernel<15>); break;
+        case 1: e = go(std::integral_constant<int, 1>()); break;
+        case 3: e = go(std::integral_constant<int, 3>()); break;
+        case 5: e = go(std::integral_constant<int, 5>()); break;
+        case 7: e = go(std::integral_constant<int, 7>()); break;
+        case 9: e = go(std::integral_constant<int, 9>()); break;
+        case 11: e = go(std::integral_constant<int, 11>()); break;
+        case 13: e = go(std::integral_constant<int, 13>()); break;
+        case 15: e = go(std::integral_constant<int, 15>()); break;
         default: return VPT_ERR_ARG;
     }
     if (e != cudaSuccess) return VPT_ERR_CUDA;

@@ -5,6 +5,7 @@ Tolerances: fp32 outputs of bf16 x bf16 -> fp32 products: |gpu - ref| <= 1e-5 * 
 (fp32 accumulation over K <= 2592 terms); bf16 outputs: one bf16 rounding, |gpu - ref| <=
 2^-8 * |ref| + 1e-6 * rms(ref)."""
 import ctypes
+import threading
 
 import numpy as np
 import pytest
@@ -417,3 +418,70 @@ def test_weight_gradient_of_runs_of_pixels(lib, case):
         own[k * pps:(k + 1) * pps] = dy.reshape(P, cout)[k * pps:(k + 1) * pps]
         ref = uo.conv3x3_weight_grad(x, own.reshape(n, h, w, cout))
         close_f32(host(part[k, :9 * cin]), ref.transpose(1, 2, 0).reshape(9 * cin, cout))
+
+
+def test_threads_launch_layers_of_different_sizes(lib):
+    """Threads on streams of their own run layers whose launches take different amounts of shared memory: every call
+    succeeds and gives what it gives alone."""
+    shapes = [(1, 16, 16, 16, 16), (1, 16, 16, 64, 256), (1, 8, 128, 32, 32), (1, 8, 256, 96, 64), (1, 24, 8, 224, 96)]
+
+    class Layer:
+        def __init__(self, n, h, w, cin, cout):
+            self.size = (n, h, w, cin, cout)
+            self.x, self.dy = dev_bf16(rng_data(91, n, h, w, cin)), dev_bf16(rng_data(92, n, h, w, cout))
+            self.w = dev_bf16(rng_data(93, cout, 9, cin, scale=1.0 / np.sqrt(9 * cin)))
+            self.logits, self.rad = dev_f32(rng_data(94, n, h, w, 232)), dev_f32(rng_data(95, n, 3, h, w))
+            self.splits = lib.vpt_unet_wgrad_splits(n, h, w, cin, cout, 64)
+            self.ks = 15 if cin > 32 else 3
+
+        def outputs(self):
+            n, h, w, cin, cout = self.size
+            rows = lib.vpt_unet_wgrad_rows(cin)
+            return (torch.zeros((n, h, w, cout), device="cuda"), torch.zeros((self.splits, rows, cout), device="cuda"),
+                    torch.zeros((n, 3, h, w), device="cuda"))
+
+        def run(self, out, err, stream):
+            n, h, w, cin, cout = self.size
+            hc = 232 if self.ks == 15 else 16
+            s = ctypes.c_void_p(stream.cuda_stream)
+            st = (lib.vpt_unet_conv3x3(ptr(self.x), ptr(self.w), None, None, ptr(out[0]), n, h, w, cin, cout, 0, 1,
+                                       ptr(err), s),
+                  lib.vpt_unet_conv3x3_wgrad(ptr(self.x), ptr(self.dy), ptr(out[1]), n, h, w, cin, cout, 64, ptr(err), s),
+                  lib.vpt_unet_kpn_head(ptr(self.logits), hc, self.ks, ptr(self.rad), None, ptr(out[2]), None, None, n,
+                                        h, w, ctypes.c_float(1e-2), s))
+            assert st == (0, 0, 0), (self.size, st)
+
+    layers = [Layer(*s) for s in shapes]
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = [layer.outputs() for layer in layers]
+    got = [[layer.outputs() for layer in layers] for _ in range(4)]
+    for layer, out in zip(layers, want):
+        layer.run(out, err, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(i):
+        try:
+            torch.cuda.set_device(0)
+            stream = torch.cuda.Stream()
+            for rep in range(100):
+                for k in range(len(layers)):
+                    j = (k + i) % len(layers)
+                    layers[j].run(got[i][j], err, stream)
+                if rep % 10 == 9:
+                    stream.synchronize()
+            stream.synchronize()
+        except BaseException as e:  # noqa: BLE001
+            errors.append(e)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors[0]
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    for outs in got:
+        for out, ref in zip(outs, want):
+            assert all(torch.equal(a, b) for a, b in zip(out, ref))
