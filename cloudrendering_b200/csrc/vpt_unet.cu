@@ -3294,7 +3294,7 @@ VptStatus vpt_unet_conv3x3_wgrad(const void* x, const void* dy, float* partial, 
 int vpt_unet_wgrad_rows(int cin) { return (9 * cin + kBM - 1) / kBM * kBM; }
 
 int vpt_unet_wgrad_splits(int n, int h, int width, int cin, int cout, int pixels_per_split) {
-    if (n <= 0 || h <= 0 || width <= 0 || pixels_per_split <= 0) return 0;
+    if (n <= 0 || h <= 0 || width <= 0 || !chan_ok(cin) || !chan_ok(cout) || cout > 4096 || pixels_per_split <= 0) return 0;
     if (wgrad_on_rows(width, cin, cout)) return wgrad_plan(n, h, width, cin, cout, sm_count()).grid;
     const long P = (long)n * h * width;
     return (int)((P + pixels_per_split - 1) / pixels_per_split);

@@ -54,3 +54,13 @@ def test_stateless_entry_points_reject_bad_arguments_without_gpu():
     assert lib.vpt_build_occupancy_grid(None, 8, 8, 8, 8, 0, 0.0, None, None) == 1
     assert lib.vpt_eaw_denoise_rgba(None, None, None, 4, 4, 1, 5.0, 0.1, 0.1, 0, None, None) == 1
     assert lib.vpt_build_environment_pyramid(None, 4, 4, 3, None, None) == 1
+
+
+def test_wgrad_splits_of_layers_that_do_not_exist():
+    """No partials (and no division by zero) for channel counts that the weight gradient refuses."""
+    lib = _lib.load()
+    for w in (64, 128):
+        assert lib.vpt_unet_wgrad_splits(1, 64, w, 32, 64, 64) > 0
+        for cin, cout in ((0, 32), (32, 0), (0, 0), (-16, 32), (32, -16), (24, 32), (32, 40), (32, 4112)):
+            assert lib.vpt_unet_wgrad_splits(1, 64, w, cin, cout, 64) == 0, (w, cin, cout)
+    assert lib.vpt_unet_wgrad_splits(1, 64, 64, 32, 64, 0) == 0
