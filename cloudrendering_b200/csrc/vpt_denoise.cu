@@ -1007,14 +1007,14 @@ extern "C" VptStatus vpt_svgf_filter(const float* noisy_rgba, const float* norma
     st.atrous_iterations = iterations;
     const float4* res = nullptr;
     // the last pass writes the output itself, unless the caller's output is one of the maps or histories
-    // that the passes still read
+    // that the passes still read, or no whole 16-byte words (a view into a buffer of floats)
     const struct {
         const void* p;
         size_t floats;
     } held[] = {{noisy_rgba, 4}, {normal_rgba, 4}, {color_history, 4}, {moments_history, 4}, {normal_history, 4},
                 {depth, 1},      {depth_fwidth, 1}, {motion, 2},       {depth_history, 1}};
     const uintptr_t o0 = reinterpret_cast<uintptr_t>(out_rgba);
-    bool direct = true;
+    bool direct = o0 % 16 == 0;
     for (const auto& b : held) {
         const uintptr_t p0 = reinterpret_cast<uintptr_t>(b.p);
         direct = direct && (o0 >= p0 + n * b.floats * 4 || p0 >= o0 + n * 16);

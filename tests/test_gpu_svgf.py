@@ -117,3 +117,22 @@ def test_svgf_tile_edges_match_the_oracle(w, h, iterations):
             # as above: rtol 1e-4, 0.1 % of the pixels (at least one) may take another branch
             close = (np.abs(got - exp) <= 1e-4 * (np.abs(exp) + 1e-3)).reshape(h * w, -1).all(axis=1)
             assert (~close).sum() <= max(1, h * w // 1000), (frame, name, (~close).sum())
+
+
+def test_svgf_output_at_any_float():
+    """An output that starts at any float of a larger buffer takes the same image, and nothing beside it."""
+    lib = _lib.load()
+    w, h = 70, 41
+    dev = [torch.from_numpy(a).cuda() for a in maps(h, w, 0, np.random.default_rng(12))]
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    want = None
+    for shift in range(4):
+        hist = [torch.zeros((h, w, 4), device="cuda") for _ in range(3)] + [torch.zeros((h, w), device="cuda")]
+        buf = torch.full((w * h * 4 + 8,), -7.0, device="cuda")
+        out = buf[shift:shift + w * h * 4]
+        assert lib.vpt_svgf_filter(*[p(t) for t in dev], *[p(t) for t in hist], w, h, ctypes.c_float(0.2),
+                                   ctypes.c_float(0.2), 3, p(out), None) == 0
+        torch.cuda.synchronize()
+        want = out.clone() if shift == 0 else want
+        assert torch.equal(out, want)
+        assert bool((buf[:shift] == -7.0).all()) and bool((buf[shift + w * h * 4:] == -7.0).all())
