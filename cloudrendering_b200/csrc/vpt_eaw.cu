@@ -134,7 +134,9 @@ struct EawPixel {
     }
 };
 
-// exponents' scales -log2(e) / phi, and the quirk's constant colour weight min(exp(-1 / phi_c), 1)
+// exponents' scales -log2(e) / phi.  The quirk's constant colour weight min(exp(-1 / phi_c), 1) is the same for every
+// tap: it cancels in the quotient of the sums and is left out (as a factor it would take the weights out of the
+// normal range for a small phi_c), except where it is 0, which leaves 0 / 0.
 __device__ __forceinline__ f32x2 eaw_scale(float phi) {
     const float s = -kLog2e / phi;
     return pack2(s, s);
@@ -143,7 +145,7 @@ __device__ __forceinline__ f32x2 eaw_color_scale(const EawPass& a) {
     return a.use_c && !a.quirk ? eaw_scale(a.phi_c) : 0ull;
 }
 __device__ __forceinline__ float eaw_bias(const EawPass& a) {
-    return a.use_c && a.quirk ? fminf(-kLog2e / a.phi_c, 0.0f) : 0.0f;
+    return a.use_c && a.quirk && expf(-1.0f / a.phi_c) == 0.0f ? -INFINITY : 0.0f;
 }
 
 // One pixel with the separate stops, its 25 taps taken from `taps` (fetch(i) gives the three maps).

@@ -279,6 +279,23 @@ def test_eaw_tiles_phi_and_non_finite_maps(core, w, h, iterations, phi, quirk):
                            atol=1e-6)
 
 
+@pytest.mark.parametrize("phi_color", [0.0098, 0.011, 0.012, 0.02])
+@pytest.mark.parametrize("maps", [True, False])
+def test_eaw_quirk_with_small_phi(core, phi_color, maps):
+    """The quirk's colour weight exp(-1 / phi_color) is the same for every tap and cancels, also where it is next to the
+    smallest float."""
+    w, h = 45, 38
+    g = np.random.default_rng(6)
+    color, pos, nrm = (g.random((h, w, 4), np.float32) for _ in range(3))
+    d = [torch.from_numpy(a).cuda() for a in (color, pos, nrm)]
+    out = torch.empty((h, w, 4), dtype=torch.float32, device="cuda")
+    m = (dptr(d[1]), dptr(d[2])) if maps else (None, None)
+    assert core.lib.vpt_eaw_denoise_rgba(dptr(d[0]), *m, w, h, 3, phi_color, 0.1, 0.1, 1, dptr(out), None) == 0
+    torch.cuda.synchronize()
+    ref = eaw_stops(color, pos if maps else None, nrm if maps else None, 3, (phi_color, 0.1, 0.1), 1)
+    assert np.allclose(out.cpu().numpy(), ref, rtol=3 * 4e-6, atol=1e-6)  # as above
+
+
 def test_eaw_rejects_an_output_that_overlaps_an_input(core):
     h, w = 16, 16
     imgs = [torch.rand((h, w, 4), device="cuda") for _ in range(3)]
