@@ -394,6 +394,8 @@ cudaError_t eaw_denoise(const float* color, const float* pos, const float* nrm, 
     a.quirk = s.ref_compute_quirk;
     const bool packed = s.phi_color >= 0.0f && s.phi_position >= 0.0f && s.phi_normal >= 0.0f;
     const bool lattice = s.lattice_tiles != 0;
+    // steps of 65,536 pixels and more are refused with lattice tiles
+    if (lattice && s.iterations > 16) return cudaErrorInvalidValue;
     const float* src = color;
     float* bufs[2] = {ping, pong};
     a.step = 1;
@@ -406,7 +408,7 @@ cudaError_t eaw_denoise(const float* color, const float* pos, const float* nrm, 
                            : launch_pass<false, false>(a, lattice, packed, stream));
         if (e != cudaSuccess) return e;
         src = a.out;
-        a.step *= 2;
+        a.step = std::min(a.step * 2, 1 << 28);  // (taps that far are at the edge: the same image at any larger step)
     }
     *result = const_cast<float*>(src);
     return cudaGetLastError();

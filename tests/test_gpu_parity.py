@@ -296,6 +296,18 @@ def test_eaw_quirk_with_small_phi(core, phi_color, maps):
     assert np.allclose(out.cpu().numpy(), ref, rtol=3 * 4e-6, atol=1e-6)  # as above
 
 
+def test_eaw_iteration_limit(core):
+    """Sixteen iterations are filtered, more are refused; the denoiser without lattice tiles takes them."""
+    h, w = 9, 14
+    color = np.random.default_rng(7).random((h, w, 4), np.float32)
+    d, out = torch.from_numpy(color).cuda(), torch.empty((h, w, 4), device="cuda")
+    call = lambda n: core.lib.vpt_eaw_denoise_rgba(dptr(d), None, None, w, h, n, 5.0, 0.1, 0.1, 0, dptr(out), None)
+    assert call(16) == 0
+    torch.cuda.synchronize()
+    assert np.allclose(out.cpu().numpy(), eaw_stops(color, None, None, 16, (5.0, 0.1, 0.1)), rtol=16 * 4e-6, atol=1e-6)
+    assert call(17) != 0 and call(40) != 0
+
+
 def test_eaw_rejects_an_output_that_overlaps_an_input(core):
     h, w = 16, 16
     imgs = [torch.rand((h, w, 4), device="cuda") for _ in range(3)]
