@@ -392,7 +392,9 @@ cudaError_t eaw_denoise(const float* color, const float* pos, const float* nrm, 
     a.phi_n = s.phi_normal;
     a.use_c = s.use_color;
     a.quirk = s.ref_compute_quirk;
-    const bool packed = s.phi_color >= 0.0f && s.phi_position >= 0.0f && s.phi_normal >= 0.0f;
+    // the stops in use have phi >= 0
+    const bool packed = (!a.use_c || s.phi_color >= 0.0f) && (!a.pos || s.phi_position >= 0.0f) &&
+                        (!a.nrm || s.phi_normal >= 0.0f);
     const bool lattice = s.lattice_tiles != 0;
     // steps of 65,536 pixels and more are refused with lattice tiles
     if (lattice && s.iterations > 16) return cudaErrorInvalidValue;

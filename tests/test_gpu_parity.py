@@ -296,6 +296,20 @@ def test_eaw_quirk_with_small_phi(core, phi_color, maps):
     assert np.allclose(out.cpu().numpy(), ref, rtol=3 * 4e-6, atol=1e-6)  # as above
 
 
+def test_eaw_phi_of_a_map_that_is_not_there(core):
+    """A negative phi matters where its map is filtered with; without the map the tiles serve, at their speed."""
+    from torch.profiler import ProfilerActivity, profile
+    d, out = torch.rand((64, 96, 4), device="cuda"), torch.empty((64, 96, 4), device="cuda")
+    outs = []
+    for phi in (0.1, -1.0):
+        with profile(activities=[ProfilerActivity.CUDA]) as p:
+            assert core.lib.vpt_eaw_denoise_rgba(dptr(d), None, None, 96, 64, 1, 5.0, phi, phi, 0, dptr(out), None) == 0
+            torch.cuda.synchronize()
+        assert any("eaw_lattice_kernel" in e.name for e in p.events()), phi
+        outs.append(out.clone())
+    assert torch.equal(*outs)
+
+
 def test_eaw_iteration_limit(core):
     """Sixteen iterations are filtered, more are refused; the denoiser without lattice tiles takes them."""
     h, w = 9, 14
