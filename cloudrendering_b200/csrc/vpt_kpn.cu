@@ -66,12 +66,18 @@ __device__ __forceinline__ float tap_exponentials(const float* __restrict__ wbas
     return s;
 }
 
-// sum of p[t] * tile over the taps inside the w x h output, for the thread's pixel (x, y)
+// first pixel of the block (the tiles of an image are counted along x, row by row, so that any height fits the grid)
+__device__ __forceinline__ int2 tile_origin(int w) {
+    const int tiles_x = (w + kKpnTileW - 1) / kKpnTileW, ty = (int)blockIdx.x / tiles_x;
+    return make_int2(((int)blockIdx.x - ty * tiles_x) * kKpnTileW, ty * kKpnTileH);
+}
+
+// sum of p[t] * tile over the taps inside the w x h output, for the thread's pixel of the block at (bx, by)
 template <int KS>
-__device__ __forceinline__ float4 apply_taps(const KpnTile<KS>& tile, const float* p, int x, int y, int w, int h) {
+__device__ __forceinline__ float4 apply_taps(const KpnTile<KS>& tile, const float* p, int bx, int by, int w, int h) {
     constexpr int R = KS / 2;
+    const int x = bx + threadIdx.x, y = by + threadIdx.y;
     // every tap of every pixel of the block lies inside: no test per tap
-    const int bx = blockIdx.x * kKpnTileW, by = blockIdx.y * kKpnTileH;
     const bool inner = bx >= R && by >= R && bx + kKpnTileW + R <= w && by + kKpnTileH + R <= h;
     float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 #pragma unroll
@@ -102,14 +108,14 @@ __global__ void __launch_bounds__(kKpnTileW* kKpnTileH)
                      int C, int H, int W, int Hw, int Ww, int h, int w, int softmax) {
     constexpr int K = KS * KS;
     __shared__ KpnTile<KS> tile;
-    const int x = blockIdx.x * kKpnTileW + threadIdx.x;
-    const int y = blockIdx.y * kKpnTileH + threadIdx.y;
+    const int2 org = tile_origin(w);
+    const int x = org.x + threadIdx.x, y = org.y + threadIdx.y;
     const int n = blockIdx.z;
     const float* img = image + (size_t)n * C * H * W;
     for (int q = threadIdx.y * kKpnTileW + threadIdx.x; q < KpnTile<KS>::kW * KpnTile<KS>::kH;
          q += kKpnTileW * kKpnTileH) {
         const int tx = q % KpnTile<KS>::kW, ty = q / KpnTile<KS>::kW;
-        const int gx = (int)blockIdx.x * kKpnTileW + tx - KS / 2, gy = (int)blockIdx.y * kKpnTileH + ty - KS / 2;
+        const int gx = org.x + tx - KS / 2, gy = org.y + ty - KS / 2;
         float v[kMaxKpnChannels] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (gx >= 0 && gx < w && gy >= 0 && gy < h) {
 #pragma unroll
@@ -133,7 +139,7 @@ __global__ void __launch_bounds__(kKpnTileW* kKpnTileH)
     }
     __syncthreads();
     if (!in) return;
-    const float4 acc = apply_taps<KS>(tile, p, x, y, w, h);
+    const float4 acc = apply_taps<KS>(tile, p, org.x, org.y, w, h);
     const float r[kMaxKpnChannels] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
     for (int c = 0; c < kMaxKpnChannels; c++)
@@ -185,13 +191,13 @@ template <int KS>
 __global__ void __launch_bounds__(kKpnTileW* kKpnTileH) kpn_inv_iter_kernel(const InvIterArgs a) {
     constexpr int K = KS * KS;
     __shared__ KpnTile<KS> tile;
-    const int x = blockIdx.x * kKpnTileW + threadIdx.x;
-    const int y = blockIdx.y * kKpnTileH + threadIdx.y;
+    const int2 org = tile_origin(a.w);
+    const int x = org.x + threadIdx.x, y = org.y + threadIdx.y;
     const int n = blockIdx.z;
     for (int q = threadIdx.y * kKpnTileW + threadIdx.x; q < KpnTile<KS>::kW * KpnTile<KS>::kH;
          q += kKpnTileW * kKpnTileH) {
         const int tx = q % KpnTile<KS>::kW, ty = q / KpnTile<KS>::kW;
-        const int gx = (int)blockIdx.x * kKpnTileW + tx - KS / 2, gy = (int)blockIdx.y * kKpnTileH + ty - KS / 2;
+        const int gx = org.x + tx - KS / 2, gy = org.y + ty - KS / 2;
         float v[kMaxKpnChannels] = {0.0f, 0.0f, 0.0f, 0.0f};
         if (gx >= 0 && gx < a.w && gy >= 0 && gy < a.h) inv_iter_base(a, n, gx, gy, v);
         tile.px[ty][tx] = make_float4(v[0], v[1], v[2], v[3]);
@@ -203,7 +209,7 @@ __global__ void __launch_bounds__(kKpnTileW* kKpnTileH) kpn_inv_iter_kernel(cons
     if (in) s = tap_exponentials<KS>(a.fused + (size_t)n * (K + 3) * plane + (size_t)y * a.Ww + x, plane, p);
     __syncthreads();
     if (!in) return;
-    const float4 acc = apply_taps<KS>(tile, p, x, y, a.w, a.h);
+    const float4 acc = apply_taps<KS>(tile, p, org.x, org.y, a.w, a.h);
     const float r[kMaxKpnChannels] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
     for (int c = 0; c < kMaxKpnChannels; c++)
@@ -260,7 +266,7 @@ __global__ void kpn_reproject_kernel(const float* __restrict__ prev, const float
 
 dim3 grid2d(int w, int h, int n) { return dim3((w + 15) / 16, (h + 15) / 16, n); }
 dim3 tile_grid(int w, int h, int n) {
-    return dim3((w + kKpnTileW - 1) / kKpnTileW, (h + kKpnTileH - 1) / kKpnTileH, n);
+    return dim3((unsigned)((w + kKpnTileW - 1) / kKpnTileW) * (unsigned)((h + kKpnTileH - 1) / kKpnTileH), 1, n);
 }
 
 }  // namespace

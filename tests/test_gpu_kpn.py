@@ -178,3 +178,15 @@ def test_apply_without_softmax_skips_taps_outside():
     wts[0, 2::3, :, -1] = np.inf  # the column right of the last
     got = kpn.apply_kernels(cuda(img), cuda(wts), 3, softmax=False).cpu().numpy()
     assert np.all(np.isfinite(got)) and got[0, 0, 5, 5] == 9.0 and got[0, 0, 0, 5] == 6.0 and got[0, 0, 0, 39] == 4.0
+
+
+@pytest.mark.parametrize("h", [524281, 1000003])
+def test_tall_images(h):
+    """More rows of tiles than a grid has in y (65,535): images of up to 1,048,560 rows are taken."""
+    img, logits = rnd(1, 1, h, 1, seed=31), rnd(1, 9, h, 1, seed=32)
+    got = kpn.apply_kernels(cuda(img), cuda(logits), 3, True).cpu().numpy()
+    assert np.allclose(got, bridge.kpn_apply(img, logits, 3, softmax=True), rtol=RTOL, atol=9 * ATOL)
+    half = rnd(1, 1, h // 2, 1, seed=33)
+    fused = rnd(1, 12, h, 1, seed=34)
+    got = kpn.inv_iter(cuda(img), cuda(half), cuda(half), None, cuda(fused), 3).cpu().numpy()
+    assert np.allclose(got, bridge.kpn_inv_iter(img, half, half, img, fused, 3, False), rtol=RTOL, atol=9 * ATOL)
