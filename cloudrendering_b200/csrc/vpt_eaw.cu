@@ -196,8 +196,10 @@ struct GlobalTaps {
 // clamp.
 template <bool POS, bool NRM>
 __global__ void eaw_iteration_kernel(const __grid_constant__ EawPass a, int packed) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    const int y = blockIdx.y * blockDim.y + threadIdx.y;
+    // blocks of 32 x 4 pixels, counted along x row by row, so that any height fits the grid
+    const int blocks_x = (a.w + 31) / 32, by = (int)blockIdx.x / blocks_x;
+    const int x = ((int)blockIdx.x - by * blocks_x) * 32 + (int)threadIdx.x;
+    const int y = by * 4 + (int)threadIdx.y;
     if (x >= a.w || y >= a.h) return;
     const GlobalTaps taps{a, x, y};
     float4 o;
@@ -350,8 +352,8 @@ static cudaError_t launch_pass(EawPass a, bool lattice, bool packed, cudaStream_
         constexpr int smem = (1 + POS + NRM) * kEawPatchW * kEawPatchH * (int)sizeof(float4);
         eaw_lattice_kernel<POS, NRM><<<(unsigned)blocks, kEawTileW * kEawTileH / kEawRowsOf<POS, NRM>, smem, s>>>(a);
     } else {
-        const dim3 b(32, 4), g((a.w + 31) / 32, (a.h + 3) / 4);
-        eaw_iteration_kernel<POS, NRM><<<g, b, 0, s>>>(a, packed);
+        const unsigned g = (unsigned)((a.w + 31) / 32) * (unsigned)((a.h + 3) / 4);
+        eaw_iteration_kernel<POS, NRM><<<g, dim3(32, 4), 0, s>>>(a, packed);
     }
     count_launches(1);
     return cudaGetLastError();

@@ -310,6 +310,16 @@ def test_eaw_phi_of_a_map_that_is_not_there(core):
     assert torch.equal(*outs)
 
 
+@pytest.mark.parametrize("w,h", [(1, 300001), (2, 1000000), (300001, 1)])
+def test_eaw_long_images(core, w, h):
+    """Images of few columns, whose passes read their taps directly, of more rows than a grid has 4-row blocks in y."""
+    color = np.random.default_rng(8).random((h, w, 4), np.float32)
+    d, out = torch.from_numpy(color).cuda(), torch.empty((h, w, 4), device="cuda")
+    assert core.lib.vpt_eaw_denoise_rgba(dptr(d), None, None, w, h, 2, 5.0, 0.1, 0.1, 0, dptr(out), None) == 0
+    torch.cuda.synchronize()
+    assert np.allclose(out.cpu().numpy(), eaw_stops(color, None, None, 2, (5.0, 0.1, 0.1)), rtol=2 * 4e-6, atol=1e-6)
+
+
 def test_eaw_iteration_limit(core):
     """Sixteen iterations are filtered, more are refused; the denoiser without lattice tiles takes them."""
     h, w = 9, 14
