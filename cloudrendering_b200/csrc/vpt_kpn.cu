@@ -30,7 +30,8 @@ constexpr int kMaxTaps = 49;  // kernels up to 7 x 7
 // or the inv_iter base) of its pixels and their KS / 2 neighbourhood in shared memory, one float4 a pixel,
 // and each thread applies its pixel's kernel to it.  The k*k logits are read once, coalesced, while the
 // staging is in flight; they are the traffic that bounds the kernels ((k^2 + 2C) x 4 bytes a pixel).
-// The softmax divides once, after the weighted sum, instead of once per tap.
+// The softmax divides once, after the weighted sum, instead of once per tap; a sum that overflows for that (values
+// above FLT_MAX / k^2) is taken again with the weights divided first.
 // Measured, the three-scale reconstruction of a 1280 x 720 image with 4 channels and 5 x 5 kernels: 625 us with the
 // base recomputed for every tap, 105 us so (164 MB: 25 us at 6.65 TB/s); error against 64 bits 7.4e-8 (was 1.03e-7).
 constexpr int kKpnTileW = 32, kKpnTileH = 8;
@@ -102,6 +103,37 @@ __device__ __forceinline__ float4 apply_taps(const KpnTile<KS>& tile, const floa
     return acc;
 }
 
+// The thread's weighted sum with every weight divided by the sum of exponentials first: where the undivided sum
+// overflows.  Reads the logits again (a second use of apply_taps' registers made the three-scale reconstruction 124 us).
+template <int KS>
+__device__ __noinline__ float4 apply_divided(const KpnTile<KS>& tile, const float* __restrict__ wbase, size_t plane, float s,
+                                             int bx, int by, int w, int h) {
+    constexpr int R = KS / 2;
+    float m = -INFINITY;
+    for (int k = 0; k < KS * KS; k++) m = fmaxf(m, __ldg(wbase + (size_t)k * plane));
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int k = 0; k < KS * KS; k++) {
+        const int dy = k / KS - R, dx = k % KS - R, x = bx + threadIdx.x + dx, y = by + threadIdx.y + dy;
+        if (x < 0 || x >= w || y < 0 || y >= h) continue;
+        const float4 v = tile.px[threadIdx.y + R + dy][threadIdx.x + R + dx];
+        const float wt = expf(__ldg(wbase + (size_t)k * plane) - m) / s;
+        acc.x = fmaf(wt, v.x, acc.x);
+        acc.y = fmaf(wt, v.y, acc.y);
+        acc.z = fmaf(wt, v.z, acc.z);
+        acc.w = fmaf(wt, v.w, acc.w);
+    }
+    return acc;
+}
+
+// acc / s, or apply_divided's sum where acc is not finite
+template <int KS>
+__device__ __forceinline__ float4 divide_taps(float4 acc, const KpnTile<KS>& tile, const float* __restrict__ wbase,
+                                              size_t plane, float s, int bx, int by, int w, int h) {
+    if (!(isfinite(acc.x) && isfinite(acc.y) && isfinite(acc.z) && isfinite(acc.w)))
+        return apply_divided<KS>(tile, wbase, plane, s, bx, by, w, h);
+    return make_float4(acc.x / s, acc.y / s, acc.z / s, acc.w / s);
+}
+
 template <int KS>
 __global__ void __launch_bounds__(kKpnTileW* kKpnTileH)
     kpn_apply_kernel(const float* __restrict__ image, const float* __restrict__ weights, float* __restrict__ out, int N,
@@ -126,10 +158,10 @@ __global__ void __launch_bounds__(kKpnTileW* kKpnTileH)
     }
     const bool in = x < w && y < h;
     const size_t plane = (size_t)Hw * Ww;
+    const float* wb = weights + (size_t)n * K * plane + (in ? (size_t)y * Ww + x : 0);
     float p[K];
     float s = 1.0f;
     if (in) {
-        const float* wb = weights + (size_t)n * K * plane + (size_t)y * Ww + x;
         if (softmax) {
             s = tap_exponentials<KS>(wb, plane, p);
         } else {
@@ -139,11 +171,12 @@ __global__ void __launch_bounds__(kKpnTileW* kKpnTileH)
     }
     __syncthreads();
     if (!in) return;
-    const float4 acc = apply_taps<KS>(tile, p, org.x, org.y, w, h);
+    float4 acc = apply_taps<KS>(tile, p, org.x, org.y, w, h);
+    if (softmax) acc = divide_taps<KS>(acc, tile, wb, plane, s, org.x, org.y, w, h);
     const float r[kMaxKpnChannels] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
     for (int c = 0; c < kMaxKpnChannels; c++)
-        if (c < C) out[(((size_t)n * C + c) * h + y) * w + x] = softmax ? r[c] / s : r[c];
+        if (c < C) out[(((size_t)n * C + c) * h + y) * w + x] = r[c];
 }
 
 __device__ __forceinline__ float sigmoidf(float v) { return 1.0f / (1.0f + expf(-v)); }
@@ -206,14 +239,16 @@ __global__ void __launch_bounds__(kKpnTileW* kKpnTileH) kpn_inv_iter_kernel(cons
     const size_t plane = (size_t)a.Hw * a.Ww;
     float p[K];
     float s = 1.0f;
-    if (in) s = tap_exponentials<KS>(a.fused + (size_t)n * (K + 3) * plane + (size_t)y * a.Ww + x, plane, p);
+    const float* wb = a.fused + (size_t)n * (K + 3) * plane + (in ? (size_t)y * a.Ww + x : 0);
+    if (in) s = tap_exponentials<KS>(wb, plane, p);
     __syncthreads();
     if (!in) return;
-    const float4 acc = apply_taps<KS>(tile, p, org.x, org.y, a.w, a.h);
+    const float4 acc = divide_taps<KS>(apply_taps<KS>(tile, p, org.x, org.y, a.w, a.h), tile, wb, plane, s, org.x, org.y,
+                                       a.w, a.h);
     const float r[kMaxKpnChannels] = {acc.x, acc.y, acc.z, acc.w};
 #pragma unroll
     for (int c = 0; c < kMaxKpnChannels; c++)
-        if (c < a.C) a.out[(((size_t)n * a.C + c) * a.h + y) * a.w + x] = r[c] / s;
+        if (c < a.C) a.out[(((size_t)n * a.C + c) * a.h + y) * a.w + x] = r[c];
 }
 
 // torch::avg_pool2d(x, 2, 2): floor(H/2) x floor(W/2), mean of each 2 x 2 block

@@ -190,3 +190,21 @@ def test_tall_images(h):
     fused = rnd(1, 12, h, 1, seed=34)
     got = kpn.inv_iter(cuda(img), cuda(half), cuda(half), None, cuda(fused), 3).cpu().numpy()
     assert np.allclose(got, bridge.kpn_inv_iter(img, half, half, img, fused, 3, False), rtol=RTOL, atol=9 * ATOL)
+
+
+def test_softmax_of_values_near_the_largest_float():
+    """Weighted means of values up to the largest float are finite, although the sum of the undivided weights
+    times the values is not; a pixel beside them is as accurate as before."""
+    big = np.float32(3e38)
+    img = np.full((1, 3, 20, 40), big, np.float32)
+    img[0, 1] = rnd(20, 40, seed=41)
+    logits = rnd(1, 25, 20, 40, seed=42)
+    got = kpn.apply_kernels(cuda(img), cuda(logits), 5, True).cpu().numpy()
+    assert np.allclose(got, bridge.kpn_apply(img, logits, 5, softmax=True), rtol=RTOL, atol=25 * ATOL)
+    fused = rnd(1, 28, 20, 40, seed=43)
+    fused[0, 25] = 30.0  # the base is the low-resolution prediction
+    fused[0, 26] = -90.0
+    lo = np.full((1, 3, 10, 20), big, np.float32)
+    got = kpn.inv_iter(cuda(img), cuda(lo), cuda(lo), None, cuda(fused), 5).cpu().numpy()
+    want = bridge.kpn_inv_iter(img, lo, lo, img, fused, 5, False)
+    assert np.isfinite(want).all() and np.allclose(got, want, rtol=RTOL, atol=25 * ATOL)
