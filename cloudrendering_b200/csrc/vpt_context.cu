@@ -149,7 +149,7 @@ struct VptContext {
     float pending_voxel_size[3] = {1.0f, 1.0f, 1.0f};  // spacing for the next grid
     int use_ess = 0;
     int ess_ref_compat = 0;
-    int schedule = vpt::kScheduleRefill;
+    int schedule = vpt::kScheduleAuto;
     int persistent_blocks_per_sm = 0;  // 0 = occupancy calculator (one resident wave)
     uint32_t max_steps = vpt::kMaxStepsPerPath;
     float fbm_contrast = 3.5f;  // remap of the fBm generator: clamp(0.5 + contrast * fbm, 0, 1)

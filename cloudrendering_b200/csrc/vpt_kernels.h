@@ -8,7 +8,8 @@ namespace vpt {
 
 constexpr int kTraceBlock = 128;
 
-enum Schedule : int { kScheduleTiles = 0, kSchedulePersistent = 1, kScheduleRefill = 2 };
+// kScheduleAuto (no schedule asked for): kScheduleRefill, and small delta and ratio launches kSchedulePersistent
+enum Schedule : int { kScheduleTiles = 0, kSchedulePersistent = 1, kScheduleRefill = 2, kScheduleAuto = 3 };
 
 struct FbmParams {
     int octaves;

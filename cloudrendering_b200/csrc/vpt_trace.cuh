@@ -1247,22 +1247,26 @@ static cudaError_t launch_trace_t(const TraceParams& P, int schedule, int featur
     constexpr bool kEvents = TRACKER == kDelta || TRACKER == kRatio || TRACKER == kNextEvent ||
                              TRACKER == kNextEvent + 100 || (TRACKER == kDecomposition && GRID != kNanoVdb);
     constexpr bool kRefillable = TRACKER == kDeltaIso || (TRACKER == kResidualRatioNee && GRID != kNanoVdb);
+    const bool refill = schedule == kScheduleRefill || schedule == kScheduleAuto;
     if constexpr (kEvents) {
-        if (schedule == kScheduleRefill && !features) {
+        if (refill && !features) {
             static int per_sm = 0;
-            const int blocks = resident_blocks(trace_event_kernel<TRACKER, INTERP, GRID, TF>, per_sm, persistent_blocks);
-            const uint64_t share = total / ((uint64_t)blocks * (kTraceBlock / 32));
+            const int resident = resident_blocks(trace_event_kernel<TRACKER, INTERP, GRID, TF>, per_sm, 0);
+            const int blocks = persistent_blocks > 0 ? persistent_blocks : resident;
             // Delta and ratio tracking with fewer than five paths per resident lane: the launch lasts as long as
             // its longest path, whose steps are shortest on persistent batches (nothing to wait for): 256^2 paths of
             // the 128^3 cloud 580 against 655 us, 512^2 690 / 810, 2 x 512^2 930 / 1040, 4 x 512^2 1370 / 1360,
             // 8 x 512^2 2290 / 2200.  The other trackers' events make batches two to three times slower at any size.
+            // (A schedule that was asked for is taken at any size.)
             constexpr bool kShortEvents = TRACKER == kDelta || TRACKER == kRatio;
-            if (!kShortEvents || share >= 160 || persistent_blocks > 0)
-                return launch_events<TRACKER, INTERP, GRID, TF>(P, total, blocks, share, stream);
+            constexpr uint64_t kWarps = kTraceBlock / 32;
+            if (!kShortEvents || total / ((uint64_t)resident * kWarps) >= 160 || schedule == kScheduleRefill)
+                return launch_events<TRACKER, INTERP, GRID, TF>(P, total, blocks, total / ((uint64_t)blocks * kWarps),
+                                                                stream);
         }
     }
     // the refill loop's surface check has no closing surfaces (CLOSE_ISOSURFACES): persistent batches then
-    if (schedule == kScheduleRefill && kRefillable && !features && !P.iso_close) {
+    if (refill && kRefillable && !features && !P.iso_close) {
         if constexpr (kRefillable) {
             static int per_sm = 0;
             const int blocks = resident_blocks(trace_refill_kernel<TRACKER, INTERP, GRID, TF>, per_sm, persistent_blocks);
@@ -1272,7 +1276,7 @@ static cudaError_t launch_trace_t(const TraceParams& P, int schedule, int featur
             return cudaGetLastError();
         }
     }
-    if (schedule == kScheduleRefill) schedule = kSchedulePersistent;
+    if (refill) schedule = kSchedulePersistent;
     if (schedule == kScheduleTiles) {
         uint64_t blocks = (total + kTraceBlock - 1) / kTraceBlock;
         trace_tiles_kernel<TRACKER, INTERP, GRID, TF><<<(unsigned)blocks, kTraceBlock, 0, stream>>>(P, features);

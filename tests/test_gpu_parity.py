@@ -541,8 +541,8 @@ def test_schedules_trace_identical_paths(core_dr, mode):
 def test_deferred_events_trace_identical_paths(core_dr, mode, interp, size):
     """The refill schedule's loop that defers path events traces the paths of the tile schedule: launches of less
     than a path per lane (the decomposition tracker spreads those over the warps), of part of a warp and of
-    several waves, shadow rays that walk ahead of their lookups, and one block per SM (which also takes the
-    small delta and ratio launches to this loop).  Same film up to the order of the FP64 additions."""
+    several waves, shadow rays that walk ahead of their lookups, and one block per SM.  Same film up to the order
+    of the FP64 additions."""
     core = core_dr
     kw = dict(PATH_CASES["nee_lights"]) if mode == "nee_lights" else dict(mode=mode)
     if mode == "nee_ess":
@@ -644,3 +644,30 @@ def test_eaw_compute_path_matches_reference_shader(core):
                                              dptr(out), None) == 0
         torch.cuda.synchronize()
         assert np.allclose(out.cpu().numpy(), ref, rtol=1e-5, atol=2e-5), key
+
+
+def traced_with(core, sp, frames):
+    """Names of the tracer kernels of one render call."""
+    from torch.profiler import ProfilerActivity, profile
+    with profile(activities=[ProfilerActivity.CUDA]) as p:
+        gpu_render(core, sp, frames, stats=False)
+        torch.cuda.synchronize()
+    return [k for k in ("trace_event", "trace_persistent", "trace_refill", "trace_tiles")
+            if any(k in e.name for e in p.events())]
+
+
+def test_a_schedule_that_is_set_is_taken():
+    """Until a schedule is set a small delta launch runs on persistent batches, a large one on the refill schedule, at
+    any number of blocks; a schedule that is set is taken at every size."""
+    core = Core()
+    small, large = (fbm_scene(width=w, height=w, mode="delta") for w in (40, 512))
+    for sp, frames, kernel in ((small, 1, "trace_persistent"), (large, 8, "trace_event")):
+        setup_core(core, sp)
+        for blocks in (0.0, 1.0):
+            core("vpt_set_option", b"persistent_blocks_per_sm", blocks)
+            assert traced_with(core, sp, frames) == [kernel], (frames, blocks)
+    core("vpt_set_option", b"persistent_blocks_per_sm", 0.0)
+    setup_core(core, small)
+    for sched, kernel in ((2.0, "trace_event"), (1.0, "trace_persistent"), (0.0, "trace_tiles"), (2.0, "trace_event")):
+        core("vpt_set_option", b"schedule", sched)
+        assert traced_with(core, small, 1) == [kernel], sched
