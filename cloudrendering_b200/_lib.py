@@ -105,6 +105,7 @@ SIGNATURES = {
     "vpt_build_occupancy_grid": (c_int, [c_void_p, c_int, c_int, c_int, c_int, c_int, c_float, c_void_p,
                                          c_void_p]),
     "vpt_build_environment_pyramid": (c_int, [c_void_p, c_int, c_int, c_int, c_void_p, c_void_p]),
+    "vpt_release_scratch": (c_int, []),
     "vpt_eaw_denoise_rgba": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_float, c_float, c_float,
                                      c_int, c_void_p, c_void_p]),
     "vpt_batch_create": (c_int, [c_void_p, c_void_p, c_int]),

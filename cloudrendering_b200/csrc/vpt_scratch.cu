@@ -5,10 +5,12 @@
 // call maps it again: 0.5 ms of a 1920 x 1080 EAW call that starts on an idle device (0.94 ms; 0.46 ms when calls
 // follow one another, and here either way).  These calls allocate from a pool of their own, one per device, which
 // keeps up to kScratchKeep bytes across synchronisations.  The pool orders reuse between streams and threads by
-// itself; a destroyed context and an allocation that fails for want of memory give it back (scratch_trim).
+// itself; a destroyed context, an allocation that fails for want of memory (the driver's own allocations take what a
+// pool keeps before they fail) and vpt_release_scratch give it back (scratch_trim).
 #include "vpt_scratch.h"
 
 #include <mutex>
+#include "../../include/vpt_b200.h"
 
 namespace vpt {
 namespace {
@@ -38,6 +40,7 @@ cudaMemPool_t scratch_pool(bool create) {
             else
                 cudaMemPoolDestroy(pool);
         }
+        if (!scratch_pools[dev]) cudaGetLastError();  // the default pool serves; no error of the call
     }
     return scratch_pools[dev];
 }
@@ -63,3 +66,8 @@ void scratch_trim() {
 }
 
 }  // namespace vpt
+
+extern "C" VptStatus vpt_release_scratch(void) {
+    vpt::scratch_trim();
+    return VPT_OK;
+}

@@ -450,9 +450,15 @@ VptStatus vpt_kpn_avg_pool2(const float* in, int n, int c, int h, int w, float* 
 VptStatus vpt_kpn_reproject(const float* prev, const float* uv, int n, int c, int prev_h, int prev_w, int h, int w,
                             float* out, void* stream);
 
+/* vpt_eaw_denoise_rgba, vpt_svgf_filter and vpt_unet_conv3x3 take their scratch, in stream order, from a pool
+ * of the library's own for each device, which keeps up to 256 MiB between calls.  It is given back when a
+ * context is destroyed on the device and when an allocation of this process would fail; this call gives it back
+ * at any time, for the current device, but for what a call in flight uses (another process may want it). */
+VptStatus vpt_release_scratch(void);
+
 /* EAW a-trous chain (EAWBlitPass::_renderCompute, src/Denoiser/EAWDenoiser.cpp:345-391; weights of
- * EAWDenoise.glsl) on RGBA images; position/normal may be NULL.  Allocates its ping-pong images
- * on `stream` with the stream-ordered allocator and frees them before returning.  `out` must not
+ * EAWDenoise.glsl) on RGBA images; position/normal may be NULL.  Takes its ping-pong image from the
+ * library's scratch (vpt_release_scratch) in the order of `stream`.  `out` must not
  * overlap color, position or normal (in-place filtering is rejected with VPT_ERR_ARG). */
 VptStatus vpt_eaw_denoise_rgba(const float* color, const float* position, const float* normal, int width,
                                int height, int iterations, float phi_color, float phi_position, float phi_normal,

@@ -3,10 +3,13 @@ on streams of their own do not disturb one another, what is kept is bounded, and
 import ctypes
 import threading
 
+import numpy as np
 import pytest
 import torch
 
 from cloudrendering_b200 import _lib
+from cloudrendering_b200._lib import VptSparseInfo
+from tests.harness import Core
 
 pytestmark = pytest.mark.gpu
 
@@ -62,7 +65,7 @@ def test_threads_and_streams_share_the_pool():
             assert torch.equal(a, b)
 
 
-@pytest.mark.parametrize("size", [(720, 1280), (3000, 8000)], ids=["below_the_bound", "above_the_bound"])
+@pytest.mark.parametrize("size", [(3000, 3000), (3000, 8000)], ids=["below_the_bound", "above_the_bound"])
 def test_kept_scratch_is_bounded_and_given_back(size):
     lib = _lib.load()
     c = torch.rand(size + (4,), device="cuda")
@@ -77,6 +80,47 @@ def test_kept_scratch_is_bounded_and_given_back(size):
     assert lib.vpt_create(ctypes.byref(ctx), 0) == 0
     eaw(lib, c, out, torch.cuda.current_stream())
     torch.cuda.synchronize()
-    assert free0 - torch.cuda.mem_get_info()[0] <= KEPT + SLACK
+    held = free0 - torch.cuda.mem_get_info()[0]
+    assert held <= KEPT + SLACK
+    if size[0] * size[1] * 16 <= KEPT:  # the image is kept across the synchronisation ...
+        assert held >= size[0] * size[1] * 16
+        assert lib.vpt_release_scratch() == 0  # ... until it is asked for
+        assert free0 - torch.cuda.mem_get_info()[0] <= SLACK
+        eaw(lib, c, out, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        assert free0 - torch.cuda.mem_get_info()[0] >= size[0] * size[1] * 16
     lib.vpt_destroy(ctx)
-    assert free0 - torch.cuda.mem_get_info()[0] <= SLACK
+    assert free0 - torch.cuda.mem_get_info()[0] <= SLACK  # less than the image
+
+
+def test_allocations_take_the_kept_scratch():
+    """With the device's memory used up, an allocation of a context finds the memory that the scratch keeps."""
+    lib = _lib.load()
+    core = Core()
+    n = 192
+    grid = np.random.default_rng(3).random((n, n, n), np.float32)
+    core("vpt_set_dense_grid", grid.ctypes.data_as(ctypes.c_void_p), n, n, n, 0)
+
+    def sparse(on):
+        core("vpt_set_use_sparse_grid", on)
+        info = VptSparseInfo()
+        if on:
+            core("vpt_get_sparse_grid_info", ctypes.byref(info))
+        return info.leaves
+
+    leaves = sparse(1)  # loads the kernels
+    assert leaves * 2048 > 24 << 20  # bytes of values
+    sparse(0)
+    core("vpt_set_dense_grid", grid.ctypes.data_as(ctypes.c_void_p), n, n, n, 0)  # drops the sparse copy
+    c = torch.rand((3000, 3000, 4), device="cuda")
+    out = torch.empty_like(c)
+    eaw(lib, c, out, torch.cuda.current_stream())
+    torch.cuda.synchronize()
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - (16 << 20), dtype=torch.uint8, device="cuda")
+    try:
+        assert torch.cuda.mem_get_info()[0] <= 20 << 20
+        assert sparse(1) == leaves
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+        core.close()
