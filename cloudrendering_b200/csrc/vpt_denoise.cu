@@ -1,9 +1,10 @@
 // vpt_denoise.cu - EAW feature inputs and entry points, SVGF, and feature-map readout.
 //
 // EAW: edge-avoiding a-trous wavelet filter (Dammertz et al. 2010) as in
-// Data/Shaders/Denoiser/EAWDenoise.glsl; its passes are in vpt_eaw.cu (one launch per iteration, each
-// thread one pixel; by default a block stages the taps of 16 x 16 pixels of one residue class modulo
-// the step in shared memory, eaw_lattice_kernel; the direct kernel reads every tap through L1).
+// Data/Shaders/Denoiser/EAWDenoise.glsl; its passes are in vpt_eaw.cu (one launch per iteration; by
+// default a block stages the taps of 32 x 16 pixels of one or two residue classes modulo the step in
+// shared memory and a thread filters 2 or 4 of them, eaw_lattice_kernel; the direct kernel, a pixel a
+// thread, reads every tap through L1).
 //
 // SVGF: Data/Shaders/Denoiser/SVGF/SVGF.glsl (reproject 210-267, filter moments 286-347, a-trous
 // 401-495) with compute_weight from svgf_common.glsl:29-41.
@@ -281,8 +282,9 @@ __device__ __forceinline__ float exp2_sfu(float x) {
     return r;
 }
 
-// x^128 for x >= 0.  A squaring doubles the relative error so far, so the first three carry their rounding
-// errors along (h + l = x^2k); the last four add about 3 ulp, as much as powf's own argument error.
+// x^128 for x >= 0.  A squaring doubles the relative error so far and adds half an ulp, so the first three carry
+// their rounding errors along (h + l = x^8 to 2^-24) and the last four bring it to at most 31 x 2^-24 (seven plain
+// squarings: 127 x 2^-24).  A rounding of x itself, whose dot product has several, counts 128 x 2^-24.
 __device__ __forceinline__ float pow128(float x) {
     float h = x * x, l = fmaf(x, x, -h);
 #pragma unroll

@@ -1049,10 +1049,10 @@ __global__ void __launch_bounds__(kWsThreads, 2) conv_ws_kernel(const __grid_con
 // the three output rows y-1, y, y+1 that read input row y have adjacent accumulators, and one MMA of N = 3 cout
 // columns adds input row y's contribution to all of them, its B operand being the taps dy = +1, 0, -1 stacked:
 // 3 x cin/16 (+ 1) MMAs a row.  A launch computes `cout` <= 80 of the layer's output channels.
-//   Layer, us, 8 images of 256 x 256 (conv_ws_kernel / here): 96 -> 32 93.0 / 56.0, 32 -> 32 29.0 / 23.3, 16 -> 32
-// 24.2 / 18.6; one image of 256 x 256, 32 -> 32 10.0 / 10.2, 48 -> 48 at half that size 17.2 / 13.2.  Bound: 8 us
+//   Layer, us, 8 images of 256 x 256 (conv_ws_kernel / here): 96 -> 32 93.0 / 52.6, 32 -> 32 29.0 / 22.5, 16 -> 32
+// 23.7 / 17.9; one image of 256 x 256, 32 -> 32 10.0 / 10.2, 48 -> 48 at half that size 17.2 / 13.2.  Bound: 8 us
 // to start, load the weights and drain, then the bytes (32 -> 32 67 MB, 10 us at 6.65 TB/s; 96 -> 32 134 MB, 20 us)
-// and the MMAs' issue (96 -> 32: 19 of about 90 cycles a row and 28 rows an SM, 25 us), which overlap in part.
+// and the MMAs' issue (96 -> 32: 19 of about 90 cycles a row and 28 rows an SM, 25 us), which overlap in part.  (One loop over the pairs of group and dx, for both orders: 66.8.)
 //   ring      input rows as in conv_ws_kernel, but a slot is free again after its own row's MMAs: two slots do.
 //   TMEM      a ring of `blocks` accumulators of cout columns, output row g of the CTA in block g % blocks;
 //             three adjacent rows are contiguous columns except around the ring's end (then two MMAs).
@@ -1272,7 +1272,6 @@ __global__ void __launch_bounds__(kStackThreads, 2)
         const uint32_t id_n = (uint32_t)(cout >> 3) << 17;  // one more block of columns
         const int ngroups = wa.ngroups;
         const uint32_t set_cols = (uint32_t)(blocks * cout);
-        // the (group, dx) pairs of a row: dx inner, or the group inner
         const int by_tap = st.by_tap;
         int slot = 0;
         uint32_t phase = 0;
@@ -1304,17 +1303,10 @@ __global__ void __launch_bounds__(kStackThreads, 2)
                     const uint32_t p0 = (uint32_t)((2 - q + lo) * cout), p_rest = p0 + (uint32_t)(n_first * cout);
                     const uint32_t id_first = id1 + (uint32_t)(n_first - 1) * id_n;
                     const uint32_t id_rest = id1 + (uint32_t)(n_rest - 1) * id_n;
-                    int k = 0, dx = 0;
-                    for (int u = 0; u < 3 * ngroups; ++u) {
-                        const int gw = wa.gw[k];
-                        const uint32_t ahi = a_hi_of(gw);
-                        // a ring of accumulators for each pass; its first step overwrites the new row's
-                        const uint32_t acc0 = tmem + (k >= st.groups0 ? set_cols : 0u);
-                        bool first = fresh && dx == 0 && (k == 0 || k == st.groups0);
-                        uint32_t aj = a_lo1 + row16 + ((uint32_t)wa.goff[k] >> 4) + (uint32_t)dx * ((uint32_t)gw >> 3);
-                        uint32_t bj = b_lo0 + (uint32_t)(wa.gc[k] >> 3) * n3 + (uint32_t)dx * b_dx;
+                    // 16-channel steps of a group and a dx; the first of a pass overwrites the new row's accumulator
+                    auto steps = [&](uint32_t acc0, int gw, uint32_t ahi, uint32_t aj, uint32_t bj, bool first) {
                         for (int j = 0; j < gw / 16; ++j) {
-                            if (first) {  // the new row overwrites its block, the older ones accumulate
+                            if (first) {  // (the older rows accumulate)
                                 first = false;
                                 for (int i = lo; i <= hi; ++i) {
                                     const int bi = blo + (i - lo) < blocks ? blo + (i - lo) : blo + (i - lo) - blocks;
@@ -1328,15 +1320,29 @@ __global__ void __launch_bounds__(kStackThreads, 2)
                             aj += 2u;
                             bj += b_step;
                         }
-                        if (by_tap) {
-                            if (++k == ngroups) {
-                                k = 0;
-                                ++dx;
-                            }
-                        } else if (++dx == 3) {
-                            dx = 0;
-                            ++k;
+                    };
+                    if (!by_tap) {
+                        for (int k = 0; k < ngroups; ++k) {
+                            const int gw = wa.gw[k];
+                            const uint32_t ahi = a_hi_of(gw);
+                            const uint32_t line16 = (uint32_t)gw >> 3;
+                            // a ring of accumulators for each pass
+                            const uint32_t acc0 = tmem + (k >= st.groups0 ? set_cols : 0u);
+                            const bool first = fresh && (k == 0 || k == st.groups0);
+                            const uint32_t al = a_lo1 + row16 + ((uint32_t)wa.goff[k] >> 4);
+                            const uint32_t bl = b_lo0 + (uint32_t)(wa.gc[k] >> 3) * n3;
+#pragma unroll
+                            for (uint32_t dx = 0; dx < 3; ++dx)
+                                steps(acc0, gw, ahi, al + dx * line16, bl + dx * b_dx, first && dx == 0);
                         }
+                    } else {
+                        for (uint32_t dx = 0; dx < 3; ++dx)
+                            for (int k = 0; k < ngroups; ++k) {
+                                const int gw = wa.gw[k];
+                                steps(tmem, gw, a_hi_of(gw),
+                                      a_lo1 + row16 + ((uint32_t)wa.goff[k] >> 4) + dx * ((uint32_t)gw >> 3),
+                                      b_lo0 + (uint32_t)(wa.gc[k] >> 3) * n3 + dx * b_dx, fresh && dx == 0 && k == 0);
+                            }
                     }
                     mma_commit(smem_u32(&empty[slot]));
                     if (q >= 2) mma_commit(smem_u32(&acc_full[b2]));
@@ -1643,11 +1649,10 @@ __global__ void __launch_bounds__(kBoxThreads)
 // bound of N <= 96), 4-7 zero the accumulators at the start and write the CTA's sums to
 // partial[blockIdx.x][t * cin + ci][co] at the end (reduced in fixed order by reduce_grads_kernel).  M = 64
 // accumulators occupy lanes 0-15 of each 32-lane quarter of TMEM.
-//   Kernel and reduction, us, 8 images of 256 x 256 (the strip kernel that copied both rows into 8-channel planes
-// and issued one MMA a tap and 16 pixels, or the gather kernel below 64 channels / here): 96 -> 32 179 / 65,
-// 32 -> 32 176 / 50, 16 -> 32 134 / 49, 32 -> 176 380 / 153; 144 -> 48 at half that size 200 / 94.  Bound: the rows'
-// bytes (96 -> 32: 134 MB, 20 us) and the MMAs (24 a row and 28 rows an SM), which overlap, then writing the
-// accumulators.
+//   us, 8 images of 256 x 256 (a strip kernel that copied both rows into 8-channel planes and issued one MMA a tap and
+// 16 pixels / here): 96 -> 32 150 / 66, 32 -> 176 289 / 100; at half that size 64 -> 64 58 / 35, 160 -> 64 132 / 72.
+// Bound: the rows' bytes (96 -> 32: 134 MB, 21 us) and the MMAs (24 a row and 28 to 42 rows an SM: the segments are not
+// split further, since their rows' order is part of the result), which overlap, then writing the accumulators.
 constexpr int kWgThreads = 256;
 constexpr int kWgMaxRing = 8;
 constexpr int kWgURing = 3;

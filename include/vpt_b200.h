@@ -508,15 +508,16 @@ VptStatus vpt_gather_bench(const float* buffer, size_t bytes, int blocks, int lo
 VptStatus vpt_unet_conv3x3(const void* x, const void* w, const float* bias, const void* mask, void* y, int n, int h,
                            int width, int cin, int cout, int relu, int out_f32, int* err, void* stream);
 /* Selects the convolution kernels: 0 (default) = by shape (the persistent row-strip kernels for images
- * at least 128 pixels wide where they are measured faster; input channels in up to 4 groups through an
- * fp32 partial allocated on the stream; the weight gradient on image rows for 2,048 pixels and more),
- * 1 = the per-tile gather kernels everywhere, 2 = the row kernels wherever they apply.  (By default tiles
- * whose 128 pixels are a box of rows or images are loaded by the tensor-memory-access unit.) */
+ * at least 128 pixels wide where they are measured faster; input channels in up to 4 passes; the weight
+ * gradient on image rows for images at least 128 pixels wide with 64 channels on a side whose operands
+ * fit), 1 = the per-tile gather kernels everywhere, 2 = the row kernels wherever they apply.  (By default
+ * tiles whose 128 pixels are a box of rows or images are loaded by the tensor-memory-access unit.)  The
+ * order of a layer's sums is the same for all kernels of a path; paths differ in it. */
 VptStatus vpt_unet_set_conv_path(int path);
 /* Row-strip convolution kernel: 0 (default) = warp-specialised (input rows loaded by the tensor-memory-
  * access unit into a ring; up to 80 output channels a launch with the three output rows that read an input
- * row in one MMA, or all of them one row at a time; input channel groups when the weights and the ring do
- * not fit), 1 = the cp.async row-strip kernel. */
+ * row in one MMA, or all of them one row at a time; input channels in passes when the weights and the ring
+ * do not fit), 1 = the cp.async row-strip kernel. */
 VptStatus vpt_unet_set_strip_kernel(int kind);
 /* K splits of the per-tile convolutions: 0 (default) = by grid size (grids of at most half an SM wave
  * split their K stages over up to 8 CTAs, whose fp32 sums, allocated on the stream, are added in split
@@ -531,8 +532,8 @@ VptStatus vpt_unet_conv3x3_wgrad(const void* x, const void* dy, float* partial, 
                                  int cout, int pixels_per_split, int* err, void* stream);
 int vpt_unet_wgrad_rows(int cin);
 /* Number of partial sums (splits) vpt_unet_conv3x3_wgrad writes for this shape and the selected path: the
- * kernel on image rows (by default from 2,048 pixels) writes one per CTA, the gather kernel one per
- * pixels_per_split pixels. */
+ * kernel on image rows (vpt_unet_set_conv_path) writes one per CTA, the gather kernel one per
+ * pixels_per_split pixels; 0 for arguments that it refuses. */
 int vpt_unet_wgrad_splits(int n, int h, int width, int cin, int cout, int pixels_per_split);
 /* wrot[ci][t][co] = w[co][8 - t][ci] */
 VptStatus vpt_unet_rotate_weights(const void* w, void* wrot, int cin, int cout, void* stream);
