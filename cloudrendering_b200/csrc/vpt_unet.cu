@@ -1632,9 +1632,10 @@ __global__ void __launch_bounds__(kBoxThreads)
 // ---------------------------------------------------------------------------------------------
 // the weight gradient on image rows
 // ---------------------------------------------------------------------------------------------
-// dw[co][t][ci] = sum over pixels p of dy[p][co] * x[p + off(t)][ci].  Pixels are K: a CTA walks segments of rows of
-// an image column 128 pixels wide, every row a contraction over its pixels in steps of 16, and sums
-// all its rows in TMEM, one after the other.  Both operands are rows as they lie in memory, [pixel][channels], read by the TMA
+// dw[co][t][ci] = sum over pixels p of dy[p][co] * x[p + off(t)][ci].  Pixels are K, in steps of 16: a CTA walks
+// segments of rows of an image column 128 pixels wide, or the rows of a run of pixels_per_split pixels (of images whose
+// width is a multiple of 16, in tiles of 128 from left to right, the first and the last row in part), and sums
+// them in TMEM, one after the other.  Both operands are rows as they lie in memory, [pixel][channels], read by the TMA
 // into the MN-major swizzled layout (channels contiguous: MN; pixels: K), lines of 32 or 16 channels.  A tap's
 // horizontal shift dx is a start moved by dx pixel lines, as in conv_stack_kernel; pixels and channels outside
 // arrive as zeros.
@@ -1650,7 +1651,8 @@ __global__ void __launch_bounds__(kBoxThreads)
 // partial[blockIdx.x][t * cin + ci][co] at the end (reduced in fixed order by reduce_grads_kernel).  M = 64
 // accumulators occupy lanes 0-15 of each 32-lane quarter of TMEM.
 //   us, 8 images of 256 x 256 (a strip kernel that copied both rows into 8-channel planes and issued one MMA a tap and
-// 16 pixels / here): 96 -> 32 150 / 66, 32 -> 176 289 / 100; at half that size 64 -> 64 58 / 35, 160 -> 64 132 / 72.
+// 16 pixels / here): 96 -> 32 150 / 66, 32 -> 176 289 / 100; at half that size 64 -> 64 58 / 35, 160 -> 64 132 / 72;
+// by the gather kernel in runs of pixels / here: 16 -> 32 108 / 41, 32 -> 32 154 / 55, 224 -> 96 at a quarter 123 / 47.
 // Bound: the rows' bytes (96 -> 32: 134 MB, 21 us) and the MMAs (24 a row and 28 to 42 rows an SM: the segments are not
 // split further, since their rows' order is part of the result), which overlap, then writing the accumulators.
 constexpr int kWgThreads = 256;
@@ -1665,24 +1667,57 @@ struct WgradArgs {
     int s_group;               // channels of an S chunk: 32, or 16 when S has 16
     int u_chunks, s_chunks;    // blockIdx.y = u_chunk * s_chunks + s_chunk
     int xtiles, seg_rows, segs_per_col;  // segments of seg_rows rows of a column; CTA i takes i, i + gridDim.x, ...
-    int u_slot, u_group_bytes, s_slot, s_ring;  // shared-memory strides; ring depth of S
+    int pps;                   // or the run of pixels [i pps, (i + 1) pps) (0: segments)
+    int tiles, row_groups;     // 128-pixel tiles and 16-pixel groups of a row of a segment
+    int u_slot, u_group_bytes, s_tile, s_slot, s_ring;  // shared-memory strides (an S slot: a row's tiles); ring depth of S
     int u_lines, s_lines;      // pixel lines of a row (the x tensor's rows carry a halo of one)
     int tmem_cols;
 };
 
-// the segments of a CTA in order
+// rows [y0, y1) of an image from x0; of the first row only the 16-pixel groups from g0 on, of the last those below g1
+struct WgSegment {
+    int n_img, x0, y0, y1, g0, g1;
+};
+
+// the segments of a CTA in order (RUNS: of a run of pixels)
+template <bool RUNS>
 struct SegWalk {
     const WgradArgs& a;
-    int seg = (int)blockIdx.x;
-    __device__ __forceinline__ bool next(WsSegment& g) {
-        if (seg >= a.n * a.xtiles * a.segs_per_col) return false;
-        const int col = seg / a.segs_per_col, part = seg - col * a.segs_per_col;
+    long at, end;  // segment, or pixel of the run
+    __device__ __forceinline__ explicit SegWalk(const WgradArgs& a_) : a(a_) {
+        const long pixels = (long)a.n * a.h * a.w_;
+        at = RUNS ? min((long)blockIdx.x * a.pps, pixels) : (long)blockIdx.x;
+        end = RUNS ? min(at + a.pps, pixels) : (long)a.n * a.xtiles * a.segs_per_col;
+    }
+    __device__ __forceinline__ bool next(WgSegment& g) {
+        if (at >= end) return false;
+        if (RUNS) {  // the rest of the run, or of its image
+            const int row = (int)(at / a.w_), img = row / a.h;
+            const long stop = min(end, (long)(img + 1) * a.h * a.w_);
+            const int last = (int)((stop - 1) / a.w_);
+            g.n_img = img;
+            g.x0 = 0;
+            g.y0 = row - img * a.h;
+            g.y1 = last + 1 - img * a.h;
+            g.g0 = (int)(at - (long)row * a.w_) / 16;
+            g.g1 = (int)(stop - (long)last * a.w_ + 15) / 16;
+            at = stop;
+            return true;
+        }
+        const int seg = (int)at, col = seg / a.segs_per_col, part = seg - col * a.segs_per_col;
         g.n_img = col / a.xtiles;
         g.x0 = (col % a.xtiles) * kBM;
         g.y0 = part * a.seg_rows;
         g.y1 = min(a.h, g.y0 + a.seg_rows);
-        seg += (int)gridDim.x;
+        g.g0 = 0;
+        g.g1 = a.row_groups;
+        at += gridDim.x;
         return true;
+    }
+    // the 16-pixel groups [lo, hi) of dy row y that count, within tile t
+    __device__ __forceinline__ int2 groups(const WgSegment& g, int y, int t) const {
+        const int lo = (y == g.y0 ? g.g0 : 0) - t * (kBM / 16), hi = (y == g.y1 - 1 ? g.g1 : a.row_groups) - t * (kBM / 16);
+        return make_int2(max(lo, 0), min(hi, kBM / 16));
     }
 };
 
@@ -1696,6 +1731,7 @@ __device__ __forceinline__ uint64_t smem_desc_mn(uint32_t line, uint32_t lbo) {
     return d;
 }
 
+template <bool RUNS>
 __global__ void __launch_bounds__(kWgThreads, 1)
     wgrad_rows_kernel(const __grid_constant__ CUtensorMap umap, const __grid_constant__ CUtensorMap smap,
                       const __grid_constant__ WgradArgs a) {
@@ -1707,7 +1743,7 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     const int u_total = a.role == 0 ? a.cin : a.cout;
     const int u0 = ((int)blockIdx.y / a.s_chunks) * 128, s0 = ((int)blockIdx.y % a.s_chunks) * a.s_group;
     const int ma = u_total - u0 > 64 ? 128 : 64;
-    const int n3 = 3 * a.s_group;
+    const int n3 = 3 * a.s_group, tiles = RUNS ? a.tiles : 1;
     const uint32_t su = smem_u32(smem), ss = su + (uint32_t)(kWgURing * a.u_slot);
     if (tid == 0) {
         for (int k = 0; k < kWgURing; ++k) {
@@ -1742,45 +1778,49 @@ __global__ void __launch_bounds__(kWgThreads, 1)
     if (warp == 0) {
         if (lane == 0) {
             const int ugroups = ma / 32;
-            const uint32_t u_tx = (uint32_t)(ugroups * a.u_lines * 64), s_tx = (uint32_t)(a.s_lines * a.s_group * 2);
+            const uint32_t u_tx = (uint32_t)(ugroups * a.u_lines * 64), s_tx = (uint32_t)(tiles * a.s_lines * a.s_group * 2);
             int us = 0, sl = 0;
             uint32_t uph = 0, sph = 0;
             long ui = 0, si = 0;
-            auto load_s = [&](const WsSegment& g, int row) {
+            auto load_s = [&](const WgSegment& g, int row) {
                 if (!mbar_wait(smem_u32(&s_empty[sl]), sph ^ 1u)) {
                     fail = true;
                     return;
                 }
                 const uint32_t fb = smem_u32(&s_full[sl]);
                 mbar_arrive_expect_tx(fb, s_tx);
-                tma_load_4d(ss + (uint32_t)(sl * a.s_slot), &smap, s0, g.x0 - (a.role == 1 ? 1 : 0), row, g.n_img, fb);
+                for (int t = 0; t < tiles; ++t)
+                    tma_load_4d(ss + (uint32_t)(sl * a.s_slot + t * a.s_tile), &smap, s0,
+                                g.x0 + t * kBM - (a.role == 1 ? 1 : 0), row, g.n_img, fb);
                 ++si;
                 if (++sl == a.s_ring) {
                     sl = 0;
                     sph ^= 1u;
                 }
             };
-            SegWalk range{a};
-            WsSegment g;
+            SegWalk<RUNS> range(a);
+            WgSegment g;
             while (!fail && range.next(g)) {
                 const int r0 = a.role == 0 ? g.y0 - 1 : g.y0, r1 = a.role == 0 ? g.y1 : g.y1 - 1;
                 const int slo = a.role == 0 ? g.y0 : g.y0 - 1, shi = a.role == 0 ? g.y1 - 1 : g.y1;
                 int next = slo;
                 for (int r = r0; r <= r1 && !fail; ++r) {
                     while (next <= min(r + 1, shi) && !fail) load_s(g, next++);
-                    if (fail || !mbar_wait(smem_u32(&u_empty[us]), uph ^ 1u)) {
-                        fail = true;
-                        break;
-                    }
-                    const uint32_t fb = smem_u32(&u_full[us]);
-                    mbar_arrive_expect_tx(fb, u_tx);
-                    for (int k = 0; k < ugroups; ++k)
-                        tma_load_4d(su + (uint32_t)(us * a.u_slot + k * a.u_group_bytes), &umap, u0 + 32 * k,
-                                    g.x0 - (a.role == 0 ? 1 : 0), r, g.n_img, fb);
-                    ++ui;
-                    if (++us == kWgURing) {
-                        us = 0;
-                        uph ^= 1u;
+                    for (int t = 0; t < tiles; ++t) {
+                        if (fail || !mbar_wait(smem_u32(&u_empty[us]), uph ^ 1u)) {
+                            fail = true;
+                            break;
+                        }
+                        const uint32_t fb = smem_u32(&u_full[us]);
+                        mbar_arrive_expect_tx(fb, u_tx);
+                        for (int k = 0; k < ugroups; ++k)
+                            tma_load_4d(su + (uint32_t)(us * a.u_slot + k * a.u_group_bytes), &umap, u0 + 32 * k,
+                                        g.x0 + t * kBM - (a.role == 0 ? 1 : 0), r, g.n_img, fb);
+                        ++ui;
+                        if (++us == kWgURing) {
+                            us = 0;
+                            uph ^= 1u;
+                        }
                     }
                 }
             }
@@ -1820,49 +1860,81 @@ __global__ void __launch_bounds__(kWgThreads, 1)
         uint32_t uph = 0;
         int ws = 0;         // ring slot of the oldest S row in use
         uint32_t wph = 0;   // its phase
-        SegWalk range{a};
-        WsSegment g;
+        SegWalk<RUNS> range(a);
+        WgSegment g;
         while (!fail && range.next(g)) {
             const int r0 = a.role == 0 ? g.y0 - 1 : g.y0, r1 = a.role == 0 ? g.y1 : g.y1 - 1;
             const int slo = a.role == 0 ? g.y0 : g.y0 - 1, shi = a.role == 0 ? g.y1 - 1 : g.y1;
             int oldest = slo;  // S row in slot ws
-            for (int r = r0; r <= r1; ++r) {
+            for (int r = r0; r <= r1 && !fail; ++r) {
                 const int lo = max(r - 1, slo), hi = min(r + 1, shi);  // S rows of this step (lo == oldest)
-                bool ok = mbar_wait(smem_u32(&u_full[us]), uph);
-                for (int k = 0; k <= hi - oldest; ++k) {
-                    const int q = ws + k < a.s_ring ? ws + k : ws + k - a.s_ring;
-                    ok = ok && mbar_wait(smem_u32(&s_full[q]), ws + k < a.s_ring ? wph : wph ^ 1u);
-                }
-                if (!__all_sync(0xffffffffu, ok)) {
-                    fail = true;
-                    break;
-                }
-                tc_fence_after();
+                const int cnt = hi - lo + 1, n_first = min(cnt, a.s_ring - ws), n_rest = cnt - n_first;
                 // S row r - 1 is last used here; the segment's last step releases the rest
                 const int keep = r == r1 ? shi + 1 : max(r, slo);
-                if (elect_one()) {
-                    const int cnt = hi - lo + 1, n_first = min(cnt, a.s_ring - ws), n_rest = cnt - n_first;
-                    const uint32_t d0 = dacc + (uint32_t)((lo - (r - 1)) * a.s_group);
-                    const uint32_t d1 = d0 + (uint32_t)(n_first * a.s_group);
-                    const uint32_t id_first = id1 + (uint32_t)(n_first - 1) * id_n;
-                    const uint32_t id_rest = id1 + (uint32_t)(n_rest - 1) * id_n;
-                    uint32_t ul = u_lo + ((uint32_t)(us * a.u_slot) >> 4);
-                    uint32_t sl = s_lo + ((uint32_t)(ws * a.s_slot) >> 4), sw = s_lo;
-                    for (int j = 0; j < kBM / 16; ++j) {
-                        mma_bf16_halves(d0, ul, u_hi, sl, s_hi, id_first, 1u);
-                        if (n_rest > 0) mma_bf16_halves(d1, ul, u_hi, sw, s_hi, id_rest, 1u);
-                        ul += u_step;
-                        sl += s_step;
-                        sw += s_step;
+                for (int t = 0; t < tiles; ++t) {
+                    bool ok = mbar_wait(smem_u32(&u_full[us]), uph);
+                    for (int k = 0; t == 0 && k < cnt; ++k) {
+                        const int q = ws + k < a.s_ring ? ws + k : ws + k - a.s_ring;
+                        ok = ok && mbar_wait(smem_u32(&s_full[q]), ws + k < a.s_ring ? wph : wph ^ 1u);
                     }
-                    mma_commit(smem_u32(&u_empty[us]));
-                    for (int k = 0; k < keep - oldest; ++k)
-                        mma_commit(smem_u32(&s_empty[ws + k < a.s_ring ? ws + k : ws + k - a.s_ring]));
-                }
-                __syncwarp();
-                if (++us == kWgURing) {
-                    us = 0;
-                    uph ^= 1u;
+                    if (!__all_sync(0xffffffffu, ok)) {
+                        fail = true;
+                        break;
+                    }
+                    tc_fence_after();
+                    if (elect_one()) {
+                        const uint32_t d0 = dacc + (uint32_t)((lo - (r - 1)) * a.s_group);
+                        const uint32_t ub = u_lo + ((uint32_t)(us * a.u_slot) >> 4);
+                        const uint32_t wrap = s_lo + ((uint32_t)(t * a.s_tile) >> 4);  // ring slot 0
+                        const uint32_t sb = wrap + ((uint32_t)(ws * a.s_slot) >> 4);
+                        const uint32_t d1 = d0 + (uint32_t)(n_first * a.s_group);
+                        const uint32_t id_first = id1 + (uint32_t)(n_first - 1) * id_n;
+                        const uint32_t id_rest = id1 + (uint32_t)(n_rest - 1) * id_n;
+                        // the groups of the rows' dy that count: of row r, or (role 0) of each S row its own
+                        int2 j0 = make_int2(0, kBM / 16);
+                        bool same = true;
+                        if (RUNS) {
+                            j0 = range.groups(g, a.role == 1 ? r : lo, t);
+                            if (a.role == 0) {
+                                const int2 jm = range.groups(g, min(lo + 1, hi), t), j2 = range.groups(g, hi, t);
+                                same = j0.x == jm.x && j0.y == jm.y && j0.x == j2.x && j0.y == j2.y;
+                            }
+                        }
+                        if (same && j0.x == 0 && j0.y == kBM / 16) {
+                            uint32_t ul = ub, sl = sb, sw = wrap;
+                            for (int j = 0; j < kBM / 16; ++j) {
+                                mma_bf16_halves(d0, ul, u_hi, sl, s_hi, id_first, 1u);
+                                if (n_rest > 0) mma_bf16_halves(d1, ul, u_hi, sw, s_hi, id_rest, 1u);
+                                ul += u_step;
+                                sl += s_step;
+                                sw += s_step;
+                            }
+                        } else if (same) {
+                            for (uint32_t j = (uint32_t)j0.x; (int)j < j0.y; ++j) {
+                                mma_bf16_halves(d0, ub + j * u_step, u_hi, sb + j * s_step, s_hi, id_first, 1u);
+                                if (n_rest > 0)
+                                    mma_bf16_halves(d1, ub + j * u_step, u_hi, wrap + j * s_step, s_hi, id_rest, 1u);
+                            }
+                        } else {  // around the ends of a run
+                            for (int k = 0; k < cnt; ++k) {
+                                const int2 jk = range.groups(g, lo + k, t);
+                                const int q = ws + k < a.s_ring ? ws + k : ws + k - a.s_ring;
+                                const uint32_t sk = wrap + ((uint32_t)(q * a.s_slot) >> 4);
+                                for (uint32_t j = (uint32_t)jk.x; (int)j < jk.y; ++j)
+                                    mma_bf16_halves(d0 + (uint32_t)(k * a.s_group), ub + j * u_step, u_hi, sk + j * s_step,
+                                                    s_hi, id1, 1u);
+                            }
+                        }
+                        mma_commit(smem_u32(&u_empty[us]));
+                        if (t == tiles - 1)
+                            for (int k = 0; k < keep - oldest; ++k)
+                                mma_commit(smem_u32(&s_empty[ws + k < a.s_ring ? ws + k : ws + k - a.s_ring]));
+                    }
+                    __syncwarp();
+                    if (++us == kWgURing) {
+                        us = 0;
+                        uph ^= 1u;
+                    }
                 }
                 for (; oldest < keep; ++oldest)
                     if (++ws == a.s_ring) {
@@ -2644,7 +2716,7 @@ inline void strip_segments(int n, int h, int w, int slots, int& xtiles, int& seg
 // of the result: one flipped rounding in the sum of a layer is as large as the error of a training step.  So
 // images at least 128 pixels wide with 64 channels on a side are split by segments of rows, one partial for each CTA of
 // a pass, where five 130-pixel rows of x and three 128-pixel rows of dy with their channels (one of the two in
-// chunks of 64 or 128) take at most 220 KB; everything else in runs of pixels_per_split (conv_tile_kernel).
+// chunks of 64 or 128) take at most 220 KB; everything else in runs of pixels_per_split (wgrad_runs, conv_tile_kernel).
 // `any`: also with fewer channels.
 inline bool wgrad_by_rows(int width, int cin, int cout, bool any) {
     if (width < kBM || (!any && cin < 64 && cout < 64)) return false;
@@ -2659,7 +2731,31 @@ inline bool wgrad_by_rows(int width, int cin, int cout, bool any) {
 struct WgradPlan {
     int role = 0, s_group = 32, u_chunks = 1, s_chunks = 1, passes = 1;
     int xtiles = 1, seg_rows = 1, segs_per_col = 1, grid = 1;
+    int pps = 0, tiles = 1, row_groups = kBM / 16;  // runs of pixels
 };
+
+// Shared memory of wgrad_rows_kernel: strides and ring depth of S (as deep as fits, 0: less than the four rows it needs).
+struct WgradSmem {
+    int u_lines, s_lines, u_group_bytes, u_slot, s_tile, s_slot, s_ring;
+    size_t bytes;
+};
+inline WgradSmem wgrad_smem(const WgradPlan& p, int cin, int cout) {
+    WgradSmem m;
+    const int pixels = std::min(kBM, p.row_groups * 16);
+    m.u_lines = pixels + (p.role == 0 ? 2 : 0);
+    m.s_lines = pixels + (p.role == 1 ? 2 : 0);
+    // group, tile and slot strides: whole 1024-byte blocks (the swizzle acts on absolute addresses)
+    auto up = [](int b) { return (b + 1023) / 1024 * 1024; };
+    m.u_group_bytes = up(m.u_lines * 64);
+    m.u_slot = m.u_group_bytes * ((p.role == 0 ? cin : cout) > 64 ? 4 : 2);
+    m.s_tile = up(m.s_lines * p.s_group * 2);
+    m.s_slot = m.s_tile * p.tiles;
+    const int left = (int)kSmPerCta - 1024 - kWgURing * m.u_slot;
+    m.s_ring = std::min(kWgMaxRing, left / m.s_slot);
+    if (m.s_ring < 4) m.s_ring = 0;
+    m.bytes = (size_t)kWgURing * m.u_slot + (size_t)m.s_ring * m.s_slot;
+    return m;
+}
 
 inline WgradPlan wgrad_plan(int n, int h, int w, int cin, int cout, int sms) {
     WgradPlan p;
@@ -2680,6 +2776,24 @@ inline WgradPlan wgrad_plan(int n, int h, int w, int cin, int cout, int sms) {
     strip_segments(n, h, w, sms, p.xtiles, p.seg_rows, p.segs_per_col, total);
     p.grid = std::min(total, sms);
     return p;
+}
+
+// The row kernel on runs of pixels_per_split pixels, for whole 16-pixel groups a row: the gather kernel's order of pixels.
+// For runs of 512 pixels (192 from 128 channels on both sides on), below which a CTA's nine accumulators cost more
+// than the gather, and rows of 32 (a row costs its barriers).  us, gather / here, pixels of a run in brackets:
+//     32 -> 32    8 x 64^2 [384] 14.4 / 15.1   256^2 [704] 22.4 / 16.5   512^2 [2,688] 72.3 / 31.5   8 x 256^2 [5,312] 141 / 53
+//     48 -> 48    8 x 64^2 [448] 17.5 / 16.9   256^2 [896] 29.6 / 17.4   8 x 256^2 [7,104] 198 / 68
+//     96 -> 96    64^2 [128] 12.9 / 14.5       112^2 [320] 19.0 / 18.4   8 x 64^2 [768] 49.2 / 26.6
+//    224 -> 96    64^2 [256] 17.1 / 18.7       8 x 32^2 [448] 24.4 / 28.3   112^2 [704] 31.6 / 25.4   8 x 64^2 [1,728] 115 / 44
+//    128 -> 128   64^2 [128] 14.4 / 13.6       8 x 32^2 [256] 19.6 / 18.3   8 x 64^2 [1,024] 55.3 / 29.0
+inline bool wgrad_runs(int n, int h, int w, int cin, int cout, int pps, WgradPlan& p) {
+    if (w % 16 || w < 32 || pps < w || pps < (cin >= 128 && cout >= 128 ? 192 : 512)) return false;
+    p = wgrad_plan(n, h, w, cin, cout, sm_count());
+    p.pps = pps;
+    p.tiles = (w + kBM - 1) / kBM;
+    p.row_groups = w / 16;
+    p.grid = (int)(((long)n * h * w + pps - 1) / pps);
+    return wgrad_smem(p, cin, cout).s_ring > 0;
 }
 
 cudaError_t launch_strip_pass(StripArgs a, cudaStream_t s) {
@@ -2773,16 +2887,19 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* partial, int
     a.xtiles = p.xtiles;
     a.seg_rows = p.seg_rows;
     a.segs_per_col = p.segs_per_col;
-    a.u_lines = kBM + (p.role == 0 ? 2 : 0);
-    a.s_lines = kBM + (p.role == 1 ? 2 : 0);
-    // group and slot strides: whole 1024-byte blocks (the swizzle acts on absolute addresses)
-    auto up = [](int b) { return (b + 1023) / 1024 * 1024; };
-    a.u_group_bytes = up(a.u_lines * 64);
+    a.pps = p.pps;
+    a.tiles = p.tiles;
+    a.row_groups = p.row_groups;
+    const WgradSmem m = wgrad_smem(p, cin, cout);
+    a.u_lines = m.u_lines;
+    a.s_lines = m.s_lines;
+    a.u_group_bytes = m.u_group_bytes;
+    a.u_slot = m.u_slot;
+    a.s_tile = m.s_tile;
+    a.s_slot = m.s_slot;
+    a.s_ring = m.s_ring;
     const int u_total = p.role == 0 ? cin : cout;
-    a.u_slot = a.u_group_bytes * (u_total > 64 ? 4 : 2);
-    a.s_slot = up(a.s_lines * p.s_group * 2);
-    a.s_ring = kWgMaxRing;
-    const size_t smem = (size_t)kWgURing * a.u_slot + (size_t)a.s_ring * a.s_slot;
+    const size_t smem = m.bytes;
     a.tmem_cols = pow2_cols(9 * p.s_group);
     CUtensorMap umap, smap;
     const bf16* ut = p.role == 0 ? x : dy;
@@ -2790,9 +2907,11 @@ cudaError_t launch_wgrad_rows(const bf16* x, const bf16* dy, float* partial, int
     if (!encode_wgrad(&umap, ut, n, h, w, u_total, 32, a.u_lines) ||
         !encode_wgrad(&smap, st, n, h, w, p.role == 0 ? cout : cin, p.s_group, a.s_lines))
         return cudaErrorInvalidValue;
-    const cudaError_t e = allow_smem<wgrad_rows_kernel>();
+    const dim3 grid((unsigned)p.grid, (unsigned)p.passes);
+    const cudaError_t e = p.pps ? allow_smem<wgrad_rows_kernel<true>>() : allow_smem<wgrad_rows_kernel<false>>();
     if (e != cudaSuccess) return e;
-    wgrad_rows_kernel<<<dim3((unsigned)p.grid, (unsigned)p.passes), kWgThreads, smem, s>>>(umap, smap, a);
+    if (p.pps) wgrad_rows_kernel<true><<<grid, kWgThreads, smem, s>>>(umap, smap, a);
+    else wgrad_rows_kernel<false><<<grid, kWgThreads, smem, s>>>(umap, smap, a);
     count_launches(1);
     return cudaGetLastError();
 }
@@ -3290,6 +3409,11 @@ VptStatus vpt_unet_conv3x3_wgrad(const void* x, const void* dy, float* partial, 
         return launch_wgrad_rows(a.x, a.w, partial, err, n, h, width, cin, cout, plan,
                                  static_cast<cudaStream_t>(stream)) == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
     }
+    WgradPlan runs;
+    if (!g_force_gather && reinterpret_cast<uintptr_t>(x) % 16 == 0 && reinterpret_cast<uintptr_t>(dy) % 16 == 0 &&
+        encode_tiled() && wgrad_runs(n, h, width, cin, cout, pixels_per_split, runs))
+        return launch_wgrad_rows(a.x, a.w, partial, err, n, h, width, cin, cout, runs,
+                                 static_cast<cudaStream_t>(stream)) == cudaSuccess ? VPT_OK : VPT_ERR_CUDA;
     const long P = (long)n * h * width;
     const dim3 grid((unsigned)mtiles, (unsigned)((cout + a.n_tile - 1) / a.n_tile),
                     (unsigned)((P + pixels_per_split - 1) / pixels_per_split));

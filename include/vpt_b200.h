@@ -532,7 +532,7 @@ VptStatus vpt_unet_conv3x3_wgrad(const void* x, const void* dy, float* partial, 
                                  int cout, int pixels_per_split, int* err, void* stream);
 int vpt_unet_wgrad_rows(int cin);
 /* Number of partial sums (splits) vpt_unet_conv3x3_wgrad writes for this shape and the selected path: the
- * kernel on image rows (vpt_unet_set_conv_path) writes one per CTA, the gather kernel one per
+ * kernel on segments of image rows (vpt_unet_set_conv_path) writes one per CTA, otherwise there is one per
  * pixels_per_split pixels; 0 for arguments that it refuses. */
 int vpt_unet_wgrad_splits(int n, int h, int width, int cin, int cout, int pixels_per_split);
 /* wrot[ci][t][co] = w[co][8 - t][ci] */

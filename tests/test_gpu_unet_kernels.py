@@ -485,3 +485,27 @@ def test_threads_launch_layers_of_different_sizes(lib):
     for outs in got:
         for out, ref in zip(outs, want):
             assert all(torch.equal(a, b) for a, b in zip(out, ref))
+
+
+@pytest.mark.parametrize("case", [
+    # n, h, w, cin, cout, pixels per split: a tile, part of one, several and a part; runs that end within a row and an
+    # image; rows as long as a run; both roles; operands that leave no ring (the gather kernel)
+    (2, 20, 32, 128, 128, 192), (3, 7, 48, 32, 48, 512), (1, 40, 64, 48, 32, 576), (2, 11, 112, 16, 64, 640),
+    (1, 9, 128, 16, 48, 512), (2, 16, 144, 48, 16, 704), (1, 30, 256, 32, 32, 5312), (3, 5, 272, 32, 16, 1024),
+    (1, 6, 512, 48, 48, 512), (1, 6, 512, 48, 32, 576), (1, 4, 528, 32, 32, 576), (5, 8, 64, 144, 96, 512),
+    (2, 33, 64, 96, 224, 768), (1, 64, 32, 288, 128, 192), (2, 9, 96, 80, 272, 512), (1, 1, 512, 16, 16, 512),
+    (1, 24, 384, 16, 16, 448 + 64)])
+def test_weight_gradient_of_runs_equals_the_gather_kernels(lib, request, case):
+    """Partials of runs of pixels by the row kernel and by the gather kernel: the same sums in the same order, bit for bit."""
+    n, h, w, cin, cout, pps = case
+    request.addfinalizer(lambda: lib.vpt_unet_set_conv_path(0))
+    d_x, d_dy = dev_bf16(rng_data(85, n, h, w, cin)), dev_bf16(rng_data(86, n, h, w, cout))
+    rows, splits, parts = lib.vpt_unet_wgrad_rows(cin), -(-n * h * w // pps), []
+    for path in (1, 0):
+        assert lib.vpt_unet_set_conv_path(path) == 0
+        assert lib.vpt_unet_wgrad_splits(n, h, w, cin, cout, pps) == splits
+        part = torch.full((splits + 1, rows, cout), -7.0, device="cuda")
+        run(lib, "vpt_unet_conv3x3_wgrad", ptr(d_x), ptr(d_dy), ptr(part), n, h, w, cin, cout, pps)
+        assert bool((part[splits] == -7.0).all()) and bool((part[:, 9 * cin:] == -7.0).all())
+        parts.append(part[:splits, :9 * cin])
+    assert torch.equal(*parts)
