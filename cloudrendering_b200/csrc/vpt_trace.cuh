@@ -422,7 +422,7 @@ VPT_DEV void flush_counters_to(unsigned long long* counters, int* error_flags, u
 // events: a scatter (phase function, new ray interval, for next event tracking a light sample), the end
 // of a shadow ray, the end of the path.  Run as they occur, an event's 100 to 300 instructions hold up the
 // whole warp for the one or two lanes that have it in an iteration.  So a lane with an event waits: the
-// others go on colliding until kEventShare eighths of the warp's live lanes wait, and then the events run
+// others go on colliding until `share` eighths of the warp's live lanes wait (event_share), and then the events run
 // together.  (The paths' own order of operations and random numbers is that of the recursive trackers in
 // vpt_trackers.cuh: a lane that waits draws nothing.)  Path ids come from a global counter in batches of
 // `batch`; lanes beyond `lanes` stay empty, so that a launch with fewer paths than resident lanes spreads
@@ -436,22 +436,35 @@ enum : int {
     kPendEnd       // the path ends with `color` (step guard)
 };
 
+// Events run once this many eighths (1 .. 8) of a warp's live lanes wait.  ms, eighths 1 .. 5: delta tracking of a 512^3
+// grid of optical depth 1,000 57.6 at 2, 56.5 at 3, 59.6 at 4; of a sparse grid 14.6 at 2, 15.5 at 3, 17.2 at 4; next event
+// tracking 23.1 at 1, 22.6 at 2, 25.4 at 3.  Thin clouds, whose paths are short and mostly events: 12 frames of 1280 x 720
+// of optical depth 100, delta tracking 2.40 at 1, 1.98 at 2, 1.79 at 3, 1.70 at 4 (events as they come 1.67); 200: 2.34 at
+// 3, 2.27 at 4; 400: 3.09 at 3 and 4.
+constexpr float kThin = 300.0f;  // optical depth along the box's longest side
+__host__ __device__ constexpr int event_share(int tracker, int grid, bool thin) {
+    return tracker == kNextEvent || tracker == kNextEvent + 100 ? 2
+           : tracker == kDecomposition                          ? 3
+           : grid == kNanoVdb                                   ? 2
+           : thin                                               ? 4
+                                                                : 3;
+}
+
 template <int TRACKER, int INTERP, int GRID, bool TF, class SRC>
 VPT_DEV void event_loop(const SRC& src, uint64_t total, unsigned long long* work_counter,
-                        unsigned long long* counters, int* error_flags, int refill_min, int batch, int lanes) {
+                        unsigned long long* counters, int* error_flags, int refill_min, int batch, int lanes,
+                        int share) {
     // next event tracking; kNextEvent + 100: its sky shadow rays skip the occupancy grid's empty blocks
     constexpr bool kNee = TRACKER == kNextEvent || TRACKER == kNextEvent + 100;
     constexpr bool kEss = TRACKER == kNextEvent + 100;
     constexpr bool kDec = TRACKER == kDecomposition;
-    // events run once kEventShare eighths of the warp's live lanes wait (measured, 1 .. 5 eighths: delta tracking of
-    // a 512^3 grid 57.6 ms at 2, 56.5 at 3, 59.6 at 4; of a sparse grid 14.6 at 2, 15.5 at 3, 17.2 at 4; next event
-    // tracking 23.1 at 1, 22.6 at 2, 25.4 at 3)
-    constexpr int kEventShare = kNee ? 2 : (!kDec && GRID == kNanoVdb ? 2 : 3);
+    // a constant where it does not depend on the cloud (as a variable the sparse case took 6 % longer)
+    constexpr int kShare = event_share(TRACKER, GRID, false);
+    const int eighths = event_share(TRACKER, GRID, true) != kShare ? share : kShare;
     // collisions a shadow ray goes ahead of its lookups (a trilinear lookup is eight fetches); measured, stochastic
     // lookups of a 512^3 grid: 23.6 ms at 1, 22.5 at 2, 19.1 at 4, 19.4 at 6 (events one by one 26.4); 256^2 paths of a
     // 128^3 grid 12.7 / 10.0 / 9.0 / 9.2 ms
     constexpr int kAhead = kNee ? (INTERP == kTrilinear ? 2 : 4) : 1;
-    static_assert(kEventShare >= 1 && kEventShare <= 8, "0 would never let a lane collide");
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -571,7 +584,7 @@ VPT_DEV void event_loop(const SRC& src, uint64_t total, unsigned long long* work
 
         // ---- collisions, until enough lanes wait with an event ----
         const int live_n = __popc(live);
-        while (__popc(__ballot_sync(FULL, pend != kPendNone)) * 8 < live_n * kEventShare) {
+        while (__popc(__ballot_sync(FULL, pend != kPendNone)) * 8 < live_n * eighths) {
             if (!has || pend != kPendNone) continue;
             const TraceParams& P = src.scene(scene);
             Sampler<INTERP, GRID, TF> sample{P};
@@ -1155,10 +1168,10 @@ __global__ void __launch_bounds__(kTraceBlock) trace_refill_kernel(const __grid_
 
 template <int TRACKER, int INTERP, int GRID, bool TF>
 __global__ void __launch_bounds__(kTraceBlock) trace_event_kernel(const __grid_constant__ TraceParams P, uint64_t total,
-                                                                  int batch, int lanes) {
+                                                                  int batch, int lanes, int share) {
     event_loop<TRACKER, INTERP, GRID, TF>(OneScene{P}, total,
                                                 reinterpret_cast<unsigned long long*>(P.work_counter), P.counters,
-                                                P.error_flags, P.refill_min, batch, lanes);
+                                                P.error_flags, P.refill_min, batch, lanes, share);
 }
 
 // Many independent scenes (own grid, camera, image size, spp, medium) traced by one persistent
@@ -1170,7 +1183,8 @@ __global__ void __launch_bounds__(kTraceBlock) trace_batch_kernel(const TracePar
                                                                   int num, unsigned long long* work_counter,
                                                                   unsigned long long* counters, int* error_flags) {
     event_loop<TRACKER, INTERP, GRID, false>(SceneBatch{scenes, offsets, num}, __ldg(offsets + num), work_counter,
-                                                    counters, error_flags, scenes[0].refill_min, kRefillBatch, 32);
+                                                    counters, error_flags, scenes[0].refill_min, kRefillBatch, 32,
+                                                    event_share(TRACKER, GRID, false));
 }
 
 
@@ -1235,7 +1249,11 @@ static cudaError_t launch_events(const TraceParams& P, uint64_t total, int block
     const int lanes = share >= 32 || !kSpread ? 32 : (share < 4 ? 4 : (int)share + 1);
     const int batch = share >= 256 ? kRefillBatch : lanes;
     cudaMemsetAsync(P.work_counter, 0, sizeof(unsigned long long), stream);
-    trace_event_kernel<TRACKER, INTERP, GRID, TF><<<blocks, kTraceBlock, 0, stream>>>(P, total, batch, lanes);
+    const float side = fmaxf(P.box_max.x - P.box_min.x,
+                             fmaxf(P.box_max.y - P.box_min.y, P.box_max.z - P.box_min.z));
+    const bool thin = side < kThin * P.inv_extinction;
+    trace_event_kernel<TRACKER, INTERP, GRID, TF><<<blocks, kTraceBlock, 0, stream>>>(P, total, batch, lanes,
+                                                                                      event_share(TRACKER, GRID, thin));
     count_launches(1);
     return cudaGetLastError();
 }

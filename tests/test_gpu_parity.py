@@ -671,3 +671,17 @@ def test_a_schedule_that_is_set_is_taken():
     for sched, kernel in ((2.0, "trace_event"), (1.0, "trace_persistent"), (0.0, "trace_tiles"), (2.0, "trace_event")):
         core("vpt_set_option", b"schedule", sched)
         assert traced_with(core, small, 1) == [kernel], sched
+
+
+@pytest.mark.parametrize("extinction", [30.0, 299.0, 301.0])
+@pytest.mark.parametrize("mode", ["delta", "ratio"])
+def test_events_of_thin_clouds_trace_identical_paths(core_dr, mode, extinction):
+    """Around the optical depth below which events wait for more company: the paths of the tile schedule."""
+    core = core_dr
+    sp = fbm_scene(width=70, height=51, mode=mode, extinction=extinction)
+    setup_core(core, sp)
+    films = []
+    for sched in (0.0, 2.0):
+        core("vpt_set_option", b"schedule", sched)
+        films.append(gpu_render(core, sp, 3, stats=False)[0])
+    assert np.allclose(*films, rtol=1e-12, atol=1e-12)
